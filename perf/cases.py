@@ -254,9 +254,13 @@ def run(state):
 
 
 def _fields(state, names):
-    """The force structs' fields; `names` are the ones FP32C forms in single precision."""
+    """The force structs' fields; `names` are the ones FP32C forms in single
+    precision.  Its neighbour count is left out: a neighbour at the edge of the
+    support is counted or not by the rounding of those fields."""
     f = state["force"]
-    return {k: f[k].astype(np.float32) if state["single"] and k in names else f[k] for k in f.dtype.names}
+    if not state["single"]:
+        return {k: f[k] for k in f.dtype.names}
+    return {k: f[k].astype(np.float32) if k in names else f[k] for k in f.dtype.names if k != "np"}
 
 
 SINGLE = {"density": ("dens", "divv", "rotv", "grdh", "ksr"), "hydro": ("vsmx",), "gravity": ("acc", "pot", "eta")}
