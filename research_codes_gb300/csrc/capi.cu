@@ -77,8 +77,9 @@ static int occupancy_grid(K kernel, int threads, int sm_count, int *out) {
 int init_grids(sph_context *ctx) {
     const int th = PAIR_WARPS * 32;
     int e = 0;
-    e |= occupancy_grid(sphk::density_kernel<false, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[0][0]);
-    e |= occupancy_grid(sphk::density_kernel<true, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[0][1]);
+    e |= occupancy_grid(sphk::mark_rows<false, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[0][0]);
+    e |= occupancy_grid(sphk::density_stream<PAIR_WARPS>, th, ctx->sm_count, &ctx->grid_stream);
+    ctx->grid[0][1] = ctx->grid[0][0];   // the rows are marked in FP32 in both precisions
     e |= occupancy_grid(sphk::hydro_kernel<false, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[1][0]);
     e |= occupancy_grid(sphk::hydro_kernel<true, HYDRO64_WARPS>, HYDRO64_WARPS * 32, ctx->sm_count,
                         &ctx->grid[1][1]);
@@ -96,11 +97,59 @@ int pair_grid(const sph_context *ctx, int kind, int precision, int n_items) {
     return std::max(1, std::min(full, need));
 }
 
-void launch_density(const sphk::DensityArgs &a, int precision, int grid, cudaStream_t s) {
-    if (precision == SPH_PREC_FP64)
-        sphk::density_kernel<true, PAIR_WARPS><<<grid, PAIR_WARPS * 32, 0, s>>>(a);
-    else
-        sphk::density_kernel<false, PAIR_WARPS><<<grid, PAIR_WARPS * 32, 0, s>>>(a);
+// The queued long items: a block each.
+template <bool SYM>
+static void mark_long(const sph_context *ctx, const sphk::MarkArgs &m, int n_max, cudaStream_t s) {
+    sphk::mark_rows<SYM, sphk::MARK_LONG_WARPS, true>
+        <<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), sphk::MARK_LONG_WARPS * 32, 0, s>>>(m);
+}
+
+// FP64 recomputation of the FP32C results queued as ambiguous (their number
+// is added to amb_total).
+static void recheck_density(const sph_context *ctx, const sphk::DensityArgs &a, int n_max, cudaStream_t s,
+                            int *amb_total) {
+    sphk::DensityArgs f = a;
+    f.amb_count = nullptr;
+    f.n_eval = nullptr;
+    sphk::density_sweep<true><<<std::max(1, std::min(n_max, ctx->sm_count)), sphk::DSWEEP_THREADS, 0, s>>>(
+        f, a.amb, a.amb_count, a.amb_cap, amb_total);
+}
+
+// The density sums of the particles of a.i_list (at most n_max) over their
+// rows, the sweep of the queued particles and, in FP32C, the FP64
+// recomputation of the ambiguous ones.  *a.n_ovf and *a.amb_count hold the
+// queues' counts.
+static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs &a, int n_max, int precision,
+                                cudaStream_t s, int *amb_total) {
+    const int per_block = sphk::DROWS_THREADS / sphk::DROWS_LANES;
+    const int rg = std::max(1, std::min((n_max + per_block - 1) / per_block, ctx->sm_count * 16));
+    const int sg = std::max(1, std::min(n_max, ctx->sm_count * 6));
+    if (precision == SPH_PREC_FP64) {
+        sphk::density_rows<true><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
+        sphk::density_sweep<true><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr);
+        return;
+    }
+    sphk::density_rows<false><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
+    sphk::density_sweep<false><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr);
+    recheck_density(ctx, a, n_max, s, amb_total);
+}
+
+// Rows of the items of m, then the density sums over them.
+void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
+                    int n_max, int precision, cudaStream_t s, int *amb_total) {
+    sphk::mark_rows<false, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
+    mark_long<false>(ctx, m, n_max, s);
+    launch_density_sums(ctx, a, n_max, precision, s, amb_total);
+}
+
+// The FP32C first walk of a particle system (n_max particles): the streamed
+// walk, then rows for the items it left (m and a cover them), the sweep of
+// what has no row and the FP64 recomputation of the ambiguous particles.
+void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, const sphk::MarkArgs &m,
+                           const sphk::DensityArgs &a, int n_max, cudaStream_t s, int *amb_total) {
+    sphk::density_stream<PAIR_WARPS><<<ctx->grid_stream, PAIR_WARPS * 32, 0, s>>>(w);
+    mark_long<false>(ctx, m, n_max, s);
+    launch_density_sums(ctx, a, n_max, SPH_PREC_FP32C, s, amb_total);
 }
 
 // FP32C: the signal-velocity / marking kernel, then the double-float pass
@@ -256,20 +305,38 @@ inline int eltwise_grid(long long n) {
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// Splits every walk into work items of <= 32 i-particles; largest first.
-void build_items(int n_walk, const int *i_off, const int *j_off, std::vector<WorkItem> &items) {
+// Warps that the pair kernels keep resident, about (4 blocks of 4 per SM).
+int resident_warps(const sph_context *ctx) { return 16 * ctx->sm_count; }
+
+// Splits every walk into work items of <= chunk i-particles; largest first.
+// split_nj > 0: walks with longer lists are cut finer (down to 4), so that no
+// item outlasts the rest.
+void build_items(int n_walk, const int *i_off, const int *j_off, int chunk, int split_nj,
+                 std::vector<WorkItem> &items) {
     items.clear();
     for (int w = 0; w < n_walk; ++w) {
         const int ni = i_off[w + 1] - i_off[w];
         const int nj = j_off[w + 1] - j_off[w];
-        for (int k = 0; k < ni; k += 32) {
-            const int c = std::min(32, ni - k);
+        int ch = chunk;
+        if (split_nj > 0)
+            for (long long lim = split_nj; ch > 4 && nj > lim; lim <<= 1) ch >>= 1;
+        for (int k = 0; k < ni; k += ch) {
+            const int c = std::min(ch, ni - k);
             const long long cost = (long long)nj * c;
             items.push_back(make_int4(w, i_off[w] + k, c, (int)std::min<long long>(cost, 0x7fffffff)));
         }
     }
     std::stable_sort(items.begin(), items.end(),
                      [](const WorkItem &a, const WorkItem &b) { return a.w > b.w; });
+}
+
+// i-particles per work item: halved from 32 while that leaves resident warps
+// without an item (a small call's time is the streaming of one item's list,
+// whatever its number of i-particles).
+int item_size(const sph_context *ctx, long long n_i) {
+    int chunk = 32;
+    while (chunk > 1 && n_i < (long long)chunk * resident_warps(ctx)) chunk >>= 1;
+    return chunk;
 }
 
 }  // namespace
@@ -326,7 +393,7 @@ extern "C" int sph_context_create(const sph_params *p, sph_context **out) {
     int cc_major = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, prm.device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_queue, 9 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_queue, 10 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_flags, 8 * sizeof(int));
     if (e == cudaSuccess && init_grids(ctx) != 0) e = cudaErrorInvalidDeviceFunction;
     if (e != cudaSuccess) {
@@ -426,6 +493,8 @@ extern "C" int sph_context_last_error(const sph_context *ctx, char *buf, size_t 
 namespace {
 
 enum { K_DENS = 0, K_HYDRO = 1, K_GRAV = 2 };
+constexpr float ROW_SLACK = 1.03f;   // row radius of the density over the first guess of h
+constexpr int SPLIT_NJ = 1024;   // density and hydro: lists beyond this make smaller items
 
 // Validates walk counts and fills the int32 offsets.  n_extra (gravity SPJ
 // counts) may be null.
@@ -471,9 +540,10 @@ Layout make_layout(int n_walk, size_t n_items, size_t bytes_epi, size_t bytes_ep
 }
 
 int stage_common(sph_context *ctx, KindState &ks, const std::vector<int> &i_off,
-                 const std::vector<int> &j_off, size_t epi_size, size_t epj_size, Layout &L) {
+                 const std::vector<int> &j_off, size_t epi_size, size_t epj_size, int chunk, int split_nj,
+                 Layout &L) {
     const int n_walk = (int)i_off.size() - 1;
-    build_items(n_walk, i_off.data(), j_off.data(), ks.items);
+    build_items(n_walk, i_off.data(), j_off.data(), chunk, split_nj, ks.items);
     L = make_layout(n_walk, ks.items.size(), epi_size * (size_t)i_off[n_walk],
                     epj_size * (size_t)j_off[n_walk]);
     if (ks.h_in.ensure(L.total) || ks.d_in.ensure(L.total))
@@ -568,7 +638,8 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
     if ((st = walk_offsets(ctx, n_walk, n_epi, n_epj, nullptr, i_off, j_off))) return st;
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
     Layout L;
-    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_DensityEPI), sizeof(sph_DensityEPJ), L))) return st;
+    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_DensityEPI), sizeof(sph_DensityEPJ),
+                           item_size(ctx, i_off[n_walk]), SPLIT_NJ, L))) return st;
     for (int w = 0; w < n_walk; ++w) {
         if ((n_epi[w] && !epi[w]) || (n_epj[w] && !epj[w]))
             return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
@@ -590,57 +661,57 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         unpack_density_j<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
             (const sph_DensityEPJ *)(d + L.off_epj), nj, ks.a4[2].p, ks.a4[3].p, ks.id[1].p);
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
-    if (f32 && ni > 0)
-        sphk::make_density_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.a4[0].p, ks.a4[1].p, ks.f4[0].p,
-                                                                             ks.f4[1].p, ks.f4[2].p, ks.f4[3].p);
-    if (f32 && nj > 0)
-        sphk::make_density_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(nj, ks.a4[2].p, ks.a4[3].p, ks.f4[4].p,
-                                                                             ks.f4[5].p, ks.f4[6].p, ks.f4[7].p);
+    if (ni > 0) {
+        if (f32)
+            sphk::make_density_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
+                ni, ks.a4[0].p, ks.a4[1].p, ks.d1[0].p, ks.f4[0].p, ks.f4[1].p, ks.f4[2].p, ks.f4[3].p);
+        else
+            sphk::make_row_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.a4[0].p, ks.d1[0].p, false,
+                                                                             ks.f4[0].p, ks.f4[1].p);
+    }
+    if (nj > 0) {
+        if (f32)
+            sphk::make_density_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
+                nj, ks.a4[2].p, ks.a4[3].p, nullptr, ks.f4[4].p, ks.f4[5].p, ks.f4[6].p, ks.f4[7].p);
+        else
+            sphk::make_row_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(nj, ks.a4[2].p, nullptr, false,
+                                                                             ks.f4[4].p, ks.f4[5].p);
+    }
     if (!ks.items.empty()) {
+        const int cap = std::max(256, ni / 16);
+        if (ks.amb.ensure(cap) || ks.long_items.ensure(ks.items.size())) return set_error(ctx, SPH_ERR_CUDA, "allocation failed");
+        // the sweep queue and the ambiguous particles' count start empty
+        cudaError_t e = cudaMemsetAsync(ctx->d_queue + 3, 0, sizeof(int), ctx->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_queue + 7, 0, 3 * sizeof(int), ctx->stream);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
+        sphk::MarkArgs m{};
+        m.i_hi = ks.f4[0].p; m.i_lo = ks.f4[1].p; m.j_hi = ks.f4[4].p; m.j_lo = ks.f4[5].p;
+        m.slack = ROW_SLACK;
+        m.items = (const WorkItem *)(d + L.off_items);
+        m.n_items = (int)ks.items.size();
+        m.j_off = (const int *)(d + L.off_joff);
+        m.queue = ctx->d_queue + K_DENS;
+        m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 7;
+        m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9;
         sphk::DensityArgs a{};
-        a.n_eval = nullptr;
         a.i_pm = ks.a4[0].p; a.i_vel = ks.a4[1].p; a.i_id = ks.id[0].p; a.i_ksr = ks.d1[0].p; a.i_rs = ks.d1[1].p;
         a.j_pm = ks.a4[2].p; a.j_vel = ks.a4[3].p; a.j_id = ks.id[1].p;
         a.fi = sphk::F32Part{ks.f4[0].p, ks.f4[1].p, ks.f4[2].p, ks.f4[3].p};
         a.fj = sphk::F32Part{ks.f4[4].p, ks.f4[5].p, ks.f4[6].p, ks.f4[7].p};
-        a.i_list = nullptr;
-        a.items = (const WorkItem *)(d + L.off_items);
-        a.n_items = (int)ks.items.size();
-        a.n_items_dev = nullptr;
-        a.j_off = (const int *)(d + L.off_joff);
-        a.j_idx = nullptr;
-        a.queue = ctx->d_queue + K_DENS;
+        a.n_i = ni;
+        a.j_off = m.j_off;
+        a.rows = m.rows; a.info = m.info; a.ovf = m.ovf; a.n_ovf = m.n_ovf;
+        a.slack = m.slack;
         a.o_dens = ks.o[0].p; a.o_divv = ks.o[1].p; a.o_rotv = ks.o[2].p; a.o_grdh = ks.o[3].p;
         a.o_ksr = ks.o[4].p; a.o_np = ks.o_np.p; a.o_itr = ks.o_itr.p;
         a.eta_ksrh = ctx->prm.eta * sphk::KSRH;
         a.ksr_max = ctx->prm.ksr_max > 0.0 ? ctx->prm.ksr_max : std::numeric_limits<double>::infinity();
-        a.ksr_max_dev = nullptr;
-        const int cap = std::max(256, ni / 16);
-        if (ks.amb_i.ensure(cap) || ks.amb_w.ensure(cap) || ks.fitems.ensure(cap))
-            return set_error(ctx, SPH_ERR_CUDA, "allocation failed");
         a.amb_count = f32 ? ctx->d_queue + 3 : nullptr;
-        a.amb_i = ks.amb_i.p;
-        a.amb_w = ks.amb_w.p;
+        a.amb = ks.amb.p;
         a.amb_cap = cap;
         a.amb_tol = AMB_TOL;
-        if (f32) {
-            cudaError_t e = cudaMemsetAsync(ctx->d_queue + 3, 0, sizeof(int), ctx->stream);
-            if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
-        }
-        launch_density(a, ctx->prm.precision, pair_grid(ctx, K_DENS, ctx->prm.precision, a.n_items), ctx->stream);
-        if (f32) {
-            // FP64 recomputation of the particles queued as decision-ambiguous
-            sphk::make_fixup_items<<<1, 256, 0, ctx->stream>>>(ctx->d_queue + 3, ks.amb_w.p, cap, ks.fitems.p,
-                                                                ctx->d_queue + 7);
-            cudaError_t e = cudaMemsetAsync(ctx->d_queue + K_DENS, 0, sizeof(int), ctx->stream);
-            if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
-            sphk::DensityArgs f = a;
-            f.items = ks.fitems.p;
-            f.n_items_dev = ctx->d_queue + 7;
-            f.i_list = ks.amb_i.p;
-            f.amb_count = nullptr;
-            launch_density(f, SPH_PREC_FP64, pair_grid(ctx, K_DENS, SPH_PREC_FP64, cap), ctx->stream);
-        }
+        launch_density(ctx, m, pair_grid(ctx, K_DENS, ctx->prm.precision, m.n_items), a, ni, ctx->prm.precision,
+                       ctx->stream);
     }
     if (ni > 0)
         pack_density<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
@@ -669,7 +740,8 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
     if ((st = walk_offsets(ctx, n_walk, n_epi, n_epj, nullptr, i_off, j_off))) return st;
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
     Layout L;
-    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_HydroEPI), sizeof(sph_HydroEPJ), L))) return st;
+    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_HydroEPI), sizeof(sph_HydroEPJ),
+                           item_size(ctx, i_off[n_walk]), SPLIT_NJ, L))) return st;
     for (int w = 0; w < n_walk; ++w) {
         if ((n_epi[w] && !epi[w]) || (n_epj[w] && !epj[w]))
             return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
@@ -763,7 +835,7 @@ extern "C" int sph_dispatch_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
     if (n_spj && !spj) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null spj");
     Layout L;
-    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_GravityEPI), sizeof(sph_GravityEPJ), L))) return st;
+    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_GravityEPI), sizeof(sph_GravityEPJ), 32, 0, L))) return st;
     static_assert(sizeof(sph_GravitySPJ) == sizeof(sph_GravityEPJ), "SPJ appended to EPJ");
     for (int w = 0; w < n_walk; ++w) {
         const int ns = n_spj ? n_spj[w] : 0;

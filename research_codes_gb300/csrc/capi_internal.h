@@ -83,16 +83,17 @@ struct KindState {
     DevBuf<char> d_in, d_out;
     DevBuf<dbl4> a4[8];
     DevBuf<float4> f4[16];   // FP32C double-float records
-    DevBuf<int> hl_list, hl_cnt;       // FP32C hydro: marked-pair rows and counts
-    DevBuf<int2> hl_ovf;               // FP32C hydro: overflowed rows (particle, walk)
+    DevBuf<int> hl_list, hl_cnt;       // rows of the density and hydro sums, hydro counts
+    DevBuf<int2> hl_ovf;               // particles without a row (particle, walk)
     DevBuf<double2> a2[2];
     DevBuf<long long> id[2];
     DevBuf<double> d1[2];
     DevBuf<double> o[5];
     DevBuf<long long> o_np;
     DevBuf<unsigned char> o_itr;
-    DevBuf<int> amb_i, amb_w;          // FP64 re-check queue of the density
-    DevBuf<int4> fitems;
+    DevBuf<int2> r_info;               // density rows (in hl_list): entries and walk per particle
+    DevBuf<int2> amb;                  // FP64 re-check queue of the density
+    DevBuf<int4> long_items;           // items with lists beyond LONG_LIST
     std::vector<int4> items;
     std::vector<int> i_off;
     bool pending = false;
@@ -106,6 +107,7 @@ struct KindState {
         for (int k = 0; k < 5; ++k) e |= o[k].ensure(ni);
         e |= o_np.ensure(ni) | o_itr.ensure(ni);
         for (int k = 0; k < 4; ++k) e |= f4[k].ensure(ni) | f4[4 + k].ensure(nj);
+        e |= hl_list.ensure(ni * sphk::ROW_CAP) | r_info.ensure(ni) | hl_ovf.ensure(ni);
         return e;
     }
     int ensure_hydro(size_t ni, size_t nj) {
@@ -145,9 +147,9 @@ struct KindState {
         for (auto &b : o) b.release();
         o_np.release();
         o_itr.release();
-        amb_i.release();
-        amb_w.release();
-        fitems.release();
+        r_info.release();
+        amb.release();
+        long_items.release();
     }
 };
 
@@ -158,10 +160,11 @@ struct sph_context {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     int *d_queue = nullptr;   // [0..2] work-queue counters, [3] density re-check count,
-                              // [4..6] finite flags, [7] re-check item count,
-                              // [8] FP32C hydro rows that overflowed
+                              // [4..6] finite flags, [7] density sweep queue,
+                              // [8] FP32C hydro rows that overflowed, [9] long items
     int *h_flags = nullptr;   // pinned copies of the flags
     int grid[3][2] = {{0}};   // persistent grid per kind and precision
+    int grid_stream = 0;      // persistent grid of the FP32C streamed density walk
     int grid_df = 0;          // resident blocks of the double-float hydro pass
     int grid_g64 = 0;         // persistent grid of the FP32C gravity kernel with a 64-entry j-tile
     sphrt::KindState kind[3];
@@ -174,7 +177,10 @@ extern const float AMB_TOL;
 int set_error(sph_context *ctx, int status, const char *fmt, ...);
 int cuda_error(sph_context *ctx, cudaError_t e, const char *what);
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items);
-void launch_density(const sphk::DensityArgs &a, int precision, int grid, cudaStream_t s);
+void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
+                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr);
+void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, const sphk::MarkArgs &m,
+                           const sphk::DensityArgs &a, int n_max, cudaStream_t s, int *amb_total);
 void launch_hydro(const sphk::HydroArgs &a, int precision, int grid, cudaStream_t s, int dfgrid,
                   cudaEvent_t mid = nullptr, bool mid_external = false);
 void launch_gravity(const sphk::GravityArgs &a, int precision, int grid, cudaStream_t s, int jtile);

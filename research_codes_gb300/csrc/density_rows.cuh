@@ -1,0 +1,539 @@
+// density_rows.cuh — the density sums over per-particle neighbour rows.
+//
+// The functor of hdr_density.hpp:252-350: three fixed-point passes
+// rho(h) -> h = eta ksrh (m / rho)^(1/3) from the first guess, then the
+// gradient pass (grdh, divv, rotv) with the final h.
+//
+//   density_rows   eight lanes per particle over its row (mark_rows): the
+//                  separations are formed once and kept in registers as
+//                  (r, m), so the three passes read no memory; the gradient
+//                  pass gathers the velocities.  A row holds every j within
+//                  slack * (first guess of h): a particle whose h leaves that
+//                  radius before the last pass is queued for the sweep.
+//   density_sweep  one block per queued particle over its walk's whole list:
+//                  particles without a row (overflow, very long lists, h
+//                  outside the row range), re-walks of few particles, and the
+//                  FP64 recomputation of FP32C results whose search-radius
+//                  decision is ambiguous.
+//
+// Both form the separations relative to the particle itself; FP32C sums a few
+// terms in FP32, folds them into Kahan pairs per lane and adds the lanes with
+// error-free transformations.
+#pragma once
+
+#include "rows.cuh"
+
+namespace sphk {
+
+// Double-float particle records of FP32C mode.
+struct F32Part {
+    const float4 *phi;   // x_hi, y_hi, z_hi, mass
+    const float4 *plo;   // x_lo, y_lo, z_lo, aux
+    const float4 *vhi;   // vx_hi, vy_hi, vz_hi, aux
+    const float4 *vlo;   // vx_lo, vy_lo, vz_lo, aux
+};
+
+struct DensityArgs {
+    // FP64 records (i_pm is read in both modes for the i-particle's mass)
+    const dbl4 *i_pm;       // x, y, z, mass
+    const dbl4 *i_vel;      // vx, vy, vz, -
+    const dbl4 *j_pm;
+    const dbl4 *j_vel;
+    // double-float positions (both modes: the sweep's distance test) and
+    // velocities (FP32C)
+    F32Part fi, fj;
+    const long long *i_id;
+    const long long *j_id;
+    const double *i_ksr;    // first guess of h (DensityEPI::ksr)
+    const double *i_rs;     // search radius (DensityEPI::rs)
+    const int *i_list;      // null: particles [0, n_i)
+    int n_i;
+    const int *n_i_dev;     // when set, the particle count is read from device memory
+    const int *j_off;       // per walk: [j_off[w], j_off[w+1]) in j index space
+    const int *j_idx;       // null: entries are j indices themselves
+    // rows (mark_rows)
+    const int *rows;
+    const int2 *info;
+    int2 *ovf;              // sweep queue
+    int *n_ovf;
+    float slack;            // row radius over the first guess of h
+    // when set: nothing runs while any of these error bits / this flag is set
+    const int *err;
+    int err_mask;
+    const int *skip_rows;
+    // bounds of the sweep's indices (n_j > 0: an index outside sets bounds_bit
+    // in *err_out and that access is skipped)
+    int n_j;
+    long long list_cap;
+    int *err_out;
+    int bounds_bit;
+    // outputs, indexed like the i arrays
+    double *o_dens, *o_divv, *o_rotv, *o_grdh, *o_ksr;
+    long long *o_np;
+    unsigned char *o_itr;
+    double eta_ksrh;        // eta * ksrh
+    double ksr_max;         // clamp of h (+inf disables)
+    const double *ksr_max_dev;  // when set, the clamp is read from device memory
+    // FP32C only: particles whose final h lies within amb_tol of rs (where
+    // the search-radius decision h > rs of hdr_density.hpp:299 could come out
+    // differently in FP64) are queued here for an FP64 recomputation
+    int *amb_count;         // null disables the queue
+    int2 *amb;              // (particle, walk)
+    int amb_cap;
+    float amb_tol;
+    // when set: pair evaluations performed, [0] the three density passes,
+    // [1] the gradient pass
+    unsigned long long *n_eval = nullptr;
+    // when set: particle passes after the first (second, third, gradient)
+    // [0] served from rows, [1] that swept the walk's j-list
+    unsigned long long *n_pass = nullptr;
+};
+
+// Two-float sum of a value over the L lanes of a segment, every lane
+// receiving the total (hi + lo); exact but for the rounding of lo.
+struct sum2 {
+    float h, l;
+};
+template <int L>
+__device__ __forceinline__ sum2 lane_sum(sum2 v) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+        const float oh = __shfl_xor_sync(FULL, v.h, o), ol = __shfl_xor_sync(FULL, v.l, o);
+        const float s = v.h + oh, b = s - v.h;
+        const float e = (v.h - (s - b)) + (oh - b);
+        v.l = (v.l + ol) + e;
+        v.h = s;
+    }
+    return v;
+}
+template <int L>
+__device__ __forceinline__ float lane_total(const Acc<false> &a) {
+    const sum2 t = lane_sum<L>(sum2{a.s, -a.c});
+    return t.h + t.l;
+}
+template <int L>
+__device__ __forceinline__ double lane_total(const Acc<true> &a) {
+    return seg_sum(a.s, L);
+}
+
+__device__ __forceinline__ float sqrt_r(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
+__device__ __forceinline__ float cbrt_r(float x) { return cbrtf(x); }
+__device__ __forceinline__ double cbrt_r(double x) { return cbrt(x); }
+
+// rho and the next h of one pass from its sum of m W0 / c0 (FP32C: FP32
+// arithmetic, relative error ~1e-7)
+template <typename R>
+struct HState {
+    R h, hinv, rho;
+    bool clamped;
+    __device__ __forceinline__ void start(double h0) {
+        h = (R)h0;
+        hinv = (R)1 / h;
+        clamped = false;
+    }
+    __device__ __forceinline__ void update(R sum, R mass, R eta_ksrh, R ksr_max) {
+        rho = (R)CEFF0 * hinv * hinv * hinv * sum;
+        const R hn = eta_ksrh * cbrt_r(mass / rho);
+        clamped = !(hn < ksr_max);   // also NaN, as the reference's comparison
+        h = clamped ? ksr_max : hn;
+        hinv = (R)1 / h;
+    }
+};
+
+// Gradient-pass sums and one pair's terms (hdr_density.hpp:304-349).
+template <bool F64>
+struct GradSums {
+    typedef typename Real<F64>::T R;
+    Acc<F64> g, d, rx, ry, rz;
+    R pg, pd, px, py, pz;
+    __device__ __forceinline__ GradSums() : pg(0), pd(0), px(0), py(0), pz(0) {}
+    // separation d, velocity difference u, mass m; self: equal ids
+    __device__ __forceinline__ void add(R dx, R dy, R dz, R ux, R uy, R uz, R m, bool self, R hinv) {
+        const R r2 = dx * dx + dy * dy + dz * dz;
+        const R ri = self ? (R)0 : rsqrt_r(r2);
+        const R q = r2 * ri * hinv;
+        const R u = max0((R)1 - q);
+        const R u2 = u * u;
+        const R u3 = u2 * u;
+        const R p14 = (R)1 + (R)4 * q;
+        const R w0 = u2 * u2 * p14;               // W0 / c0
+        const R w1 = w1_term(q, u, u2, u3, p14);  // W1 / c1
+        pg += m * ((R)(3.0 * CEFF0) * w0 + (R)CEFF1 * q * w1);
+        const R dw = m * w1 * ri;
+        pd += (ux * dx + uy * dy + uz * dz) * dw;
+        px += (uy * dz - uz * dy) * dw;
+        py += (uz * dx - ux * dz) * dw;
+        pz += (ux * dy - uy * dx) * dw;
+    }
+    __device__ __forceinline__ void fold() {
+        g.add(pg);
+        d.add(pd);
+        rx.add(px);
+        ry.add(py);
+        rz.add(pz);
+        pg = 0; pd = 0; px = 0; py = 0; pz = 0;
+    }
+};
+
+// Omega, div v, |rot v| and the write-back of one particle.
+template <typename R>
+__device__ __forceinline__ void density_finish(const DensityArgs &a, int ii, int walk, const HState<R> &s, R sg, R sd,
+                                               R sx, R sy, R sz, int np, double ksr_max) {
+    const R hinv4 = s.hinv * s.hinv * s.hinv * s.hinv;
+    const R rinv = (R)1 / s.rho;
+    const R grdh = -hinv4 * sg;
+    const R rx = (R)CEFF1 * hinv4 * sx, ry = (R)CEFF1 * hinv4 * sy, rz = (R)CEFF1 * hinv4 * sz;
+    const R om = (R)1 / ((R)1 + s.h * rinv * grdh / (R)3);
+    const R rot2 = rx * rx + ry * ry + rz * rz;
+    const R rot = (rot2 != (R)0) ? sqrt(rot2) : (R)0;
+    // the clamp itself is FP64
+    const double h = s.clamped ? ksr_max : (double)s.h;
+    const double rs_i = a.i_rs[ii];
+    a.o_dens[ii] = (double)s.rho;
+    a.o_divv[ii] = (double)(-(R)CEFF1 * hinv4 * sd * rinv * om);
+    a.o_rotv[ii] = (double)(rot * rinv * om);
+    a.o_grdh[ii] = (double)om;
+    a.o_ksr[ii] = h;
+    a.o_np[ii] = (long long)np;
+    a.o_itr[ii] = h > rs_i ? 1 : 0;   // the search-radius decision, hdr_density.hpp:299
+    if (a.amb_count && fabs(h - rs_i) <= (double)a.amb_tol * rs_i) {
+        const int k = atomicAdd(a.amb_count, 1);
+        if (k < a.amb_cap) a.amb[k] = make_int2(ii, walk);
+    }
+}
+
+// j-particle q of particle i: separation (i - j), in the precision of the sums.
+template <bool F64>
+struct PairPos {
+    typedef typename Real<F64>::T R;
+    float4 hi, lo;   // FP32C
+    dbl4 p;          // FP64
+    __device__ __forceinline__ void load_i(const DensityArgs &a, int ii) {
+        if constexpr (F64) {
+            p = a.i_pm[ii];
+        } else {
+            hi = a.fi.phi[ii];
+            lo = a.fi.plo[ii];
+        }
+    }
+    __device__ __forceinline__ R rel(const DensityArgs &a, int j, R &dx, R &dy, R &dz) const {
+        if constexpr (F64) {
+            const dbl4 q = a.j_pm[j];
+            dx = p.x - q.x; dy = p.y - q.y; dz = p.z - q.z;
+            return q.w;
+        } else {
+            const float4 qh = __ldg(&a.fj.phi[j]), ql = __ldg(&a.fj.plo[j]);
+            dx = -df_diff(qh.x, ql.x, hi.x, lo.x);
+            dy = -df_diff(qh.y, ql.y, hi.y, lo.y);
+            dz = -df_diff(qh.z, ql.z, hi.z, lo.z);
+            return qh.w;
+        }
+    }
+};
+template <bool F64>
+struct PairVel {
+    typedef typename Real<F64>::T R;
+    float4 hi, lo;
+    dbl4 v;
+    __device__ __forceinline__ void load_i(const DensityArgs &a, int ii) {
+        if constexpr (F64) {
+            v = a.i_vel[ii];
+        } else {
+            hi = a.fi.vhi[ii];
+            lo = a.fi.vlo[ii];
+        }
+    }
+    // velocity difference; FP32C differences hi and lo parts apart, so that
+    // it keeps FP32 relative accuracy across two colliding streams
+    __device__ __forceinline__ void rel(const DensityArgs &a, int j, R &ux, R &uy, R &uz) const {
+        if constexpr (F64) {
+            const dbl4 w = a.j_vel[j];
+            ux = v.x - w.x; uy = v.y - w.y; uz = v.z - w.z;
+        } else {
+            const float4 wh = __ldg(&a.fj.vhi[j]), wl = __ldg(&a.fj.vlo[j]);
+            ux = (hi.x - wh.x) + (lo.x - wl.x);
+            uy = (hi.y - wh.y) + (lo.y - wl.y);
+            uz = (hi.z - wh.z) + (lo.z - wl.z);
+        }
+    }
+};
+
+template <typename R>
+__device__ __forceinline__ R density_term(R q, R m) {   // m W0(q) / c0
+    const R u = max0((R)1 - q);
+    const R u2 = u * u;
+    return m * (u2 * u2 * ((R)1 + (R)4 * q));
+}
+
+constexpr int DROWS_LANES = 8;        // lanes per particle
+constexpr int DROWS_THREADS = 128;
+constexpr int DROWS_GROUPS = ROW_CAP / (4 * DROWS_LANES);   // int4 row reads per lane
+#ifndef SPH_DROWS_MIN_BLOCKS
+#define SPH_DROWS_MIN_BLOCKS 4
+#endif
+
+template <bool F64>
+__global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS) density_rows(const DensityArgs a) {
+    typedef typename Real<F64>::T R;
+    constexpr int L = DROWS_LANES, G = DROWS_GROUPS;
+    if (a.err && (*a.err & a.err_mask)) return;
+    if (a.skip_rows && *a.skip_rows) return;
+    const int n = a.n_i_dev ? *a.n_i_dev : a.n_i;
+    const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
+    const int lane = threadIdx.x & 31, sub = lane & (L - 1);
+    const int per_warp = 32 / L;
+    const int gw = (blockIdx.x * DROWS_THREADS + threadIdx.x) >> 5, nw = (gridDim.x * DROWS_THREADS) >> 5;
+    unsigned ev_rows = 0, ev_swept = 0;   // of this lane's particles (sub 0): row entries; particles queued
+    unsigned n_rows = 0;
+    for (int k0 = gw * per_warp; k0 < n; k0 += nw * per_warp) {
+        const int k = k0 + lane / L;
+        const int ii = (k < n) ? (a.i_list ? a.i_list[k] : k) : -1;
+        int2 inf = make_int2(ROW_CAP + 1, 0);
+        if (ii >= 0) inf = a.info[ii];
+        const bool row_ok = inf.x <= ROW_CAP;
+        const int cnt = row_ok ? inf.x : 0;
+        const int is = ii >= 0 ? ii : 0;
+        const int cmax = (int)__reduce_max_sync(FULL, (unsigned)cnt);
+        const double h0 = a.i_ksr[is];
+        PairPos<F64> P;
+        P.load_i(a, is);
+        R mi;
+        if constexpr (F64) mi = P.p.w;
+        else mi = P.hi.w;
+        const int *row = a.rows + (size_t)is * ROW_CAP;
+        int4 jv[G];
+        R r[4 * G], m[4 * G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (g * 4 * L < cmax) {
+                const int e = g * 4 * L + 4 * sub;
+                jv[g] = make_int4(-1, -1, -1, -1);
+                if (e < cnt) {
+                    jv[g] = *reinterpret_cast<const int4 *>(row + e);
+                    if (e + 1 >= cnt) jv[g].y = -1;
+                    if (e + 2 >= cnt) jv[g].z = -1;
+                    if (e + 3 >= cnt) jv[g].w = -1;
+                }
+                const int jj[4] = {jv[g].x, jv[g].y, jv[g].z, jv[g].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    R dx, dy, dz;
+                    r[4 * g + u] = 0;
+                    m[4 * g + u] = 0;   // a missing entry adds 0 * W0(0)
+                    if (jj[u] >= 0) {
+                        m[4 * g + u] = P.rel(a, jj[u], dx, dy, dz);
+                        r[4 * g + u] = sqrt_r(dx * dx + dy * dy + dz * dz);
+                    }
+                }
+            }
+        }
+        // three fixed-point passes, hdr_density.hpp:264-302
+        HState<R> s;
+        s.start(h0);
+        // every pair with q < 1 is in the row while h stays below this
+        const R h_row = (R)(h0 * (double)a.slack * 0.99998);
+        bool valid = row_ok && s.h <= (R)(h0 * (double)a.slack);
+        int np = 0;
+#pragma unroll
+        for (int pass = 0; pass < 3; ++pass) {
+            Acc<F64> acc;
+            int c = 0;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                if (g * 4 * L < cmax) {
+                    const int jj[4] = {jv[g].x, jv[g].y, jv[g].z, jv[g].w};
+                    R part = 0;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const R q = r[4 * g + u] * s.hinv;
+                        part += density_term(q, m[4 * g + u]);
+                        if (pass == 2) c += (jj[u] >= 0 && q < (R)1) ? 1 : 0;
+                    }
+                    acc.add(part);
+                }
+            }
+            const R sum = (R)lane_total<L>(acc);
+            if (pass == 2) {
+                for (int o = L / 2; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
+                np = c;
+            }
+            s.update(sum, mi, (R)a.eta_ksrh, (R)ksr_max);
+            valid = valid && s.h <= h_row;
+        }
+        // gradient pass with the final h, hdr_density.hpp:304-349
+        GradSums<F64> gs;
+        const long long idi = a.i_id[is];
+        PairVel<F64> V;
+        V.load_i(a, is);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (g * 4 * L < cmax) {
+                const int jj[4] = {jv[g].x, jv[g].y, jv[g].z, jv[g].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (jj[u] >= 0 && r[4 * g + u] * s.hinv < (R)1.0001) {
+                        R dx, dy, dz, ux, uy, uz;
+                        const R mj = P.rel(a, jj[u], dx, dy, dz);
+                        V.rel(a, jj[u], ux, uy, uz);
+                        gs.add(dx, dy, dz, ux, uy, uz, mj, a.j_id[jj[u]] == idi, s.hinv);
+                    }
+                }
+                gs.fold();
+            }
+        }
+        const R sg = (R)lane_total<L>(gs.g), sd = (R)lane_total<L>(gs.d);
+        const R sx = (R)lane_total<L>(gs.rx), sy = (R)lane_total<L>(gs.ry), sz = (R)lane_total<L>(gs.rz);
+        if (sub == 0 && ii >= 0) {
+            if (valid) {
+                density_finish<R>(a, ii, inf.y, s, sg, sd, sx, sy, sz, np, ksr_max);
+                ev_rows += (unsigned)cnt;
+                ++n_rows;
+            } else {
+                ++ev_swept;
+                if (row_ok) a.ovf[atomicAdd(a.n_ovf, 1)] = make_int2(ii, inf.y);
+            }
+        }
+    }
+    if (a.n_eval) {
+        const unsigned e = __reduce_add_sync(FULL, ev_rows);
+        const unsigned nr = __reduce_add_sync(FULL, n_rows), ns = __reduce_add_sync(FULL, ev_swept);
+        if (lane == 0 && (nr | ns)) {
+            atomicAdd(a.n_eval, 3ull * e);
+            atomicAdd(a.n_eval + 1, (unsigned long long)e);
+            atomicAdd(a.n_pass, 3ull * nr);
+            atomicAdd(a.n_pass + 1, 3ull * ns);
+        }
+    }
+}
+
+constexpr int DSWEEP_THREADS = 256;
+template <int N>
+__device__ __forceinline__ void block_sum(double (&v)[N], double (*red)[DSWEEP_THREADS / 32]) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(FULL, v[q], o);
+        if (lane == 0) red[q][wid] = v[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        double t = 0.0;
+        for (int u = 0; u < DSWEEP_THREADS / 32; ++u) t += red[q][u];
+        v[q] = t;
+    }
+    __syncthreads();
+}
+
+// queue / n_queue: (particle, walk) to sweep (n_queue capped at queue_cap);
+// total (optional): the count is added to it.
+template <bool F64>
+__global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArgs a, const int2 *queue,
+                                                               const int *n_queue, int queue_cap, int *total) {
+    typedef typename Real<F64>::T R;
+    constexpr int T = DSWEEP_THREADS, U = 4;   // U list entries per thread in flight
+    __shared__ double red[5][T / 32];
+    if (a.err && (*a.err & a.err_mask)) return;
+    const int nq = min(*n_queue, queue_cap);
+    if (total && blockIdx.x == 0 && threadIdx.x == 0) *total += *n_queue;
+    const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
+    for (int e = blockIdx.x; e < nq; e += gridDim.x) {
+        const int2 pw = queue[e];
+        const int ii = pw.x;
+        if (a.n_j > 0 && (ii < 0 || ii >= a.n_j)) {
+            if (threadIdx.x == 0) atomicOr(a.err_out, a.bounds_bit);
+            continue;   // block-uniform
+        }
+        const int jb = a.j_off[pw.y], je = a.j_off[pw.y + 1];
+        if (a.n_j > 0 && (jb < 0 || je < jb || (long long)je > a.list_cap)) {
+            if (threadIdx.x == 0) atomicOr(a.err_out, a.bounds_bit);
+            continue;   // block-uniform
+        }
+        PairPos<F64> P;
+        P.load_i(a, ii);
+        const float4 ph = a.fi.phi[ii], pl = a.fi.plo[ii];
+        const double mi = a.i_pm[ii].w;
+        // visits the list entries that can lie within h of the particle: an
+        // FP32 distance test on the double-float positions, with the margins
+        // of mark_rows (h outside its range: every entry)
+        auto over_list = [&](R h, auto &&f) {
+            const float hf = (float)h;
+            const float pad = 3.0e-14f * (fabsf(ph.x) + fabsf(ph.y) + fabsf(ph.z));
+            const float rad = hf * 1.0001f + pad;
+            const bool test = hf >= ROW_HMIN && hf <= ROW_HMAX;
+            const float lim = test ? rad * rad : INFINITY;
+            for (int k0 = jb + threadIdx.x; k0 < je; k0 += T * U) {
+                int j[U];
+                float4 qh[U], ql[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int k = k0 + u * T;
+                    j[u] = (k < je) ? (a.j_idx ? a.j_idx[k] : k) : -1;
+                    if (a.n_j > 0 && j[u] >= a.n_j) {
+                        atomicOr(a.err_out, a.bounds_bit);
+                        j[u] = -1;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (j[u] >= 0) {
+                        qh[u] = __ldg(&a.fj.phi[j[u]]);
+                        ql[u] = __ldg(&a.fj.plo[j[u]]);
+                    }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (j[u] >= 0) {
+                        const float dx = df_diff(qh[u].x, ql[u].x, ph.x, pl.x);
+                        const float dy = df_diff(qh[u].y, ql[u].y, ph.y, pl.y);
+                        const float dz = df_diff(qh[u].z, ql[u].z, ph.z, pl.z);
+                        if (!(dx * dx + dy * dy + dz * dz > lim)) f(j[u]);
+                    }
+            }
+        };
+        HState<R> s;
+        s.start(a.i_ksr[ii]);
+        int np = 0;
+        for (int pass = 0; pass < 3; ++pass) {
+            Acc<F64> acc;
+            int cnt = 0;
+            over_list(s.h, [&](int j) {
+                R dx, dy, dz;
+                const R m = P.rel(a, j, dx, dy, dz);
+                const R q = sqrt_r(dx * dx + dy * dy + dz * dz) * s.hinv;
+                cnt += (q < (R)1) ? 1 : 0;
+                acc.add(density_term(q, m));
+            });
+            double v[2] = {acc.value(), (double)cnt};
+            block_sum(v, red);
+            np = (int)v[1];
+            s.update((R)v[0], (R)mi, (R)a.eta_ksrh, (R)ksr_max);
+        }
+        GradSums<F64> gs;
+        const long long idi = a.i_id[ii];
+        PairVel<F64> V;
+        V.load_i(a, ii);
+        over_list(s.h, [&](int j) {
+            R dx, dy, dz, ux, uy, uz;
+            const R m = P.rel(a, j, dx, dy, dz);
+            V.rel(a, j, ux, uy, uz);
+            gs.add(dx, dy, dz, ux, uy, uz, m, a.j_id[j] == idi, s.hinv);
+            gs.fold();
+        });
+        double v[5] = {gs.g.value(), gs.d.value(), gs.rx.value(), gs.ry.value(), gs.rz.value()};
+        block_sum(v, red);
+        if (threadIdx.x == 0) {
+            density_finish<R>(a, ii, pw.y, s, (R)v[0], (R)v[1], (R)v[2], (R)v[3], (R)v[4], np, ksr_max);
+            if (a.n_eval) {
+                atomicAdd(a.n_eval, 3ull * (unsigned long long)(je - jb));
+                atomicAdd(a.n_eval + 1, (unsigned long long)(je - jb));
+            }
+        }
+    }
+}
+
+}  // namespace sphk

@@ -22,26 +22,21 @@
 //    coordinates without compensation: the "plain FP64 GPU" comparator.
 #pragma once
 
+#include "density_rows.cuh"
+#include "density_stream.cuh"
 #include "hydro_df.cuh"
+#include "rows.cuh"
 #include "sph_device.cuh"
 
 // Minimum resident blocks per SM requested from the compiler for the FP32C
-// density, gravity and hydro kernels (register budget 65536 / (128 threads x
-// blocks)).
-#ifndef SPH_DENSITY_MIN_BLOCKS
-#define SPH_DENSITY_MIN_BLOCKS 4
-#endif
+// gravity and hydro kernels (register budget 65536 / (128 threads x blocks)).
 #ifndef SPH_GRAVITY_MIN_BLOCKS
 #define SPH_GRAVITY_MIN_BLOCKS 4
 #endif
 // Unroll factors of the full-tile FP32C loops: f32x2 iterations (two entries
-// each) of the gravity and packed density loops, entries of the hydro
-// mark-only loop.
+// each) of the gravity loop, entries of the hydro mark-only loop.
 #ifndef SPH_GRAVITY_UNROLL
 #define SPH_GRAVITY_UNROLL 16
-#endif
-#ifndef SPH_DENSITY_UNROLL
-#define SPH_DENSITY_UNROLL 4
 #endif
 #ifndef SPH_HYDRO_MARK_UNROLL
 #define SPH_HYDRO_MARK_UNROLL 16
@@ -57,860 +52,7 @@
 namespace sphk {
 
 constexpr int GRAVITY_UNROLL = SPH_GRAVITY_UNROLL;
-constexpr int DENSITY_UNROLL = SPH_DENSITY_UNROLL;
 constexpr int HYDRO_MARK_UNROLL = SPH_HYDRO_MARK_UNROLL;
-
-// Double-float particle records of FP32C mode.
-struct F32Part {
-    const float4 *phi;   // x_hi, y_hi, z_hi, mass
-    const float4 *plo;   // x_lo, y_lo, z_lo, aux
-    const float4 *vhi;   // vx_hi, vy_hi, vz_hi, aux
-    const float4 *vlo;   // vx_lo, vy_lo, vz_lo, aux
-};
-
-__device__ __forceinline__ float df_diff(float hi, float lo, float chi, float clo) {
-    return (hi - chi) + (lo - clo);
-}
-
-// Double-float split of an FP64 value: hi = float(x), lo = float(x - hi).
-__device__ __forceinline__ float2 df_split(double x) {
-    const float h = (float)x;
-    return make_float2(h, (float)(x - (double)h));
-}
-
-struct ItemRef {   // decoded work item
-    int walk, jb, nj, ni, tpi, sub, li, ii, ic;
-    bool act;
-};
-
-__device__ __forceinline__ ItemRef decode(const WorkItem &it, const int *j_off, const int *i_list, int lane) {
-    ItemRef r;
-    r.walk = it.x;
-    r.jb = j_off[it.x];
-    r.nj = j_off[it.x + 1] - r.jb;
-    r.ni = it.z;
-    r.tpi = lanes_per_i(it.z);
-    const int sh = ilog2_pow2(r.tpi);
-    r.li = lane >> sh;
-    r.sub = lane & (r.tpi - 1);
-    r.act = r.li < it.z;
-    const int k = it.y + (r.act ? r.li : 0);
-    r.ii = i_list ? i_list[k] : k;
-    r.ic = i_list ? i_list[it.y] : it.y;   // the item's centre particle
-    return r;
-}
-
-// ---------------------------------------------------------------- density
-struct DensityArgs {
-    // FP64 records (i_pm is read in both modes for the i-particle's mass)
-    const dbl4 *i_pm;       // x, y, z, mass
-    const dbl4 *i_vel;      // vx, vy, vz, -
-    const dbl4 *j_pm;
-    const dbl4 *j_vel;
-    // FP32C mode records (phi.w = mass)
-    F32Part fi, fj;
-    const long long *i_id;
-    const long long *j_id;
-    const double *i_ksr;    // first guess of h (DensityEPI::ksr)
-    const double *i_rs;     // search radius (DensityEPI::rs)
-    // work
-    const WorkItem *items;
-    int n_items;
-    const int *n_items_dev; // when set, the item count is read from device memory
-    const int *j_off;       // per walk: [j_off[w], j_off[w+1]) in j index space
-    const int *j_idx;       // null: entries are j indices themselves
-    const int *i_list;      // null: item i-particles are contiguous
-    int *queue;             // item counter, 0 at launch
-    // outputs, indexed like the i arrays
-    double *o_dens, *o_divv, *o_rotv, *o_grdh, *o_ksr;
-    long long *o_np;
-    unsigned char *o_itr;
-    double eta_ksrh;        // eta * ksrh
-    double ksr_max;         // clamp of h (+inf disables)
-    const double *ksr_max_dev;  // when set, the clamp is read from device memory
-    // FP32C only: particles whose final h lies within amb_tol of rs (where
-    // the search-radius decision h > rs of hdr_density.hpp:299 could come out
-    // differently in FP64) are queued here for an FP64 recomputation
-    int *amb_count;         // null disables the queue
-    int *amb_i;             // queued particle index
-    int *amb_w;             // its walk
-    int amb_cap;
-    float amb_tol;
-    // Per-warp neighbour lists; null: every pass sweeps the walk's j-list.
-    // Warp w of the grid (blockIdx.x * WARPS + warp) owns the int array
-    // nbr[w * nbr_cap * 32, (w + 1) * nbr_cap * 32), entry c of lane l at
-    // [c * 32 + l]; warps w >= nbr_warps sweep.  nbr_slack (> 1) is the list
-    // radius in units of each i-particle's first-pass h.
-    int *nbr = nullptr;
-    int nbr_cap = 0;
-    int nbr_warps = 0;
-    float nbr_slack = 1.0f;
-    // when set: pair evaluations performed, [0] the three density passes
-    // ((j-entries kept by the support test x i-particles) of the swept passes
-    // plus the list entries of the listed ones), [1] the gradient pass
-    unsigned long long *n_eval = nullptr;
-    // when set: [0] item passes (second, third, gradient) served from the
-    // neighbour lists, [1] item passes that swept the walk's j-list
-    unsigned long long *n_pass = nullptr;
-};
-
-template <bool B>
-struct BTag {
-    static constexpr bool value = B;
-};
-
-// The density functor of hdr_density.hpp:252-350 for one work item per warp:
-// three fixed-point passes rho(h) -> h = eta ksrh (m / rho)^(1/3) from the
-// first guess, then the gradient pass (grdh, divv, rotv) with the final h.
-//
-// Every pass can stream the walk's j-list through a shared ring (kept entries
-// of each 32-entry chunk compacted by the item-box support test), which
-// evaluates every kept entry for every i-particle of the item: ~10x more
-// pairs than the kernel support holds.  With neighbour lists the first pass
-// streams the list once with the support widened by nbr_slack and also writes,
-// per lane, the j indices within nbr_slack * (first-pass h) of its
-// i-particle; the second and third passes and the gradient pass then loop over
-// each lane's own list (gathering the j records) whenever every h of the item
-// has stayed within that radius and no lane's list overflowed nbr_cap;
-// otherwise the pass sweeps.  Entries beyond a particle's support add exactly
-// zero in both forms, so the two differ only in the grouping of the FP32
-// partial sums.
-template <bool F64, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, F64 ? 1 : SPH_DENSITY_MIN_BLOCKS)
-density_kernel(const DensityArgs a) {
-    typedef typename Real<F64>::T R;
-    typedef typename Real<F64>::T4 R4;
-    // per warp a 64-entry ring of compacted j records: entries accumulate
-    // until 32 are ready, the pair loop consumes one 32-entry half at a time
-    __shared__ R4 s_p[WARPS][64];
-    __shared__ R4 s_v[WARPS][64];
-    __shared__ float2 s_vl[WARPS][64];
-    __shared__ long long s_id[WARPS][64];
-    // FP32C density passes: the same ring as a structure of arrays, so that
-    // two consecutive entries load as one f32x2 operand
-    __shared__ __align__(16) float s_rx[F64 ? 1 : WARPS][64], s_ry[F64 ? 1 : WARPS][64],
-        s_rz[F64 ? 1 : WARPS][64], s_rm[F64 ? 1 : WARPS][64];
-    __shared__ int s_j[WARPS][64];   // j index of each ring entry (list-building pass)
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    const unsigned lt = lanemask_lt();
-    const int n_items = a.n_items_dev ? *a.n_items_dev : a.n_items;
-    const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
-    const int gw = blockIdx.x * WARPS + wid;
-    // this lane's neighbour list: entry c at a.nbr[nlb + c * 32]
-    const bool has_nl = a.nbr != nullptr && gw < a.nbr_warps;
-    const int nlb = has_nl ? gw * a.nbr_cap * 32 + lane : 0;
-    // list radius^2 over (first-pass h)^2, and the largest h (over the
-    // first-pass h) a listed pass accepts: every pair with q < 1 then has r^2
-    // below the list radius with a margin of 2e-5 over the rounding of both
-    // tests
-    const R nl_lim = (R)a.nbr_slack * (R)a.nbr_slack;
-    const double nl_hmax = (double)a.nbr_slack * 0.99998;
-
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(a.queue, 1);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= n_items) return;
-        const ItemRef r = decode(a.items[item], a.j_off, a.i_list, lane);
-        const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;
-
-        // i-particle relative to the centre particle c (velocity, id, mass
-        // and search radius are read where they are used, keeping the
-        // registers of the passes free)
-        R xi, yi, zi;
-        float4 cph = make_float4(0, 0, 0, 0), cpl = cph;
-        if (F64) {
-            const dbl4 p = a.i_pm[ii];
-            xi = (R)p.x; yi = (R)p.y; zi = (R)p.z;
-        } else {
-            cph = a.fi.phi[r.ic]; cpl = a.fi.plo[r.ic];
-            const float4 ph = a.fi.phi[ii], pl = a.fi.plo[ii];
-            xi = (R)df_diff(ph.x, pl.x, cph.x, cpl.x);
-            yi = (R)df_diff(ph.y, pl.y, cph.y, cpl.y);
-            zi = (R)df_diff(ph.z, pl.z, cph.z, cpl.z);
-        }
-        // The kernel is zero for r >= h, so a j-particle farther than the
-        // largest h of the item from the item's box adds nothing to any sum
-        // or count of this item: staging drops it before the pair loop.
-        IBox<R> box;
-        box.from_lanes(xi, yi, zi);
-        double h = a.i_ksr[ii];
-        // largest h a listed pass accepts for this lane
-        const float nl_h = (float)(h * nl_hmax);
-        R rho = 0;
-        int np = 0;
-
-        // One j record as loaded from memory (FP32C double-float or FP64).
-        struct JRec {
-            float4 ph, pl, vh, vl;
-            dbl4 p, v;
-            long long id;
-        };
-        auto jlist = [&](int k) -> int { return a.j_idx ? a.j_idx[jb + k] : jb + k; };
-        auto load = [&](int j, bool with_v, JRec &q) {
-            if constexpr (F64) {
-                q.p = a.j_pm[j];
-                if (with_v) q.v = a.j_vel[j];
-            } else {
-                q.ph = a.fj.phi[j];
-                q.pl = a.fj.plo[j];
-                if (with_v) {
-                    q.vh = a.fj.vhi[j];
-                    q.vl = a.fj.vlo[j];
-                }
-            }
-            if (with_v) q.id = a.j_id[j];
-        };
-        // position of particle j in the frame of the pair loops (FP32C:
-        // relative to the centre particle; FP64: absolute) and its mass
-        auto jpos = [&](int j) -> R4 {
-            if constexpr (F64) {
-                const dbl4 p = a.j_pm[j];
-                return Real<F64>::make4((R)p.x, (R)p.y, (R)p.z, (R)p.w);
-            } else {
-                const float4 ph = __ldg(&a.fj.phi[j]), pl = __ldg(&a.fj.plo[j]);
-                return Real<F64>::make4(df_diff(ph.x, pl.x, cph.x, cpl.x), df_diff(ph.y, pl.y, cph.y, cpl.y),
-                                        df_diff(ph.z, pl.z, cph.z, cpl.z), ph.w);
-            }
-        };
-        // Streams the walk's list through the ring: lane k takes entry t+k,
-        // entries that can lie within sqrt(rf2) of the item box are
-        // compacted into the ring, and consume(base, n) runs whenever 32 are
-        // ready (and once more for the rest).  Loads run one 32-entry chunk
-        // ahead of their use (the list index two chunks ahead) so that their
-        // latency overlaps the box test and the pair loops.  with_v also
-        // stages velocities and ids (gradient pass), with_j the j indices.
-        unsigned kept = 0;   // j-entries kept by the support test, all sweeps
-        auto sweep = [&](const R rf2, const bool with_v, const bool with_j, auto &&consume) {
-            int head = 0, fill = 0;
-            JRec cur, nxt;
-            int jn = 0, jnx = 0;
-            if (lane < nj) {
-                jnx = jlist(lane);
-                load(jnx, with_v, nxt);
-            }
-            if (32 + lane < nj) jn = jlist(32 + lane);
-            for (int t = 0; t < nj; t += 32) {
-                cur = nxt;
-                const int jc = jnx;
-                const bool valid = t + lane < nj;
-                if (t + 32 + lane < nj) {
-                    jnx = jn;
-                    load(jn, with_v, nxt);
-                }
-                if (t + 64 + lane < nj) jn = jlist(t + 64 + lane);
-                bool keep = false;
-                R4 p4;
-                if (valid) {
-                    if constexpr (F64) {
-                        p4 = Real<F64>::make4((R)cur.p.x, (R)cur.p.y, (R)cur.p.z, (R)cur.p.w);
-                    } else {
-                        p4 = Real<F64>::make4((R)df_diff(cur.ph.x, cur.pl.x, cph.x, cpl.x),
-                                              (R)df_diff(cur.ph.y, cur.pl.y, cph.y, cpl.y),
-                                              (R)df_diff(cur.ph.z, cur.pl.z, cph.z, cpl.z), (R)cur.ph.w);
-                    }
-                    keep = !(box.d2(p4.x, p4.y, p4.z) > rf2);
-                }
-                const unsigned m = __ballot_sync(FULL, keep);
-                if (keep) {
-                    const int slot = (head + fill + __popc(m & lt)) & 63;
-                    if (!F64 && !with_v) {
-                        s_rx[wid][slot] = (float)p4.x;
-                        s_ry[wid][slot] = (float)p4.y;
-                        s_rz[wid][slot] = (float)p4.z;
-                        s_rm[wid][slot] = (float)p4.w;
-                    } else {
-                        s_p[wid][slot] = p4;
-                    }
-                    if (with_v) {
-                        if constexpr (F64) {
-                            s_v[wid][slot] = Real<F64>::make4((R)cur.v.x, (R)cur.v.y, (R)cur.v.z, (R)0);
-                        } else {
-                            s_v[wid][slot] = Real<F64>::make4((R)cur.vh.x, (R)cur.vh.y, (R)cur.vh.z, (R)cur.vl.x);
-                            s_vl[wid][slot] = make_float2(cur.vl.y, cur.vl.z);
-                        }
-                        s_id[wid][slot] = cur.id;
-                    }
-                    if (with_j) s_j[wid][slot] = jc;
-                }
-                fill += __popc(m);
-                kept += __popc(m);
-                __syncwarp();
-                if (fill >= 32) {
-                    consume(head, 32);
-                    head ^= 32;
-                    fill -= 32;
-                }
-            }
-            if (fill > 0) consume(head, fill);
-        };
-
-        // neighbour list of this lane: its length (above nbr_cap the list is
-        // unusable), appended by the first pass from the ring
-        int ncnt = 0;
-        bool nl_ok = false;
-        unsigned ev_list = 0, ev_list_g = 0;   // list entries evaluated (this lane)
-        int n_listed = 0;                      // of the 3 item passes after the first
-        auto nl_push = [&](int head, unsigned msk) {
-            while (msk) {
-                const int k = __ffs(msk) - 1;
-                msk &= msk - 1;
-                if (ncnt < a.nbr_cap) a.nbr[nlb + ncnt * 32] = s_j[wid][head + k];
-                ++ncnt;
-            }
-        };
-
-        // three fixed-point passes, hdr_density.hpp:264-302
-        for (int pass = 0; pass < 3; ++pass) {
-            const R hinv = (R)1 / (R)h;
-            const R hinv2 = hinv * hinv;
-            const bool build = has_nl && pass == 0;
-            const bool listed = pass > 0 && nl_ok && __all_sync(FULL, (float)h <= nl_h);
-            Acc<F64> acc;
-            int cnt = 0;
-            R part = 0;
-            // rho pair term m_j W0(q)/c0; neighbour count only in the last
-            // pass (the only np the reference stores, :297)
-            auto term = [&](const R4 pj, bool count) -> R {
-                const R dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
-                const R r2 = dx * dx + dy * dy + dz * dz;
-                const R q = sqrt_q(r2, hinv2);
-                const R u = max0((R)1 - q);
-                const R u2 = u * u;
-                if (count) cnt += (q < (R)1) ? 1 : 0;
-                return pj.w * (u2 * u2 * ((R)1 + (R)4 * q));
-            };
-            // ring entry k; with mark set, bit k of *mark flags an entry
-            // within the list radius
-            auto pair = [&](int k, bool count, unsigned *mark) {
-                R4 pj;
-                if constexpr (F64) {
-                    pj = s_p[wid][k];
-                } else {
-                    pj = Real<F64>::make4(s_rx[wid][k], s_ry[wid][k], s_rz[wid][k], s_rm[wid][k]);
-                }
-                part += term(pj, count);
-                if (mark) {
-                    const R dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
-                    if ((dx * dx + dy * dy + dz * dz) * hinv2 < nl_lim) *mark |= 1u << (k & 31);
-                }
-            };
-            // full FP32C tile: two entries per instruction (f32x2); even and
-            // odd entries summed apart and combined at the end of the tile;
-            // the list-building form also flags the entries within the list
-            // radius
-            auto run_packed = [&](int head, bool count, auto build_tag) {
-                constexpr bool B = decltype(build_tag)::value;
-                const f2 XI = f2_make((float)xi, (float)xi), YI = f2_make((float)yi, (float)yi);
-                const f2 ZI = f2_make((float)zi, (float)zi), H2 = f2_make((float)hinv2, (float)hinv2);
-                const f2 NEG = f2_make(-1.0f, -1.0f), ONE = f2_make(1.0f, 1.0f), FOUR = f2_make(4.0f, 4.0f);
-                const float lim = (float)nl_lim;
-                f2 PART = f2_make(0.0f, 0.0f);
-                int c2 = 0;
-                unsigned msk = 0;
-#pragma unroll DENSITY_UNROLL
-                for (int k = 0; k < 32; k += 2) {
-                    const f2 DX = f2_fma(f2_lds(&s_rx[wid][head + k]), NEG, XI);
-                    const f2 DY = f2_fma(f2_lds(&s_ry[wid][head + k]), NEG, YI);
-                    const f2 DZ = f2_fma(f2_lds(&s_rz[wid][head + k]), NEG, ZI);
-                    const float2 x2 = f2_get(f2_mul(f2_fma(DZ, DZ, f2_fma(DY, DY, f2_mul(DX, DX))), H2));
-                    if constexpr (B) msk |= (x2.x < lim ? 1u << k : 0u) | (x2.y < lim ? 2u << k : 0u);
-                    float q0, q1;
-                    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(q0) : "f"(x2.x));
-                    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(q1) : "f"(x2.y));
-                    const f2 Q = f2_make(q0, q1);
-                    const float2 u = f2_get(f2_fma(Q, NEG, ONE));
-                    const f2 U = f2_make(max0(u.x), max0(u.y));
-                    const f2 U2 = f2_mul(U, U);
-                    PART = f2_fma(f2_lds(&s_rm[wid][head + k]), f2_mul(f2_mul(U2, U2), f2_fma(Q, FOUR, ONE)), PART);
-                    if (count) c2 += (q0 < 1.0f ? 1 : 0) + (q1 < 1.0f ? 1 : 0);
-                }
-                const float2 ps = f2_get(PART);
-                part = (R)(ps.x + ps.y);
-                cnt += c2;
-                if constexpr (B) nl_push(head, msk);
-            };
-            auto run = [&](int head, int n) {
-                part = 0;
-                if (!F64 && tpi == 1 && n == 32) {
-                    if (build)
-                        run_packed(head, false, BTag<true>());
-                    else
-                        run_packed(head, pass == 2, BTag<false>());
-                } else {
-                    unsigned msk = 0;
-                    unsigned *mark = build ? &msk : nullptr;
-                    if (tpi == 1 && n == 32) {
-                        if (pass == 2) {
-#pragma unroll 8
-                            for (int k = 0; k < 32; ++k) pair(head + k, true, nullptr);
-                        } else {
-#pragma unroll 8
-                            for (int k = 0; k < 32; ++k) pair(head + k, false, mark);
-                        }
-                    } else {
-                        for (int k = sub; k < n; k += tpi) pair(head + k, pass == 2, mark);
-                    }
-                    if (build) nl_push(head, msk);
-                }
-                acc.add(part);
-                __syncwarp();
-            };
-            if (listed) {
-                // this lane's list, four entries per round (gathers first)
-                const int cmax = (int)__reduce_max_sync(FULL, (unsigned)ncnt);
-                for (int c0 = 0; c0 < cmax; c0 += 4) {
-                    int jj[4];
-                    R4 pj[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) jj[u] = (c0 + u < ncnt) ? a.nbr[nlb + (c0 + u) * 32] : -1;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (jj[u] >= 0) pj[u] = jpos(jj[u]);
-                    part = 0;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (jj[u] >= 0) part += term(pj[u], pass == 2);
-                    acc.add(part);
-                }
-                if (r.act) ev_list += (unsigned)ncnt;
-                ++n_listed;
-            } else {
-                const R rf2 = support2<R>(build ? h * (double)a.nbr_slack : h);
-                sweep(rf2, false, build, run);
-            }
-            if (build) nl_ok = __all_sync(FULL, ncnt <= a.nbr_cap);
-            const double sum = seg_sum(acc.value(), tpi);
-            const int c = (int)seg_sum((long long)cnt, tpi);
-            const double mi = a.i_pm[ii].w;
-            double hn;
-            if (F64) {
-                const double hinv_d = 1.0 / h;
-                rho = (R)(CEFF0 * hinv_d * hinv_d * hinv_d * sum);
-                hn = a.eta_ksrh * cbrt(mi / (double)rho);
-            } else {
-                // FP32 per-particle update (relative error ~1e-7, far inside
-                // the 1e-5 budget) keeps the FP64 pipe out of the loop
-                const float hinv_f = (float)hinv;
-                const float rho_f = (float)CEFF0 * hinv_f * hinv_f * hinv_f * (float)sum;
-                rho = (R)rho_f;
-                hn = (double)((float)a.eta_ksrh * cbrtf((float)mi / rho_f));
-            }
-            hn = (hn < ksr_max) ? hn : ksr_max;
-            np = c;
-            h = hn;
-        }
-        // the search-radius decision of the last pass (hdr_density.hpp:299)
-        const double rs_i = a.i_rs[ii];
-        const bool itr = h > rs_i;
-        if (!F64 && a.amb_count && r.act && sub == 0 && fabs(h - rs_i) <= (double)a.amb_tol * rs_i) {
-            const int k = atomicAdd(a.amb_count, 1);
-            if (k < a.amb_cap) {
-                a.amb_i[k] = ii;
-                a.amb_w[k] = r.walk;
-            }
-        }
-
-        const unsigned kept_rho = kept;
-        // gradient pass with the final h, hdr_density.hpp:304-349
-        {
-            const long long idi = a.i_id[ii];
-            R vxi, vyi, vzi;
-            float lxi = 0.0f, lyi = 0.0f, lzi = 0.0f;
-            if (F64) {
-                const dbl4 v = a.i_vel[ii];
-                vxi = (R)v.x; vyi = (R)v.y; vzi = (R)v.z;
-            } else {
-                // velocities stay absolute hi/lo pairs and are differenced
-                // per pair: an item may straddle two colliding streams
-                const float4 vh = a.fi.vhi[ii], vl = a.fi.vlo[ii];
-                vxi = vh.x; vyi = vh.y; vzi = vh.z;
-                lxi = vl.x; lyi = vl.y; lzi = vl.z;
-            }
-            const R hinv = (R)1 / (R)h;
-            Acc<F64> g_acc, d_acc, rx_acc, ry_acc, rz_acc;
-            R pg = 0, pd = 0, prx = 0, pry = 0, prz = 0;
-            // pair terms; (vx, vy, vz) the j velocity (FP32C: hi parts, with
-            // the lo parts (lx, ly, lz) differenced apart)
-            auto gpair = [&](const R4 pj, R vx, R vy, R vz, float lx, float ly, float lz, long long idj) {
-                const R dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
-                R ux = vxi - vx, uy = vyi - vy, uz = vzi - vz;
-                if (!F64) {
-                    ux += (R)(lxi - lx);
-                    uy += (R)(lyi - ly);
-                    uz += (R)(lzi - lz);
-                }
-                const R r2 = dx * dx + dy * dy + dz * dz;
-                const R ri = (idi != idj) ? rsqrt_r(r2) : (R)0;
-                const R q = r2 * ri * hinv;
-                const R u = max0((R)1 - q);
-                const R u2 = u * u;
-                const R u3 = u2 * u;
-                const R p14 = (R)1 + (R)4 * q;
-                const R w0 = u2 * u2 * p14;            // W0 / c0
-                const R w1 = w1_term(q, u, u2, u3, p14);   // W1 / c1
-                pg += pj.w * ((R)(3.0 * CEFF0) * w0 + (R)CEFF1 * q * w1);
-                const R dw = pj.w * w1 * ri;
-                pd += (ux * dx + uy * dy + uz * dz) * dw;
-                prx += (uy * dz - uz * dy) * dw;
-                pry += (uz * dx - ux * dz) * dw;
-                prz += (ux * dy - uy * dx) * dw;
-            };
-            auto pair = [&](int k) {
-                const R4 vj = s_v[wid][k];
-                const float2 vl = s_vl[wid][k];
-                gpair(s_p[wid][k], vj.x, vj.y, vj.z, (float)vj.w, vl.x, vl.y, s_id[wid][k]);
-            };
-            auto fold = [&]() {
-                g_acc.add(pg);
-                d_acc.add(pd);
-                rx_acc.add(prx);
-                ry_acc.add(pry);
-                rz_acc.add(prz);
-                pg = 0; pd = 0; prx = 0; pry = 0; prz = 0;
-            };
-            // Each lane first marks the tile entries inside its own support
-            // (r^2/h^2 below 1 + 2e-5, so every pair with q < 1 is marked),
-            // then evaluates the gradient terms of the marked entries only, in
-            // tile order; the unmarked pairs contribute exactly zero.
-            const R lim = hinv * hinv * (R)1.00002;
-            auto mark = [&](int k, unsigned &msk) {
-                const R4 pj = s_p[wid][k];
-                const R dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
-                const R r2 = dx * dx + dy * dy + dz * dz;
-                if (!(r2 * lim >= (R)1)) msk |= 1u << (k & 31);
-            };
-            auto run = [&](int head, int n) {
-                unsigned msk = 0;
-                if (tpi == 1 && n == 32) {
-#pragma unroll 8
-                    for (int k = 0; k < 32; ++k) mark(head + k, msk);
-                } else {
-                    for (int k = sub; k < n; k += tpi) mark(head + k, msk);
-                }
-                while (msk) {
-                    const int k = __ffs(msk) - 1;
-                    msk &= msk - 1;
-                    pair(head + k);
-                }
-                fold();
-                __syncwarp();
-            };
-            if (nl_ok && __all_sync(FULL, (float)h <= nl_h)) {
-                // this lane's list, two entries per round (gathers first)
-                const int cmax = (int)__reduce_max_sync(FULL, (unsigned)ncnt);
-                for (int c0 = 0; c0 < cmax; c0 += 2) {
-                    int jj[2];
-                    R4 pj[2];
-                    R4 vh[2];
-                    float4 vl[2];
-                    long long idj[2];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) jj[u] = (c0 + u < ncnt) ? a.nbr[nlb + (c0 + u) * 32] : -1;
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        if (jj[u] >= 0) {
-                            pj[u] = jpos(jj[u]);
-                            if constexpr (F64) {
-                                const dbl4 v = a.j_vel[jj[u]];
-                                vh[u] = Real<F64>::make4((R)v.x, (R)v.y, (R)v.z, (R)0);
-                                vl[u] = make_float4(0, 0, 0, 0);
-                            } else {
-                                vh[u] = __ldg(&a.fj.vhi[jj[u]]);
-                                vl[u] = __ldg(&a.fj.vlo[jj[u]]);
-                            }
-                            idj[u] = __ldg(&a.j_id[jj[u]]);
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        if (jj[u] >= 0) gpair(pj[u], vh[u].x, vh[u].y, vh[u].z, vl[u].x, vl[u].y, vl[u].z, idj[u]);
-                    if ((c0 & 7) == 6) fold();
-                }
-                fold();
-                if (r.act) ev_list_g += (unsigned)ncnt;
-                ++n_listed;
-            } else {
-                sweep(support2<R>(h), true, false, run);
-            }
-            const double sg = seg_sum(g_acc.value(), tpi);
-            const double sd = seg_sum(d_acc.value(), tpi);
-            const double sx = seg_sum(rx_acc.value(), tpi);
-            const double sy = seg_sum(ry_acc.value(), tpi);
-            const double sz = seg_sum(rz_acc.value(), tpi);
-            if (r.act && sub == 0) {
-                double divv, rotv, omega;
-                if (F64) {
-                    const double hinv_d = 1.0 / h;
-                    const double hinv4 = hinv_d * hinv_d * hinv_d * hinv_d;
-                    const double grdh = -hinv4 * sg;
-                    const double rx = CEFF1 * hinv4 * sx, ry = CEFF1 * hinv4 * sy, rz = CEFF1 * hinv4 * sz;
-                    const double rhoinv = 1.0 / (double)rho;
-                    omega = 1.0 / (1.0 + h * rhoinv * grdh / 3.0);
-                    const double rot2 = rx * rx + ry * ry + rz * rz;
-                    const double rot = (rot2 != 0.0) ? sqrt(rot2) : 0.0;
-                    divv = -CEFF1 * hinv4 * sd * rhoinv * omega;
-                    rotv = rot * rhoinv * omega;
-                } else {
-                    const float hf = (float)h;
-                    const float hinv_f = 1.0f / hf;
-                    const float hinv4 = hinv_f * hinv_f * hinv_f * hinv_f;
-                    const float rinv = 1.0f / (float)rho;
-                    const float g = -hinv4 * (float)sg;
-                    const float xf = (float)CEFF1 * hinv4 * (float)sx, yf = (float)CEFF1 * hinv4 * (float)sy,
-                                zf = (float)CEFF1 * hinv4 * (float)sz;
-                    const float om = 1.0f / (1.0f + hf * rinv * g / 3.0f);
-                    const float rot2 = xf * xf + yf * yf + zf * zf;
-                    omega = om;
-                    divv = -(float)CEFF1 * hinv4 * (float)sd * rinv * om;
-                    rotv = ((rot2 != 0.0f) ? sqrtf(rot2) : 0.0f) * rinv * om;
-                }
-                a.o_dens[ii] = (double)rho;
-                a.o_divv[ii] = divv;
-                a.o_rotv[ii] = rotv;
-                a.o_grdh[ii] = omega;
-                a.o_ksr[ii] = h;
-                a.o_np[ii] = (long long)np;
-                a.o_itr[ii] = itr ? 1 : 0;
-            }
-        }
-        if (a.n_eval) {
-            const unsigned long long l0 = __reduce_add_sync(FULL, ev_list);
-            const unsigned long long l1 = __reduce_add_sync(FULL, ev_list_g);
-            if (lane == 0) {
-                atomicAdd(a.n_eval, (unsigned long long)kept_rho * (unsigned long long)r.ni + l0);
-                atomicAdd(a.n_eval + 1, (unsigned long long)(kept - kept_rho) * (unsigned long long)r.ni + l1);
-            }
-        }
-        if (a.n_pass && lane == 0) {
-            atomicAdd(a.n_pass, (unsigned long long)n_listed);
-            atomicAdd(a.n_pass + 1, (unsigned long long)(3 - n_listed));
-        }
-    }
-}
-
-// Re-walks of few particles (the search-radius loop of hdr_density.hpp:
-// 382-414 late in its course: typically a handful of particles whose h
-// grew past 1.1^k times its first guess).  density_kernel gives such a walk
-// one warp, which streams the walk's list 32 entries at a time and waits on
-// every chunk's loads; here one block takes a walk and evaluates its
-// iterating particles one after another, every pass spreading the whole
-// list over the block's threads.  Same pair terms, per-particle updates,
-// search-radius decision, ambiguity queue and outputs as density_kernel
-// (for a one-particle item: positions relative to the particle itself);
-// each thread sums its entries (FP32C: Kahan) and the block adds the
-// threads' sums in FP64.  Runs only when *small is set (the caller then
-// leaves density_kernel no items).
-constexpr int REWALK_THREADS = 256;
-template <int N>
-__device__ __forceinline__ void block_sum(double (&v)[N], double (*red)[REWALK_THREADS / 32]) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < N; ++q) {
-        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(FULL, v[q], o);
-        if (lane == 0) red[q][wid] = v[q];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < N; ++q) {
-        double t = 0.0;
-        for (int u = 0; u < REWALK_THREADS / 32; ++u) t += red[q][u];
-        v[q] = t;
-    }
-    __syncthreads();
-}
-// Error bits (scal[err_slot]): list_err_mask marks lists that cannot be
-// used (a failed build: nothing runs), bounds_bit is raised for an index
-// outside the particle or list arrays (that access is skipped).
-struct RewalkBounds {
-    int n;                 // particles
-    long long list_cap;    // entries of the walks' lists
-    int *err;              // error word
-    int list_err_mask;
-    int bounds_bit;
-};
-template <bool F64>
-__global__ void __launch_bounds__(REWALK_THREADS) density_rewalk_blocks(const DensityArgs a, const int *n_walks,
-                                                                       const int *seg_first, const int *seg_count,
-                                                                       const int *small, RewalkBounds bnd) {
-    typedef typename Real<F64>::T R;
-    __shared__ double red[6][REWALK_THREADS / 32];
-    if (!*small || (*bnd.err & bnd.list_err_mask)) return;
-    const int nw = *n_walks;
-    const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
-    for (int w = blockIdx.x; w < nw; w += gridDim.x) {
-        const int jb = a.j_off[w], je = a.j_off[w + 1];
-        if (jb < 0 || je < jb || (long long)je > bnd.list_cap) {
-            if (threadIdx.x == 0) atomicOr(bnd.err, bnd.bounds_bit);
-            continue;   // block-uniform
-        }
-        for (int s = 0; s < seg_count[w]; ++s) {
-            const int u = seg_first[w] + s;
-            const int ii = (u >= 0 && u < bnd.n) ? a.i_list[u] : -1;
-            if (ii < 0 || ii >= bnd.n) {
-                if (threadIdx.x == 0) atomicOr(bnd.err, bnd.bounds_bit);
-                continue;   // block-uniform
-            }
-            float4 cph = make_float4(0, 0, 0, 0), cpl = cph;
-            dbl4 ci = make_dbl4(0, 0, 0, 0);
-            if (F64) ci = a.i_pm[ii];
-            else { cph = a.fi.phi[ii]; cpl = a.fi.plo[ii]; }
-            // position of j relative to i (FP32C) or absolute (FP64), and its mass
-            auto rel = [&](int j, R &dx, R &dy, R &dz) -> R {
-                if constexpr (F64) {
-                    const dbl4 p = a.j_pm[j];
-                    dx = (R)ci.x - (R)p.x; dy = (R)ci.y - (R)p.y; dz = (R)ci.z - (R)p.z;
-                    return (R)p.w;
-                } else {
-                    const float4 ph = a.fj.phi[j], pl = a.fj.plo[j];
-                    dx = -df_diff(ph.x, pl.x, cph.x, cpl.x);
-                    dy = -df_diff(ph.y, pl.y, cph.y, cpl.y);
-                    dz = -df_diff(ph.z, pl.z, cph.z, cpl.z);
-                    return (R)ph.w;
-                }
-            };
-            double h = a.i_ksr[ii];
-            const double mi = a.i_pm[ii].w;
-            R rho = 0;
-            long long np = 0;
-            // three fixed-point passes, hdr_density.hpp:264-302
-            for (int pass = 0; pass < 3; ++pass) {
-                const R hinv = (R)1 / (R)h;
-                const R hinv2 = hinv * hinv;
-                Acc<F64> acc;
-                long long cnt = 0;
-                for (int k = jb + threadIdx.x; k < je; k += REWALK_THREADS) {
-                    const int j = a.j_idx ? a.j_idx[k] : k;
-                    if (j < 0 || j >= bnd.n) {
-                        atomicOr(bnd.err, bnd.bounds_bit);
-                        continue;
-                    }
-                    R dx, dy, dz;
-                    const R m = rel(j, dx, dy, dz);
-                    const R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
-                    const R u = max0((R)1 - q);
-                    const R u2 = u * u;
-                    if (pass == 2) cnt += (q < (R)1) ? 1 : 0;
-                    acc.add(m * (u2 * u2 * ((R)1 + (R)4 * q)));
-                }
-                double v[2] = {acc.value(), (double)cnt};
-                block_sum(v, red);
-                double hn;
-                if (F64) {
-                    const double hinv_d = 1.0 / h;
-                    rho = (R)(CEFF0 * hinv_d * hinv_d * hinv_d * v[0]);
-                    hn = a.eta_ksrh * cbrt(mi / (double)rho);
-                } else {
-                    const float hinv_f = (float)hinv;
-                    const float rho_f = (float)CEFF0 * hinv_f * hinv_f * hinv_f * (float)v[0];
-                    rho = (R)rho_f;
-                    hn = (double)((float)a.eta_ksrh * cbrtf((float)mi / rho_f));
-                }
-                hn = (hn < ksr_max) ? hn : ksr_max;
-                np = (long long)v[1];
-                h = hn;
-            }
-            // the search-radius decision of the last pass (hdr_density.hpp:299)
-            const double rs_i = a.i_rs[ii];
-            const bool itr = h > rs_i;
-            if (!F64 && a.amb_count && threadIdx.x == 0 && fabs(h - rs_i) <= (double)a.amb_tol * rs_i) {
-                const int q = atomicAdd(a.amb_count, 1);
-                if (q < a.amb_cap) {
-                    a.amb_i[q] = ii;
-                    a.amb_w[q] = w;
-                }
-            }
-            // gradient pass with the final h, hdr_density.hpp:304-349
-            const long long idi = a.i_id[ii];
-            R vxi, vyi, vzi;
-            float lxi = 0.0f, lyi = 0.0f, lzi = 0.0f;
-            if (F64) {
-                const dbl4 vv = a.i_vel[ii];
-                vxi = (R)vv.x; vyi = (R)vv.y; vzi = (R)vv.z;
-            } else {
-                const float4 vh = a.fi.vhi[ii], vl = a.fi.vlo[ii];
-                vxi = vh.x; vyi = vh.y; vzi = vh.z;
-                lxi = vl.x; lyi = vl.y; lzi = vl.z;
-            }
-            const R hinv = (R)1 / (R)h;
-            Acc<F64> g_acc, d_acc, rx_acc, ry_acc, rz_acc;
-            for (int k = jb + threadIdx.x; k < je; k += REWALK_THREADS) {
-                const int j = a.j_idx ? a.j_idx[k] : k;
-                if (j < 0 || j >= bnd.n) {
-                    atomicOr(bnd.err, bnd.bounds_bit);
-                    continue;
-                }
-                R dx, dy, dz;
-                const R m = rel(j, dx, dy, dz);
-                R ux, uy, uz;
-                if constexpr (F64) {
-                    const dbl4 vv = a.j_vel[j];
-                    ux = vxi - (R)vv.x; uy = vyi - (R)vv.y; uz = vzi - (R)vv.z;
-                } else {
-                    const float4 vh = a.fj.vhi[j], vl = a.fj.vlo[j];
-                    ux = vxi - vh.x; uy = vyi - vh.y; uz = vzi - vh.z;
-                    ux += (R)(lxi - vl.x);
-                    uy += (R)(lyi - vl.y);
-                    uz += (R)(lzi - vl.z);
-                }
-                const R r2 = dx * dx + dy * dy + dz * dz;
-                const R ri = (idi != a.j_id[j]) ? rsqrt_r(r2) : (R)0;
-                const R q = r2 * ri * hinv;
-                const R u = max0((R)1 - q);
-                const R u2 = u * u;
-                const R u3 = u2 * u;
-                const R p14 = (R)1 + (R)4 * q;
-                const R w0 = u2 * u2 * p14;
-                const R w1 = w1_term(q, u, u2, u3, p14);
-                g_acc.add(m * ((R)(3.0 * CEFF0) * w0 + (R)CEFF1 * q * w1));
-                const R dw = m * w1 * ri;
-                d_acc.add((ux * dx + uy * dy + uz * dz) * dw);
-                rx_acc.add((uy * dz - uz * dy) * dw);
-                ry_acc.add((uz * dx - ux * dz) * dw);
-                rz_acc.add((ux * dy - uy * dx) * dw);
-            }
-            double v[5] = {g_acc.value(), d_acc.value(), rx_acc.value(), ry_acc.value(), rz_acc.value()};
-            block_sum(v, red);
-            if (threadIdx.x == 0) {
-                const double sg = v[0], sd = v[1], sx = v[2], sy = v[3], sz = v[4];
-                double divv, rotv, omega;
-                if (F64) {
-                    const double hinv_d = 1.0 / h;
-                    const double hinv4 = hinv_d * hinv_d * hinv_d * hinv_d;
-                    const double grdh = -hinv4 * sg;
-                    const double rx = CEFF1 * hinv4 * sx, ry = CEFF1 * hinv4 * sy, rz = CEFF1 * hinv4 * sz;
-                    const double rhoinv = 1.0 / (double)rho;
-                    omega = 1.0 / (1.0 + h * rhoinv * grdh / 3.0);
-                    const double rot2 = rx * rx + ry * ry + rz * rz;
-                    const double rot = (rot2 != 0.0) ? sqrt(rot2) : 0.0;
-                    divv = -CEFF1 * hinv4 * sd * rhoinv * omega;
-                    rotv = rot * rhoinv * omega;
-                } else {
-                    const float hf = (float)h;
-                    const float hinv_f = 1.0f / hf;
-                    const float hinv4 = hinv_f * hinv_f * hinv_f * hinv_f;
-                    const float rinv = 1.0f / (float)rho;
-                    const float g = -hinv4 * (float)sg;
-                    const float xf = (float)CEFF1 * hinv4 * (float)sx, yf = (float)CEFF1 * hinv4 * (float)sy,
-                                zf = (float)CEFF1 * hinv4 * (float)sz;
-                    const float om = 1.0f / (1.0f + hf * rinv * g / 3.0f);
-                    const float rot2 = xf * xf + yf * yf + zf * zf;
-                    omega = om;
-                    divv = -(float)CEFF1 * hinv4 * (float)sd * rinv * om;
-                    rotv = ((rot2 != 0.0f) ? sqrtf(rot2) : 0.0f) * rinv * om;
-                }
-                a.o_dens[ii] = (double)rho;
-                a.o_divv[ii] = divv;
-                a.o_rotv[ii] = rotv;
-                a.o_grdh[ii] = omega;
-                a.o_ksr[ii] = h;
-                a.o_np[ii] = np;
-                a.o_itr[ii] = itr ? 1 : 0;
-            }
-        }
-    }
-}
 
 // ---------------------------------------------------------------- hydro
 struct HydroArgs {
@@ -1897,27 +1039,19 @@ gravity_kernel(const GravityArgs a) {
     }
 }
 
-// One FP64 work item per queued particle (single-i items use all 32 lanes).
-__global__ inline void make_fixup_items(const int *amb_count, const int *amb_w, int cap, WorkItem *items,
-                                        int *n_items) {
-    const int n = min(*amb_count, cap);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        items[k] = make_int4(amb_w[k], k, 1, 0);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *n_items = n;
-}
-
 // ---------------------------------------------------------------- records
 // Builders of the FP32C double-float records from FP64 arrays (one thread
 // per particle).  Each fills hi/lo pairs; aux lanes as documented at the
 // consumers above.
-__global__ inline void make_density_records(int n, const dbl4 *pm, const dbl4 *vel, float4 *phi, float4 *plo,
-                                            float4 *vhi, float4 *vlo) {
+// Density records; lo.w: h rounded up (the row radius; 0 without h).
+__global__ inline void make_density_records(int n, const dbl4 *pm, const dbl4 *vel, const double *h, float4 *phi,
+                                            float4 *plo, float4 *vhi, float4 *vlo) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const dbl4 p = pm[k], v = vel[k];
         const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
         const float2 u = df_split(v.x), w = df_split(v.y), s = df_split(v.z);
         phi[k] = make_float4(x.x, y.x, z.x, (float)p.w);
-        plo[k] = make_float4(x.y, y.y, z.y, 0.0f);
+        plo[k] = make_float4(x.y, y.y, z.y, h ? __double2float_ru(h[k]) : 0.0f);
         vhi[k] = make_float4(u.x, w.x, s.x, 0.0f);
         vlo[k] = make_float4(u.y, w.y, s.y, 0.0f);
     }

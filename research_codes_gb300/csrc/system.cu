@@ -31,9 +31,9 @@ namespace {
 constexpr double KSRH = sphk::KSRH;
 constexpr double INV_KSRH2 = 1.0 / (KSRH * KSRH);   // eps^2 = h^2 / ksrh^2 without an FP64 divide
 constexpr int ITEM_SPLIT_NJ = 4096;   // default list length above which a walk's items are halved (down to 4 i)
-// density neighbour lists: entries per lane (a lane with more sweeps) and
-// the default list radius over the first-pass h (later passes whose h grew
-// beyond it sweep)
+// density neighbour lists and rows: entries per lane of the streamed walk (a
+// lane with more sweeps) and the default radius over the first-pass h (a
+// particle whose h grows beyond it sweeps its walk's list)
 constexpr int NBR_CAP = 96;
 constexpr float NBR_SLACK = 1.03f;
 constexpr float MAX_NBR_SLACK = 2.0f;
@@ -47,8 +47,9 @@ constexpr int MAX_RED = 8;
 // below 2^31 (lists that would need more are a capacity error).
 constexpr long long MAX_POOL_CHUNKS = 0x7fffffffLL / sphtree::LIST_CHUNK;
 constexpr int NBKT = 32;   // cost classes of work items (log2 of the estimated cost)
-enum { S_NGROUPS = 0, S_NACTIVE, S_NITEMS, S_QUEUE, S_ERROR, S_UNCONV, S_TOTAL, S_ITERS, S_AMB, S_NFIX, S_AMBTOT,
-       S_NTASKS, S_NROOTS, S_POOL, S_POOLERR, S_TQUEUE, S_POOLMAX, S_HOVF, S_SMALL, S_BKT,
+enum { S_NGROUPS = 0, S_NACTIVE, S_NITEMS, S_QUEUE, S_ERROR, S_UNCONV, S_TOTAL, S_ITERS, S_AMB, S_AMBTOT,
+       S_NTASKS, S_NROOTS, S_POOL, S_POOLERR, S_TQUEUE, S_POOLMAX, S_HOVF, S_SMALL, S_NITER, S_DOVF, S_NLONG, S_NLEFT,
+       S_BKT,
        S_NI = S_BKT + 2 * NBKT + 2 };
 // double scalars
 enum { D_TIME = 0, D_DT, D_KSRMAX, D_EPSU, D_DTC, D_XC, D_YC, D_ZC, D_MC, D_EKIN, D_ETHM, D_EPOT,
@@ -393,7 +394,6 @@ __global__ void compact_active(int n, const int *scal, const int *flag, const in
 }
 
 __global__ void set_int(int *p, int v) { *p = v; }
-__global__ void accumulate_int(const int *src, int *dst) { *dst += *src; }
 __global__ void copy_int(const int *src, int *dst) { *dst = *src; }
 
 // list totals: offset[n-1] + count[n-1] (counts beyond the walk count are 0)
@@ -541,21 +541,30 @@ __global__ void scatter_list(int n, const int *flag, const int *scan, int *list)
     }
 }
 
-// Re-walks with at most REWALK_SMALL iterating particles run on
-// density_rewalk_blocks (a block per walk) instead of density_kernel.
+// Number of i-particles of a walk over the iterating ones.  Re-walks (first =
+// 0) of at most REWALK_SMALL particles run on density_sweep (a block per
+// particle): their sweep queue holds all of them (walk_segments fills it) and
+// no row is marked.
 constexpr int REWALK_SMALL = 1024;
-__global__ void rewalk_small(int n, const int *flag, const int *scan, int *scal) {
+__global__ void walk_particles(int n, const int *flag, const int *scan, int first, int *scal) {
     const int total = scan[n - 1] + flag[n - 1];
-    scal[S_SMALL] = (total <= REWALK_SMALL) ? 1 : 0;
+    const int small = (!first && total <= REWALK_SMALL) ? 1 : 0;
+    scal[S_NITER] = total;
+    scal[S_SMALL] = small;
+    scal[S_DOVF] = small ? total : 0;
+    scal[S_NLONG] = 0;
+    scal[S_NLEFT] = 0;
 }
 __global__ void drop_items_if_small(int *scal) {
     if (scal[S_SMALL]) scal[S_NITEMS] = 0;
 }
 
-// the index-list segment of each active walk
+// the index-list segment of each active walk; when the walk is small, its
+// particles as (particle, walk) into the sweep queue
 __global__ void walk_segments(int n, const int *scal, const int *a_first, const int *a_count, const int *flag,
-                              const int *scan, int *seg_first, int *seg_count) {
+                              const int *scan, const int *list, int *seg_first, int *seg_count, int2 *queue) {
     const int nw = scal[S_NACTIVE];
+    const bool small = scal[S_SMALL] != 0;
     GRID_STRIDE(k, n) {
         if (k < nw) {
             const int f = a_first[k], e = a_first[k] + a_count[k];
@@ -563,6 +572,8 @@ __global__ void walk_segments(int n, const int *scal, const int *a_first, const 
             const int se = (e < n) ? scan[e] : scan[n - 1] + flag[n - 1];
             seg_first[k] = sf;
             seg_count[k] = se - sf;
+            if (small)
+                for (int u = sf; u < se; ++u) queue[u] = make_int2(list[u], k);
         }
     }
 }
@@ -957,17 +968,20 @@ struct sph_system {
     DevBuf<float4> flo, fhi, fmom, ptest;
     // FP32C double-float records (particles, hydro fields, tree monopoles)
     DevBuf<float4> f_phi, f_plo, f_vhi, f_vlo, f_g1, f_g2, f_g3, f_g4, f_shi, f_slo;
-    // FP32C hydro: per particle the j indices of its marked pairs
-    // (HYDRO_LIST_CAP per row), their number, and the rows that overflowed
+    // per particle the j indices of its pairs (ROW_CAP per row; density rows,
+    // then the hydro rows of the same evaluation), their number (density: with
+    // the walk), and the particles without a row
     DevBuf<int> hl_list, hl_cnt;
-    DevBuf<int2> hl_ovf;
+    DevBuf<int2> hl_ovf, r_info;
+    // items with long lists, left to a block each, and their particles
+    DevBuf<WorkItem> long_items;
+    DevBuf<int> left;
     // re-walk index list (particles still iterating) and its per-walk segments
     DevBuf<int> uflag, uscan, ulist, a_sfirst, a_scount;
     // FP64 re-check queue of decision-ambiguous density results
-    DevBuf<int> amb_i, amb_w;
-    DevBuf<WorkItem> fitems;
+    DevBuf<int2> amb;
     int amb_cap = 0;
-    // per-warp neighbour lists of the density kernel (scratch)
+    // per-warp neighbour lists of the streamed density walk (scratch)
     DevBuf<int> nbr;
     int nbr_warps = 0;
     DevBuf<double> w_csmax;   // per hydro walk: largest sound speed of its list
@@ -1083,9 +1097,10 @@ int alloc_all(sph_system *s) {
     e |= s->f_shi.ensure(nn) | s->f_slo.ensure(nn);
     e |= s->uflag.ensure(n) | s->uscan.ensure(n) | s->ulist.ensure(n) | s->a_sfirst.ensure(n) | s->a_scount.ensure(n);
     s->amb_cap = std::max<int>(1024, s->n / 16);
-    e |= s->amb_i.ensure(s->amb_cap) | s->amb_w.ensure(s->amb_cap) | s->fitems.ensure(s->amb_cap);
-    s->nbr_warps = std::max(s->ctx->grid[0][0], s->ctx->grid[0][1]) * PAIR_WARPS;
-    e |= s->nbr.ensure((size_t)s->nbr_warps * NBR_CAP * 32) | s->w_csmax.ensure(n);
+    e |= s->amb.ensure(s->amb_cap) | s->r_info.ensure(n) | s->w_csmax.ensure(n);
+    e |= s->long_items.ensure(n) | s->left.ensure(n);
+    s->nbr_warps = s->ctx->grid_stream * PAIR_WARPS;
+    e |= s->nbr.ensure((size_t)s->nbr_warps * NBR_CAP * 32);
     DevBuf<int> *i1[] = {&s->gflag, &s->groot, &s->gscan, &s->group_node, &s->group_first, &s->group_count,
                          &s->aflag, &s->ascan, &s->a_node, &s->a_first, &s->a_count};
     for (auto *b : i1) e |= b->ensure(n);
@@ -1271,6 +1286,14 @@ __global__ void pool_usage(int *scal) {
     atomicMax(&scal[S_POOLMAX], scal[S_POOL]);
 }
 
+// i-particles per density and hydro work item: halved from 32 (down to 4)
+// while that leaves resident warps without an item.
+int item_size(const sph_system *s) {
+    int chunk = 32;
+    while (chunk > 4 && (long long)s->n < (long long)chunk * 16 * s->ctx->sm_count) chunk >>= 1;
+    return chunk;
+}
+
 // Builds the lists of `kind` over the walks (group nodes + radii) and the
 // matching work items.  In eager mode (no capture) the list capacity grows to
 // the counted total first.
@@ -1452,72 +1475,73 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
     r = exclusive_scan(s, s->uflag.p, s->uscan.p);
     if (r) return r;
     scatter_list<<<grid_for(n), 256, 0, st>>>(n, s->uflag.p, s->uscan.p, s->ulist.p);
+    walk_particles<<<1, 1, 0, st>>>(n, s->uflag.p, s->uscan.p, first ? 1 : 0, s->scal.p);
     walk_segments<<<grid_for(n), 256, 0, st>>>(n, s->scal.p, s->a_first.p, s->a_count.p, s->uflag.p,
-                                               s->uscan.p, s->a_sfirst.p, s->a_scount.p);
-    if (!first) rewalk_small<<<1, 1, 0, st>>>(n, s->uflag.p, s->uscan.p, s->scal.p);
+                                               s->uscan.p, s->ulist.p, s->a_sfirst.p, s->a_scount.p, s->hl_ovf.p);
     const int kind = first ? 0 : 3;
     r = build_lists_and_items(s, kind, s->a_node.p, s->a_r.p, eager, s->lscal.p + (first ? L_PAIRS_D1 : L_PAIRS_D),
-                              s->a_sfirst.p, s->a_scount.p, first ? 32 : 8);
+                              s->a_sfirst.p, s->a_scount.p, !first ? std::min(8, item_size(s)) : f32 ? 32 : item_size(s));
     if (r) return r;
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
+    sphk::MarkArgs m{};
+    m.i_hi = s->f_phi.p; m.i_lo = s->f_plo.p; m.j_hi = s->f_phi.p; m.j_lo = s->f_plo.p;
+    m.slack = s->prm.density_list_slack > 0.0f ? s->prm.density_list_slack : 0.0f;
+    m.items = s->ls[0].items.p; m.n_items_dev = s->scal.p + S_NITEMS;
+    m.j_off = s->loff[kind].p; m.j_idx = s->jidx[kind].p; m.queue = s->scal.p + S_QUEUE;
+    m.i_list = s->ulist.p;
+    m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
+    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG;
     sphk::DensityArgs a{};
     a.n_eval = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_D1) : nullptr;
     a.n_pass = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_DLISTED) : nullptr;
-    const bool lists = s->prm.density_list_slack > 0.0f;
-    a.nbr = lists ? s->nbr.p : nullptr;
-    a.nbr_cap = NBR_CAP;
-    a.nbr_warps = s->nbr_warps;
-    a.nbr_slack = lists ? s->prm.density_list_slack : 1.0f;
     a.i_pm = s->pos[0].p; a.i_vel = s->vel[0].p; a.i_id = s->id[0].p; a.i_ksr = s->ksr[0].p;
     a.i_rs = s->rs.p;
     a.j_pm = s->pos[0].p; a.j_vel = s->vel[0].p; a.j_id = s->id[0].p;
-    a.items = s->ls[0].items.p; a.n_items = 0; a.n_items_dev = s->scal.p + S_NITEMS;
-    a.j_off = s->loff[kind].p; a.j_idx = s->jidx[kind].p; a.queue = s->scal.p + S_QUEUE;
-    a.i_list = s->ulist.p;
     a.fi = sphk::F32Part{s->f_phi.p, s->f_plo.p, s->f_vhi.p, s->f_vlo.p};
     a.fj = a.fi;
+    a.i_list = s->ulist.p; a.n_i_dev = s->scal.p + S_NITER;
+    a.j_off = m.j_off; a.j_idx = m.j_idx;
+    a.rows = m.rows; a.info = m.info; a.ovf = m.ovf; a.n_ovf = m.n_ovf; a.slack = m.slack;
+    a.err = s->scal.p + S_ERROR; a.err_mask = E_LISTCAP | E_STACK; a.skip_rows = s->scal.p + S_SMALL;
+    a.n_j = n; a.list_cap = s->lcap[kind]; a.err_out = s->scal.p + S_ERROR; a.bounds_bit = E_BOUNDS;
     a.o_dens = tmp.dens; a.o_divv = tmp.divv; a.o_rotv = tmp.rotv; a.o_grdh = tmp.grdh; a.o_ksr = tmp.ksr;
     a.o_np = tmp.np; a.o_itr = tmp.itr;
     a.eta_ksrh = ctx->prm.eta * KSRH;
     a.ksr_max = ctx->prm.ksr_max > 0.0 ? ctx->prm.ksr_max : std::numeric_limits<double>::infinity();
     a.ksr_max_dev = (s->prm.ksr_max_mode == 1) ? s->dscal.p + D_KSRMAX : nullptr;
     a.amb_count = f32 ? s->scal.p + S_AMB : nullptr;
-    a.amb_i = s->amb_i.p;
-    a.amb_w = s->amb_w.p;
+    a.amb = s->amb.p;
     a.amb_cap = s->amb_cap;
     a.amb_tol = sphrt::AMB_TOL;
     if (f32) CUDA_TRY(cudaMemsetAsync(s->scal.p + S_AMB, 0, sizeof(int), st));
     if (first) phase_event(s, EV_DENSK_B, st);
     if (!first) drop_items_if_small<<<1, 1, 0, st>>>(s->scal.p);
-    sphrt::launch_density(a, ctx->prm.precision, ctx->grid[0][ctx->prm.precision == SPH_PREC_FP64], st);
-    if (!first) {
-        // few iterating particles: a block per walk instead (see density_rewalk_blocks)
-        const int rg = ctx->sm_count * 4;
-        const sphk::RewalkBounds bnd{n, s->lcap[kind], s->scal.p + S_ERROR, E_LISTCAP | E_STACK, E_BOUNDS};
-        if (f32)
-            sphk::density_rewalk_blocks<false><<<rg, sphk::REWALK_THREADS, 0, st>>>(
-                a, s->scal.p + S_NACTIVE, s->a_sfirst.p, s->a_scount.p, s->scal.p + S_SMALL, bnd);
-        else
-            sphk::density_rewalk_blocks<true><<<rg, sphk::REWALK_THREADS, 0, st>>>(
-                a, s->scal.p + S_NACTIVE, s->a_sfirst.p, s->a_scount.p, s->scal.p + S_SMALL, bnd);
+    if (f32 && first) {
+        sphk::StreamArgs w{};
+        w.i_pm = a.i_pm; w.fi = a.fi; w.fj = a.fj; w.i_id = a.i_id; w.j_id = a.j_id;
+        w.i_ksr = a.i_ksr; w.i_rs = a.i_rs;
+        w.items = m.items; w.n_items_dev = m.n_items_dev; w.j_off = m.j_off; w.j_idx = m.j_idx;
+        w.i_list = m.i_list; w.queue = m.queue;
+        w.o_dens = a.o_dens; w.o_divv = a.o_divv; w.o_rotv = a.o_rotv; w.o_grdh = a.o_grdh; w.o_ksr = a.o_ksr;
+        w.o_np = a.o_np; w.o_itr = a.o_itr;
+        w.eta_ksrh = a.eta_ksrh; w.ksr_max = a.ksr_max; w.ksr_max_dev = a.ksr_max_dev;
+        w.amb_count = a.amb_count; w.amb = a.amb; w.amb_cap = a.amb_cap; w.amb_tol = a.amb_tol;
+        const bool lists = s->prm.density_list_slack > 0.0f;
+        w.nbr = lists ? s->nbr.p : nullptr;
+        w.nbr_cap = NBR_CAP;
+        w.nbr_warps = s->nbr_warps;
+        w.nbr_slack = lists ? s->prm.density_list_slack : 1.0f;
+        w.long_items = m.long_items; w.n_long = m.n_long;
+        w.left = s->left.p; w.n_left = s->scal.p + S_NLEFT;
+        w.n_eval = a.n_eval; w.n_pass = a.n_pass;
+        a.i_list = w.left;
+        a.n_i_dev = w.n_left;
+        sphrt::launch_density_stream(ctx, w, m, a, n, st, s->scal.p + S_AMBTOT);
+    } else {
+        sphrt::launch_density(ctx, m, ctx->grid[0][0], a, n, ctx->prm.precision, st,
+                              f32 ? s->scal.p + S_AMBTOT : nullptr);
     }
     if (first) phase_event(s, EV_DENSK_E, st);
-    if (f32) {
-        // FP64 recomputation of decision-ambiguous particles (same lists)
-        sphk::make_fixup_items<<<8, 256, 0, st>>>(s->scal.p + S_AMB, s->amb_w.p, s->amb_cap, s->fitems.p,
-                                                  s->scal.p + S_NFIX);
-        accumulate_int<<<1, 1, 0, st>>>(s->scal.p + S_AMB, s->scal.p + S_AMBTOT);
-        CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
-        sphk::DensityArgs f = a;
-        f.n_eval = nullptr;
-        f.n_pass = nullptr;
-        f.nbr = nullptr;
-        f.items = s->fitems.p;
-        f.n_items_dev = s->scal.p + S_NFIX;
-        f.i_list = s->amb_i.p;
-        f.amb_count = nullptr;
-        sphrt::launch_density(f, SPH_PREC_FP64, ctx->grid[0][1], st);
-    }
     commit_density<<<grid_for(n), 256, 0, st>>>(n, s->rs.p, tmp, out, s->scal.p);
     if (it >= 0)
         iteration_end<<<1, 1, 0, st>>>(s->scal.p, max_it, it);
@@ -1584,8 +1608,11 @@ int density_phase(sph_system *s, bool eager) {
     phase_event(s, EV_DENS_B, st);
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
     if (f32)
-        sphk::make_density_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->f_phi.p,
+        sphk::make_density_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->ksr[0].p, s->f_phi.p,
                                                                 s->f_plo.p, s->f_vhi.p, s->f_vlo.p);
+    else
+        sphk::make_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->ksr[0].p, false, s->f_phi.p,
+                                                            s->f_plo.p);
     init_rs<<<grid_for(n), 256, 0, st>>>(n, s->ksr[0].p, s->rs.p);
     // the first guess, kept for the derivative of this evaluation
     CUDA_TRY(cudaMemcpyAsync(s->h_guess.p, s->ksr[0].p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, st));
@@ -1710,7 +1737,8 @@ int hydro_phase(sph_system *s, bool eager) {
                                                               s->h3.p, s->f_phi.p, s->f_plo.p, s->f_vhi.p,
                                                               s->f_vlo.p, s->f_g1.p, s->f_g2.p, s->f_g3.p,
                                                               s->f_g4.p);
-    int r = build_lists_and_items(s, 1, s->group_node.p, nullptr, eager, s->lscal.p + L_PAIRS_H);
+    int r = build_lists_and_items(s, 1, s->group_node.p, nullptr, eager, s->lscal.p + L_PAIRS_H, nullptr, nullptr,
+                                  item_size(s));
     if (r) return r;
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
     const bool skip = s->prm.hydro_signal_skip != 0;
@@ -1981,7 +2009,7 @@ extern "C" int sph_system_destroy(sph_system *s) {
     for (auto *b : f1) b->release();
     s->hl_list.release(); s->hl_cnt.release(); s->hl_ovf.release();
     s->uflag.release(); s->uscan.release(); s->ulist.release(); s->a_sfirst.release(); s->a_scount.release();
-    s->amb_i.release(); s->amb_w.release(); s->fitems.release(); s->nbr.release(); s->w_csmax.release();
+    s->amb.release(); s->r_info.release(); s->long_items.release(); s->left.release(); s->nbr.release(); s->w_csmax.release();
     DevBuf<int> *i1[] = {&s->gflag, &s->groot, &s->gscan, &s->group_node, &s->group_first, &s->group_count,
                          &s->aflag, &s->ascan, &s->a_node, &s->a_first, &s->a_count,
                          &s->scal};
