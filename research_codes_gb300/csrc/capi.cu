@@ -77,12 +77,11 @@ static int occupancy_grid(K kernel, int threads, int sm_count, int *out) {
 int init_grids(sph_context *ctx) {
     const int th = PAIR_WARPS * 32;
     int e = 0;
-    e |= occupancy_grid(sphk::mark_rows<false, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[0][0]);
+    e |= occupancy_grid(sphk::mark_rows<sphk::ROWS_DENSITY, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[0][0]);
     e |= occupancy_grid(sphk::density_stream<PAIR_WARPS>, th, ctx->sm_count, &ctx->grid_stream);
     ctx->grid[0][1] = ctx->grid[0][0];   // the rows are marked in FP32 in both precisions
-    e |= occupancy_grid(sphk::hydro_kernel<false, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[1][0]);
-    e |= occupancy_grid(sphk::hydro_kernel<true, HYDRO64_WARPS>, HYDRO64_WARPS * 32, ctx->sm_count,
-                        &ctx->grid[1][1]);
+    e |= occupancy_grid(sphk::mark_rows<sphk::ROWS_HYDRO32, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[1][0]);
+    e |= occupancy_grid(sphk::mark_rows<sphk::ROWS_HYDRO64, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[1][1]);
     e |= occupancy_grid(sphk::gravity_kernel<false, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[2][0]);
     e |= occupancy_grid(sphk::gravity_kernel<true, PAIR_WARPS>, th, ctx->sm_count, &ctx->grid[2][1]);
     e |= occupancy_grid(sphk::hydro_df_lists, sphk::HYDRO_DF_THREADS, ctx->sm_count, &ctx->grid_df);
@@ -92,16 +91,15 @@ int init_grids(sph_context *ctx) {
 
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items) {
     const int full = ctx->grid[kind][precision == SPH_PREC_FP64 ? 1 : 0];
-    const int warps = (kind == 1 && precision == SPH_PREC_FP64) ? HYDRO64_WARPS : PAIR_WARPS;
-    const int need = (n_items + warps - 1) / warps;
+    const int need = (n_items + PAIR_WARPS - 1) / PAIR_WARPS;
     return std::max(1, std::min(full, need));
 }
 
 // The queued long items: a block each.
-template <bool SYM>
+template <int KIND>
 static void mark_long(const sph_context *ctx, const sphk::MarkArgs &m, int n_max, cudaStream_t s) {
-    sphk::mark_rows<SYM, sphk::MARK_LONG_WARPS, true>
-        <<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), sphk::MARK_LONG_WARPS * 32, 0, s>>>(m);
+    constexpr int W = KIND == sphk::ROWS_DENSITY ? sphk::MARK_LONG_WARPS : sphk::HYDRO_LONG_WARPS;
+    sphk::mark_rows<KIND, W, true><<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), W * 32, 0, s>>>(m);
 }
 
 // FP64 recomputation of the FP32C results queued as ambiguous (their number
@@ -137,43 +135,54 @@ static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs 
 // Rows of the items of m, then the density sums over them.
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
                     int n_max, int precision, cudaStream_t s, int *amb_total) {
-    sphk::mark_rows<false, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-    mark_long<false>(ctx, m, n_max, s);
+    sphk::mark_rows<sphk::ROWS_DENSITY, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
+    mark_long<sphk::ROWS_DENSITY>(ctx, m, n_max, s);
     launch_density_sums(ctx, a, n_max, precision, s, amb_total);
 }
 
-// The FP32C first walk of a particle system (n_max particles): the streamed
-// walk, then rows for the items it left (m and a cover them), the sweep of
-// what has no row and the FP64 recomputation of the ambiguous particles.
-void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, const sphk::MarkArgs &m,
-                           const sphk::DensityArgs &a, int n_max, cudaStream_t s, int *amb_total) {
+// The FP32C density of a particle system (n_max particles): the streamed walk
+// over the items of w (those with long lists a block each), the sweep of the queued particles (re-walks of few) and
+// the FP64 recomputation of the ambiguous ones.
+void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
+                           int n_max, cudaStream_t s, int *amb_total) {
     sphk::density_stream<PAIR_WARPS><<<ctx->grid_stream, PAIR_WARPS * 32, 0, s>>>(w);
-    mark_long<false>(ctx, m, n_max, s);
-    launch_density_sums(ctx, a, n_max, SPH_PREC_FP32C, s, amb_total);
+    sphk::density_stream<sphk::STREAM_LONG_WARPS, true>
+        <<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), sphk::STREAM_LONG_WARPS * 32, 0, s>>>(w);
+    if (sweep)
+        sphk::density_sweep<false><<<std::max(1, std::min(n_max, ctx->sm_count * 6)), sphk::DSWEEP_THREADS, 0, s>>>(
+            a, a.ovf, a.n_ovf, n_max, nullptr);
+    recheck_density(ctx, a, n_max, s, amb_total);
 }
 
-// FP32C: the signal-velocity / marking kernel, then the double-float pass
-// over the marked-pair rows and over the overflowed particles (a.df_novf
-// must be zero at launch; dfgrid: resident blocks of the double-float pass).
-// mid (optional) is recorded between the two (as an external record node
+// Hydro: signal velocities and rows of the items of m, then the pair sums
+// over them (FP32C: the double-float pass) and over the lists of the particles
+// without a row.  *a.n_ovf and *m.n_long must be zero at launch.  mid
+// (optional) is recorded between the two parts (as an external record node
 // when mid_external: inside a stream capture).
-void launch_hydro(const sphk::HydroArgs &a, int precision, int grid, cudaStream_t s, int dfgrid,
-                  cudaEvent_t mid, bool mid_external) {
-    auto record_mid = [&]() {
-        if (mid) cudaEventRecordWithFlags(mid, s, mid_external ? cudaEventRecordExternal : cudaEventRecordDefault);
-    };
-    if (precision == SPH_PREC_FP64) {
-        sphk::hydro_kernel<true, HYDRO64_WARPS><<<grid, HYDRO64_WARPS * 32, 0, s>>>(a);
-        record_mid();
+void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
+                  int precision, cudaStream_t s, cudaEvent_t mid, bool mid_external) {
+    const bool f64 = precision == SPH_PREC_FP64;
+    if (f64) {
+        sphk::mark_rows<sphk::ROWS_HYDRO64, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
+        mark_long<sphk::ROWS_HYDRO64>(ctx, m, a.n_i, s);
+    } else {
+        sphk::mark_rows<sphk::ROWS_HYDRO32, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
+        mark_long<sphk::ROWS_HYDRO32>(ctx, m, a.n_i, s);
+    }
+    if (mid) cudaEventRecordWithFlags(mid, s, mid_external ? cudaEventRecordExternal : cudaEventRecordDefault);
+    if (a.n_i <= 0) return;
+    if (f64) {
+        const int per_block = sphk::HROWS_THREADS / sphk::HROWS_LANES;
+        sphk::hydro64_rows<<<std::max(1, std::min((a.n_i + per_block - 1) / per_block, 16 * ctx->sm_count)),
+                             sphk::HROWS_THREADS, 0, s>>>(a);
+        sphk::hydro64_sweep<<<std::max(1, std::min(a.n_i, 2 * ctx->sm_count)), sphk::DSWEEP_THREADS, 0, s>>>(a);
         return;
     }
-    sphk::hydro_kernel<false, PAIR_WARPS><<<grid, PAIR_WARPS * 32, 0, s>>>(a);
-    record_mid();
-    if (a.n_i <= 0) return;
     const int need = (a.n_i + sphk::HYDRO_DF_THREADS - 1) / sphk::HYDRO_DF_THREADS;
-    sphk::hydro_df_lists<<<std::max(1, std::min(need, dfgrid)), sphk::HYDRO_DF_THREADS, 0, s>>>(a);
-    // one block per overflowed particle, up to one per SM and round
-    sphk::hydro_df_sweep<<<std::max(1, std::min(a.n_i, 2 * dfgrid / 5 + 1)), sphk::HYDRO_SWEEP_THREADS, 0, s>>>(a);
+    sphk::hydro_df_lists<<<std::max(1, std::min(need, ctx->grid_df)), sphk::HYDRO_DF_THREADS, 0, s>>>(a);
+    // one block per particle without a row, up to one per SM and round
+    sphk::hydro_df_sweep<<<std::max(1, std::min(a.n_i, 2 * ctx->grid_df / 5 + 1)), sphk::HYDRO_SWEEP_THREADS, 0, s>>>(
+        a);
 }
 
 // jtile: entries a warp stages per pass in FP32C (32 or 64; FP64 uses 32).
@@ -494,6 +503,7 @@ namespace {
 
 enum { K_DENS = 0, K_HYDRO = 1, K_GRAV = 2 };
 constexpr float ROW_SLACK = 1.03f;   // row radius of the density over the first guess of h
+constexpr int LONG_NJ = 4096;    // lists beyond this are marked by a block per item
 constexpr int SPLIT_NJ = 1024;   // density and hydro: lists beyond this make smaller items
 
 // Validates walk counts and fills the int32 offsets.  n_extra (gravity SPJ
@@ -666,7 +676,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
             sphk::make_density_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
                 ni, ks.a4[0].p, ks.a4[1].p, ks.d1[0].p, ks.f4[0].p, ks.f4[1].p, ks.f4[2].p, ks.f4[3].p);
         else
-            sphk::make_row_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.a4[0].p, ks.d1[0].p, false,
+            sphk::make_row_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.a4[0].p, ks.d1[0].p,
                                                                              ks.f4[0].p, ks.f4[1].p);
     }
     if (nj > 0) {
@@ -674,7 +684,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
             sphk::make_density_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
                 nj, ks.a4[2].p, ks.a4[3].p, nullptr, ks.f4[4].p, ks.f4[5].p, ks.f4[6].p, ks.f4[7].p);
         else
-            sphk::make_row_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(nj, ks.a4[2].p, nullptr, false,
+            sphk::make_row_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(nj, ks.a4[2].p, nullptr,
                                                                              ks.f4[4].p, ks.f4[5].p);
     }
     if (!ks.items.empty()) {
@@ -692,7 +702,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         m.j_off = (const int *)(d + L.off_joff);
         m.queue = ctx->d_queue + K_DENS;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 7;
-        m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9;
+        m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
         sphk::DensityArgs a{};
         a.i_pm = ks.a4[0].p; a.i_vel = ks.a4[1].p; a.i_id = ks.id[0].p; a.i_ksr = ks.d1[0].p; a.i_rs = ks.d1[1].p;
         a.j_pm = ks.a4[2].p; a.j_vel = ks.a4[3].p; a.j_id = ks.id[1].p;
@@ -740,8 +750,11 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
     if ((st = walk_offsets(ctx, n_walk, n_epi, n_epj, nullptr, i_off, j_off))) return st;
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
     Layout L;
+    // FP32C: items of 32 i-particles, whose rows and so sums do not depend on
+    // the size of the call
+    const bool f64 = ctx->prm.precision == SPH_PREC_FP64;
     if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_HydroEPI), sizeof(sph_HydroEPJ),
-                           item_size(ctx, i_off[n_walk]), SPLIT_NJ, L))) return st;
+                           f64 ? item_size(ctx, i_off[n_walk]) : 32, f64 ? SPLIT_NJ : 0, L))) return st;
     for (int w = 0; w < n_walk; ++w) {
         if ((n_epi[w] && !epi[w]) || (n_epj[w] && !epj[w]))
             return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
@@ -765,18 +778,41 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
             (const sph_HydroEPJ *)(d + L.off_epj), nj, true, ks.a4[2].p, ks.a4[3].p, ks.id[1].p,
             ks.a4[6].p, ks.a4[7].p, ks.a2[1].p);
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
-    if (f32 && ni > 0)
-        sphk::make_hydro_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-            ni, ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.a2[0].p, ks.f4[0].p, ks.f4[1].p, ks.f4[2].p,
-            ks.f4[3].p, ks.f4[8].p, ks.f4[9].p, ks.f4[10].p, ks.f4[14].p);
-    if (f32 && nj > 0)
-        sphk::make_hydro_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
-            nj, ks.a4[2].p, ks.a4[3].p, ks.a4[6].p, ks.a4[7].p, ks.a2[1].p, ks.f4[4].p, ks.f4[5].p, ks.f4[6].p,
-            ks.f4[7].p, ks.f4[11].p, ks.f4[12].p, ks.f4[13].p, ks.f4[15].p);
+    if (ni > 0) {
+        if (f32)
+            sphk::make_hydro_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
+                ni, ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.a2[0].p, ks.f4[0].p, ks.f4[1].p, ks.f4[2].p,
+                ks.f4[3].p, ks.f4[8].p, ks.f4[9].p, ks.f4[10].p, ks.f4[14].p, ks.f4[16].p, ks.f4[17].p);
+        else
+            sphk::make_hydro_row_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
+                ni, ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.f4[16].p, ks.f4[1].p, ks.f4[17].p);
+    }
+    if (nj > 0) {
+        if (f32)
+            sphk::make_hydro_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
+                nj, ks.a4[2].p, ks.a4[3].p, ks.a4[6].p, ks.a4[7].p, ks.a2[1].p, ks.f4[4].p, ks.f4[5].p, ks.f4[6].p,
+                ks.f4[7].p, ks.f4[11].p, ks.f4[12].p, ks.f4[13].p, ks.f4[15].p, ks.f4[18].p, ks.f4[19].p);
+        else
+            sphk::make_hydro_row_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
+                nj, ks.a4[2].p, ks.a4[3].p, ks.a4[6].p, ks.a4[7].p, ks.f4[18].p, ks.f4[5].p, ks.f4[19].p);
+    }
     if (!ks.items.empty()) {
+        if (ks.long_items.ensure(ks.items.size())) return set_error(ctx, SPH_ERR_CUDA, "allocation failed");
+        // no particle without a row and no long item yet
+        cudaError_t e = cudaMemsetAsync(ctx->d_queue + 8, 0, 2 * sizeof(int), ctx->stream);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
+        sphk::MarkArgs m{};
+        m.i_hi = ks.f4[16].p; m.i_lo = ks.f4[1].p; m.j_hi = ks.f4[18].p; m.j_lo = ks.f4[5].p;
+        m.i_v = ks.f4[17].p; m.j_v = ks.f4[19].p;
+        m.items = (const WorkItem *)(d + L.off_items);
+        m.n_items = (int)ks.items.size();
+        m.j_off = (const int *)(d + L.off_joff);
+        m.queue = ctx->d_queue + K_HYDRO;
+        m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 8;
+        m.long_items = f64 ? ks.long_items.p : nullptr; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
+        m.o_vsmx = ks.o[3].p;
+        m.sv_skip = 1;
         sphk::HydroArgs a{};
-        a.n_eval_near = nullptr;
-        a.n_eval_far = nullptr;
         a.i_pm = ks.a4[0].p; a.i_vel = ks.a4[1].p; a.i_id = ks.id[0].p;
         a.i_h1 = ks.a4[4].p; a.i_h2 = ks.a4[5].p; a.i_h3 = ks.a2[0].p;
         a.j_pm = ks.a4[2].p; a.j_vel = ks.a4[3].p; a.j_id = ks.id[1].p;
@@ -785,26 +821,15 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         a.fj = sphk::F32Part{ks.f4[4].p, ks.f4[5].p, ks.f4[6].p, ks.f4[7].p};
         a.fi_g1 = ks.f4[8].p; a.fi_g2 = ks.f4[9].p; a.fi_g3 = ks.f4[10].p;
         a.fj_g1 = ks.f4[11].p; a.fj_g2 = ks.f4[12].p; a.fj_g3 = ks.f4[13].p;
-        a.i_list = nullptr;
-        a.items = (const WorkItem *)(d + L.off_items);
-        a.n_items = (int)ks.items.size();
-        a.n_items_dev = nullptr;
-        a.j_off = (const int *)(d + L.off_joff);
-        a.j_idx = nullptr;
-        a.queue = ctx->d_queue + K_HYDRO;
-        a.o_acch = ks.o[0].p; a.o_accg = ks.o[1].p; a.o_udot = ks.o[2].p; a.o_vsmx = ks.o[3].p;
-        a.o_diffu = ks.o[4].p;
         a.fi_g4 = ks.f4[14].p; a.fj_g4 = ks.f4[15].p;
-        a.df_list = ks.hl_list.p; a.df_cap = sphk::HYDRO_LIST_CAP; a.df_cnt = ks.hl_cnt.p;
-        a.df_ovf = ks.hl_ovf.p; a.df_novf = ctx->d_queue + 8; a.n_i = ni;
-        if (f32) {
-            // walks without items leave their rows empty; no overflow yet
-            cudaError_t e = cudaMemsetAsync(ks.hl_cnt.p, 0, sizeof(int) * (size_t)ni, ctx->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_queue + 8, 0, sizeof(int), ctx->stream);
-            if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
-        }
-        launch_hydro(a, ctx->prm.precision, pair_grid(ctx, K_HYDRO, ctx->prm.precision, a.n_items), ctx->stream,
-                     ctx->grid_df);
+        a.j_off = m.j_off;
+        a.o_acch = ks.o[0].p; a.o_accg = ks.o[1].p; a.o_udot = ks.o[2].p; a.o_diffu = ks.o[4].p;
+        a.rows = m.rows; a.info = m.info; a.ovf = m.ovf; a.n_ovf = m.n_ovf; a.n_i = ni;
+        a.mi_p = m.i_hi; a.mi_l = m.i_lo; a.mj_p = m.j_hi; a.mj_l = m.j_lo;
+        m.i_id = a.i_id; m.j_id = a.j_id; m.fi = a.fi; m.fj = a.fj; m.fi_g2 = a.fi_g2; m.fj_g2 = a.fj_g2;
+        m.i_pm = a.i_pm; m.i_vel = a.i_vel; m.i_h2 = a.i_h2; m.j_pm = a.j_pm; m.j_vel = a.j_vel; m.j_h2 = a.j_h2;
+        launch_hydro(ctx, m, pair_grid(ctx, K_HYDRO, ctx->prm.precision, m.n_items), a, ctx->prm.precision,
+                     ctx->stream);
     }
     if (ni > 0)
         pack_hydro<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(

@@ -10,9 +10,6 @@
 #include "pair_kernels.cuh"
 
 #define PAIR_WARPS 4
-// the FP64 hydro kernel's shared rings need half the warps per block to stay
-// within the 48 KB static shared-memory limit
-#define HYDRO64_WARPS 2
 
 namespace sphrt {
 
@@ -82,8 +79,8 @@ struct KindState {
     HostBuf<char> h_in, h_out;
     DevBuf<char> d_in, d_out;
     DevBuf<dbl4> a4[8];
-    DevBuf<float4> f4[16];   // FP32C double-float records
-    DevBuf<int> hl_list, hl_cnt;       // rows of the density and hydro sums, hydro counts
+    DevBuf<float4> f4[20];   // FP32C double-float records; 16..19 hydro mark records
+    DevBuf<int> hl_list;               // rows of the density and hydro sums
     DevBuf<int2> hl_ovf;               // particles without a row (particle, walk)
     DevBuf<double2> a2[2];
     DevBuf<long long> id[2];
@@ -91,9 +88,9 @@ struct KindState {
     DevBuf<double> o[5];
     DevBuf<long long> o_np;
     DevBuf<unsigned char> o_itr;
-    DevBuf<int2> r_info;               // density rows (in hl_list): entries and walk per particle
+    DevBuf<int2> r_info;               // rows: entries and walk per particle
     DevBuf<int2> amb;                  // FP64 re-check queue of the density
-    DevBuf<int4> long_items;           // items with lists beyond LONG_LIST
+    DevBuf<int4> long_items;           // items with lists left to a block each
     std::vector<int4> items;
     std::vector<int> i_off;
     bool pending = false;
@@ -121,7 +118,8 @@ struct KindState {
         for (int k = 0; k < 4; ++k) e |= f4[k].ensure(ni) | f4[4 + k].ensure(nj);
         for (int k = 8; k < 11; ++k) e |= f4[k].ensure(ni) | f4[k + 3].ensure(nj);
         e |= f4[14].ensure(ni) | f4[15].ensure(nj);
-        e |= hl_list.ensure(ni * sphk::HYDRO_LIST_CAP) | hl_cnt.ensure(ni) | hl_ovf.ensure(ni);
+        e |= f4[16].ensure(ni) | f4[17].ensure(ni) | f4[18].ensure(nj) | f4[19].ensure(nj);
+        e |= hl_list.ensure(ni * sphk::ROW_CAP) | r_info.ensure(ni) | hl_ovf.ensure(ni);
         return e;
     }
     int ensure_gravity(size_t ni, size_t nj) {
@@ -139,7 +137,6 @@ struct KindState {
         for (auto &b : a4) b.release();
         for (auto &b : f4) b.release();
         hl_list.release();
-        hl_cnt.release();
         hl_ovf.release();
         for (auto &b : a2) b.release();
         for (auto &b : id) b.release();
@@ -179,9 +176,9 @@ int cuda_error(sph_context *ctx, cudaError_t e, const char *what);
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items);
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
                     int n_max, int precision, cudaStream_t s, int *amb_total = nullptr);
-void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, const sphk::MarkArgs &m,
-                           const sphk::DensityArgs &a, int n_max, cudaStream_t s, int *amb_total);
-void launch_hydro(const sphk::HydroArgs &a, int precision, int grid, cudaStream_t s, int dfgrid,
-                  cudaEvent_t mid = nullptr, bool mid_external = false);
+void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
+                           int n_max, cudaStream_t s, int *amb_total);
+void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
+                  int precision, cudaStream_t s, cudaEvent_t mid = nullptr, bool mid_external = false);
 void launch_gravity(const sphk::GravityArgs &a, int precision, int grid, cudaStream_t s, int jtile);
 }  // namespace sphrt

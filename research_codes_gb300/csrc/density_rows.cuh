@@ -25,14 +25,6 @@
 
 namespace sphk {
 
-// Double-float particle records of FP32C mode.
-struct F32Part {
-    const float4 *phi;   // x_hi, y_hi, z_hi, mass
-    const float4 *plo;   // x_lo, y_lo, z_lo, aux
-    const float4 *vhi;   // vx_hi, vy_hi, vz_hi, aux
-    const float4 *vlo;   // vx_lo, vy_lo, vz_lo, aux
-};
-
 struct DensityArgs {
     // FP64 records (i_pm is read in both modes for the i-particle's mass)
     const dbl4 *i_pm;       // x, y, z, mass
@@ -222,12 +214,17 @@ struct PairPos {
         }
     }
     __device__ __forceinline__ R rel(const DensityArgs &a, int j, R &dx, R &dy, R &dz) const {
+        if constexpr (F64) return rel(a, j, hi, lo, dx, dy, dz);
+        else return rel(a, j, __ldg(&a.fj.phi[j]), __ldg(&a.fj.plo[j]), dx, dy, dz);
+    }
+    // FP32C: (qh, ql) are j's records
+    __device__ __forceinline__ R rel(const DensityArgs &a, int j, const float4 &qh, const float4 &ql, R &dx, R &dy,
+                                     R &dz) const {
         if constexpr (F64) {
             const dbl4 q = a.j_pm[j];
             dx = p.x - q.x; dy = p.y - q.y; dz = p.z - q.z;
             return q.w;
         } else {
-            const float4 qh = __ldg(&a.fj.phi[j]), ql = __ldg(&a.fj.plo[j]);
             dx = -df_diff(qh.x, ql.x, hi.x, lo.x);
             dy = -df_diff(qh.y, ql.y, hi.y, lo.y);
             dz = -df_diff(qh.z, ql.z, hi.z, lo.z);
@@ -458,10 +455,35 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         P.load_i(a, ii);
         const float4 ph = a.fi.phi[ii], pl = a.fi.plo[ii];
         const double mi = a.i_pm[ii].w;
-        // visits the list entries that can lie within h of the particle: an
-        // FP32 distance test on the double-float positions, with the margins
-        // of mark_rows (h outside its range: every entry)
+        // visits the list entries; FP64: those that can lie within h of the
+        // particle by an FP32 distance test on the double-float positions,
+        // with the margins of mark_rows (h outside its range: every entry)
         auto over_list = [&](R h, auto &&f) {
+            if constexpr (!F64) {   // the test would cost what the sum does
+                for (int k0 = jb + threadIdx.x; k0 < je; k0 += T * U) {
+                    int j[U];
+                    float4 qh[U], ql[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int k = k0 + u * T;
+                        j[u] = (k < je) ? (a.j_idx ? a.j_idx[k] : k) : -1;
+                        if (a.n_j > 0 && j[u] >= a.n_j) {
+                            atomicOr(a.err_out, a.bounds_bit);
+                            j[u] = -1;
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (j[u] >= 0) {
+                            qh[u] = __ldg(&a.fj.phi[j[u]]);
+                            ql[u] = __ldg(&a.fj.plo[j[u]]);
+                        }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (j[u] >= 0) f(j[u], qh[u], ql[u]);
+                }
+                return;
+            }
             const float hf = (float)h;
             const float pad = 3.0e-14f * (fabsf(ph.x) + fabsf(ph.y) + fabsf(ph.z));
             const float rad = hf * 1.0001f + pad;
@@ -491,7 +513,7 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
                         const float dx = df_diff(qh[u].x, ql[u].x, ph.x, pl.x);
                         const float dy = df_diff(qh[u].y, ql[u].y, ph.y, pl.y);
                         const float dz = df_diff(qh[u].z, ql[u].z, ph.z, pl.z);
-                        if (!(dx * dx + dy * dy + dz * dz > lim)) f(j[u]);
+                        if (!(dx * dx + dy * dy + dz * dz > lim)) f(j[u], qh[u], ql[u]);
                     }
             }
         };
@@ -501,10 +523,11 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         for (int pass = 0; pass < 3; ++pass) {
             Acc<F64> acc;
             int cnt = 0;
-            over_list(s.h, [&](int j) {
+            const R hinv2 = s.hinv * s.hinv;
+            over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
                 R dx, dy, dz;
-                const R m = P.rel(a, j, dx, dy, dz);
-                const R q = sqrt_r(dx * dx + dy * dy + dz * dz) * s.hinv;
+                const R m = P.rel(a, j, qh, ql, dx, dy, dz);
+                const R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
                 cnt += (q < (R)1) ? 1 : 0;
                 acc.add(density_term(q, m));
             });
@@ -517,9 +540,9 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         const long long idi = a.i_id[ii];
         PairVel<F64> V;
         V.load_i(a, ii);
-        over_list(s.h, [&](int j) {
+        over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
             R dx, dy, dz, ux, uy, uz;
-            const R m = P.rel(a, j, dx, dy, dz);
+            const R m = P.rel(a, j, qh, ql, dx, dy, dz);
             V.rel(a, j, ux, uy, uz);
             gs.add(dx, dy, dz, ux, uy, uz, m, a.j_id[j] == idi, s.hinv);
             gs.fold();

@@ -1,10 +1,17 @@
-// density_stream.cuh — the FP32C density of a particle system's first walk,
-// over work items of up to 32 i-particles.
+// density_stream.cuh — the FP32C density of a particle system, over work items
+// of up to 32 i-particles.
 //
 // One warp streams its item's whole list; entries inside the list radius go
-// to per-lane neighbour lists that the later passes read.  The rows kernels
-// (density_rows.cuh) serve every other density: FP64, the functors and the
-// re-walks.
+// to per-lane neighbour lists that the later passes read.  Items with longer
+// lists are left to the LONG form, in which a block streams one item: same
+// ring order, same tiles, same folds, so the same results bit for bit, with
+// the loads, support tests and tiles of a round spread over its warps.
+//
+// The rows kernels (density_rows.cuh) serve the FP64 density, the functors and
+// the re-walks of few particles.  They are not used here: the hydro sums
+// amplify a change of rounding in h and rho by up to 10^3, and the h of a few
+// surface particles by more from evaluation to evaluation, so that runs would
+// leave the trajectories they had before.
 #pragma once
 
 #include "density_rows.cuh"
@@ -20,8 +27,7 @@ namespace sphk {
 
 // f32x2 iterations (two entries each) of the packed loop per unrolled round
 constexpr int DENSITY_UNROLL = SPH_DENSITY_UNROLL;
-// Longer lists go to the LONG form of mark_rows.
-constexpr int STREAM_LONG = 8192;
+constexpr int STREAM_LONG_WARPS = 8;
 
 struct StreamArgs {
     const dbl4 *i_pm;       // x, y, z, mass
@@ -61,11 +67,11 @@ struct StreamArgs {
     int nbr_cap = 0;
     int nbr_warps = 0;
     float nbr_slack = 1.0f;
-    // walks beyond STREAM_LONG entries are left to the rows kernels: their
-    // items and particles are queued
+    // items left to the LONG form (null: none) and their number; the listed
+    // pairs of the walk, which say what a long list is
     WorkItem *long_items;
     int *n_long;
-    int *left, *n_left;
+    const long long *pairs;
     // when set: pair evaluations performed, [0] the three density passes
     // ((j-entries kept by the support test x i-particles) of the swept passes
     // plus the list entries of the listed ones), [1] the gradient pass
@@ -96,24 +102,45 @@ struct BTag {
 // otherwise the pass sweeps.  Entries beyond a particle's support add exactly
 // zero in both forms, so the two differ only in the grouping of the FP32
 // partial sums.
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_stream(const StreamArgs a) {
+//
+// LONG: a block takes an item of the long-item queue.  Its warps hold the same
+// lanes; a round of 32 WARPS U list entries is loaded and tested by all of
+// them, compacted in list order, cut into 32-entry tiles that the warps sum
+// one each, and every warp folds the tiles' partial sums in order.
+template <int WARPS, bool LONG = false>
+__global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS) density_stream(const StreamArgs a) {
+    // LONG: the compacted entries (< 32 left over + a round) and the tiles'
+    // partial sums (1 or 5 per lane; the list-building pass keeps its marks in
+    // the second slot)
+    constexpr int U = 4, ROUND = 32 * U * WARPS, LBUF = LONG ? ROUND + 32 : 1, LT = LONG ? LBUF / 32 : 1;
+    __shared__ __align__(16) float l_x[LBUF], l_y[LBUF], l_z[LBUF], l_m[LBUF];
+    __shared__ int l_j[LBUF];
+    __shared__ float l_part[LT][5][32];
+    __shared__ int l_cnt[LONG ? WARPS : 1];
+    __shared__ unsigned l_any[LT];
+    constexpr int RW = LONG ? 1 : WARPS, RN = LONG ? 1 : 64;   // the per-warp ring
     // per warp a 64-entry ring of compacted j records: entries accumulate
     // until 32 are ready, the pair loop consumes one 32-entry half at a time
-    __shared__ float4 s_p[WARPS][64];
-    __shared__ float4 s_v[WARPS][64];
-    __shared__ float2 s_vl[WARPS][64];
-    __shared__ long long s_id[WARPS][64];
+    __shared__ float4 s_p[RW][RN];
+    __shared__ float4 s_v[RW][RN];
+    __shared__ float2 s_vl[RW][RN];
+    __shared__ long long s_id[RW][RN];
     // density passes: the same ring as a structure of arrays, so that
     // two consecutive entries load as one f32x2 operand
-    __shared__ __align__(16) float s_rx[WARPS][64], s_ry[WARPS][64], s_rz[WARPS][64], s_rm[WARPS][64];
-    __shared__ int s_j[WARPS][64];   // j index of each ring entry (list-building pass)
+    __shared__ __align__(16) float s_rx[RW][RN], s_ry[RW][RN], s_rz[RW][RN], s_rm[RW][RN];
+    __shared__ int s_j[RW][RN];   // j index of each ring entry (list-building pass)
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
     const unsigned lt = lanemask_lt();
-    const int n_items = a.n_items_dev ? *a.n_items_dev : a.n_items;
+    const int n_items = LONG ? *a.n_long : (a.n_items_dev ? *a.n_items_dev : a.n_items);
     const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
-    const int gw = blockIdx.x * WARPS + wid;
+    const int gw = LONG ? blockIdx.x : blockIdx.x * WARPS + wid;
+    // the ring (LONG: the compacted entries)
+    const float *bx = LONG ? l_x : s_rx[LONG ? 0 : wid], *by = LONG ? l_y : s_ry[LONG ? 0 : wid];
+    const float *bz = LONG ? l_z : s_rz[LONG ? 0 : wid], *bm = LONG ? l_m : s_rm[LONG ? 0 : wid];
+    const int *bj = LONG ? l_j : s_j[LONG ? 0 : wid];
+    int next = blockIdx.x;   // LONG
+    const int long_nj = a.pairs ? long_list(*a.pairs) : 0;
     // this lane's neighbour list: entry c at a.nbr[nlb + c * 32]
     const bool has_nl = a.nbr != nullptr && gw < a.nbr_warps;
     const int nlb = has_nl ? gw * a.nbr_cap * 32 + lane : 0;
@@ -126,20 +153,20 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
 
     for (;;) {
         int item = 0;
-        if (lane == 0) item = atomicAdd(a.queue, 1);
-        item = __shfl_sync(FULL, item, 0);
+        if (LONG) {
+            item = next;
+            next += gridDim.x;
+        } else {
+            if (lane == 0) item = atomicAdd(a.queue, 1);
+            item = __shfl_sync(FULL, item, 0);
+        }
         if (item >= n_items) return;
-        const ItemRef r = decode(a.items[item], a.j_off, a.i_list, lane);
+        const WorkItem wi = LONG ? a.long_items[item] : a.items[item];
+        const ItemRef r = decode(wi, a.j_off, a.i_list, lane);
         const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;
 
-        if (nj > STREAM_LONG) {
-            int p = 0;
-            if (lane == 0) {
-                a.long_items[atomicAdd(a.n_long, 1)] = a.items[item];
-                p = atomicAdd(a.n_left, r.ni);
-            }
-            p = __shfl_sync(FULL, p, 0);
-            if (r.act && sub == 0) a.left[p + r.li] = ii;
+        if (!LONG && a.long_items && nj > long_nj) {
+            if (lane == 0) a.long_items[atomicAdd(a.n_long, 1)] = wi;
             continue;
         }
         // i-particle relative to the centre particle c (velocity, id, mass
@@ -223,10 +250,10 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                 if (keep) {
                     const int slot = (head + fill + __popc(m & lt)) & 63;
                     if (!with_v) {
-                        s_rx[wid][slot] = p4.x;
-                        s_ry[wid][slot] = p4.y;
-                        s_rz[wid][slot] = p4.z;
-                        s_rm[wid][slot] = p4.w;
+                        s_rx[LONG ? 0 : wid][slot] = p4.x;
+                        s_ry[LONG ? 0 : wid][slot] = p4.y;
+                        s_rz[LONG ? 0 : wid][slot] = p4.z;
+                        s_rm[LONG ? 0 : wid][slot] = p4.w;
                     } else {
                         s_p[wid][slot] = p4;
                     }
@@ -249,6 +276,103 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
             if (fill > 0) consume(head, fill);
         };
 
+        // The LONG sweep: tile(head, n, out) sums the compacted entries
+        // [head, head + n) for this lane into out[0..NV); fold(t, head) adds the
+        // NV sums of tile t.  A run of tiles without any sum folds one zero
+        // (further zeros leave a compensated sum as it is).
+        auto sweep_long = [&](const float rf2, auto &&tile, auto &&fold) {
+            int fill = 0;
+            bool zero = false;
+            int jn[U];   // the next round's list entries
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = 32 * (U * wid + u) + lane;
+                jn[u] = (k < nj) ? jlist(k) : -1;
+            }
+            for (int t = 0; t < nj; t += ROUND) {
+                float4 p4[U], lo[U];
+                int jc[U];
+                unsigned m[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    jc[u] = jn[u];
+                    if (jc[u] >= 0) {
+                        p4[u] = a.fj.phi[jc[u]];
+                        lo[u] = a.fj.plo[jc[u]];
+                    }
+                    const int k = t + ROUND + 32 * (U * wid + u) + lane;
+                    jn[u] = (k < nj) ? jlist(k) : -1;
+                }
+                int mine = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    bool keep = false;
+                    if (jc[u] >= 0) {
+                        p4[u] = make_float4(df_diff(p4[u].x, lo[u].x, cph.x, cpl.x),
+                                            df_diff(p4[u].y, lo[u].y, cph.y, cpl.y),
+                                            df_diff(p4[u].z, lo[u].z, cph.z, cpl.z), p4[u].w);
+                        keep = !(box.d2(p4[u].x, p4[u].y, p4[u].z) > rf2);
+                    }
+                    m[u] = __ballot_sync(FULL, keep);
+                    mine += __popc(m[u]);
+                }
+                if (lane == 0) l_cnt[wid] = mine;
+                __syncthreads();   // counts; the last round's tiles are folded
+                int pos = fill, total = 0;
+                for (int w = 0; w < WARPS; ++w) {
+                    const int c = l_cnt[w];
+                    if (w < wid) pos += c;
+                    total += c;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (m[u] >> lane & 1u) {
+                        const int q = pos + __popc(m[u] & lt);
+                        l_x[q] = p4[u].x;
+                        l_y[q] = p4[u].y;
+                        l_z[q] = p4[u].z;
+                        l_m[q] = p4[u].w;
+                        l_j[q] = jc[u];
+                    }
+                    pos += __popc(m[u]);
+                }
+                fill += total;
+                kept += total;
+                __syncthreads();   // entries
+                const int nt = fill >> 5;
+                for (int q = wid; q < nt; q += WARPS) {
+                    const bool any = tile(32 * q, 32, q);
+                    if (lane == 0) l_any[q] = any ? 1u : 0u;
+                }
+                __syncthreads();   // tiles
+                for (int q = 0; q < nt; ++q) {
+                    const bool any = l_any[q] != 0u;
+                    if (any || !zero) fold(q, 32 * q);
+                    zero = !any;
+                }
+                // the entries left over move to the front (one warp)
+                if (wid == 0 && nt > 0) {
+                    const int q = 32 * nt + lane;
+                    const bool mv = q < fill;
+                    const float x = mv ? l_x[q] : 0.0f, y = mv ? l_y[q] : 0.0f, z = mv ? l_z[q] : 0.0f;
+                    const float w = mv ? l_m[q] : 0.0f;
+                    const int j = mv ? l_j[q] : 0;
+                    __syncwarp();
+                    if (mv) {
+                        l_x[lane] = x; l_y[lane] = y; l_z[lane] = z; l_m[lane] = w; l_j[lane] = j;
+                    }
+                }
+                fill &= 31;
+            }
+            __syncthreads();   // the last round's folds and move
+            if (fill > 0) {
+                if (wid == 0) tile(0, fill, 0);
+                __syncthreads();
+                fold(0, 0);
+                __syncthreads();
+            }
+        };
+
         // neighbour list of this lane: its length (above nbr_cap the list is
         // unusable), appended by the first pass from the ring
         int ncnt = 0;
@@ -259,7 +383,7 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
             while (msk) {
                 const int k = __ffs(msk) - 1;
                 msk &= msk - 1;
-                if (ncnt < a.nbr_cap) a.nbr[nlb + ncnt * 32] = s_j[wid][head + k];
+                if (ncnt < a.nbr_cap && (!LONG || wid == 0)) a.nbr[nlb + ncnt * 32] = bj[head + k];
                 ++ncnt;
             }
         };
@@ -287,7 +411,7 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
             // ring entry k; with mark set, bit k of *mark flags an entry
             // within the list radius
             auto pair = [&](int k, bool count, unsigned *mark) {
-                const float4 pj = make_float4(s_rx[wid][k], s_ry[wid][k], s_rz[wid][k], s_rm[wid][k]);
+                const float4 pj = make_float4(bx[k], by[k], bz[k], bm[k]);
                 part += term(pj, count);
                 if (mark) {
                     const float dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
@@ -309,9 +433,9 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                 unsigned msk = 0;
 #pragma unroll DENSITY_UNROLL
                 for (int k = 0; k < 32; k += 2) {
-                    const f2 DX = f2_fma(f2_lds(&s_rx[wid][head + k]), NEG, XI);
-                    const f2 DY = f2_fma(f2_lds(&s_ry[wid][head + k]), NEG, YI);
-                    const f2 DZ = f2_fma(f2_lds(&s_rz[wid][head + k]), NEG, ZI);
+                    const f2 DX = f2_fma(f2_lds(&bx[head + k]), NEG, XI);
+                    const f2 DY = f2_fma(f2_lds(&by[head + k]), NEG, YI);
+                    const f2 DZ = f2_fma(f2_lds(&bz[head + k]), NEG, ZI);
                     const float2 x2 = f2_get(f2_mul(f2_fma(DZ, DZ, f2_fma(DY, DY, f2_mul(DX, DX))), H2));
                     if constexpr (B) msk |= (x2.x < lim ? 1u << k : 0u) | (x2.y < lim ? 2u << k : 0u);
                     float q0, q1;
@@ -321,27 +445,32 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                     const float2 u = f2_get(f2_fma(Q, NEG, ONE));
                     const f2 U = f2_make(max0(u.x), max0(u.y));
                     const f2 U2 = f2_mul(U, U);
-                    PART = f2_fma(f2_lds(&s_rm[wid][head + k]), f2_mul(f2_mul(U2, U2), f2_fma(Q, FOUR, ONE)), PART);
+                    PART = f2_fma(f2_lds(&bm[head + k]), f2_mul(f2_mul(U2, U2), f2_fma(Q, FOUR, ONE)), PART);
                     if (count) c2 += (q0 < 1.0f ? 1 : 0) + (q1 < 1.0f ? 1 : 0);
                 }
                 const float2 ps = f2_get(PART);
                 part = (float)(ps.x + ps.y);
                 cnt += c2;
-                if constexpr (B) nl_push(head, msk);
+                return msk;
             };
-            auto run = [&](int head, int n) {
+            // sum of one tile in part, and its marks
+            auto tile = [&](int head, int n) -> unsigned {
                 part = 0;
+                unsigned msk = 0;
                 if (tpi == 1 && n == 32) {
                     if (build)
-                        run_packed(head, false, BTag<true>());
+                        msk = run_packed(head, false, BTag<true>());
                     else
                         run_packed(head, pass == 2, BTag<false>());
                 } else {
-                    unsigned msk = 0;
                     unsigned *mark = build ? &msk : nullptr;
                     for (int k = sub; k < n; k += tpi) pair(head + k, pass == 2, mark);
-                    if (build) nl_push(head, msk);
                 }
+                return msk;
+            };
+            auto run = [&](int head, int n) {
+                const unsigned msk = tile(head, n);
+                if (build) nl_push(head, msk);
                 acc.add(part);
                 __syncwarp();
             };
@@ -366,8 +495,34 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                 ++n_listed;
             } else {
                 const float rf2 = support2<float>(build ? h * (double)a.nbr_slack : h);
-                sweep(rf2, false, build, run);
+                if constexpr (LONG) {
+                    sweep_long(rf2,
+                               [&](int head, int n, int q) {
+                                   const unsigned msk = tile(head, n);
+                                   l_part[q][0][lane] = part;
+                                   if (build) l_part[q][1][lane] = __uint_as_float(msk);
+                                   return __any_sync(FULL, part != 0.0f || msk != 0u);
+                               },
+                               [&](int q, int head) {
+                                   if (build) nl_push(head, __float_as_uint(l_part[q][1][lane]));
+                                   acc.add(l_part[q][0][lane]);
+                               });
+                    // the warps' counts
+                    __syncthreads();
+                    if (pass == 2) {
+                        int *sum = reinterpret_cast<int *>(&l_part[0][0][0]);
+                        if (wid == 0) sum[lane] = 0;
+                        __syncthreads();
+                        atomicAdd(&sum[lane], cnt);
+                        __syncthreads();
+                        cnt = sum[lane];
+                        __syncthreads();
+                    }
+                } else {
+                    sweep(rf2, false, build, run);
+                }
             }
+            if (LONG && build) __syncthreads();   // the lists
             if (build) nl_ok = __all_sync(FULL, ncnt <= a.nbr_cap);
             const double sum = seg_sum(acc.value(), tpi);
             const int c = (int)seg_sum((long long)cnt, tpi);
@@ -385,7 +540,7 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
         // the search-radius decision of the last pass (hdr_density.hpp:299)
         const double rs_i = a.i_rs[ii];
         const bool itr = h > rs_i;
-        if (a.amb_count && r.act && sub == 0 && fabs(h - rs_i) <= (double)a.amb_tol * rs_i) {
+        if (a.amb_count && (!LONG || wid == 0) && r.act && sub == 0 && fabs(h - rs_i) <= (double)a.amb_tol * rs_i) {
             const int k = atomicAdd(a.amb_count, 1);
             if (k < a.amb_cap) a.amb[k] = make_int2(ii, r.walk);
         }
@@ -427,9 +582,16 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                 prz += (ux * dy - uy * dx) * dw;
             };
             auto pair = [&](int k) {
-                const float4 vj = s_v[wid][k];
-                const float2 vl = s_vl[wid][k];
-                gpair(s_p[wid][k], vj.x, vj.y, vj.z, (float)vj.w, vl.x, vl.y, s_id[wid][k]);
+                if constexpr (LONG) {
+                    const int j = bj[k];
+                    const float4 vh = __ldg(&a.fj.vhi[j]), vl = __ldg(&a.fj.vlo[j]);
+                    gpair(make_float4(bx[k], by[k], bz[k], bm[k]), vh.x, vh.y, vh.z, vl.x, vl.y, vl.z,
+                          __ldg(&a.j_id[j]));
+                } else {
+                    const float4 vj = s_v[wid][k];
+                    const float2 vl = s_vl[wid][k];
+                    gpair(s_p[wid][k], vj.x, vj.y, vj.z, (float)vj.w, vl.x, vl.y, s_id[wid][k]);
+                }
             };
             auto fold = [&]() {
                 g_acc.add(pg);
@@ -445,12 +607,13 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
             // tile order; the unmarked pairs contribute exactly zero.
             const float lim = hinv * hinv * (float)1.00002;
             auto mark = [&](int k, unsigned &msk) {
-                const float4 pj = s_p[wid][k];
+                const float4 pj = LONG ? make_float4(bx[k], by[k], bz[k], bm[k]) : s_p[LONG ? 0 : wid][LONG ? 0 : k];
                 const float dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
                 const float r2 = dx * dx + dy * dy + dz * dz;
                 if (!(r2 * lim >= (float)1)) msk |= 1u << (k & 31);
             };
-            auto run = [&](int head, int n) {
+            // sums of one tile in pg .. prz
+            auto tile = [&](int head, int n) {
                 unsigned msk = 0;
                 if (tpi == 1 && n == 32) {
 #pragma unroll 8
@@ -463,6 +626,9 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                     msk &= msk - 1;
                     pair(head + k);
                 }
+            };
+            auto run = [&](int head, int n) {
+                tile(head, n);
                 fold();
                 __syncwarp();
             };
@@ -495,14 +661,38 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
                 if (r.act) ev_list_g += (unsigned)ncnt;
                 ++n_listed;
             } else {
-                sweep(support2<float>(h), true, false, run);
+                if constexpr (LONG) {
+                    sweep_long(support2<float>(h),
+                               [&](int head, int n, int q) {
+                                   tile(head, n);
+                                   l_part[q][0][lane] = pg;
+                                   l_part[q][1][lane] = pd;
+                                   l_part[q][2][lane] = prx;
+                                   l_part[q][3][lane] = pry;
+                                   l_part[q][4][lane] = prz;
+                                   const bool any = pg != 0.0f || pd != 0.0f || prx != 0.0f || pry != 0.0f || prz != 0.0f;
+                                   pg = 0; pd = 0; prx = 0; pry = 0; prz = 0;
+                                   return __any_sync(FULL, any);
+                               },
+                               [&](int q, int head) {
+                                   (void)head;
+                                   pg = l_part[q][0][lane];
+                                   pd = l_part[q][1][lane];
+                                   prx = l_part[q][2][lane];
+                                   pry = l_part[q][3][lane];
+                                   prz = l_part[q][4][lane];
+                                   fold();
+                               });
+                } else {
+                    sweep(support2<float>(h), true, false, run);
+                }
             }
             const double sg = seg_sum(g_acc.value(), tpi);
             const double sd = seg_sum(d_acc.value(), tpi);
             const double sx = seg_sum(rx_acc.value(), tpi);
             const double sy = seg_sum(ry_acc.value(), tpi);
             const double sz = seg_sum(rz_acc.value(), tpi);
-            if (r.act && sub == 0) {
+            if (r.act && sub == 0 && (!LONG || wid == 0)) {
                 const float hf = (float)h;
                 const float hinv_f = 1.0f / hf;
                 const float hinv4 = hinv_f * hinv_f * hinv_f * hinv_f;
@@ -527,12 +717,12 @@ __global__ void __launch_bounds__(WARPS * 32, SPH_DENSITY_MIN_BLOCKS) density_st
         if (a.n_eval) {
             const unsigned long long l0 = __reduce_add_sync(FULL, ev_list);
             const unsigned long long l1 = __reduce_add_sync(FULL, ev_list_g);
-            if (lane == 0) {
+            if (lane == 0 && (!LONG || wid == 0)) {
                 atomicAdd(a.n_eval, (unsigned long long)kept_rho * (unsigned long long)r.ni + l0);
                 atomicAdd(a.n_eval + 1, (unsigned long long)(kept - kept_rho) * (unsigned long long)r.ni + l1);
             }
         }
-        if (a.n_pass && lane == 0) {
+        if (a.n_pass && lane == 0 && (!LONG || wid == 0)) {
             atomicAdd(a.n_pass, (unsigned long long)n_listed);
             atomicAdd(a.n_pass + 1, (unsigned long long)(3 - n_listed));
         }

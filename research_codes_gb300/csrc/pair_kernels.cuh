@@ -34,25 +34,18 @@
 #define SPH_GRAVITY_MIN_BLOCKS 4
 #endif
 // Unroll factors of the full-tile FP32C loops: f32x2 iterations (two entries
-// each) of the gravity loop, entries of the hydro mark-only loop.
+// each) of the gravity loop.
 #ifndef SPH_GRAVITY_UNROLL
 #define SPH_GRAVITY_UNROLL 16
-#endif
-#ifndef SPH_HYDRO_MARK_UNROLL
-#define SPH_HYDRO_MARK_UNROLL 16
 #endif
 // The double-float hydro pass (128 threads): 3 blocks per SM, 168 registers.
 #ifndef SPH_HYDRO_DF_MIN_BLOCKS
 #define SPH_HYDRO_DF_MIN_BLOCKS 3
 #endif
-#ifndef SPH_HYDRO_MIN_BLOCKS
-#define SPH_HYDRO_MIN_BLOCKS 4
-#endif
 
 namespace sphk {
 
 constexpr int GRAVITY_UNROLL = SPH_GRAVITY_UNROLL;
-constexpr int HYDRO_MARK_UNROLL = SPH_HYDRO_MARK_UNROLL;
 
 // ---------------------------------------------------------------- hydro
 struct HydroArgs {
@@ -74,552 +67,145 @@ struct HydroArgs {
     const float4 *fi_g1, *fi_g2, *fi_g3, *fj_g1, *fj_g2, *fj_g3;
     const long long *i_id;
     const long long *j_id;
-    const WorkItem *items;
-    int n_items;
-    const int *n_items_dev;
     const int *j_off;
     const int *j_idx;
-    const int *i_list;
-    int *queue;
-    // outputs
+    // outputs (the signal velocity is mark_rows')
     double *o_acch;      // 3 per particle
     double *o_accg;      // 3 per particle
-    double *o_udot, *o_vsmx, *o_diffu;
-    // when set: pair evaluations performed in full (near) and for the
-    // signal velocity only (far), j-entries x i-particles
-    unsigned long long *n_eval_near, *n_eval_far;
-    // when set: per walk, the largest sound speed of its j-list (the signal
-    // velocity of every i-particle of the walk is at least its own sound
-    // speed plus this), which lets tiles that cannot raise the maximum skip
-    // their signal-velocity terms
-    const double *walk_csmax = nullptr;
-    int sv_skip = 0;   // nonzero: tiles test the bound and skip (0: every term evaluated)
-    // when set: [0] 32-entry tiles whose signal-velocity terms were skipped,
-    // [1] tiles evaluated
-    unsigned long long *n_skip = nullptr;
-    // when set: [0] marked pairs (inside either support, evaluated in
-    // full), [1] lane slots their loops occupied (per 32-entry tile, 32 x
-    // the largest per-lane count)
-    unsigned long long *n_mark = nullptr;
-    // FP32C: the kernel evaluates the signal velocities and writes, per
-    // i-particle, the j indices of its marked pairs (self pairs excluded) to
-    // row i of df_list (df_cap entries) and their number to df_cnt[i]; a
-    // particle with more than df_cap appends (i, walk) to df_ovf and counts
-    // it in *df_novf.  The double-float pass (hydro_df_lists /
-    // hydro_df_sweep) then forms acch, accg, udot and diffu.  g4 records:
-    // (1/h hi, 1/h lo, h^-4 hi, h^-4 lo).
+    double *o_udot, *o_diffu;
+    // rows (mark_rows): the pairs inside either support, self pairs excluded;
+    // particles without a row in the sweep queue.  g4 records: (1/h hi, 1/h lo,
+    // h^-4 hi, h^-4 lo).
     const float4 *fi_g4 = nullptr, *fj_g4 = nullptr;
-    int *df_list = nullptr;
-    int df_cap = 0;
-    int *df_cnt = nullptr;
-    int2 *df_ovf = nullptr;
-    int *df_novf = nullptr;
-    int n_i = 0;   // i-particles (the double-float pass covers [0, n_i))
+    const int *rows = nullptr;
+    const int2 *info = nullptr;
+    const int2 *ovf = nullptr;
+    const int *n_ovf = nullptr;
+    int n_i = 0;   // i-particles (the sums cover [0, n_i))
+    // FP64: double-float positions with h in hi.w, for the sweep's distance test
+    const float4 *mi_p = nullptr, *mi_l = nullptr, *mj_p = nullptr, *mj_l = nullptr;
 };
 
-// Capacity of a particle's row of marked pairs in the FP32C hydro lists
-// (~50-60 marked pairs are typical; a particle whose row overflows is summed
-// over its walk's whole list instead).
-constexpr int HYDRO_LIST_CAP = 128;
-static_assert(HYDRO_LIST_CAP % 4 == 0, "rows of marked pairs start 16-byte aligned");
+// ---- FP64 hydro sums over the rows, hdr_hydro.hpp:349-398 ----
+struct Hydro64P {   // one particle's fields
+    dbl4 p, v, h1, h2;
+    double2 h3;
+    double hinv4;
+};
+__device__ __forceinline__ Hydro64P hydro64_load(const dbl4 *pm, const dbl4 *vel, const dbl4 *h1, const dbl4 *h2,
+                                                 const double2 *h3, int k) {
+    Hydro64P q;
+    q.p = pm[k]; q.v = vel[k]; q.h1 = h1[k]; q.h2 = h2[k]; q.h3 = h3[k];
+    q.hinv4 = q.h1.x * q.h1.x * q.h1.x * q.h1.x;
+    return q;
+}
+struct Hydro64Acc {
+    double ax = 0, ay = 0, az = 0, gx = 0, gy = 0, gz = 0, ud = 0, df = 0;
+};
+__device__ __forceinline__ void hydro64_pair(const Hydro64P &i, const Hydro64P &j, Hydro64Acc &s) {
+    const double dx = i.p.x - j.p.x, dy = i.p.y - j.p.y, dz = i.p.z - j.p.z;
+    const double ux = i.v.x - j.v.x, uy = i.v.y - j.v.y, uz = i.v.z - j.v.z;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double ri = rsqrt_r(r2);
+    const double rr = r2 * ri;
+    // kernel gradients W1(q) for both smoothing lengths
+    const double qi = rr * i.h1.x, qj = rr * j.h1.x;
+    if (qi >= 1.0 && qj >= 1.0) return;   // beyond both supports: every term is zero
+    const double ui = max0(1.0 - qi), uj = max0(1.0 - qj);
+    const double ui2 = ui * ui, uj2 = uj * uj;
+    const double w1i = w1_term(qi, ui, ui2, ui2 * ui, 1.0 + 4.0 * qi);
+    const double w1j = w1_term(qj, uj, uj2, uj2 * uj, 1.0 + 4.0 * qj);
+    const double dw_i = CEFF1 * i.hinv4 * w1i;
+    const double dw_j = CEFF1 * j.hinv4 * w1j;
+    const double mj = j.p.w;
+    const double ka = (dw_i + dw_j) * mj;
+    // viscosity, :368-376
+    const double w = (dx * ux + dy * uy + dz * uz) * ri;
+    const double wneg = w < 0.0 ? w : 0.0;
+    const double vs = i.h2.y + j.h2.y - 3.0 * wneg;
+    const double rhi = rcp_r(i.h2.x + j.h2.x);
+    const double av = (i.h1.w + j.h1.w) * (i.h2.z + j.h2.z) * vs * wneg;
+    // pressure gradient, :378-382
+    const double ta = (i.h1.z + j.h1.z - 0.5 * av * rhi) * ka * ri;
+    s.ax -= ta * dx;
+    s.ay -= ta * dy;
+    s.az -= ta * dz;
+    // energy equation with conduction, :384-393
+    const double du = i.h3.x - j.h3.x;
+    const double alphu = i.h2.w + j.h2.w;
+    double cond = 0.0;
+    if (alphu != 0.0) {
+        const double vsu2 = fabs(i.h1.y - j.h1.y) * rhi * 2.0;
+        cond = alphu * (vsu2 > 0.0 ? vsu2 * rsqrt_r(vsu2) : 0.0) * du;
+    }
+    s.ud += ka * (i.h1.z * w - rhi * (0.25 * av * wneg - cond));
+    s.df += rhi * du * ka * ri;
+    // softening correction, :395-398
+    const double dg = mj * ri * (i.h3.y * dw_i + j.h3.y * dw_j);
+    s.gx += dg * dx;
+    s.gy += dg * dy;
+    s.gz += dg * dz;
+}
+__device__ __forceinline__ void hydro64_store(const HydroArgs &a, int p, const double (&v)[8]) {
+    for (int c = 0; c < 3; ++c) {
+        a.o_acch[3 * p + c] = 0.5 * v[c];
+        a.o_accg[3 * p + c] = 0.5 * v[3 + c];
+    }
+    a.o_udot[p] = 0.5 * v[6];
+    a.o_diffu[p] = 2.0 * v[7];
+}
 
-template <bool F64, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, F64 ? 1 : SPH_HYDRO_MIN_BLOCKS)
-hydro_kernel(const HydroArgs a) {
-    typedef typename Real<F64>::T R;
-    typedef typename Real<F64>::T4 R4;
-    // Two 64-entry rings of compacted j records per warp.  Near ring: the
-    // j-particles that can lie within the kernel support of some i-particle
-    // of the item (r < max(h_i, h_j)), with every field of the pair formula.
-    // Far ring: the others, whose pair terms all vanish except the
-    // signal-velocity maximum (hdr_hydro.hpp:372 takes it over every j of
-    // the list), kept as position + sound speed and velocity only.
-    // Near-ring layout (FP32C; FP64 keeps the lo parts at zero):
-    __shared__ R4 s_p1[WARPS][64];    // dx, dy, dz (exact hi parts, item frame), hinv
-    __shared__ R4 s_p2[WARPS][64];    // position lo parts, vsnd
-    __shared__ R4 s_v1[WARPS][64];    // velocity hi, mass
-    __shared__ R4 s_v2[WARPS][64];    // velocity lo, hinv^4
-    // pair-formula fields (FP64 mode only: FP32C forms the pair sums in a
-    // separate double-float pass)
-    __shared__ R4 s_c[F64 ? WARPS : 1][64];     // P (hi), presc, bswt, dens
-    __shared__ R4 s_d[F64 ? WARPS : 1][64];     // alph, alphu, u (hi), eta
-    __shared__ float2 s_f[F64 ? WARPS : 1][64]; // P lo, u lo
-    __shared__ long long s_id[WARPS][64];
-    __shared__ R4 s_fp[WARPS][64];    // far: centred position, vsnd
-    __shared__ R4 s_fv[WARPS][64];    // far: velocity (hi), signal-velocity bound b_j
-    __shared__ R s_nb[WARPS][64];     // near: signal-velocity bound b_j
-    // FP32C near entries for the mark test: position in the item frame as one
-    // float (as the support test has it) and h_j^2 widened by 2e-4; and the
-    // entry's j index (written to the marked-pair lists)
-    __shared__ float4 s_m[F64 ? 1 : WARPS][64];
-    __shared__ int s_jx[F64 ? 1 : WARPS][64];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    const unsigned lt = lanemask_lt();
-    const int n_items = a.n_items_dev ? *a.n_items_dev : a.n_items;
-
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(a.queue, 1);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= n_items) return;
-        const ItemRef r = decode(a.items[item], a.j_off, a.i_list, lane);
-        const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;
-
-        R xi, yi, zi, vxi, vyi, vzi, hi_i, hi4_i, pp_i, pc_i, bs_i, dn_i, cs_i, al_i, au_i, eg_i, et_i;
-        float lxi = 0.0f, lyi = 0.0f, lzi = 0.0f, plo_i = 0.0f, elo_i = 0.0f;
-        float xlo = 0.0f, ylo = 0.0f, zlo = 0.0f;
-        float4 cph = make_float4(0, 0, 0, 0), cpl = cph;
-        if (F64) {
-            const dbl4 p = a.i_pm[ii], v = a.i_vel[ii], h1 = a.i_h1[ii], h2 = a.i_h2[ii];
-            const double2 h3 = a.i_h3[ii];
-            xi = p.x; yi = p.y; zi = p.z; vxi = v.x; vyi = v.y; vzi = v.z;
-            hi_i = h1.x; hi4_i = h1.x * h1.x * h1.x * h1.x; pp_i = h1.y; pc_i = h1.z; bs_i = h1.w;
-            dn_i = h2.x; cs_i = h2.y; al_i = h2.z; au_i = h2.w; eg_i = h3.x; et_i = h3.y;
-        } else {
-            cph = a.fi.phi[r.ic]; cpl = a.fi.plo[r.ic];
-            const float4 ph = a.fi.phi[ii], pl = a.fi.plo[ii], vh = a.fi.vhi[ii], vl = a.fi.vlo[ii];
-            const float4 g1 = a.fi_g1[ii], g2 = a.fi_g2[ii], g3 = a.fi_g3[ii];
-            xi = ph.x - cph.x; yi = ph.y - cph.y; zi = ph.z - cph.z;   // exact hi parts
-            xlo = pl.x - cpl.x; ylo = pl.y - cpl.y; zlo = pl.z - cpl.z;
-            vxi = vh.x; vyi = vh.y; vzi = vh.z;       // absolute hi/lo, differenced per pair
-            lxi = vl.x; lyi = vl.y; lzi = vl.z;
-            hi_i = vh.w; hi4_i = vl.w;
-            pp_i = g1.x; plo_i = g1.y; pc_i = g1.z; bs_i = g1.w;   // P and u as hi/lo,
-            dn_i = g2.x; cs_i = g2.y; al_i = g2.z; au_i = g2.w;    // differenced per pair
-            eg_i = g3.x; elo_i = g3.y; et_i = g3.z;
+// Eight lanes per particle over its row; particles without one are left to
+// the sweep.  FP64 pipe bound (~120 instructions per pair).
+constexpr int HROWS_LANES = 8, HROWS_THREADS = 128;
+__global__ inline void __launch_bounds__(HROWS_THREADS) hydro64_rows(const HydroArgs a) {
+    constexpr int L = HROWS_LANES;
+    const int lane = threadIdx.x & 31, sub = lane & (L - 1);
+    const int gw = (blockIdx.x * HROWS_THREADS + threadIdx.x) >> 5, nw = (gridDim.x * HROWS_THREADS) >> 5;
+    for (int k0 = gw * (32 / L); k0 < a.n_i; k0 += nw * (32 / L)) {
+        const int p = k0 + lane / L;
+        const int cnt = p < a.n_i ? a.info[p].x : ROW_CAP + 1;
+        const bool ok = cnt <= ROW_CAP;
+        Hydro64Acc s;
+        if (ok) {
+            const Hydro64P I = hydro64_load(a.i_pm, a.i_vel, a.i_h1, a.i_h2, a.i_h3, p);
+            const int *row = a.rows + (size_t)p * ROW_CAP;
+            for (int e = sub; e < cnt; e += L)
+                hydro64_pair(I, hydro64_load(a.j_pm, a.j_vel, a.j_h1, a.j_h2, a.j_h3, row[e]), s);
         }
-        const long long idi = a.i_id[ii];
-        // Signal-velocity bounds.  With v_c the velocity of the item's centre
-        // particle, |v_i - v_j| <= d_i + d_j (d = |v - v_c|, FP32C with the
-        // hi and lo differences added per component) and |w| <= |v_i - v_j|,
-        // so every pair term cs_i + cs_j - 3 min(w, 0) of a tile is at most
-        // cs_i + 3 d_i + max_j b_j with b_j = cs_j + 3 d_j.  The maximum over
-        // the list starts at cs_i + (largest cs_j of the walk), which no pair
-        // term undercuts; a tile whose bound (with a 1e-5 relative margin over
-        // the rounding of both) stays below every lane's running maximum adds
-        // nothing to it and skips those terms: the maximum is unchanged bit
-        // for bit.  The margin also covers the approximate square root of d.
-        // Entries beyond both supports are tested as each 32-entry chunk of
-        // the list arrives, against the running maximum at that point (which
-        // only grows), and are staged in the far ring only when the test
-        // fails.
-        R vcx, vcy, vcz;
-        float lcx = 0.0f, lcy = 0.0f, lcz = 0.0f;
-        if (F64) {
-            const dbl4 v = a.i_vel[r.ic];
-            vcx = v.x; vcy = v.y; vcz = v.z;
-        } else {
-            const float4 vh = a.fi.vhi[r.ic], vl = a.fi.vlo[r.ic];
-            vcx = vh.x; vcy = vh.y; vcz = vh.z;
-            lcx = vl.x; lcy = vl.y; lcz = vl.z;
-        }
-        auto dvel = [&](R hx, R hy, R hz, float lx, float ly, float lz) -> R {
-            const R ex = fabs(hx - vcx) + (R)fabsf(lx - lcx);
-            const R ey = fabs(hy - vcy) + (R)fabsf(ly - lcy);
-            const R ez = fabs(hz - vcz) + (R)fabsf(lz - lcz);
-            return sqrt_bound(ex * ex + ey * ey + ez * ez);
-        };
-        auto sv_bound = [&](R cs, R d) -> R {
-            const R b = cs + (R)3 * d;
-            return (b < (R)0) ? (R)0 : b;   // NaN stays NaN (no skip)
-        };
-        const R ub_i = cs_i + (R)3 * dvel(vxi, vyi, vzi, lxi, lyi, lzi);
-        // i position in the item frame as one number (box and far pairs)
-        const R xc = xi + (R)xlo, yc = yi + (R)ylo, zc = zi + (R)zlo;
-        IBox<R> box;
-        box.from_lanes(xc, yc, zc);
-        const R hm2 = support2<R>(1.0 / (double)hi_i);
-        const R hi2_i = hi_i * hi_i;
-        const R h2m_i = rcp_r(hi2_i) * (R)1.0002;   // h_i^2 widened as the support test's
-
-        Acc<F64> ax, ay, az, ud, df, gx, gy, gz;
-        R vsmx = 0;
-        if (a.walk_csmax) {
-            const R v0 = cs_i + (R)a.walk_csmax[r.walk];
-            vsmx = (v0 > (R)0) ? v0 : (R)0;
-        }
-        unsigned n_skipped = 0, n_tiles = 0, n_marked = 0, n_slots = 0;
-        // true when no pair term with any lane's bound b can exceed any
-        // lane's running maximum
-        auto below = [&](R b) -> bool {
-            R t;
-            if constexpr (F64) {
-                t = b;
+        double v[8] = {s.ax, s.ay, s.az, s.gx, s.gy, s.gz, s.ud, s.df};
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const R u = __shfl_xor_sync(FULL, t, o);
-                    t = (u > t || u != u) ? u : t;
-                }
-            } else {
-                // non-negative floats (or NaN) order like their bit patterns
-                t = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(b)));
-            }
-            const bool ok = (ub_i + t) * (R)1.00001 <= vsmx;
-            const bool all = __all_sync(FULL, ok);
-            ++n_tiles;
-            if (all) ++n_skipped;
-            return all;
-        };
-        // the same for the n-entry ring tile at bound[]
-        auto skip_tile = [&](const R *bound, int stride, int n) -> bool {
-            if (!a.sv_skip) return false;
-            return below((lane < n) ? bound[lane * stride] : (R)0);
-        };
-        int nhead = 0, nfill = 0, fhead = 0, ffill = 0;
-        int lcount = 0;   // FP32C: marked pairs of this lane's particle so far
-        long long kept_n = 0, kept_f = 0;
-        R pax = 0, pay = 0, paz = 0, pud = 0, pdf = 0, pgx = 0, pgy = 0, pgz = 0;
-        // pair separation and velocity difference of near entry k
-        auto diffs = [&](int k, R &dx, R &dy, R &dz, R &ux, R &uy, R &uz, R &r2, R &ri) {
-            const R4 P1 = s_p1[wid][k];
-            const R4 V1 = s_v1[wid][k];
-            dx = xi - P1.x; dy = yi - P1.y; dz = zi - P1.z;
-            ux = vxi - V1.x; uy = vyi - V1.y; uz = vzi - V1.z;
-            if (!F64) {
-                const R4 P2 = s_p2[wid][k];
-                const R4 V2 = s_v2[wid][k];
-                dx += (R)(xlo - (float)P2.x);
-                dy += (R)(ylo - (float)P2.y);
-                dz += (R)(zlo - (float)P2.z);
-                ux += (R)(lxi - (float)V2.x);
-                uy += (R)(lyi - (float)V2.y);
-                uz += (R)(lzi - (float)V2.z);
-            }
-            r2 = dx * dx + dy * dy + dz * dz;
-            ri = (idi != s_id[wid][k]) ? rsqrt_r(r2) : (R)0;
-        };
-        // Every near entry: the signal velocity (hdr_hydro.hpp:368-372) and
-        // a mark when the pair is inside either support (FP64: r^2
-        // min(1/h_i^2, 1/h_j^2) below 1 + 2e-5, so every pair with q_i < 1 or
-        // q_j < 1 is marked; FP32C: the test of mark_only below, so that a
-        // particle's row holds the same pairs whether or not its tiles skip
-        // their signal-velocity terms).  Unmarked pairs add exactly zero to
-        // every sum.
-        auto signal = [&](int k, unsigned &msk) {
-            R dx, dy, dz, ux, uy, uz, r2, ri;
-            diffs(k, dx, dy, dz, ux, uy, uz, r2, ri);
-            const R w = (dx * ux + dy * uy + dz * uz) * ri;
-            const R wneg = w < (R)0 ? w : (R)0;
-            const R vs = cs_i + s_p2[wid][k].w - (R)3 * wneg;
-            vsmx = vs > vsmx ? vs : vsmx;
-            if constexpr (F64) {
-                const R hj = s_p1[wid][k].w;
-                const R hmin2 = hi2_i < hj * hj ? hi2_i : hj * hj;
-                if (!(r2 * hmin2 >= (R)1.00002)) msk |= 1u << (k & 31);
-            } else {
-                const float4 M = s_m[wid][k];
-                const float ex = xc - M.x, ey = yc - M.y, ez = zc - M.z;
-                const float lim = h2m_i > M.w ? h2m_i : M.w;
-                if (!(ex * ex + ey * ey + ez * ez >= lim)) msk |= 1u << (k & 31);
-            }
-        };
-        // the mark alone (tiles whose signal-velocity terms are skipped).
-        // FP32C tests r^2 < max(h_i, h_j)^2 (1 + 2e-4) on the one-float item
-        // frame positions of the support test (whose rounding the 2e-4 margin
-        // covers), which marks every pair the exact test marks and a few
-        // beyond both supports; those add exactly zero (W1 = 0 there).
-        auto mark_only = [&](int k, unsigned &msk) {
-            if constexpr (!F64) {
-                const float4 M = s_m[wid][k];
-                const float dx = xc - M.x, dy = yc - M.y, dz = zc - M.z;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                const float lim = h2m_i > M.w ? h2m_i : M.w;
-                if (!(r2 >= lim)) msk |= 1u << (k & 31);
-                return;
-            }
-            const R4 P1 = s_p1[wid][k];
-            R dx = xi - P1.x, dy = yi - P1.y, dz = zi - P1.z;
-            if (!F64) {
-                const R4 P2 = s_p2[wid][k];
-                dx += (R)(xlo - (float)P2.x);
-                dy += (R)(ylo - (float)P2.y);
-                dz += (R)(zlo - (float)P2.z);
-            }
-            const R r2 = dx * dx + dy * dy + dz * dz;
-            const R hj = P1.w;
-            const R hmin2 = hi2_i < hj * hj ? hi2_i : hj * hj;
-            if (!(r2 * hmin2 >= (R)1.00002)) msk |= 1u << (k & 31);
-        };
-        // The remaining terms of a marked pair, hdr_hydro.hpp:349-398
-        auto pair = [&](int k) {
-            R dx, dy, dz, ux, uy, uz, r2, ri;
-            diffs(k, dx, dy, dz, ux, uy, uz, r2, ri);
-            const R4 P1 = s_p1[wid][k];
-            const R4 V1 = s_v1[wid][k];
-            const R4 C = s_c[wid][k];
-            const R4 D = s_d[wid][k];
-            const R hinv4_j = s_v2[wid][k].w;
-            const R cs_j = s_p2[wid][k].w;
-            R dp = pp_i - C.x, du = eg_i - D.z;
-            if (!F64) {
-                const float2 F = s_f[wid][k];
-                dp += (R)(plo_i - F.x);
-                du += (R)(elo_i - F.y);
-            }
-            const R rr = r2 * ri;
-            // kernel gradients W1(q) for both smoothing lengths
-            const R qi = rr * hi_i, qj = rr * P1.w;
-            const R ui = max0((R)1 - qi), uj = max0((R)1 - qj);
-            const R ui2 = ui * ui, uj2 = uj * uj;
-            const R w1i = w1_term(qi, ui, ui2, ui2 * ui, (R)1 + (R)4 * qi);
-            const R w1j = w1_term(qj, uj, uj2, uj2 * uj, (R)1 + (R)4 * qj);
-            const R dw_i = (R)CEFF1 * hi4_i * w1i;
-            const R dw_j = (R)CEFF1 * hinv4_j * w1j;
-            const R ka = (dw_i + dw_j) * V1.w;
-            // viscosity, hdr_hydro.hpp:368-376
-            const R w = (dx * ux + dy * uy + dz * uz) * ri;
-            const R wneg = w < (R)0 ? w : (R)0;
-            const R vs = cs_i + cs_j - (R)3 * wneg;
-            const R rhi = rcp_r(dn_i + C.w);
-            const R av = (bs_i + C.z) * (al_i + D.x) * vs * wneg;
-            // pressure gradient, :378-382
-            const R ta = (pc_i + C.y - (R)0.5 * av * rhi) * ka * ri;
-            pax -= ta * dx;
-            pay -= ta * dy;
-            paz -= ta * dz;
-            // energy equation with conduction, :384-393
-            const R vsu2 = fabs(dp) * rhi * (R)2;
-            const R vsu = vsu2 > (R)0 ? vsu2 * rsqrt_r(vsu2) : (R)0;
-            pud += ka * (pc_i * w - rhi * ((R)0.25 * av * wneg - (au_i + D.y) * vsu * du));
-            pdf += rhi * du * ka * ri;
-            // softening correction, :395-398
-            const R dg = V1.w * ri * (et_i * dw_i + D.w * dw_j);
-            pgx += dg * dx;
-            pgy += dg * dy;
-            pgz += dg * dz;
-        };
-        // a j beyond both supports: only the signal velocity (r > 0 here)
-        auto far_pair = [&](int k) {
-            const R4 P = s_fp[wid][k];
-            const R4 V = s_fv[wid][k];
-            const R dx = xc - P.x, dy = yc - P.y, dz = zc - P.z;
-            const R ux = vxi - V.x, uy = vyi - V.y, uz = vzi - V.z;
-            const R r2 = dx * dx + dy * dy + dz * dz;
-            const R w = (dx * ux + dy * uy + dz * uz) * rsqrt_r(r2);
-            const R wneg = w < (R)0 ? w : (R)0;
-            const R vs = cs_i + P.w - (R)3 * wneg;
-            vsmx = vs > vsmx ? vs : vsmx;
-        };
-        auto run_near = [&](int n) {
-            pax = 0; pay = 0; paz = 0; pud = 0; pdf = 0; pgx = 0; pgy = 0; pgz = 0;
-            unsigned msk = 0;
-            if (skip_tile(&s_nb[wid][nhead], 1, n)) {
-                if (tpi == 1 && n == 32) {
-#pragma unroll HYDRO_MARK_UNROLL
-                    for (int k = 0; k < 32; ++k) mark_only(nhead + k, msk);
-                } else {
-                    for (int k = sub; k < n; k += tpi) mark_only(nhead + k, msk);
-                }
-            } else if (tpi == 1 && n == 32) {
-#pragma unroll 4
-                for (int k = 0; k < 32; ++k) signal(nhead + k, msk);
-            } else {
-                for (int k = sub; k < n; k += tpi) signal(nhead + k, msk);
-            }
-            if (a.n_mark) {
-                const unsigned c = __popc(msk);
-                n_marked += c;
-                n_slots += 32u * __reduce_max_sync(FULL, c);
-            }
-            if constexpr (F64) {
-                while (msk) {
-                    const int k = __ffs(msk) - 1;
-                    msk &= msk - 1;
-                    pair(nhead + k);
-                }
-                ax.add(pax);
-                ay.add(pay);
-                az.add(paz);
-                ud.add(pud);
-                df.add(pdf);
-                gx.add(pgx);
-                gy.add(pgy);
-                gz.add(pgz);
-            } else {
-                // append the marked j to the particle's row, self pairs (equal
-                // ids, hdr_hydro.hpp:356) dropped; the tpi lanes of one
-                // particle write consecutive segments (prefix over the lanes)
-                unsigned m = r.act ? msk : 0u;
-                for (unsigned t = m; t; t &= t - 1) {
-                    const int k = __ffs(t) - 1;
-                    if (s_id[wid][nhead + k] == idi) m &= ~(1u << k);
-                }
-                const int c = __popc(m);
-                int incl = c;
-                for (int o = 1; o < tpi; o <<= 1) {
-                    const int v = __shfl_up_sync(FULL, incl, o, tpi);
-                    if (sub >= o) incl += v;
-                }
-                const int tot = __shfl_sync(FULL, incl, tpi - 1, tpi);
-                int pos = lcount + incl - c;
-                int *row = a.df_list + (size_t)ii * a.df_cap;
-                for (; m; m &= m - 1) {
-                    const int k = __ffs(m) - 1;
-                    if (pos < a.df_cap) row[pos] = s_jx[wid][nhead + k];
-                    ++pos;
-                }
-                lcount += tot;
-            }
-            __syncwarp();
-        };
-        auto run_far = [&](int n) {
-            if (skip_tile(&s_fv[wid][fhead].w, 4, n)) {
-                __syncwarp();
-                return;
-            }
-            if (tpi == 1 && n == 32) {
-#pragma unroll 8
-                for (int k = 0; k < 32; ++k) far_pair(fhead + k);
-            } else {
-                for (int k = sub; k < n; k += tpi) far_pair(fhead + k);
-            }
-            __syncwarp();
-        };
-        for (int t = 0; t < nj; t += 32) {
-            const int jk = t + lane;
-            bool near = false, far = false;
-            int j = 0;
-            float4 ph, pl, vh, g2;
-            dbl4 p64, v64, g1_64, g2_64;
-            R px = 0, py = 0, pz = 0, hj_inv = 0, hj2m = 0;
-            if (jk < nj) {
-                j = a.j_idx ? a.j_idx[jb + jk] : jb + jk;
-                if (F64) {
-                    p64 = a.j_pm[j];
-                    v64 = a.j_vel[j];
-                    g1_64 = a.j_h1[j];
-                    g2_64 = a.j_h2[j];
-                    px = p64.x; py = p64.y; pz = p64.z; hj_inv = g1_64.x;
-                } else {
-                    ph = a.fj.phi[j];
-                    pl = a.fj.plo[j];
-                    vh = a.fj.vhi[j];
-                    g2 = a.fj_g2[j];
-                    px = df_diff(ph.x, pl.x, cph.x, cpl.x);
-                    py = df_diff(ph.y, pl.y, cph.y, cpl.y);
-                    pz = df_diff(ph.z, pl.z, cph.z, cpl.z);
-                    hj_inv = vh.w;
-                }
-                const R hj = rcp_r(hj_inv);
-                const R hj2 = hj * hj * (R)1.0002;
-                hj2m = hj2;
-                const R rf2 = hj2 > hm2 ? hj2 : hm2;
-                near = !(box.d2(px, py, pz) > rf2) || !(hj2 >= (R)0);
-                far = !near;
-            }
-            const unsigned mn = __ballot_sync(FULL, near);
-            const unsigned mf = __ballot_sync(FULL, far);
-            if (near) {
-                const int k = (nhead + nfill + __popc(mn & lt)) & 63;
-                if (F64) {
-                    const double2 g3 = a.j_h3[j];
-                    const double h4 = g1_64.x * g1_64.x * g1_64.x * g1_64.x;
-                    s_p1[wid][k] = Real<F64>::make4(p64.x, p64.y, p64.z, g1_64.x);
-                    s_p2[wid][k] = Real<F64>::make4(0.0, 0.0, 0.0, g2_64.y);
-                    s_v1[wid][k] = Real<F64>::make4(v64.x, v64.y, v64.z, p64.w);
-                    s_v2[wid][k] = Real<F64>::make4(0.0, 0.0, 0.0, h4);
-                    s_c[wid][k] = Real<F64>::make4(g1_64.y, g1_64.z, g1_64.w, g2_64.x);
-                    s_d[wid][k] = Real<F64>::make4(g2_64.z, g2_64.w, g3.x, g3.y);
-                    s_f[wid][k] = make_float2(0.0f, 0.0f);
-                    s_nb[wid][k] = sv_bound(g2_64.y, dvel(v64.x, v64.y, v64.z, 0.0f, 0.0f, 0.0f));
-                } else {
-                    // the signal velocity and the mark only: the pair sums are
-                    // formed in double-float from the lists (hydro_df_lists)
-                    const float4 vl = a.fj.vlo[j];
-                    s_p1[wid][k] = Real<F64>::make4((R)(ph.x - cph.x), (R)(ph.y - cph.y), (R)(ph.z - cph.z),
-                                                    (R)vh.w);
-                    s_p2[wid][k] = Real<F64>::make4((R)(pl.x - cpl.x), (R)(pl.y - cpl.y), (R)(pl.z - cpl.z),
-                                                    (R)g2.y);
-                    s_v1[wid][k] = Real<F64>::make4((R)vh.x, (R)vh.y, (R)vh.z, (R)ph.w);
-                    s_v2[wid][k] = Real<F64>::make4((R)vl.x, (R)vl.y, (R)vl.z, (R)vl.w);
-                    s_nb[wid][k] = sv_bound((R)g2.y, dvel(vh.x, vh.y, vh.z, vl.x, vl.y, vl.z));
-                    if constexpr (!F64) {
-                        s_m[wid][k] = make_float4(px, py, pz, hj2m);
-                        s_jx[wid][k] = j;
-                    }
-                }
-                s_id[wid][k] = a.j_id[j];
-            }
-            // far entries: their signal-velocity bound, and the whole chunk's
-            // far entries dropped when none can raise any lane's maximum
-            R bfar = 0;
-            if (far) {
-                if constexpr (F64)
-                    bfar = sv_bound(g2_64.y, dvel(v64.x, v64.y, v64.z, 0.0f, 0.0f, 0.0f));
-                else
-                    bfar = sv_bound((R)g2.y, dvel(vh.x, vh.y, vh.z, lcx, lcy, lcz));
-            }
-            unsigned ms = mf;
-            if (a.sv_skip && mf && below(far ? bfar : (R)0)) ms = 0;
-            if (ms & (1u << lane)) {
-                const int k = (fhead + ffill + __popc(ms & lt)) & 63;
-                if constexpr (F64) {
-                    s_fp[wid][k] = Real<F64>::make4(px, py, pz, g2_64.y);
-                    s_fv[wid][k] = Real<F64>::make4(v64.x, v64.y, v64.z, bfar);
-                } else {
-                    s_fp[wid][k] = Real<F64>::make4(px, py, pz, (R)g2.y);
-                    s_fv[wid][k] = Real<F64>::make4((R)vh.x, (R)vh.y, (R)vh.z, bfar);
-                }
-            }
-            nfill += __popc(mn);
-            ffill += __popc(ms);
-            kept_n += __popc(mn);
-            kept_f += __popc(mf);
-            __syncwarp();
-            if (nfill >= 32) {
-                run_near(32);
-                nhead ^= 32;
-                nfill -= 32;
-            }
-            if (ffill >= 32) {
-                run_far(32);
-                fhead ^= 32;
-                ffill -= 32;
-            }
+        for (int q = 0; q < 8; ++q) v[q] = seg_sum(v[q], L);
+        if (ok && sub == 0) hydro64_store(a, p, v);
+    }
+}
+
+// One block per particle of the sweep queue over its walk's whole list.
+__global__ inline void __launch_bounds__(DSWEEP_THREADS) hydro64_sweep(const HydroArgs a) {
+    __shared__ double red[8][DSWEEP_THREADS / 32];
+    const int n = *a.n_ovf;
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const int p = a.ovf[e].x, w = a.ovf[e].y;
+        const Hydro64P I = hydro64_load(a.i_pm, a.i_vel, a.i_h1, a.i_h2, a.i_h3, p);
+        const long long idi = a.i_id[p];
+        const float4 ph = a.mi_p[p], pl = a.mi_l[p];
+        const float pad = 3.0e-14f * (fabsf(ph.x) + fabsf(ph.y) + fabsf(ph.z));
+        Hydro64Acc s;
+        for (int k = a.j_off[w] + threadIdx.x; k < a.j_off[w + 1]; k += DSWEEP_THREADS) {
+            const int j = a.j_idx ? a.j_idx[k] : k;
+            // pairs beyond both supports add zero: an FP32 distance test with
+            // the margins of mark_rows (h outside its range: no test)
+            const float4 qh = a.mj_p[j], ql = a.mj_l[j];
+            const float dx = df_diff(qh.x, ql.x, ph.x, pl.x), dy = df_diff(qh.y, ql.y, ph.y, pl.y);
+            const float dz = df_diff(qh.z, ql.z, ph.z, pl.z);
+            const float h = fmaxf(ph.w, qh.w) * 1.0001f + pad;
+            const bool test = ph.w >= ROW_HMIN && ph.w <= ROW_HMAX && qh.w >= ROW_HMIN && qh.w <= ROW_HMAX;
+            if ((test && dx * dx + dy * dy + dz * dz > h * h) || a.j_id[j] == idi) continue;
+            hydro64_pair(I, hydro64_load(a.j_pm, a.j_vel, a.j_h1, a.j_h2, a.j_h3, j), s);
         }
-        if (nfill > 0) run_near(nfill);
-        if (ffill > 0) run_far(ffill);
-        const double svs = seg_max((double)vsmx, tpi);
-        if constexpr (F64) {
-            const double sax = seg_sum(ax.value(), tpi), say = seg_sum(ay.value(), tpi);
-            const double saz = seg_sum(az.value(), tpi), sud = seg_sum(ud.value(), tpi);
-            const double sdf = seg_sum(df.value(), tpi), sgx = seg_sum(gx.value(), tpi);
-            const double sgy = seg_sum(gy.value(), tpi), sgz = seg_sum(gz.value(), tpi);
-            if (r.act && sub == 0) {
-                a.o_acch[3 * ii + 0] = 0.5 * sax;
-                a.o_acch[3 * ii + 1] = 0.5 * say;
-                a.o_acch[3 * ii + 2] = 0.5 * saz;
-                a.o_accg[3 * ii + 0] = 0.5 * sgx;
-                a.o_accg[3 * ii + 1] = 0.5 * sgy;
-                a.o_accg[3 * ii + 2] = 0.5 * sgz;
-                a.o_udot[ii] = 0.5 * sud;
-                a.o_vsmx[ii] = svs;
-                a.o_diffu[ii] = 2.0 * sdf;
-            }
-        } else if (r.act && sub == 0) {
-            a.o_vsmx[ii] = svs;
-            a.df_cnt[ii] = lcount;
-            if (lcount > a.df_cap) {
-                const int e = atomicAdd(a.df_novf, 1);
-                a.df_ovf[e] = make_int2(ii, r.walk);
-            }
-        }
-        if (a.n_eval_near && lane == 0) {
-            atomicAdd(a.n_eval_near, (unsigned long long)kept_n * (unsigned long long)r.ni);
-            atomicAdd(a.n_eval_far, (unsigned long long)kept_f * (unsigned long long)r.ni);
-        }
-        if (a.n_skip && lane == 0) {
-            atomicAdd(a.n_skip, (unsigned long long)n_skipped);
-            atomicAdd(a.n_skip + 1, (unsigned long long)n_tiles);
-        }
-        if (a.n_mark) {
-            const unsigned m = __reduce_add_sync(FULL, n_marked);
-            if (lane == 0) {
-                atomicAdd(a.n_mark, (unsigned long long)m);
-                atomicAdd(a.n_mark + 1, (unsigned long long)n_slots);
-            }
-        }
+        double v[8] = {s.ax, s.ay, s.az, s.gx, s.gy, s.gz, s.ud, s.df};
+        block_sum(v, red);
+        if (threadIdx.x == 0) hydro64_store(a, p, v);
     }
 }
 
@@ -650,13 +236,13 @@ __device__ __forceinline__ void hydro_df_store(const HydroArgs &a, int p, const 
 __global__ inline void __launch_bounds__(HYDRO_DF_THREADS, SPH_HYDRO_DF_MIN_BLOCKS) hydro_df_lists(const HydroArgs a) {
     using dfk::pk;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n_i; p += gridDim.x * blockDim.x) {
-        const int c = a.df_cnt[p];
-        if (c > a.df_cap) continue;
+        const int c = a.info[p].x;
+        if (c > ROW_CAP) continue;
         const HydroDFP<float> I = hydro_df_load(a.fi, a.fi_g1, a.fi_g2, a.fi_g3, a.fi_g4, p);
         const HydroDFP<pk> I2 = hydro_df_pack(I, I);
         HydroDFAcc<pk> acc2 = hydro_df_zero<pk>();
         HydroDFAcc<float> acc = hydro_df_zero<float>();
-        const int *row = a.df_list + (size_t)p * a.df_cap;
+        const int *row = a.rows + (size_t)p * ROW_CAP;
         int k = 0;
         for (; k + 1 < c; k += 2) {
             const HydroDFP<float> J0 = hydro_df_load(a.fj, a.fj_g1, a.fj_g2, a.fj_g3, a.fj_g4, row[k]);
@@ -691,9 +277,9 @@ __global__ inline void __launch_bounds__(HYDRO_SWEEP_THREADS) hydro_df_sweep(con
     constexpr int NW = HYDRO_SWEEP_THREADS / 32;
     __shared__ dfk::df part[9][NW];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int n_ovf = *a.df_novf;
+    const int n_ovf = *a.n_ovf;
     for (int e = blockIdx.x; e < n_ovf; e += gridDim.x) {
-        const int2 ent = a.df_ovf[e];
+        const int2 ent = a.ovf[e];
         const int p = ent.x, w = ent.y;
         const int jb = a.j_off[w], je = a.j_off[w + 1];
         const long long idi = a.i_id[p];
@@ -1079,10 +665,11 @@ __global__ inline void make_gravity_records_pe(int n, const dbl4 *pe, float4 *ph
 
 // Hydro records (layout in hydro_df.cuh): from h1 = (1/h, P, P Omega / rho^2,
 // bswt / 2), h2 = (rho, c_s, alpha, alpha_u), h3 = (thrm, eta); 1/h, h^-4 and
-// P Omega / rho^2 also as hi/lo splits of their FP64 values.
+// P Omega / rho^2 also as hi/lo splits of their FP64 values; and the mark
+// records (hydro_mark_records).
 __global__ inline void make_hydro_records(int n, const dbl4 *pm, const dbl4 *vel, const dbl4 *h1, const dbl4 *h2,
                                           const double2 *h3, float4 *phi, float4 *plo, float4 *vhi, float4 *vlo,
-                                          float4 *g1, float4 *g2, float4 *g3, float4 *g4) {
+                                          float4 *g1, float4 *g2, float4 *g3, float4 *g4, float4 *mp, float4 *mv) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const dbl4 p = pm[k], v = vel[k], a = h1[k], b = h2[k];
         const double2 c = h3[k];
@@ -1099,6 +686,10 @@ __global__ inline void make_hydro_records(int n, const dbl4 *pm, const dbl4 *vel
         g2[k] = make_float4((float)b.x, (float)b.y, (float)b.z, (float)b.w);
         g3[k] = make_float4(T.x, T.y, (float)c.y, Q.y);
         g4[k] = make_float4(H.x, H.y, H4.x, H4.y);
+        float4 m0, m1;
+        hydro_mark_records(p, v, a.x, b.y, m0, m1);
+        mp[k] = m0;
+        mv[k] = m1;
     }
 }
 

@@ -48,8 +48,7 @@ constexpr int MAX_RED = 8;
 constexpr long long MAX_POOL_CHUNKS = 0x7fffffffLL / sphtree::LIST_CHUNK;
 constexpr int NBKT = 32;   // cost classes of work items (log2 of the estimated cost)
 enum { S_NGROUPS = 0, S_NACTIVE, S_NITEMS, S_QUEUE, S_ERROR, S_UNCONV, S_TOTAL, S_ITERS, S_AMB, S_AMBTOT,
-       S_NTASKS, S_NROOTS, S_POOL, S_POOLERR, S_TQUEUE, S_POOLMAX, S_HOVF, S_SMALL, S_NITER, S_DOVF, S_NLONG, S_NLEFT,
-       S_BKT,
+       S_NTASKS, S_NROOTS, S_POOL, S_POOLERR, S_TQUEUE, S_POOLMAX, S_HOVF, S_SMALL, S_NITER, S_DOVF, S_NLONG, S_BKT,
        S_NI = S_BKT + 2 * NBKT + 2 };
 // double scalars
 enum { D_TIME = 0, D_DT, D_KSRMAX, D_EPSU, D_DTC, D_XC, D_YC, D_ZC, D_MC, D_EKIN, D_ETHM, D_EPOT,
@@ -553,7 +552,6 @@ __global__ void walk_particles(int n, const int *flag, const int *scan, int firs
     scal[S_SMALL] = small;
     scal[S_DOVF] = small ? total : 0;
     scal[S_NLONG] = 0;
-    scal[S_NLEFT] = 0;
 }
 __global__ void drop_items_if_small(int *scal) {
     if (scal[S_SMALL]) scal[S_NITEMS] = 0;
@@ -690,20 +688,19 @@ __global__ void gravity_writeback(int n, double G, const double *acc, const doub
     }
 }
 
-// Largest sound speed over each hydro walk's j-list (one block per walk, -inf
-// for an empty list).  The signal velocity of every i-particle of the walk,
-// a maximum of cs_i + cs_j - 3 min(w, 0) over the list (hdr_hydro.hpp:368-372),
+// Largest sound speed over each hydro walk's j-list (one block per walk, 0 for
+// an empty list).  The signal velocity of every i-particle of the walk, a
+// maximum of cs_i + cs_j - 3 min(w, 0) over the list (hdr_hydro.hpp:368-372),
 // is at least its own sound speed plus this.
 constexpr int CSMAX_THREADS = 256;
 __global__ void __launch_bounds__(CSMAX_THREADS) walk_csmax(const int *n_walks, const int *j_off, const int *j_idx,
-                                                            const float4 *f_g2, const dbl4 *h2, double *out,
-                                                            const int *scal) {
-    __shared__ double red[CSMAX_THREADS / 32];
+                                                            const float4 *mv, float *out, const int *scal) {
+    __shared__ float red[CSMAX_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (scal[S_ERROR] & (E_LISTCAP | E_STACK)) return;   // the lists overflowed (no hydro items either)
     const int nw = *n_walks;
     for (int w = blockIdx.x; w < nw; w += gridDim.x) {
-        double m = -INFINITY;
+        float m = 0.0f;
         const int e = j_off[w + 1];
         // four entries per thread and round: their loads are in flight together
         for (int k = j_off[w] + threadIdx.x; k < e; k += 4 * CSMAX_THREADS) {
@@ -711,17 +708,17 @@ __global__ void __launch_bounds__(CSMAX_THREADS) walk_csmax(const int *n_walks, 
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int kk = k + u * CSMAX_THREADS;
-                j[u] = kk < e ? (j_idx ? j_idx[kk] : kk) : -1;
+                j[u] = kk < e ? j_idx[kk] : -1;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (j[u] >= 0) m = fmax(m, f_g2 ? (double)f_g2[j[u]].y : h2[j[u]].y);   // NaN never raises it
+                if (j[u] >= 0) m = fmaxf(m, mv[j[u]].w);   // NaN never raises it
         }
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        m = sphk::warp_max(m);
         if (lane == 0) red[warp] = m;
         __syncthreads();
         if (threadIdx.x == 0) {
-            for (int k = 1; k < CSMAX_THREADS / 32; ++k) m = fmax(m, red[k]);
+            for (int k = 1; k < CSMAX_THREADS / 32; ++k) m = fmaxf(m, red[k]);
             out[w] = m;
         }
         __syncthreads();
@@ -967,15 +964,14 @@ struct sph_system {
     DevBuf<double> neps2;
     DevBuf<float4> flo, fhi, fmom, ptest;
     // FP32C double-float records (particles, hydro fields, tree monopoles)
-    DevBuf<float4> f_phi, f_plo, f_vhi, f_vlo, f_g1, f_g2, f_g3, f_g4, f_shi, f_slo;
+    DevBuf<float4> f_phi, f_plo, f_vhi, f_vlo, f_g1, f_g2, f_g3, f_g4, f_mp, f_mv, f_shi, f_slo;
     // per particle the j indices of its pairs (ROW_CAP per row; density rows,
     // then the hydro rows of the same evaluation), their number (density: with
     // the walk), and the particles without a row
-    DevBuf<int> hl_list, hl_cnt;
+    DevBuf<int> hl_list;
     DevBuf<int2> hl_ovf, r_info;
-    // items with long lists, left to a block each, and their particles
-    DevBuf<WorkItem> long_items;
-    DevBuf<int> left;
+    DevBuf<WorkItem> long_items;   // items with long lists, left to a block each
+    DevBuf<float> w_csmax;   // per hydro walk: largest sound speed of its list
     // re-walk index list (particles still iterating) and its per-walk segments
     DevBuf<int> uflag, uscan, ulist, a_sfirst, a_scount;
     // FP64 re-check queue of decision-ambiguous density results
@@ -984,7 +980,6 @@ struct sph_system {
     // per-warp neighbour lists of the streamed density walk (scratch)
     DevBuf<int> nbr;
     int nbr_warps = 0;
-    DevBuf<double> w_csmax;   // per hydro walk: largest sound speed of its list
     // groups and walks
     DevBuf<int> gflag, groot, gscan, group_node, group_first, group_count;
     DevBuf<int> aflag, ascan, a_node, a_first, a_count;
@@ -1091,14 +1086,15 @@ int alloc_all(sph_system *s) {
     e |= s->visit.ensure(n) | s->mom.ensure(nn) | s->neps2.ensure(nn);
     if (s->prm.quadrupole) e |= s->quad.ensure(6 * nn) | s->fq0.ensure(nn) | s->fq1.ensure(nn);
     e |= s->flo.ensure(nn) | s->fhi.ensure(nn) | s->fmom.ensure(nn) | s->ptest.ensure(n);
-    DevBuf<float4> *f1[] = {&s->f_phi, &s->f_plo, &s->f_vhi, &s->f_vlo, &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4};
+    DevBuf<float4> *f1[] = {&s->f_phi, &s->f_plo, &s->f_vhi, &s->f_vlo, &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4,
+                            &s->f_mp, &s->f_mv};
     for (auto *b : f1) e |= b->ensure(n);
-    e |= s->hl_list.ensure(n * sphk::HYDRO_LIST_CAP) | s->hl_cnt.ensure(n) | s->hl_ovf.ensure(n);
+    e |= s->hl_list.ensure(n * sphk::ROW_CAP) | s->hl_ovf.ensure(n);
     e |= s->f_shi.ensure(nn) | s->f_slo.ensure(nn);
     e |= s->uflag.ensure(n) | s->uscan.ensure(n) | s->ulist.ensure(n) | s->a_sfirst.ensure(n) | s->a_scount.ensure(n);
     s->amb_cap = std::max<int>(1024, s->n / 16);
-    e |= s->amb.ensure(s->amb_cap) | s->r_info.ensure(n) | s->w_csmax.ensure(n);
-    e |= s->long_items.ensure(n) | s->left.ensure(n);
+    e |= s->amb.ensure(s->amb_cap) | s->r_info.ensure(n);
+    e |= s->long_items.ensure(n) | s->w_csmax.ensure(n);
     s->nbr_warps = s->ctx->grid_stream * PAIR_WARPS;
     e |= s->nbr.ensure((size_t)s->nbr_warps * NBR_CAP * 32);
     DevBuf<int> *i1[] = {&s->gflag, &s->groot, &s->gscan, &s->group_node, &s->group_first, &s->group_count,
@@ -1480,7 +1476,7 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
                                                s->uscan.p, s->ulist.p, s->a_sfirst.p, s->a_scount.p, s->hl_ovf.p);
     const int kind = first ? 0 : 3;
     r = build_lists_and_items(s, kind, s->a_node.p, s->a_r.p, eager, s->lscal.p + (first ? L_PAIRS_D1 : L_PAIRS_D),
-                              s->a_sfirst.p, s->a_scount.p, !first ? std::min(8, item_size(s)) : f32 ? 32 : item_size(s));
+                              s->a_sfirst.p, s->a_scount.p, f32 ? (first ? 32 : 8) : std::min(first ? 32 : 8, item_size(s)));
     if (r) return r;
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
     sphk::MarkArgs m{};
@@ -1491,6 +1487,7 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
     m.i_list = s->ulist.p;
     m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
     m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG;
+    m.pairs = s->lscal.p + (first ? L_PAIRS_D1 : L_PAIRS_D);
     sphk::DensityArgs a{};
     a.n_eval = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_D1) : nullptr;
     a.n_pass = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_DLISTED) : nullptr;
@@ -1516,7 +1513,7 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
     if (f32) CUDA_TRY(cudaMemsetAsync(s->scal.p + S_AMB, 0, sizeof(int), st));
     if (first) phase_event(s, EV_DENSK_B, st);
     if (!first) drop_items_if_small<<<1, 1, 0, st>>>(s->scal.p);
-    if (f32 && first) {
+    if (f32) {
         sphk::StreamArgs w{};
         w.i_pm = a.i_pm; w.fi = a.fi; w.fj = a.fj; w.i_id = a.i_id; w.j_id = a.j_id;
         w.i_ksr = a.i_ksr; w.i_rs = a.i_rs;
@@ -1531,15 +1528,12 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
         w.nbr_cap = NBR_CAP;
         w.nbr_warps = s->nbr_warps;
         w.nbr_slack = lists ? s->prm.density_list_slack : 1.0f;
-        w.long_items = m.long_items; w.n_long = m.n_long;
-        w.left = s->left.p; w.n_left = s->scal.p + S_NLEFT;
+        w.long_items = m.long_items; w.n_long = m.n_long; w.pairs = m.pairs;
         w.n_eval = a.n_eval; w.n_pass = a.n_pass;
-        a.i_list = w.left;
-        a.n_i_dev = w.n_left;
-        sphrt::launch_density_stream(ctx, w, m, a, n, st, s->scal.p + S_AMBTOT);
+        sphrt::launch_density_stream(ctx, w, !first, a, n, st, s->scal.p + S_AMBTOT);
     } else {
         sphrt::launch_density(ctx, m, ctx->grid[0][0], a, n, ctx->prm.precision, st,
-                              f32 ? s->scal.p + S_AMBTOT : nullptr);
+                              nullptr);
     }
     if (first) phase_event(s, EV_DENSK_E, st);
     commit_density<<<grid_for(n), 256, 0, st>>>(n, s->rs.p, tmp, out, s->scal.p);
@@ -1611,8 +1605,7 @@ int density_phase(sph_system *s, bool eager) {
         sphk::make_density_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->ksr[0].p, s->f_phi.p,
                                                                 s->f_plo.p, s->f_vhi.p, s->f_vlo.p);
     else
-        sphk::make_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->ksr[0].p, false, s->f_phi.p,
-                                                            s->f_plo.p);
+        sphk::make_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->ksr[0].p, s->f_phi.p, s->f_plo.p);
     init_rs<<<grid_for(n), 256, 0, st>>>(n, s->ksr[0].p, s->rs.p);
     // the first guess, kept for the derivative of this evaluation
     CUDA_TRY(cudaMemcpyAsync(s->h_guess.p, s->ksr[0].p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, st));
@@ -1736,48 +1729,58 @@ int hydro_phase(sph_system *s, bool eager) {
         sphk::make_hydro_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->h1.p, s->h2.p,
                                                               s->h3.p, s->f_phi.p, s->f_plo.p, s->f_vhi.p,
                                                               s->f_vlo.p, s->f_g1.p, s->f_g2.p, s->f_g3.p,
-                                                              s->f_g4.p);
+                                                              s->f_g4.p, s->f_mp.p, s->f_mv.p);
+    else
+        sphk::make_hydro_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->h1.p, s->h2.p,
+                                                                  s->f_mp.p, s->f_plo.p, s->f_mv.p);
     int r = build_lists_and_items(s, 1, s->group_node.p, nullptr, eager, s->lscal.p + L_PAIRS_H, nullptr, nullptr,
                                   item_size(s));
     if (r) return r;
-    const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
-    const bool skip = s->prm.hydro_signal_skip != 0;
-    if (skip)
-        walk_csmax<<<ctx->sm_count * 8, CSMAX_THREADS, 0, st>>>(s->walk_num[1], s->loff[1].p, s->jidx[1].p,
-                                                     f32 ? s->f_g2.p : nullptr, s->h2.p, s->w_csmax.p, s->scal.p);
+    // rows of particles no work item reaches (a failed list build) stay
+    // empty; no particle without a row and no long item yet
+    CUDA_TRY(cudaMemsetAsync(s->r_info.p, 0, sizeof(int2) * (size_t)n, st));
+    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_HOVF, 0, sizeof(int), st));
+    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_NLONG, 0, sizeof(int), st));
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
+    if (s->prm.hydro_signal_skip != 0)
+        walk_csmax<<<ctx->sm_count * 8, CSMAX_THREADS, 0, st>>>(s->walk_num[1], s->loff[1].p, s->jidx[1].p, s->f_mv.p,
+                                                                s->w_csmax.p, s->scal.p);
     phase_event(s, EV_HK_B, st);
+    sphk::MarkArgs m{};
+    m.i_hi = s->f_mp.p; m.i_lo = s->f_plo.p; m.j_hi = m.i_hi; m.j_lo = m.i_lo;
+    m.i_v = s->f_mv.p; m.j_v = m.i_v;
+    m.items = s->ls[0].items.p; m.n_items_dev = s->scal.p + S_NITEMS;
+    m.j_off = s->loff[1].p; m.j_idx = s->jidx[1].p; m.queue = s->scal.p + S_QUEUE;
+    m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_HOVF;
+    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG; m.pairs = s->lscal.p + L_PAIRS_H;
+    m.i_id = s->id[0].p; m.j_id = m.i_id;
+    m.fi = sphk::F32Part{s->f_phi.p, s->f_plo.p, s->f_vhi.p, s->f_vlo.p};
+    m.fj = m.fi;
+    m.fi_g2 = s->f_g2.p; m.fj_g2 = s->f_g2.p;
+    m.i_pm = s->pos[0].p; m.i_vel = s->vel[0].p; m.i_h2 = s->h2.p;
+    m.j_pm = m.i_pm; m.j_vel = m.i_vel; m.j_h2 = m.i_h2;
+    m.o_vsmx = s->r_vsmx.p;
+    m.sv_skip = s->prm.hydro_signal_skip != 0 ? 1 : 0;
+    m.csmax = m.sv_skip ? s->w_csmax.p : nullptr;
+    m.n_near = reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_HN);
+    m.n_far = reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_HF);
+    m.n_skip = reinterpret_cast<unsigned long long *>(s->lscal.p + L_HSKIP);
+    m.n_mark = reinterpret_cast<unsigned long long *>(s->lscal.p + L_HMARK);
     sphk::HydroArgs a{};
-    a.n_eval_near = reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_HN);
-    a.n_eval_far = reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_HF);
-    a.n_skip = reinterpret_cast<unsigned long long *>(s->lscal.p + L_HSKIP);
-    a.n_mark = reinterpret_cast<unsigned long long *>(s->lscal.p + L_HMARK);
-    a.walk_csmax = skip ? s->w_csmax.p : nullptr;
-    a.sv_skip = skip ? 1 : 0;
-    a.i_pm = s->pos[0].p; a.i_vel = s->vel[0].p; a.i_id = s->id[0].p;
+    a.i_pm = m.i_pm; a.i_vel = m.i_vel; a.i_id = m.i_id;
     a.i_h1 = s->h1.p; a.i_h2 = s->h2.p; a.i_h3 = s->h3.p;
-    a.j_pm = s->pos[0].p; a.j_vel = s->vel[0].p; a.j_id = s->id[0].p;
+    a.j_pm = m.i_pm; a.j_vel = m.i_vel; a.j_id = m.i_id;
     a.j_h1 = s->h1.p; a.j_h2 = s->h2.p; a.j_h3 = s->h3.p;
-    a.fi = sphk::F32Part{s->f_phi.p, s->f_plo.p, s->f_vhi.p, s->f_vlo.p};
-    a.fj = a.fi;
-    a.fi_g1 = s->f_g1.p; a.fi_g2 = s->f_g2.p; a.fi_g3 = s->f_g3.p;
-    a.fj_g1 = s->f_g1.p; a.fj_g2 = s->f_g2.p; a.fj_g3 = s->f_g3.p;
-    a.i_list = nullptr;
-    a.items = s->ls[0].items.p; a.n_items = 0; a.n_items_dev = s->scal.p + S_NITEMS;
-    a.j_off = s->loff[1].p; a.j_idx = s->jidx[1].p; a.queue = s->scal.p + S_QUEUE;
-    a.o_acch = s->r_acch.p; a.o_accg = s->r_accg.p; a.o_udot = s->r_udot.p; a.o_vsmx = s->r_vsmx.p;
-    a.o_diffu = s->r_diffu.p;
-    a.fi_g4 = s->f_g4.p; a.fj_g4 = s->f_g4.p;
-    a.df_list = s->hl_list.p; a.df_cap = sphk::HYDRO_LIST_CAP; a.df_cnt = s->hl_cnt.p;
-    a.df_ovf = s->hl_ovf.p; a.df_novf = s->scal.p + S_HOVF; a.n_i = n;
-    if (f32) {
-        // rows of particles no work item reaches (a failed list build) stay
-        // empty; the overflow queue starts empty
-        CUDA_TRY(cudaMemsetAsync(s->hl_cnt.p, 0, sizeof(int) * (size_t)n, st));
-        CUDA_TRY(cudaMemsetAsync(s->scal.p + S_HOVF, 0, sizeof(int), st));
-    }
-    sphrt::launch_hydro(a, ctx->prm.precision, ctx->grid[1][ctx->prm.precision == SPH_PREC_FP64], st,
-                        ctx->grid_df, s->ev[EV_HK_MID], s->capturing >= 0);
+    a.fi = m.fi;
+    a.fj = m.fi;
+    a.fi_g1 = s->f_g1.p; a.fi_g2 = s->f_g2.p; a.fi_g3 = s->f_g3.p; a.fi_g4 = s->f_g4.p;
+    a.fj_g1 = s->f_g1.p; a.fj_g2 = s->f_g2.p; a.fj_g3 = s->f_g3.p; a.fj_g4 = s->f_g4.p;
+    a.j_off = m.j_off; a.j_idx = m.j_idx;
+    a.o_acch = s->r_acch.p; a.o_accg = s->r_accg.p; a.o_udot = s->r_udot.p; a.o_diffu = s->r_diffu.p;
+    a.rows = m.rows; a.info = m.info; a.ovf = m.ovf; a.n_ovf = m.n_ovf; a.n_i = n;
+    a.mi_p = m.i_hi; a.mi_l = m.i_lo; a.mj_p = m.j_hi; a.mj_l = m.j_lo;
+    sphrt::launch_hydro(ctx, m, ctx->grid[1][ctx->prm.precision == SPH_PREC_FP64], a, ctx->prm.precision, st,
+                        s->ev[EV_HK_MID], s->capturing >= 0);
     phase_event(s, EV_HK_E, st);
     AlphaParams ap{s->prm.alpha_max, s->prm.alpha_min, s->prm.alphu_max, s->prm.alphu_min};
     hydro_writeback<<<grid_for(n), 256, 0, st>>>(
@@ -2005,11 +2008,11 @@ extern "C" int sph_system_destroy(sph_system *s) {
     s->count.release(); s->visit.release(); s->mom.release(); s->quad.release(); s->fq0.release();
     s->fq1.release();
     DevBuf<float4> *f1[] = {&s->flo, &s->fhi, &s->fmom, &s->ptest, &s->f_phi, &s->f_plo, &s->f_vhi, &s->f_vlo,
-                            &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4, &s->f_shi, &s->f_slo};
+                            &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4, &s->f_mp, &s->f_mv, &s->f_shi, &s->f_slo};
     for (auto *b : f1) b->release();
-    s->hl_list.release(); s->hl_cnt.release(); s->hl_ovf.release();
+    s->hl_list.release(); s->hl_ovf.release();
     s->uflag.release(); s->uscan.release(); s->ulist.release(); s->a_sfirst.release(); s->a_scount.release();
-    s->amb.release(); s->r_info.release(); s->long_items.release(); s->left.release(); s->nbr.release(); s->w_csmax.release();
+    s->amb.release(); s->r_info.release(); s->long_items.release(); s->w_csmax.release(); s->nbr.release();
     DevBuf<int> *i1[] = {&s->gflag, &s->groot, &s->gscan, &s->group_node, &s->group_first, &s->group_count,
                          &s->aflag, &s->ascan, &s->a_node, &s->a_first, &s->a_count,
                          &s->scal};

@@ -1,4 +1,4 @@
-"""GPU tests of the neighbour-row kernels (csrc/rows.cuh, csrc/density_rows.cuh)
+"""GPU tests of the neighbour-row kernels (csrc/rows.cuh and the sums over rows)
 at the sizes where they can go wrong, against the oracle: rows of 0 to more
 than ROW_CAP entries, list lengths around a streaming step (64 entries) and
 around the length that a whole block marks (4096), group sizes that
@@ -72,3 +72,58 @@ def test_density_rows(prec, n_i, n_j, guess, neighbours):
 @pytest.mark.parametrize("scale", [1.0e-20, 1.0e25])
 def test_density_fp64_beyond_the_fp32_range(scale):
     _check("fp64", *_cloud(20, 600, 5, scale=scale))
+
+
+def _hydro_cloud(n_i, n_j, seed, neighbours=50.0, scale=1.0, speed=1.0):
+    """Hydro inputs on the same ball: a pressure gradient, sound speeds of
+    order one and random velocities of `speed` times that."""
+    rng = np.random.default_rng(seed + 1)
+    den, src = _cloud(n_i, n_j, seed, neighbours=neighbours, scale=scale)
+    out = []
+    for d, dt in ((den, abi.HydroEPI), (src, abi.HydroEPJ)):
+        a = np.zeros(len(d), dt)
+        a["id"], a["pos"], a["vel"] = d["id"], d["pos"], speed * scale * d["vel"]
+        if dt is abi.HydroEPJ:
+            a["mass"] = d["mass"]
+        r2 = ((a["pos"] / scale - 30.0) ** 2).sum(1)
+        a["ksr"] = scale * (neighbours / n_j) ** (1.0 / 3.0) * (0.8 + 0.4 * ((a["id"] * 37) % 101) / 101.0)
+        a["hinv"] = 1.0 / a["ksr"]
+        a["dens"] = 0.3 + 0.1 * r2
+        a["pres"] = scale ** 2 * (1.0 - 0.5 * r2)
+        a["presc"] = a["pres"] / a["dens"] ** 2
+        a["bswt"] = 0.5 * ((a["id"] * 13) % 7) / 7.0
+        a["vsnd"] = scale * (1.0 + 0.3 * ((a["id"] * 29) % 53) / 53.0)
+        a["alph"], a["alphu"] = 1.0, 0.05
+        a["thrm"] = a["pres"] / a["dens"]
+        a["eta"] = 0.1 * a["ksr"] ** 2
+        out.append(a)
+    return out
+
+
+@pytest.mark.parametrize("prec", ["fp32c", "fp64"])
+@pytest.mark.parametrize("n_i,n_j,neighbours,speed", [
+    (1, 40, 20.0, 1.0), (5, 64, 20.0, 0.0), (33, 65, 20.0, 1.0), (33, 1000, 50.0, 1e-3),
+    (7, 4096, 50.0, 1.0), (37, 4097, 50.0, 30.0),   # the last list of one warp, the first of a block
+    (40, 3000, 160.0, 1.0), (40, 9000, 160.0, 1.0),  # rows beyond their capacity
+])
+def test_hydro_rows(prec, n_i, n_j, neighbours, speed):
+    epi, epj = _hydro_cloud(n_i, n_j, 7 * n_i + n_j, neighbours, speed=speed)
+    out = np.zeros(n_i, abi.Hydro)
+    with functors.Context(precision=prec, eta=ETA) as ctx:
+        functors.calcHydro(ctx)(epi, n_i, epj, n_j, out)
+    ref = orc.hydro(epi, epj)
+    tol = 1e-11 if prec == "fp64" else 1e-5
+    for f in ("acch", "accg", "udot", "vsmx"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < tol, f
+    assert rel_err(out["diffu"], ref["diffu"], 1e-2).max() < (tol if prec == "fp64" else 1e-4)
+
+
+@pytest.mark.parametrize("scale", [1.0e-20, 1.0e25])
+def test_hydro_fp64_beyond_the_fp32_range(scale):
+    epi, epj = _hydro_cloud(20, 600, 5, scale=scale)
+    out = np.zeros(20, abi.Hydro)
+    with functors.Context(precision="fp64", eta=ETA) as ctx:
+        functors.calcHydro(ctx)(epi, 20, epj, 600, out)
+    ref = orc.hydro(epi, epj)
+    for f in ("acch", "accg", "udot", "vsmx", "diffu"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < 1e-11, f
