@@ -30,10 +30,20 @@
 // the value central differences converge to.  The lists, tree and time step are those of the
 // forward evaluation and are held fixed (the density and hydro kernels are
 // C2 at their support, so list membership does not change their values).
-// Arithmetic is FP64 throughout; j-side contributions are reduced over the
-// warp (whose lanes visit the same list entry) before one atomic add each.
+// Arithmetic is FP64 throughout.
+//
+// The hydro and density-gradient pairs are gathered: a pair inside either
+// support is in the rows of both particles (the forward evaluation's hydro
+// rows, ~60 entries), and each particle adds what both ends' equations pass to
+// it, without atomics; eight lanes per particle.  The three h passes have
+// supports of their own, one-sided: their j-side goes out by atomics from rows
+// marked for them.  The gravity lists are one-sided too: a warp holds 32
+// i-particles against tiles of 32 list entries, lane l starting at entry l, so
+// that each entry's adjoints are added up in shared memory and sent out once
+// per tile.
 #pragma once
 
+#include "rows.cuh"
 #include "sph_device.cuh"
 
 namespace sphadj {
@@ -42,11 +52,6 @@ using sphk::CEFF0;
 using sphk::CEFF1;
 using sphk::KSRH;
 using sphk::FULL;
-
-// One warp's share of a walk: up to 32 consecutive i-particles.
-struct AdjItem {
-    int walk, first, ni;
-};
 
 struct AdjState {
     int n;
@@ -57,6 +62,10 @@ struct AdjState {
     const double *neps2;    // tree nodes: mass-weighted eps^2
     const int *parent;      // tree nodes: parent (root: -1); leaf of particle p: n - 1 + p
     const int *d_off, *d_idx, *h_off, *h_idx, *g_off, *g_idx;   // density, hydro, gravity lists per walk
+    const int *h_rows, *d_rows;       // rows of the hydro pairs and of the h passes
+    const int2 *h_info, *d_info;      // their entries (> ROW_CAP: the walk's list instead) and walks
+    const long long *id;
+    double slack;                     // radius of the rows of the h passes over the first guess
     double G, amax, amin, eta_ksrh;
 };
 
@@ -72,6 +81,7 @@ struct AdjAcc {
     double *u, *alph, *h0;  // outputs: internal energy, alpha, first guess of h
     double *h, *rho, *omega, *divv, *rotv, *c, *b, *pc, *eta, *e2, *hinv, *etas, *bswt;
     double *node;           // 4 per tree node: centre of mass (3), eps^2
+    double *coef;           // 5 per particle: adjoints of its gradient-pass sums (D, R, Sg)
 };
 
 // Wendland C2: W0 = u^4 (1+4q), W1 = -5 q u^3 (the reference's u^4 - u^3 (1+4q)),
@@ -88,17 +98,28 @@ __device__ __forceinline__ void wendland(double q, double &w0, double &w0p, doub
     }
 }
 
-__device__ __forceinline__ double wsum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    return v;
-}
-
-// warp-summed atomic add of a j-side contribution (every lane passes its own
-// value, zero where it has none)
-__device__ __forceinline__ void wadd(double *p, double v, int lane) {
-    v = wsum(v);
-    if (lane == 0 && v != 0.0) atomicAdd(p, v);
-}
+// Eight lanes per particle: its candidate pairs are its row, or its walk's
+// whole list where it has none.
+constexpr int LANES = 8;
+__device__ __forceinline__ double lsum(double v) { return sphk::seg_sum(v, LANES); }
+struct Candidates {
+    const int *p;
+    int n;
+    __device__ __forceinline__ Candidates(const int *rows, const int2 *info, const int *off, const int *idx, int i) {
+        const int2 f = info[i];
+        if (f.x <= sphk::ROW_CAP) {
+            p = rows + (size_t)i * sphk::ROW_CAP;
+            n = f.x;
+        } else {
+            p = idx + off[f.y];
+            n = off[f.y + 1] - off[f.y];
+        }
+    }
+};
+// particle of this lane's segment (-1 beyond n), grid-stride over particles
+#define ADJ_PARTICLES(i, n)                                                                                      \
+    for (int k0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 / LANES), i = k0 + (threadIdx.x & 31) / LANES; \
+         k0 < (n); k0 += ((gridDim.x * blockDim.x) >> 5) * (32 / LANES), i = k0 + (threadIdx.x & 31) / LANES)
 
 // -------------------------------------------------------------- stage A
 // alpha source and the seeds that need no pair loop
@@ -120,136 +141,108 @@ __global__ void adj_alpha(AdjState s, AdjSeed sd, AdjAcc a) {
 
 // -------------------------------------------------------------- stage B
 // hydro pairs: seeds acch (= acc / 2 per pair sum), accg (= G acc / 2), udot / 2
-__global__ void adj_hydro(AdjState s, AdjSeed sd, AdjAcc a, const AdjItem *items, int n_items) {
-    const int lane = threadIdx.x & 31;
-    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = wg; it < n_items; it += nw) {
-        const AdjItem t = items[it];
-        const bool act = lane < t.ni;
-        const int i = t.first + (act ? lane : 0);
+// of both ends of each pair
+__global__ void __launch_bounds__(128) adj_hydro(AdjState s, AdjSeed sd, AdjAcc a) {
+    const int sub = threadIdx.x & (LANES - 1);
+    ADJ_PARTICLES(ip, s.n) {
+        const bool act = ip < s.n;
+        const int i = act ? ip : s.n - 1;
         const dbl4 xi = s.pos[i], vi = s.vel[i];
-        const double hi = 1.0 / s.h[i], hi4 = hi * hi * hi * hi;
+        const double hi_len = s.h[i], hi = 1.0 / hi_len, hi3 = hi * hi * hi, hi4 = hi3 * hi;
         const double rho_i = s.dens[i], c_i = s.vsnd[i], b_i = 0.5 * s.bswt[i], al_i = s.alph[i];
         const double pc_i = s.pres[i] * s.grdh[i] / (rho_i * rho_i), et_i = s.eta[i];
-        const double sc = act ? 1.0 : 0.0;
-        const double Ahx = 0.5 * sd.acc[3 * i] * sc, Ahy = 0.5 * sd.acc[3 * i + 1] * sc,
-                     Ahz = 0.5 * sd.acc[3 * i + 2] * sc;
-        const double Agx = s.G * Ahx, Agy = s.G * Ahy, Agz = s.G * Ahz;
-        const double Us = 0.5 * sd.udot[i] * sc;
-        double xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0};
+        const double Ahx = 0.5 * sd.acc[3 * i], Ahy = 0.5 * sd.acc[3 * i + 1], Ahz = 0.5 * sd.acc[3 * i + 2];
+        const double Us_i = 0.5 * sd.udot[i];
+        const long long idi = s.id[i];
+        double xb0 = 0, xb1 = 0, xb2 = 0, vb0 = 0, vb1 = 0, vb2 = 0;
         double hinvb = 0, cb = 0, rb = 0, bb = 0, ab = 0, pcb = 0, etb = 0;
-        const double hmax_i = s.h[i];
-        for (int k = s.h_off[t.walk]; k < s.h_off[t.walk + 1]; ++k) {
-            const int j = s.h_idx[k];
+        const Candidates cand(s.h_rows, s.h_info, s.h_off, s.h_idx, i);
+        for (int e = sub; e < (act ? cand.n : 0); e += LANES) {
+            const int j = cand.p[e];
             const dbl4 xj = s.pos[j];
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
             const double hj_len = s.h[j];
-            const double hm = hmax_i > hj_len ? hmax_i : hj_len;
-            const bool in = act && j != i && r2 < hm * hm;
-            double jx[3] = {0, 0, 0}, jv[3] = {0, 0, 0};
-            double jhinv = 0, jc = 0, jr = 0, jb = 0, ja = 0, jpc = 0, jet = 0;
-            if (in) {
-                const dbl4 vj = s.vel[j];
-                const double mj = xj.w;
-                const double hj = 1.0 / hj_len, hj4 = hj * hj * hj * hj;
-                const double rho_j = s.dens[j], c_j = s.vsnd[j], b_j = 0.5 * s.bswt[j], al_j = s.alph[j];
-                const double pc_j = s.pres[j] * s.grdh[j] / (rho_j * rho_j), et_j = s.eta[j];
-                const double ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
-                const double ri = 1.0 / sqrt(r2), r = r2 * ri;
-                const double qi = r * hi, qj = r * hj;
-                double w0, w0p, w1i, w1pi, w1j, w1pj;
-                wendland(qi, w0, w0p, w1i, w1pi);
-                wendland(qj, w0, w0p, w1j, w1pj);
-                const double dWi = CEFF1 * hi4 * w1i, dWj = CEFF1 * hj4 * w1j;
-                const double ka = (dWi + dWj) * mj;
-                const double w = (dx * ux + dy * uy + dz * uz) * ri;
-                const double wn = w < 0.0 ? w : 0.0;
-                const double vs = c_i + c_j - 3.0 * wn;
-                const double rh = 1.0 / (rho_i + rho_j);
-                const double B = b_i + b_j, A = al_i + al_j;
-                const double av = B * A * vs * wn;
-                const double T = pc_i + pc_j - 0.5 * av * rh;
-                const double ta = T * ka * ri;
-                const double dg = mj * ri * (et_i * dWi + et_j * dWj);
-                // reverse
-                const double tab = -(Ahx * dx + Ahy * dy + Ahz * dz);
-                double ddx = -ta * Ahx, ddy = -ta * Ahy, ddz = -ta * Ahz;
-                const double dgb = Agx * dx + Agy * dy + Agz * dz;
-                ddx += dg * Agx; ddy += dg * Agy; ddz += dg * Agz;
-                double kab = Us * (pc_i * w - 0.25 * rh * av * wn);
-                pcb += Us * ka * w;
-                double wb = Us * ka * pc_i;
-                double rhb = -Us * ka * 0.25 * av * wn;
-                double avb = -Us * ka * 0.25 * rh * wn;
-                double wnb = -Us * ka * 0.25 * rh * av;
-                const double Tb = tab * ka * ri;
-                kab += tab * T * ri;
-                double rib = tab * T * ka;
-                pcb += Tb;
-                jpc = Tb;
-                avb += -0.5 * rh * Tb;
-                rhb += -0.5 * av * Tb;
-                rib += dgb * mj * (et_i * dWi + et_j * dWj);
-                etb += dgb * mj * ri * dWi;
-                jet = dgb * mj * ri * dWj;
-                double dWib = dgb * mj * ri * et_i, dWjb = dgb * mj * ri * et_j;
-                bb += avb * A * vs * wn;
-                jb = avb * A * vs * wn;
-                ab += avb * B * vs * wn;
-                ja = avb * B * vs * wn;
-                const double vsb = avb * B * A * wn;
-                wnb += avb * B * A * vs;
-                cb += vsb;
-                jc = vsb;
-                wnb += -3.0 * vsb;
-                if (w < 0.0) wb += wnb;
-                else if (w == 0.0) wb += 0.5 * wnb;
-                ddx += wb * ri * ux; ddy += wb * ri * uy; ddz += wb * ri * uz;
-                const double ubx = wb * ri * dx, uby = wb * ri * dy, ubz = wb * ri * dz;
-                rib += wb * (dx * ux + dy * uy + dz * uz);
-                rb += -rhb * rh * rh;
-                jr = -rhb * rh * rh;
-                dWib += kab * mj;
-                dWjb += kab * mj;
-                // dW = c1 hinv^4 W1(r hinv)
-                hinvb += dWib * CEFF1 * (4.0 * hi * hi * hi * w1i + hi4 * w1pi * r);
-                jhinv = dWjb * CEFF1 * (4.0 * hj * hj * hj * w1j + hj4 * w1pj * r);
-                const double rb_ = dWib * CEFF1 * hi4 * w1pi * hi + dWjb * CEFF1 * hj4 * w1pj * hj;
-                const double r2b = 0.5 * rb_ * ri - 0.5 * rib * ri * ri * ri;
-                ddx += 2.0 * r2b * dx; ddy += 2.0 * r2b * dy; ddz += 2.0 * r2b * dz;
-                xb[0] += ddx; xb[1] += ddy; xb[2] += ddz;
-                jx[0] = -ddx; jx[1] = -ddy; jx[2] = -ddz;
-                vb[0] += ubx; vb[1] += uby; vb[2] += ubz;
-                jv[0] = -ubx; jv[1] = -uby; jv[2] = -ubz;
-            }
-            if (__any_sync(FULL, in)) {
-                for (int c = 0; c < 3; ++c) {
-                    wadd(&a.x[3 * j + c], jx[c], lane);
-                    wadd(&a.v[3 * j + c], jv[c], lane);
-                }
-                wadd(&a.hinv[j], jhinv, lane);
-                wadd(&a.c[j], jc, lane);
-                wadd(&a.rho[j], jr, lane);
-                wadd(&a.b[j], jb, lane);
-                wadd(&a.alph[j], ja, lane);
-                wadd(&a.pc[j], jpc, lane);
-                wadd(&a.eta[j], jet, lane);
-            }
+            const double hm = fmax(hi_len, hj_len);
+            if (!(r2 < hm * hm) || s.id[j] == idi) continue;
+            const dbl4 vj = s.vel[j];
+            const double mi = xi.w, mj = xj.w;
+            const double hj = 1.0 / hj_len, hj4 = hj * hj * hj * hj;
+            const double rho_j = s.dens[j], b_j = 0.5 * s.bswt[j], al_j = s.alph[j];
+            const double pc_j = s.pres[j] * s.grdh[j] / (rho_j * rho_j), et_j = s.eta[j];
+            const double Bhx = 0.5 * sd.acc[3 * j], Bhy = 0.5 * sd.acc[3 * j + 1], Bhz = 0.5 * sd.acc[3 * j + 2];
+            const double Us_j = 0.5 * sd.udot[j];
+            const double ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
+            const double ri = sphk::rsqrt_r(r2), r = r2 * ri;
+            double w0, w0p, w1i, w1pi, w1j, w1pj;
+            wendland(r * hi, w0, w0p, w1i, w1pi);
+            wendland(r * hj, w0, w0p, w1j, w1pj);
+            const double dWi = CEFF1 * hi4 * w1i, dWj = CEFF1 * hj4 * w1j;
+            // the equations of i and of j: separation d and -d, velocity u and
+            // -u, the same w, viscosity and pressure factor
+            const double kaI = (dWi + dWj) * mj, kaJ = (dWi + dWj) * mi;
+            const double du = dx * ux + dy * uy + dz * uz;
+            const double w = du * ri;
+            const double wn = w < 0.0 ? w : 0.0;
+            const double vs = c_i + s.vsnd[j] - 3.0 * wn;
+            const double rh = 1.0 / (rho_i + rho_j);
+            const double B = b_i + b_j, A = al_i + al_j;
+            const double av = B * A * vs * wn;
+            const double T = pc_i + pc_j - 0.5 * av * rh;
+            const double taI = T * kaI * ri, taJ = T * kaJ * ri;
+            const double Eg = et_i * dWi + et_j * dWj;
+            const double dgI = s.G * mj * ri * Eg, dgJ = s.G * mi * ri * Eg;
+            // reverse
+            const double ad = Ahx * dx + Ahy * dy + Ahz * dz, bd = Bhx * dx + Bhy * dy + Bhz * dz;
+            const double ci = dgI - taI, cj = taJ - dgJ;
+            double ddx = ci * Ahx + cj * Bhx, ddy = ci * Ahy + cj * Bhy, ddz = ci * Ahz + cj * Bhz;
+            const double TbI = -ad * kaI * ri, TbJ = bd * kaJ * ri, Tb = TbI + TbJ;
+            const double DG = s.G * (ad * mj - bd * mi);
+            const double visc = 0.25 * rh * av * wn;
+            const double KB = (Us_i * (pc_i * w - visc) - ad * T * ri) * mj + (Us_j * (pc_j * w - visc) + bd * T * ri) * mi;
+            const double UI = Us_i * kaI, UJ = Us_j * kaJ, UK = UI + UJ;
+            pcb += UI * w + Tb;
+            double wb = UI * pc_i + UJ * pc_j;
+            const double rhb = -av * (0.25 * wn * UK + 0.5 * Tb);
+            const double avb = -rh * (0.25 * wn * UK + 0.5 * Tb);
+            double rib = T * (bd * kaJ - ad * kaI) + DG * Eg;
+            etb += DG * ri * dWi;
+            const double dWib = DG * ri * et_i + KB, dWjb = DG * ri * et_j + KB;
+            const double avw = avb * wn;
+            bb += avw * A * vs;
+            ab += avw * B * vs;
+            const double vsb = avw * B * A;
+            cb += vsb;
+            const double wnb = -0.25 * rh * av * UK + avb * B * A * vs - 3.0 * vsb;
+            if (w < 0.0) wb += wnb;
+            else if (w == 0.0) wb += 0.5 * wnb;
+            const double wr = wb * ri;
+            ddx += wr * ux; ddy += wr * uy; ddz += wr * uz;
+            vb0 += wr * dx; vb1 += wr * dy; vb2 += wr * dz;
+            rib += wb * du;
+            rb -= rhb * rh * rh;
+            // dW = c1 hinv^4 W1(r hinv)
+            hinvb += dWib * CEFF1 * (4.0 * hi3 * w1i + hi4 * w1pi * r);
+            const double rb_ = CEFF1 * (dWib * hi4 * w1pi * hi + dWjb * hj4 * w1pj * hj);
+            const double r2b2 = (rb_ - rib * ri * ri) * ri;   // twice the adjoint of r^2
+            xb0 += ddx + r2b2 * dx;
+            xb1 += ddy + r2b2 * dy;
+            xb2 += ddz + r2b2 * dz;
         }
-        if (act) {
-            for (int c = 0; c < 3; ++c) {
-                atomicAdd(&a.x[3 * i + c], xb[c]);
-                atomicAdd(&a.v[3 * i + c], vb[c]);
-            }
-            atomicAdd(&a.hinv[i], hinvb);
-            atomicAdd(&a.c[i], cb);
-            atomicAdd(&a.rho[i], rb);
-            atomicAdd(&a.b[i], bb);
-            atomicAdd(&a.alph[i], ab);
-            atomicAdd(&a.pc[i], pcb);
-            atomicAdd(&a.eta[i], etb);
+        xb0 = lsum(xb0); xb1 = lsum(xb1); xb2 = lsum(xb2);
+        vb0 = lsum(vb0); vb1 = lsum(vb1); vb2 = lsum(vb2);
+        hinvb = lsum(hinvb); cb = lsum(cb); rb = lsum(rb); bb = lsum(bb);
+        ab = lsum(ab); pcb = lsum(pcb); etb = lsum(etb);
+        if (act && sub == 0) {
+            a.x[3 * i] += xb0; a.x[3 * i + 1] += xb1; a.x[3 * i + 2] += xb2;
+            a.v[3 * i] += vb0; a.v[3 * i + 1] += vb1; a.v[3 * i + 2] += vb2;
+            a.hinv[i] += hinvb;
+            a.c[i] += cb;
+            a.rho[i] += rb;
+            a.b[i] += bb;
+            a.alph[i] += ab;
+            a.pc[i] += pcb;
+            a.eta[i] += etb;
         }
     }
 }
@@ -279,61 +272,84 @@ __global__ void adj_hydro_prep(AdjState s, AdjAcc a) {
 
 // -------------------------------------------------------------- stage D
 // gravity pairs: seeds acc_sum (G acc), pot_sum (G pot), etas
-__global__ void adj_gravity(AdjState s, AdjSeed sd, AdjAcc a, const AdjItem *items, int n_items) {
-    const int lane = threadIdx.x & 31;
-    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
+constexpr int AG_WARPS = 4;
+__global__ void __launch_bounds__(AG_WARPS * 32) adj_gravity(AdjState s, AdjSeed sd, AdjAcc a,
+                                                             const sphk::WorkItem *items, int n_items, int *queue) {
+    __shared__ dbl4 s_x[AG_WARPS][32];
+    __shared__ double s_e[AG_WARPS][32], s_b[AG_WARPS][4][32];
+    __shared__ int s_j[AG_WARPS][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int n = s.n;
-    for (int it = wg; it < n_items; it += nw) {
-        const AdjItem t = items[it];
-        const bool act = lane < t.ni;
-        const int i = t.first + (act ? lane : 0);
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(queue, 1);
+        it = __shfl_sync(FULL, it, 0);
+        if (it >= n_items) return;
+        const sphk::WorkItem t = items[it];
+        const bool act = lane < t.z;
+        const int i = t.y + (act ? lane : 0);
         const dbl4 xi = s.pos[i];
         const double e2i = s.eps2[i];
         const double sc = act ? 1.0 : 0.0;
         const double Cx = s.G * sd.acc[3 * i] * sc, Cy = s.G * sd.acc[3 * i + 1] * sc,
                      Cz = s.G * sd.acc[3 * i + 2] * sc;
-        const double Pb = sd.pot ? s.G * sd.pot[i] * sc : 0.0;
-        const double Eb = a.etas[i] * sc;
+        const double Ph = sd.pot ? 0.5 * s.G * sd.pot[i] * sc : 0.0;
+        const double Eb3 = 3.0 * a.etas[i] * sc;
         double xb0 = 0, xb1 = 0, xb2 = 0, e2b = 0;
-        for (int k = s.g_off[t.walk]; k < s.g_off[t.walk + 1]; ++k) {
-            const int j = s.g_idx[k];
-            const bool node = j >= n;
-            const dbl4 xj = node ? s.mom[j - n] : s.pos[j];
-            const double e2j = node ? s.neps2[j - n] : s.eps2[j];
-            const double mj = xj.w;
-            const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            const double Ri = 1.0 / sqrt(r2 + e2i), Rj = 1.0 / sqrt(r2 + e2j);
-            const double Ri2 = Ri * Ri, Rj2 = Rj * Rj;
-            const double g = 0.5 * mj * (Ri2 * Ri + Rj2 * Rj);
-            const double gb = -(Cx * dx + Cy * dy + Cz * dz);
-            double ddx = -g * Cx, ddy = -g * Cy, ddz = -g * Cz;
-            const double Rib = gb * 1.5 * mj * Ri2 - 0.5 * mj * Pb + 3.0 * mj * Ri2 * Eb;
-            const double Rjb = gb * 1.5 * mj * Rj2 - 0.5 * mj * Pb;
-            const double aib = -0.5 * Rib * Ri2 * Ri, ajb = -0.5 * Rjb * Rj2 * Rj;
-            const double r2b = aib + ajb;
-            ddx += 2.0 * r2b * dx; ddy += 2.0 * r2b * dy; ddz += 2.0 * r2b * dz;
-            xb0 += ddx; xb1 += ddy; xb2 += ddz;
-            e2b += aib;
-            const bool self = !node && j == i;
-            if (self) e2b += ajb;   // eps_j is eps_i
-            const double jxb0 = self ? 0.0 : -ddx, jxb1 = self ? 0.0 : -ddy, jxb2 = self ? 0.0 : -ddz;
-            const double je2b = self ? 0.0 : ajb;
-            if (self) {
-                xb0 -= ddx; xb1 -= ddy; xb2 -= ddz;   // d = 0 identically for the self pair
-            }
-            if (node) {
-                double *nb = a.node + 4 * (size_t)(j - n);
-                wadd(nb + 0, jxb0, lane);
-                wadd(nb + 1, jxb1, lane);
-                wadd(nb + 2, jxb2, lane);
-                wadd(nb + 3, je2b, lane);
+        const int kb = s.g_off[t.x], ke = s.g_off[t.x + 1];
+        for (int k0 = kb; k0 < ke; k0 += 32) {
+            const int m = min(32, ke - k0);
+            __syncwarp();
+            int j = -1;
+            dbl4 xj = make_dbl4(0.0, 0.0, 0.0, 0.0);   // no entry: mass 0, at the origin
+            double e2 = 1.0;
+            if (lane < m) {
+                j = s.g_idx[k0 + lane];
+                xj = j >= n ? s.mom[j - n] : s.pos[j];
+                e2 = j >= n ? s.neps2[j - n] : s.eps2[j];
             } else {
-                wadd(&a.x[3 * j + 0], jxb0, lane);
-                wadd(&a.x[3 * j + 1], jxb1, lane);
-                wadd(&a.x[3 * j + 2], jxb2, lane);
-                wadd(&a.e2[j], je2b, lane);
+                xj.x = xi.x + 1.0; xj.y = xi.y; xj.z = xi.z;
+            }
+            s_x[wid][lane] = xj;
+            s_e[wid][lane] = e2;
+            s_j[wid][lane] = j;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) s_b[wid][c][lane] = 0.0;
+            __syncwarp();
+            // lane l takes entry l + u: the lanes' entries differ, so each
+            // entry's sums have one writer per round
+            for (int u = 0; u < 32; ++u) {
+                const int k = (lane + u) & 31;
+                const dbl4 q = s_x[wid][k];
+                const double dx = xi.x - q.x, dy = xi.y - q.y, dz = xi.z - q.z;
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const double Ri = sphk::rsqrt_r(r2 + e2i), Rj = sphk::rsqrt_r(r2 + s_e[wid][k]);
+                const double Ri2 = Ri * Ri, Rj2 = Rj * Rj;
+                const double Ri3 = Ri2 * Ri, Rj3 = Rj2 * Rj;
+                const double hm = 0.5 * q.w;
+                const double gb3 = -3.0 * (Cx * dx + Cy * dy + Cz * dz);   // 3 x the adjoint of g
+                // adjoints of a = r^2 + eps^2, R = a^(-1/2): -R^3/2 times that of R
+                const double aib = -hm * Ri3 * (0.5 * (gb3 * Ri2) - Ph + Ri2 * Eb3);
+                const double ajb = -0.5 * hm * Rj3 * (gb3 * Rj2 - 2.0 * Ph) ;
+                const double g = hm * (Ri3 + Rj3);
+                const bool self = s_j[wid][k] == i;
+                const double r2b2 = 2.0 * (aib + ajb);
+                const double ddx = self ? 0.0 : r2b2 * dx - g * Cx, ddy = self ? 0.0 : r2b2 * dy - g * Cy;
+                const double ddz = self ? 0.0 : r2b2 * dz - g * Cz;   // d = 0 identically for the self pair
+                xb0 += ddx; xb1 += ddy; xb2 += ddz;
+                e2b += self ? aib + ajb : aib;   // its eps_j is eps_i
+                s_b[wid][0][k] -= ddx;
+                s_b[wid][1][k] -= ddy;
+                s_b[wid][2][k] -= ddz;
+                s_b[wid][3][k] += self ? 0.0 : ajb;
+                __syncwarp();
+            }
+            if (lane < m) {
+                double *x = j >= n ? a.node + 4 * (size_t)(j - n) : a.x + 3 * (size_t)j;
+                double *e = j >= n ? x + 3 : a.e2 + j;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) atomicAdd(x + c, s_b[wid][c][lane]);
+                atomicAdd(e, s_b[wid][3][lane]);
             }
         }
         if (act) {
@@ -387,195 +403,200 @@ __global__ void adj_switch(AdjState s, AdjAcc a) {
 }
 
 // -------------------------------------------------------------- stage G
-// density gradient pass (final h): Omega, divv, rotv -> positions, velocities, h, rho
-__global__ void adj_density_grad(AdjState s, AdjAcc a, const AdjItem *items, int n_items) {
-    const int lane = threadIdx.x & 31;
-    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = wg; it < n_items; it += nw) {
-        const AdjItem t = items[it];
-        const bool act = lane < t.ni;
-        const int i = t.first + (act ? lane : 0);
+// density gradient pass (final h): Omega, divv, rotv -> positions, velocities, h, rho.
+// First each particle's forward sums and the adjoints of them (coef) ...
+__global__ void __launch_bounds__(128) adj_density_sums(AdjState s, AdjAcc a) {
+    const int sub = threadIdx.x & (LANES - 1);
+    ADJ_PARTICLES(ip, s.n) {
+        const bool act = ip < s.n;
+        const int i = act ? ip : s.n - 1;
         const dbl4 xi = s.pos[i], vi = s.vel[i];
         const double h = s.h[i], hinv = 1.0 / h, rho = s.dens[i];
-        const int kb = s.d_off[t.walk], ke = s.d_off[t.walk + 1];
-        // forward sums
-        double Sg = 0, D = 0, Rx = 0, Ry = 0, Rz = 0;
-        for (int k = kb; k < ke; ++k) {
-            const int j = s.d_idx[k];
+        const long long idi = s.id[i];
+        // the particle itself (not in its row): W0(0) = 1, W1(0) = 0
+        double Sg = sub == 0 ? xi.w * 3.0 * CEFF0 : 0.0, D = 0, Rx = 0, Ry = 0, Rz = 0;
+        const Candidates cand(s.h_rows, s.h_info, s.h_off, s.h_idx, i);
+        for (int e = sub; e < (act ? cand.n : 0); e += LANES) {
+            const int j = cand.p[e];
             const dbl4 xj = s.pos[j];
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            if (!(r2 < h * h)) continue;
-            const double r = sqrt(r2), q = r * hinv;
+            if (!(r2 < h * h) || s.id[j] == idi) continue;
+            const double ri = sphk::rsqrt_r(r2), q = r2 * ri * hinv;
             double w0, w0p, w1, w1p;
             wendland(q, w0, w0p, w1, w1p);
             Sg += xj.w * (3.0 * CEFF0 * w0 + CEFF1 * q * w1);
-            if (j == i) continue;
             const dbl4 vj = s.vel[j];
             const double ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
-            const double ph = xj.w * w1 / r;
+            const double ph = xj.w * w1 * ri;
             D += (ux * dx + uy * dy + uz * dz) * ph;
             Rx += (uy * dz - uz * dy) * ph;
             Ry += (uz * dx - ux * dz) * ph;
             Rz += (ux * dy - uy * dx) * ph;
         }
+        Sg = lsum(Sg); D = lsum(D); Rx = lsum(Rx); Ry = lsum(Ry); Rz = lsum(Rz);
+        if (!act || sub != 0) continue;
         const double h4i = hinv * hinv * hinv * hinv;
         const double grdh = -h4i * Sg;
         const double Z = 1.0 + h * grdh / (3.0 * rho);
         const double om = 1.0 / Z;
         const double Rn = sqrt(Rx * Rx + Ry * Ry + Rz * Rz);
-        double hb = 0, rb = 0;
-        const double dvb = act ? a.divv[i] : 0.0, rvb = act ? a.rotv[i] : 0.0;
+        const double dvb = a.divv[i], rvb = a.rotv[i];
         const double Db = dvb * (-CEFF1 * h4i * om / rho);
-        double omb = (act ? a.omega[i] : 0.0) + dvb * (-CEFF1 * h4i * D / rho) + rvb * CEFF1 * h4i * Rn / rho;
-        rb += dvb * CEFF1 * h4i * D * om / (rho * rho) - rvb * CEFF1 * h4i * Rn * om / (rho * rho);
-        hb += dvb * 4.0 * CEFF1 * h4i * hinv * D * om / rho - rvb * 4.0 * CEFF1 * h4i * hinv * Rn * om / rho;
+        const double omb = a.omega[i] + dvb * (-CEFF1 * h4i * D / rho) + rvb * CEFF1 * h4i * Rn / rho;
+        double rb = dvb * CEFF1 * h4i * D * om / (rho * rho) - rvb * CEFF1 * h4i * Rn * om / (rho * rho);
+        double hb = dvb * 4.0 * CEFF1 * h4i * hinv * D * om / rho - rvb * 4.0 * CEFF1 * h4i * hinv * Rn * om / rho;
         const double rs = Rn > 0.0 ? rvb * CEFF1 * h4i * om / rho / Rn : 0.0;
-        const double Rbx = rs * Rx, Rby = rs * Ry, Rbz = rs * Rz;
         const double Zb = -omb * om * om;
         hb += Zb * grdh / (3.0 * rho);
         const double grb = Zb * h / (3.0 * rho);
         rb += -Zb * h * grdh / (3.0 * rho * rho);
-        const double Sgb = -grb * h4i;
         hb += grb * 4.0 * h4i * hinv * Sg;
-        // pairs
-        double xb0 = 0, xb1 = 0, xb2 = 0, vb0 = 0, vb1 = 0, vb2 = 0;
-        for (int k = kb; k < ke; ++k) {
-            const int j = s.d_idx[k];
+        a.h[i] += hb;
+        a.rho[i] += rb;
+        double *c = a.coef + 5 * (size_t)i;
+        c[0] = Db;
+        c[1] = rs * Rx;
+        c[2] = rs * Ry;
+        c[3] = rs * Rz;
+        c[4] = -grb * h4i;   // adjoint of Sg
+    }
+}
+
+// ... then the pairs: what the sums of both ends pass to particle i.  The
+// terms of j's sums have -d and -u, and i stands at their other end: both
+// signs cancel, so the two ends' coefficients add.
+__global__ void __launch_bounds__(128) adj_density_grad(AdjState s, AdjAcc a) {
+    const int sub = threadIdx.x & (LANES - 1);
+    ADJ_PARTICLES(ip, s.n) {
+        const bool act = ip < s.n;
+        const int i = act ? ip : s.n - 1;
+        const dbl4 xi = s.pos[i], vi = s.vel[i];
+        const double hi_len = s.h[i], hi = 1.0 / hi_len;
+        const long long idi = s.id[i];
+        const double *c = a.coef + 5 * (size_t)i;
+        const double Dbi = c[0], Rxi = c[1], Ryi = c[2], Rzi = c[3], Sgi = c[4];
+        double hb = 0, xb0 = 0, xb1 = 0, xb2 = 0, vb0 = 0, vb1 = 0, vb2 = 0;
+        const Candidates cand(s.h_rows, s.h_info, s.h_off, s.h_idx, i);
+        for (int e = sub; e < (act ? cand.n : 0); e += LANES) {
+            const int j = cand.p[e];
             const dbl4 xj = s.pos[j];
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const bool in = act && j != i && r2 < h * h;
-            double jx0 = 0, jx1 = 0, jx2 = 0, jv0 = 0, jv1 = 0, jv2 = 0;
-            if (in) {
-                const dbl4 vj = s.vel[j];
-                const double ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
-                const double r = sqrt(r2), ri = 1.0 / r, q = r * hinv;
+            const double hj_len = s.h[j];
+            const double hm = fmax(hi_len, hj_len);
+            if (!(r2 < hm * hm) || s.id[j] == idi) continue;
+            const dbl4 vj = s.vel[j];
+            const double ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
+            const double ri = sphk::rsqrt_r(r2), r = r2 * ri;
+            const double ud = ux * dx + uy * dy + uz * dz;
+            const double cx = uy * dz - uz * dy, cy = uz * dx - ux * dz, cz = ux * dy - uy * dx;
+            double P = 0, Qx = 0, Qy = 0, Qz = 0, r2b2 = 0;   // r2b2: twice the adjoint of r^2
+            // one end's sums: coefficients, 1/h, the other end's mass
+            auto end = [&](double Db, double Rx, double Ry, double Rz, double Sg, double hinv, double m) -> double {
+                const double q = r * hinv;
                 double w0, w0p, w1, w1p;
                 wendland(q, w0, w0p, w1, w1p);
-                const double m = xj.w;
                 const double ph = m * w1 * ri;
-                double qb = Sgb * m * (3.0 * CEFF0 * w0p + CEFF1 * (w1 + q * w1p));
-                const double ud = ux * dx + uy * dy + uz * dz;
-                // D: (u.d) ph
-                double ubx = Db * ph * dx, uby = Db * ph * dy, ubz = Db * ph * dz;
-                double ddx = Db * ph * ux, ddy = Db * ph * uy, ddz = Db * ph * uz;
-                double phb = Db * ud;
-                // R: (u x d) ph
-                const double cx = uy * dz - uz * dy, cy = uz * dx - ux * dz, cz = ux * dy - uy * dx;
-                ubx += ph * (dy * Rbz - dz * Rby);
-                uby += ph * (dz * Rbx - dx * Rbz);
-                ubz += ph * (dx * Rby - dy * Rbx);
-                ddx += ph * (Rby * uz - Rbz * uy);
-                ddy += ph * (Rbz * ux - Rbx * uz);
-                ddz += ph * (Rbx * uy - Rby * ux);
-                phb += Rbx * cx + Rby * cy + Rbz * cz;
-                qb += phb * m * w1p * ri;
-                const double rib = phb * m * w1;
-                const double rbar = qb * hinv;
-                hb += -qb * r * hinv * hinv;
-                const double r2b = 0.5 * rbar * ri - 0.5 * rib * ri * ri * ri;
-                ddx += 2.0 * r2b * dx; ddy += 2.0 * r2b * dy; ddz += 2.0 * r2b * dz;
-                xb0 += ddx; xb1 += ddy; xb2 += ddz;
-                vb0 += ubx; vb1 += uby; vb2 += ubz;
-                jx0 = -ddx; jx1 = -ddy; jx2 = -ddz;
-                jv0 = -ubx; jv1 = -uby; jv2 = -ubz;
+                P += Db * ph;
+                Qx += ph * Rx; Qy += ph * Ry; Qz += ph * Rz;
+                const double phb = Db * ud + Rx * cx + Ry * cy + Rz * cz;
+                const double qb = m * (Sg * (3.0 * CEFF0 * w0p + CEFF1 * (w1 + q * w1p)) + phb * w1p * ri);
+                r2b2 += (qb * hinv - phb * m * w1 * ri * ri) * ri;
+                return qb;
+            };
+            if (r2 < hi_len * hi_len) hb -= end(Dbi, Rxi, Ryi, Rzi, Sgi, hi, xj.w) * r * hi * hi;
+            if (r2 < hj_len * hj_len) {
+                const double *cj = a.coef + 5 * (size_t)j;
+                end(cj[0], cj[1], cj[2], cj[3], cj[4], 1.0 / hj_len, xi.w);
             }
-            if (__any_sync(FULL, in)) {
-                wadd(&a.x[3 * j + 0], jx0, lane);
-                wadd(&a.x[3 * j + 1], jx1, lane);
-                wadd(&a.x[3 * j + 2], jx2, lane);
-                wadd(&a.v[3 * j + 0], jv0, lane);
-                wadd(&a.v[3 * j + 1], jv1, lane);
-                wadd(&a.v[3 * j + 2], jv2, lane);
-            }
+            vb0 += P * dx + dy * Qz - dz * Qy;
+            vb1 += P * dy + dz * Qx - dx * Qz;
+            vb2 += P * dz + dx * Qy - dy * Qx;
+            xb0 += P * ux + Qy * uz - Qz * uy + r2b2 * dx;
+            xb1 += P * uy + Qz * ux - Qx * uz + r2b2 * dy;
+            xb2 += P * uz + Qx * uy - Qy * ux + r2b2 * dz;
         }
-        if (act) {
-            atomicAdd(&a.x[3 * i + 0], xb0);
-            atomicAdd(&a.x[3 * i + 1], xb1);
-            atomicAdd(&a.x[3 * i + 2], xb2);
-            atomicAdd(&a.v[3 * i + 0], vb0);
-            atomicAdd(&a.v[3 * i + 1], vb1);
-            atomicAdd(&a.v[3 * i + 2], vb2);
-            atomicAdd(&a.h[i], hb);
-            atomicAdd(&a.rho[i], rb);
+        hb = lsum(hb);
+        xb0 = lsum(xb0); xb1 = lsum(xb1); xb2 = lsum(xb2);
+        vb0 = lsum(vb0); vb1 = lsum(vb1); vb2 = lsum(vb2);
+        if (act && sub == 0) {
+            a.x[3 * i] += xb0; a.x[3 * i + 1] += xb1; a.x[3 * i + 2] += xb2;
+            a.v[3 * i] += vb0; a.v[3 * i + 1] += vb1; a.v[3 * i + 2] += vb2;
+            a.h[i] += hb;
         }
     }
 }
 
 // -------------------------------------------------------------- stage H
 // the three smoothing-length passes: (rho_2, h_3) -> positions, first guess h_0
-__global__ void adj_density_passes(AdjState s, AdjAcc a, const AdjItem *items, int n_items) {
-    const int lane = threadIdx.x & 31;
-    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = wg; it < n_items; it += nw) {
-        const AdjItem t = items[it];
-        const bool act = lane < t.ni;
-        const int i = t.first + (act ? lane : 0);
+__global__ void __launch_bounds__(128) adj_density_passes(AdjState s, AdjAcc a) {
+    const int sub = threadIdx.x & (LANES - 1);
+    ADJ_PARTICLES(ip, s.n) {
+        const bool act = ip < s.n;
+        const int i = act ? ip : s.n - 1;
         const dbl4 xi = s.pos[i];
-        const int kb = s.d_off[t.walk], ke = s.d_off[t.walk + 1];
+        Candidates cand(s.d_rows, s.d_info, s.d_off, s.d_idx, i);
         // forward: h_k, rho_k and S'_k = sum m q W0'(q) per pass
         double hk[4], rk[3], sp[3];
         hk[0] = s.h0[i];
+        const double h_row = hk[0] * s.slack * 0.99998;
         for (int p = 0; p < 3; ++p) {
+            if (p > 0 && hk[p] > h_row) {   // beyond the row: the walk's list
+                const int w = s.d_info[i].y;
+                cand.p = s.d_idx + s.d_off[w];
+                cand.n = s.d_off[w + 1] - s.d_off[w];
+            }
             const double hinv = 1.0 / hk[p];
             double S0 = 0, S1 = 0;
-            for (int k = kb; k < ke; ++k) {
-                const int j = s.d_idx[k];
-                const dbl4 xj = s.pos[j];
+            for (int e = sub; e < cand.n; e += LANES) {
+                const dbl4 xj = s.pos[cand.p[e]];
                 const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
                 const double r2 = dx * dx + dy * dy + dz * dz;
                 if (!(r2 < hk[p] * hk[p])) continue;
-                const double q = sqrt(r2) * hinv;
+                const double q = sphk::sqrt_r(r2) * hinv;
                 double w0, w0p, w1, w1p;
                 wendland(q, w0, w0p, w1, w1p);
                 S0 += xj.w * w0;
                 S1 += xj.w * q * w0p;
             }
+            S0 = lsum(S0);
+            sp[p] = lsum(S1);
             rk[p] = CEFF0 * hinv * hinv * hinv * S0;
-            sp[p] = S1;
             hk[p + 1] = s.eta_ksrh * cbrt(xi.w / rk[p]);
         }
         // reverse over the scalars
-        double rhob[3], hb[4];
+        double rhob[3], hb[4], fk[3];
         hb[3] = act ? a.h[i] : 0.0;
         rhob[2] = (act ? a.rho[i] : 0.0) + hb[3] * (-hk[3] / (3.0 * rk[2]));
         for (int p = 2; p >= 0; --p) {
-            const double hinv = 1.0 / hk[p];
+            const double hinv = 1.0 / hk[p], hinv4 = hinv * hinv * hinv * hinv;
             // rho = c0 h^-3 S0(h): d rho/d h = -3 rho/h - c0 h^-4 sum m q W0'(q)
-            hb[p] = rhob[p] * (-3.0 * rk[p] * hinv - CEFF0 * hinv * hinv * hinv * hinv * sp[p]);
+            hb[p] = rhob[p] * (-3.0 * rk[p] * hinv - CEFF0 * hinv4 * sp[p]);
             if (p > 0) rhob[p - 1] = hb[p] * (-hk[p] / (3.0 * rk[p - 1]));
+            // d rho_k / d r = c0 h_k^-4 m W0'(q_k), W0'(q) = -20 q (1 - q)^3
+            fk[p] = -20.0 * CEFF0 * rhob[p] * hinv4 * hinv;
         }
-        // pairs: d rho_k / d r = c0 h_k^-4 m W0'(q_k)
+        // pairs: r-bar / r, times d for the separation
         double xb0 = 0, xb1 = 0, xb2 = 0;
         const double hmx = fmax(fmax(hk[0], hk[1]), hk[2]);
-        for (int k = kb; k < ke; ++k) {
-            const int j = s.d_idx[k];
+        const double hi0 = 1.0 / hk[0], hi1 = 1.0 / hk[1], hi2 = 1.0 / hk[2];
+        for (int e = sub; e < (act ? cand.n : 0); e += LANES) {
+            const int j = cand.p[e];
             const dbl4 xj = s.pos[j];
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const bool in = act && j != i && r2 < hmx * hmx;
-            double f = 0.0;
-            if (in) {
-                const double r = sqrt(r2), ri = 1.0 / r;
-                for (int p = 0; p < 3; ++p) {
-                    const double hinv = 1.0 / hk[p];
-                    double w0, w0p, w1, w1p;
-                    wendland(r * hinv, w0, w0p, w1, w1p);
-                    f += rhob[p] * CEFF0 * hinv * hinv * hinv * hinv * xj.w * w0p;
-                }
-                f *= ri;   // r-bar / r, times d for the separation
-                xb0 += f * dx; xb1 += f * dy; xb2 += f * dz;
-            }
-            if (__any_sync(FULL, in)) {
-                wadd(&a.x[3 * j + 0], -f * dx, lane);
-                wadd(&a.x[3 * j + 1], -f * dy, lane);
-                wadd(&a.x[3 * j + 2], -f * dz, lane);
-            }
+            if (j == i || !(r2 < hmx * hmx)) continue;
+            const double r = sphk::sqrt_r(r2);
+            const double u0 = sphk::max0(1.0 - r * hi0), u1 = sphk::max0(1.0 - r * hi1), u2 = sphk::max0(1.0 - r * hi2);
+            const double f = xj.w * (fk[0] * (u0 * u0 * u0) + fk[1] * (u1 * u1 * u1) + fk[2] * (u2 * u2 * u2));
+            xb0 += f * dx; xb1 += f * dy; xb2 += f * dz;
+            atomicAdd(&a.x[3 * j + 0], -f * dx);
+            atomicAdd(&a.x[3 * j + 1], -f * dy);
+            atomicAdd(&a.x[3 * j + 2], -f * dz);
         }
-        if (act) {
+        xb0 = lsum(xb0); xb1 = lsum(xb1); xb2 = lsum(xb2);
+        if (act && sub == 0) {
             atomicAdd(&a.x[3 * i + 0], xb0);
             atomicAdd(&a.x[3 * i + 1], xb1);
             atomicAdd(&a.x[3 * i + 2], xb2);
@@ -583,6 +604,7 @@ __global__ void adj_density_passes(AdjState s, AdjAcc a, const AdjItem *items, i
         }
     }
 }
+#undef ADJ_PARTICLES
 
 // work items: one per 32 i-particles of a group (offsets from an exclusive
 // scan of the per-group counts)
@@ -590,16 +612,12 @@ __global__ void adj_item_counts(int n_groups, const int *gcount, int *cnt) {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n_groups; g += gridDim.x * blockDim.x)
         cnt[g] = (gcount[g] + 31) / 32;
 }
-__global__ void adj_fill_items(int n_groups, const int *gfirst, const int *gcount, const int *off, AdjItem *items) {
+__global__ void adj_fill_items(int n_groups, const int *gfirst, const int *gcount, const int *off,
+                               sphk::WorkItem *items) {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n_groups; g += gridDim.x * blockDim.x) {
         const int c = gcount[g];
-        for (int k = 0; 32 * k < c; ++k) {
-            AdjItem t;
-            t.walk = g;
-            t.first = gfirst[g] + 32 * k;
-            t.ni = min(32, c - 32 * k);
-            items[off[g] + k] = t;
-        }
+        for (int k = 0; 32 * k < c; ++k)
+            items[off[g] + k] = make_int4(g, gfirst[g] + 32 * k, min(32, c - 32 * k), 0);
     }
 }
 

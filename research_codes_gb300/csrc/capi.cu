@@ -132,11 +132,16 @@ static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs 
     recheck_density(ctx, a, n_max, s, amb_total);
 }
 
+// Density rows of the items of m.
+void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s) {
+    sphk::mark_rows<sphk::ROWS_DENSITY, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
+    mark_long<sphk::ROWS_DENSITY>(ctx, m, n_max, s);
+}
+
 // Rows of the items of m, then the density sums over them.
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
                     int n_max, int precision, cudaStream_t s, int *amb_total) {
-    sphk::mark_rows<sphk::ROWS_DENSITY, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-    mark_long<sphk::ROWS_DENSITY>(ctx, m, n_max, s);
+    launch_mark_density(ctx, m, mark_grid, n_max, s);
     launch_density_sums(ctx, a, n_max, precision, s, amb_total);
 }
 

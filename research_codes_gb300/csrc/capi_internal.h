@@ -174,6 +174,7 @@ extern const float AMB_TOL;
 int set_error(sph_context *ctx, int status, const char *fmt, ...);
 int cuda_error(sph_context *ctx, cudaError_t e, const char *what);
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items);
+void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s);
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
                     int n_max, int precision, cudaStream_t s, int *amb_total = nullptr);
 void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,

@@ -108,12 +108,6 @@ __device__ __forceinline__ double lane_total(const Acc<true> &a) {
     return seg_sum(a.s, L);
 }
 
-__device__ __forceinline__ float sqrt_r(float x) {
-    float y;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
 __device__ __forceinline__ float cbrt_r(float x) { return cbrtf(x); }
 __device__ __forceinline__ double cbrt_r(double x) { return cbrt(x); }
 

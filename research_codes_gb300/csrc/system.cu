@@ -1007,8 +1007,9 @@ struct sph_system {
     DevBuf<double> h_guess;  // first guess of h of the last density evaluation
     // adjoint scratch, allocated on first use: accumulators, seeds, items
     DevBuf<double> adj_acc, adj_seed;
-    DevBuf<sphadj::AdjItem> adj_items;
-    DevBuf<int> adj_cnt, adj_off;
+    DevBuf<WorkItem> adj_items;
+    DevBuf<int> adj_cnt, adj_off, adj_rows;
+    DevBuf<int2> adj_info;
     // graph
     cudaGraphExec_t step_exec = nullptr;
     bool graph_valid = false;
@@ -2028,7 +2029,7 @@ extern "C" int sph_system_destroy(sph_system *s) {
     s->lscal.release(); s->an_buf.release();
     s->h_scal.release(); s->h_dscal.release(); s->h_lscal.release();
     s->h_guess.release(); s->adj_acc.release(); s->adj_seed.release(); s->adj_items.release();
-    s->adj_cnt.release(); s->adj_off.release();
+    s->adj_cnt.release(); s->adj_off.release(); s->adj_rows.release(); s->adj_info.release();
     s->ctx->n_systems--;
     delete s;
     return SPH_OK;
@@ -2642,9 +2643,10 @@ extern "C" int sph_system_adjoint_forces(sph_system *s, const double *seed, doub
                                 "the derivative needs a force evaluation with one density walk (got %d)", sc[S_ITERS]);
     const int ng = sc[S_NGROUPS];
     // scratch
-    const int NA = 26;   // doubles per particle in the accumulators (+ 4 per node, 2n nodes)
+    const int NA = 27;   // doubles per particle in the accumulators (+ 4 per node, 2n nodes)
     int e = s->adj_acc.ensure((size_t)NA * n + 8 * (size_t)n) | s->adj_seed.ensure(8 * (size_t)n + 9 * (size_t)n);
     e |= s->adj_cnt.ensure(n + 1) | s->adj_off.ensure(n + 1);
+    e |= s->adj_rows.ensure((size_t)n * sphk::ROW_CAP) | s->adj_info.ensure(n);
     if (e) return sphrt::set_error(ctx, SPH_ERR_CUDA, "adjoint scratch allocation failed");
     CUDA_TRY(cudaMemsetAsync(s->adj_acc.p, 0, sizeof(double) * ((size_t)NA * n + 8 * (size_t)n), st));
     // items: one warp per 32 particles of a group
@@ -2675,6 +2677,7 @@ extern "C" int sph_system_adjoint_forces(sph_system *s, const double *seed, doub
     acc.h = slot(9); acc.rho = slot(10); acc.omega = slot(11); acc.divv = slot(12); acc.rotv = slot(13);
     acc.c = slot(14); acc.b = slot(15); acc.pc = slot(16); acc.eta = slot(17); acc.e2 = slot(18);
     acc.hinv = slot(19); acc.etas = slot(20); acc.bswt = slot(21);
+    acc.coef = slot(22);   // 5 per particle
     acc.node = slot(NA);   // 8n doubles: 4 per node
     sphadj::AdjState as;
     as.n = n;
@@ -2686,15 +2689,34 @@ extern "C" int sph_system_adjoint_forces(sph_system *s, const double *seed, doub
     as.d_off = s->loff[0].p; as.d_idx = s->jidx[0].p; as.h_off = s->loff[1].p; as.h_idx = s->jidx[1].p;
     as.g_off = s->loff[2].p; as.g_idx = s->jidx[2].p;
     as.G = s->prm.G; as.amax = s->prm.alpha_max; as.amin = s->prm.alpha_min; as.eta_ksrh = ctx->prm.eta * KSRH;
-    const int eg = grid_for(n), wg = ctx->sm_count * 8;
+    as.h_rows = s->hl_list.p; as.h_info = s->r_info.p; as.d_rows = s->adj_rows.p; as.d_info = s->adj_info.p;
+    as.id = s->id[0].p;
+    as.slack = (double)NBR_SLACK;
+    // rows of the h passes: every j within the slack of the first guess
+    sphk::make_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->h_guess.p, s->f_phi.p, s->f_plo.p);
+    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
+    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_DOVF, 0, 2 * sizeof(int), st));   // queue of the rowless, long items
+    sphk::MarkArgs m{};
+    m.i_hi = s->f_phi.p; m.i_lo = s->f_plo.p; m.j_hi = m.i_hi; m.j_lo = m.i_lo;
+    m.slack = NBR_SLACK;
+    m.items = s->adj_items.p; m.n_items = n_items;
+    m.j_off = as.d_off; m.j_idx = as.d_idx; m.queue = s->scal.p + S_QUEUE;
+    m.rows = s->adj_rows.p; m.info = s->adj_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
+    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG; m.pairs = s->lscal.p + L_PAIRS_D1;
+    sphrt::launch_mark_density(ctx, m, sphrt::pair_grid(ctx, 0, SPH_PREC_FP64, n_items), n, st);
+    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
+    const int eg = grid_for(n), rg = std::min(grid_for(8LL * n, 128), 16 * ctx->sm_count);
+    const int gg = std::min((n_items + sphadj::AG_WARPS - 1) / sphadj::AG_WARPS, ctx->sm_count * 8);
     sphadj::adj_alpha<<<eg, 256, 0, st>>>(as, sed, acc);
-    sphadj::adj_hydro<<<wg, 128, 0, st>>>(as, sed, acc, s->adj_items.p, n_items);
+    sphadj::adj_hydro<<<rg, 128, 0, st>>>(as, sed, acc);
     sphadj::adj_hydro_prep<<<eg, 256, 0, st>>>(as, acc);
-    sphadj::adj_gravity<<<wg, 128, 0, st>>>(as, sed, acc, s->adj_items.p, n_items);
+    sphadj::adj_gravity<<<gg, sphadj::AG_WARPS * 32, 0, st>>>(as, sed, acc, s->adj_items.p, n_items,
+                                                             s->scal.p + S_QUEUE);
     sphadj::adj_nodes<<<eg, 256, 0, st>>>(as, acc);
     sphadj::adj_switch<<<eg, 256, 0, st>>>(as, acc);
-    sphadj::adj_density_grad<<<wg, 128, 0, st>>>(as, acc, s->adj_items.p, n_items);
-    sphadj::adj_density_passes<<<wg, 128, 0, st>>>(as, acc, s->adj_items.p, n_items);
+    sphadj::adj_density_sums<<<rg, 128, 0, st>>>(as, acc);
+    sphadj::adj_density_grad<<<rg, 128, 0, st>>>(as, acc);
+    sphadj::adj_density_passes<<<rg, 128, 0, st>>>(as, acc);
     // results: sorted -> upload order
     double *out = s->adj_seed.p;   // 9n doubles (the seeds are consumed)
     scatter_field<<<grid_for(n), 256, 0, st>>>(n, 3, s->orig[0].p, acc.x, out);
