@@ -257,7 +257,7 @@ int sph_calc_gravity_sp(sph_context *ctx,
  * queued on `stream` (a cudaStream_t, NULL = default stream) and the call
  * returns without waiting.  FP32C arithmetic; forces ACCUMULATE like the
  * reference functor.  Scratch lives in one file-scope __device__ array of the
- * library (~2.4 MB, held by every GPU that loads the library until the process
+ * library (~6.2 MB, held by every GPU that loads the library until the process
  * exits), which bounds a call to n_i <= SPH_NOALLOC_MAX_I and
  * n_j <= SPH_NOALLOC_MAX_J (larger calls return SPH_ERR_CAPACITY).  Every call
  * looks up the array's device address with the caller's device current

@@ -272,7 +272,7 @@ __global__ void adj_hydro_prep(AdjState s, AdjAcc a) {
 
 // -------------------------------------------------------------- stage D
 // gravity pairs: seeds acc_sum (G acc), pot_sum (G pot), etas
-constexpr int AG_WARPS = 4;
+constexpr int AG_WARPS = 4, AG_PARTS = 4;
 __global__ void __launch_bounds__(AG_WARPS * 32) adj_gravity(AdjState s, AdjSeed sd, AdjAcc a,
                                                              const sphk::WorkItem *items, int n_items, int *queue) {
     __shared__ dbl4 s_x[AG_WARPS][32];
@@ -284,10 +284,14 @@ __global__ void __launch_bounds__(AG_WARPS * 32) adj_gravity(AdjState s, AdjSeed
         int it = 0;
         if (lane == 0) it = atomicAdd(queue, 1);
         it = __shfl_sync(FULL, it, 0);
-        if (it >= n_items) return;
-        const sphk::WorkItem t = items[it];
-        const bool act = lane < t.z;
-        const int i = t.y + (act ? lane : 0);
+        if (it >= n_items * AG_PARTS) return;
+        // a quarter of an item's list per turn
+        const sphk::WorkItem t = items[it / AG_PARTS];
+        const int part = it % AG_PARTS;
+        const int tpi = sphk::lanes_per_i(t.z);
+        const int li = lane / tpi;
+        const bool act = li < t.z;
+        const int i = t.y + (act ? li : 0);
         const dbl4 xi = s.pos[i];
         const double e2i = s.eps2[i];
         const double sc = act ? 1.0 : 0.0;
@@ -296,8 +300,9 @@ __global__ void __launch_bounds__(AG_WARPS * 32) adj_gravity(AdjState s, AdjSeed
         const double Ph = sd.pot ? 0.5 * s.G * sd.pot[i] * sc : 0.0;
         const double Eb3 = 3.0 * a.etas[i] * sc;
         double xb0 = 0, xb1 = 0, xb2 = 0, e2b = 0;
-        const int kb = s.g_off[t.x], ke = s.g_off[t.x + 1];
-        for (int k0 = kb; k0 < ke; k0 += 32) {
+        const int kb = s.g_off[t.x], tiles = (s.g_off[t.x + 1] - kb + 31) / 32;
+        const int ke = min(s.g_off[t.x + 1], kb + 32 * (tiles * (part + 1) / AG_PARTS));
+        for (int k0 = kb + 32 * (tiles * part / AG_PARTS); k0 < ke; k0 += 32) {
             const int m = min(32, ke - k0);
             __syncwarp();
             int j = -1;
@@ -317,8 +322,9 @@ __global__ void __launch_bounds__(AG_WARPS * 32) adj_gravity(AdjState s, AdjSeed
             for (int c = 0; c < 4; ++c) s_b[wid][c][lane] = 0.0;
             __syncwarp();
             // lane l takes entry l + u: the lanes' entries differ, so each
-            // entry's sums have one writer per round
-            for (int u = 0; u < 32; ++u) {
+            // entry's sums have one writer per round (and the tpi lanes of a
+            // particle take the entries of their own residue)
+            for (int u = 0; u < 32; u += tpi) {
                 const int k = (lane + u) & 31;
                 const dbl4 q = s_x[wid][k];
                 const double dx = xi.x - q.x, dy = xi.y - q.y, dz = xi.z - q.z;

@@ -300,13 +300,19 @@ __global__ void pack_hydro(int n, const double *acch, const double *accg, const 
     }
 }
 
-__global__ void pack_gravity(int n, const double *acc, const double *pot, const double *eta,
+// One warp per particle, over the parts of its list.
+__global__ void pack_gravity(int n, const double *acc, const double *pot, const double *eta, int slices,
                              sph_Gravity *out, int *flag) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += nw) {
+        double v[5];
+        sphk::gravity_gather_warp(acc, pot, eta, k, slices, n, lane, v);
+        if (lane != 0) continue;
         sph_Gravity g;
-        for (int c = 0; c < 3; ++c) g.acc[c] = acc[3 * k + c];
-        g.pot = pot[k];
-        g.eta = eta[k];
+        for (int c = 0; c < 3; ++c) g.acc[c] = v[c];
+        g.pot = v[3];
+        g.eta = v[4];
         out[k] = g;
         if (!(finite3(g.acc[0], g.acc[1], g.acc[2]) && finite3(g.pot, g.eta, 0.0))) atomicOr(flag, 1);
     }
@@ -877,7 +883,9 @@ extern "C" int sph_dispatch_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
         if (ns) std::memcpy(jdst + sizeof(sph_GravityEPJ) * n_epj[w], spj[w], sizeof(sph_GravitySPJ) * ns);
     }
     const int ni = i_off[n_walk], nj = j_off[n_walk];
-    if (ks.ensure_gravity(ni, nj)) return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
+    const int slices = sphk::gravity_slices((long long)ks.items.size(), nj / std::max(n_walk, 1),
+                                            2LL * resident_warps(ctx), 512);
+    if (ks.ensure_gravity(ni, nj, slices)) return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Gravity) * (size_t)std::max(ni, 1)) ||
         ks.d_out.ensure(sizeof(sph_Gravity) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
@@ -911,11 +919,15 @@ extern "C" int sph_dispatch_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
         a.queue = ctx->d_queue + K_GRAV;
         a.o_acc = ks.o[0].p; a.o_pot = ks.o[1].p; a.o_eta = ks.o[2].p;
         a.s_quad = nullptr; a.f_sq0 = nullptr; a.f_sq1 = nullptr;   // SPJ are monopoles
-        launch_gravity(a, ctx->prm.precision, pair_grid(ctx, K_GRAV, ctx->prm.precision, a.n_items), ctx->stream, 32);
+        a.slices = slices;
+        a.o_stride = ni;
+        launch_gravity(a, ctx->prm.precision, pair_grid(ctx, K_GRAV, ctx->prm.precision, a.n_items * slices),
+                       ctx->stream, 32);
     }
     if (ni > 0)
-        pack_gravity<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.o[0].p, ks.o[1].p, ks.o[2].p,
-                                                               (sph_Gravity *)ks.d_out.p, ctx->d_queue + 4 + K_GRAV);
+        pack_gravity<<<eltwise_grid(32LL * ni), 256, 0, ctx->stream>>>(ni, ks.o[0].p, ks.o[1].p, ks.o[2].p, slices,
+                                                                      (sph_Gravity *)ks.d_out.p,
+                                                                      ctx->d_queue + 4 + K_GRAV);
     return finish_dispatch(ctx, ks, n_walk, i_off, sizeof(sph_Gravity));
 }
 

@@ -122,10 +122,10 @@ struct KindState {
         e |= hl_list.ensure(ni * sphk::ROW_CAP) | r_info.ensure(ni) | hl_ovf.ensure(ni);
         return e;
     }
-    int ensure_gravity(size_t ni, size_t nj) {
+    int ensure_gravity(size_t ni, size_t nj, size_t slices) {
         int e = 0;
         e |= a4[0].ensure(ni) | a4[2].ensure(nj) | d1[0].ensure(nj);
-        e |= o[0].ensure(3 * ni) | o[1].ensure(ni) | o[2].ensure(ni);
+        e |= o[0].ensure(3 * ni * slices) | o[1].ensure(ni * slices) | o[2].ensure(ni * slices);
         e |= f4[0].ensure(ni) | f4[1].ensure(ni) | f4[4].ensure(nj) | f4[5].ensure(nj);
         return e;
     }

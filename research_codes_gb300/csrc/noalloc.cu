@@ -13,7 +13,7 @@
 // one file-scope __device__ array, so it allocates nothing.
 //
 // The array is part of the library's device image: every GPU that loads the
-// library holds it (about 2.4 MB) until the process exits.  Its size bounds a
+// library holds it (about 6.2 MB) until the process exits.  Its size bounds a
 // call to n_i <= SPH_NOALLOC_MAX_I and n_j <= SPH_NOALLOC_MAX_J.  Every call
 // shares it and it keeps the last call's contents; the call clears the
 // work-queue counter itself before the kernels use it.  Calls that overlap on
@@ -37,6 +37,10 @@ constexpr int MAX_I = SPH_NOALLOC_MAX_I;
 constexpr int MAX_J = SPH_NOALLOC_MAX_J;
 constexpr int NOALLOC_WARPS = 4;
 constexpr int MAX_ITEMS = (MAX_I + 31) / 32;
+// Results of the parts of the lists: a call of n_i particles takes at most
+// MAX_PART / n_i parts, as many as give every resident warp (~2400) a unit.
+constexpr int MAX_PART = 98304;
+constexpr int UNITS = 4864;
 
 // Layout of the scratch array (byte offsets, each 256-byte aligned).
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -45,9 +49,9 @@ constexpr size_t OFF_FI_LO = align256(OFF_FI_HI + sizeof(float4) * MAX_I);
 constexpr size_t OFF_FJ_HI = align256(OFF_FI_LO + sizeof(float4) * MAX_I);
 constexpr size_t OFF_FJ_LO = align256(OFF_FJ_HI + sizeof(float4) * MAX_J);
 constexpr size_t OFF_ACC = align256(OFF_FJ_LO + sizeof(float4) * MAX_J);
-constexpr size_t OFF_POT = align256(OFF_ACC + sizeof(double) * 3 * MAX_I);
-constexpr size_t OFF_ETA = align256(OFF_POT + sizeof(double) * MAX_I);
-constexpr size_t OFF_ITEMS = align256(OFF_ETA + sizeof(double) * MAX_I);
+constexpr size_t OFF_POT = align256(OFF_ACC + sizeof(double) * 3 * MAX_PART);
+constexpr size_t OFF_ETA = align256(OFF_POT + sizeof(double) * MAX_PART);
+constexpr size_t OFF_ITEMS = align256(OFF_ETA + sizeof(double) * MAX_PART);
 constexpr size_t OFF_JOFF = align256(OFF_ITEMS + sizeof(sphk::WorkItem) * MAX_ITEMS);
 constexpr size_t OFF_QUEUE = align256(OFF_JOFF + sizeof(int) * 2);
 constexpr size_t SCRATCH_BYTES = align256(OFF_QUEUE + sizeof(int));
@@ -89,20 +93,25 @@ __global__ void noalloc_prepare(const sph_GravityEPI *epi, int ni, const sph_Gra
     }
 }
 
-// force[k] += result[k] (calcGravity accumulates, hdr_gravity.hpp:333-337)
-__global__ void noalloc_accumulate(int ni, const unsigned char *scr, sph_Gravity *force) {
+// force[k] += result[k] (calcGravity accumulates, hdr_gravity.hpp:333-337); one
+// warp per particle, over the parts of its list
+__global__ void noalloc_accumulate(int ni, int slices, const unsigned char *scr, sph_Gravity *force) {
     const double *acc = reinterpret_cast<const double *>(scr + OFF_ACC);
     const double *pot = reinterpret_cast<const double *>(scr + OFF_POT);
     const double *eta = reinterpret_cast<const double *>(scr + OFF_ETA);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ni; k += gridDim.x * blockDim.x) {
-        sph_Gravity f = force[k];
-        f.acc[0] += acc[3 * k];
-        f.acc[1] += acc[3 * k + 1];
-        f.acc[2] += acc[3 * k + 2];
-        f.pot += pot[k];
-        f.eta += eta[k];
-        force[k] = f;
-    }
+    const int lane = threadIdx.x & 31;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= ni) return;
+    double g[5];
+    sphk::gravity_gather_warp(acc, pot, eta, k, slices, ni, lane, g);
+    if (lane != 0) return;
+    sph_Gravity f = force[k];
+    f.acc[0] += g[0];
+    f.acc[1] += g[1];
+    f.acc[2] += g[2];
+    f.pot += g[3];
+    f.eta += g[4];
+    force[k] = f;
 }
 
 // Device address of g_noalloc_scratch on the current device.
@@ -154,9 +163,11 @@ extern "C" int sph_calc_gravity_ep_noalloc(const sph_GravityEPI *epi, int32_t n_
     a.o_acc = reinterpret_cast<double *>(scr + OFF_ACC);
     a.o_pot = reinterpret_cast<double *>(scr + OFF_POT);
     a.o_eta = reinterpret_cast<double *>(scr + OFF_ETA);
-    const int blocks = (a.n_items + NOALLOC_WARPS - 1) / NOALLOC_WARPS;
+    a.slices = sphk::gravity_slices(a.n_items, n_j, UNITS, MAX_PART / n_i);
+    a.o_stride = n_i;
+    const int blocks = (a.n_items * a.slices + NOALLOC_WARPS - 1) / NOALLOC_WARPS;
     sphk::gravity_kernel<false, NOALLOC_WARPS><<<blocks, NOALLOC_WARPS * 32, 0, s>>>(a);
     if (cudaGetLastError() != cudaSuccess) return SPH_ERR_CUDA;
-    noalloc_accumulate<<<(n_i + 255) / 256, 256, 0, s>>>(n_i, scr, force);
+    noalloc_accumulate<<<(n_i + 7) / 8, 256, 0, s>>>(n_i, a.slices, scr, force);
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }

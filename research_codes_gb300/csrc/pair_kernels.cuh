@@ -342,6 +342,10 @@ struct GravityArgs {
     int *queue;
     double *o_acc;          // 3 per particle (assigned)
     double *o_pot, *o_eta;
+    // work units: each item's list in `slices` parts (0: 1), the results of
+    // part s at particle index + s * o_stride, to be added in the order of s
+    int slices;
+    size_t o_stride;
     // quadrupole of the sources k >= n_split (tree nodes), traceless, about
     // their centre of mass; null: monopoles only (the reference's SPJ).
     // FP64: 6 per node (xx, yy, zz, xy, xz, yz); FP32C: (xx, yy, zz, xy) and
@@ -349,6 +353,45 @@ struct GravityArgs {
     const double *s_quad;
     const float4 *f_sq0, *f_sq1;
 };
+
+// Parts of an item's list so that n_items items make `units` work units, of at
+// least 128 entries each.  One unit is a warp's turn: a few more units than
+// resident warps leave most of the last round empty, and a call of a few
+// items leaves most of the chip idle.
+inline int gravity_slices(long long n_items, long long nj, long long units, int most) {
+    const long long want = n_items > 0 ? (units + n_items - 1) / n_items : 1;
+    const long long fit = nj / 128 > 1 ? nj / 128 : 1;
+    const long long s = want < fit ? want : fit;
+    return (int)(s < 1 ? 1 : (s > most ? most : s));
+}
+
+// Adds the parts' results of particle p: g = (acc, pot, eta).
+__device__ __forceinline__ void gravity_gather(const double *acc, const double *pot, const double *eta, int p,
+                                               int slices, size_t stride, double (&g)[5]) {
+    for (int q = 0; q < 5; ++q) g[q] = 0.0;
+    for (int s = 0; s < slices; ++s) {
+        const size_t o = p + s * stride;
+        g[0] += acc[3 * o];
+        g[1] += acc[3 * o + 1];
+        g[2] += acc[3 * o + 2];
+        g[3] += pot[o];
+        g[4] += eta[o];
+    }
+}
+// The same by the 32 lanes of a warp, parts l, l + 32, ... per lane.
+__device__ __forceinline__ void gravity_gather_warp(const double *acc, const double *pot, const double *eta, int p,
+                                                    int slices, size_t stride, int lane, double (&g)[5]) {
+    for (int q = 0; q < 5; ++q) g[q] = 0.0;
+    for (int s = lane; s < slices; s += 32) {
+        const size_t o = p + s * stride;
+        g[0] += acc[3 * o];
+        g[1] += acc[3 * o + 1];
+        g[2] += acc[3 * o + 2];
+        g[3] += pot[o];
+        g[4] += eta[o];
+    }
+    for (int q = 0; q < 5; ++q) g[q] = seg_sum(g[q], 32);
+}
 
 // JT: the j-tile, list entries a warp stages in shared memory per pass (32
 // or 64; each lane loads JT / 32 of them one tile ahead) and sums in FP32
@@ -373,6 +416,7 @@ gravity_kernel(const GravityArgs a) {
     __shared__ R4 q_a[WARPS][QR];
     __shared__ typename Real<F64>::T2 q_b[WARPS][QR];
     const unsigned lt = lanemask_lt();
+    const int slices = a.slices > 0 ? a.slices : 1;
     const bool quad = F64 ? (a.s_quad != nullptr) : (a.f_sq0 != nullptr);
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
@@ -382,9 +426,14 @@ gravity_kernel(const GravityArgs a) {
         int item = 0;
         if (lane == 0) item = atomicAdd(a.queue, 1);
         item = __shfl_sync(FULL, item, 0);
-        if (item >= n_items) return;
-        const ItemRef r = decode(a.items[item], a.j_off, a.i_list, lane);
-        const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;
+        if (item >= n_items * slices) return;
+        const int slice = item % slices;
+        const ItemRef r = decode(a.items[item / slices], a.j_off, a.i_list, lane);
+        const int tpi = r.tpi, sub = r.sub, ii = r.ii;
+        // whole tiles per part
+        const int tiles = (r.nj + JT - 1) / JT;
+        const int t_lo = (int)((long long)tiles * slice / slices), t_hi = (int)((long long)tiles * (slice + 1) / slices);
+        const int jb = r.jb + t_lo * JT, nj = min(r.nj, t_hi * JT) - t_lo * JT;
 
         R xi, yi, zi, e2i;
         float4 ch = make_float4(0, 0, 0, 0), cl = ch;
@@ -616,11 +665,12 @@ gravity_kernel(const GravityArgs a) {
         const double saz = seg_sum(az.value(), tpi), spt = seg_sum(pt.value(), tpi);
         const double set = seg_sum(et.value(), tpi);
         if (r.act && sub == 0) {
-            a.o_acc[3 * ii + 0] = 0.5 * sax;
-            a.o_acc[3 * ii + 1] = 0.5 * say;
-            a.o_acc[3 * ii + 2] = 0.5 * saz;
-            a.o_pot[ii] = 0.5 * spt;
-            a.o_eta[ii] = set;
+            const size_t o = ii + slice * a.o_stride;
+            a.o_acc[3 * o + 0] = 0.5 * sax;
+            a.o_acc[3 * o + 1] = 0.5 * say;
+            a.o_acc[3 * o + 2] = 0.5 * saz;
+            a.o_pot[o] = 0.5 * spt;
+            a.o_eta[o] = set;
         }
     }
 }

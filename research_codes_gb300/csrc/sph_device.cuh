@@ -65,18 +65,18 @@ __device__ __forceinline__ float rsqrt_r(float x) {
 // order iteration, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 from one fused
 // multiply-add: five FP64 operations, relative error 2^-53 from the last
 // rounding plus (5/16) e^3 < 2^-60.  GB300 retires two FP64 operations per clock
-// and SM, and the pair loops are made of little else.  Arguments whose square
-// root the approximation does not cover (zero, subnormal, negative, infinite,
-// NaN) go to the library's rsqrt.
+// and SM, and the pair loops are made of little else.  Zero and infinite
+// arguments give the exact +inf and 0 of the approximation (subnormal ones
+// count as zero), negative ones and NaN give NaN.
 __device__ __forceinline__ bool rsqrt_special(double x) {
     return (unsigned)(__double2hiint(x) - 0x00100000) >= 0x7fe00000u;
 }
 __device__ __forceinline__ double rsqrt_r(double x) {
-    if (rsqrt_special(x)) return rsqrt(x);
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
+    const double r = fma(y * e, fma(e, 0.375, 0.5), y);
+    return rsqrt_special(x) ? y : r;
 }
 
 // 1/x: FP32 via rcp.approx.ftz.f32 (relative error <= 2^-23), FP64 exact.

@@ -674,17 +674,20 @@ __global__ void post_density(int n, const dbl4 *pos, const double *dens, const d
 // Gravity write-back, hdr_gravity.hpp:107-113
 __global__ void gravity_writeback(int n, double G, const double *acc, const double *pot, const double *etas,
                                   const double *ksr, const double *grdh, const double *dens, double *accg2,
-                                  double *pot_out, double *eta_out, bool f32) {
+                                  double *pot_out, double *eta_out, bool f32, int slices, double *etas_out) {
     GRID_STRIDE(p, n) {
-        for (int c = 0; c < 3; ++c) accg2[3 * p + c] = G * acc[3 * p + c];
+        double g[5];
+        sphk::gravity_gather(acc, pot, etas, p, slices, n, g);
+        for (int c = 0; c < 3; ++c) accg2[3 * p + c] = G * g[c];
+        etas_out[p] = g[4];   // the derivative reads it
         if (f32) {   // eta feeds the FP32 hydro records
             const float h = (float)ksr[p];
             eta_out[p] = (double)(h * h / (float)(KSRH * KSRH) * (float)grdh[p] / (3.0f * (float)dens[p]) *
-                                  (float)etas[p]);
+                                  (float)g[4]);
         } else {
-            eta_out[p] = ksr[p] * ksr[p] / (KSRH * KSRH) * grdh[p] / (3.0 * dens[p]) * etas[p];
+            eta_out[p] = ksr[p] * ksr[p] / (KSRH * KSRH) * grdh[p] / (3.0 * dens[p]) * g[4];
         }
-        pot_out[p] = G * pot[p];
+        pot_out[p] = G * g[3];
     }
 }
 
@@ -1063,6 +1066,8 @@ void phase_event(sph_system *s, int k, cudaStream_t st) {
         cudaEventRecord(s->ev[k], st);
 }
 
+int gravity_slices(const sph_system *s);
+
 int alloc_all(sph_system *s) {
     const size_t n = (size_t)s->n;
     const size_t nn = 2 * n;
@@ -1075,12 +1080,13 @@ int alloc_all(sph_system *s) {
     }
     DevBuf<double> *d1[] = {&s->rs, &s->dens, &s->divv, &s->rotv, &s->grdh, &s->pres, &s->vsnd, &s->bswt,
                             &s->eps2, &s->udot, &s->vsmx, &s->diffu, &s->pot, &s->eta, &s->adot, &s->adotu,
-                            &s->t_dens, &s->t_divv, &s->t_rotv, &s->t_grdh, &s->t_ksr, &s->r_pot, &s->r_eta,
-                            &s->r_udot, &s->r_vsmx, &s->r_diffu, &s->g_r, &s->a_r};
+                            &s->t_dens, &s->t_divv, &s->t_rotv, &s->t_grdh, &s->t_ksr, &s->r_udot,
+                            &s->r_vsmx, &s->r_diffu, &s->g_r, &s->a_r};
     for (auto *b : d1) e |= b->ensure(n);
-    DevBuf<double> *d3[] = {&s->acc, &s->acch, &s->accg1, &s->accg2, &s->r_acc, &s->r_acch, &s->r_accg,
-                            &s->staging};
+    DevBuf<double> *d3[] = {&s->acc, &s->acch, &s->accg1, &s->accg2, &s->r_acch, &s->r_accg, &s->staging};
     for (auto *b : d3) e |= b->ensure(3 * n);
+    const size_t parts = n * (size_t)gravity_slices(s);
+    e |= s->r_acc.ensure(3 * parts) | s->r_pot.ensure(parts) | s->r_eta.ensure(parts);
     e |= s->np.ensure(n) | s->t_np.ensure(n) | s->t_itr.ensure(n);
     e |= s->pe.ensure(n) | s->h1.ensure(n) | s->h2.ensure(n) | s->h3.ensure(n);
     e |= s->child.ensure(n) | s->parent.ensure(nn) | s->first.ensure(nn) | s->count.ensure(nn);
@@ -1289,6 +1295,13 @@ int item_size(const sph_system *s) {
     int chunk = 32;
     while (chunk > 4 && (long long)s->n < (long long)chunk * 16 * s->ctx->sm_count) chunk >>= 1;
     return chunk;
+}
+
+// Parts of the gravity lists (~1000 entries and up, ~24 i-particles per item):
+// several units per resident warp.
+constexpr int MAX_SLICES = 8;
+int gravity_slices(const sph_system *s) {
+    return sphk::gravity_slices(s->n / 24 + 1, 1024, 6LL * 16 * s->ctx->sm_count, MAX_SLICES);
 }
 
 // Builds the lists of `kind` over the walks (group nodes + radii) and the
@@ -1709,12 +1722,14 @@ int gravity_phase(sph_system *s) {
     a.f_sq0 = q32 ? s->fq0.p : nullptr;
     a.f_sq1 = q32 ? s->fq1.p : nullptr;
     const int jt = (ctx->prm.precision == SPH_PREC_FP32C && s->prm.gravity_jtile == 64) ? 64 : 32;
+    a.slices = gravity_slices(s);
+    a.o_stride = n;
     sphrt::launch_gravity(a, ctx->prm.precision,
                           jt == 64 ? ctx->grid_g64 : ctx->grid[2][ctx->prm.precision == SPH_PREC_FP64], st, jt);
     phase_event(s, EV_GK_E, st);
     gravity_writeback<<<grid_for(n), 256, 0, st>>>(n, s->prm.G, s->r_acc.p, s->r_pot.p, s->r_eta.p, s->ksr[0].p,
                                                    s->grdh.p, s->dens.p, s->accg2.p, s->pot.p, s->eta.p,
-                                                   ctx->prm.precision == SPH_PREC_FP32C);
+                                                   ctx->prm.precision == SPH_PREC_FP32C, a.slices, s->r_eta.p);
     return SPH_OK;
 }
 
