@@ -54,6 +54,7 @@ def _declare(lib):
         "sph_retrieve_hydro": (ctypes.c_int, [_P, _I32, _I32, _PI32, _PP]),
         "sph_dispatch_gravity": (ctypes.c_int, [_P, _I32, _I32, _PP, _PI32, _PP, _PI32, _PP, _PI32]),
         "sph_retrieve_gravity": (ctypes.c_int, [_P, _I32, _I32, _PI32, _PP]),
+        "sph_member_pointers": (None, [_P, _I64, _I64, _PP]),
         "sph_abi_layout": (_I64, [ctypes.POINTER(_I64), _I64]),
         "sph_version": (ctypes.c_char_p, []),
         "sph_context_stream": (ctypes.c_int, [_P, ctypes.POINTER(_P)]),

@@ -2,12 +2,19 @@
 // functors and the batched Dispatch/Retrieve pairs.
 //
 // Data path of one dispatch (one CUDA stream per context):
-//   host  : walk arrays -> one pinned staging buffer [offsets | items | EPI | EPJ]
-//   H2D   : one cudaMemcpyAsync of that buffer
-//   device: unpack kernel (reference AoS structs -> FP64 SoA), persistent pair
-//           kernel, pack kernel (SoA -> reference Force structs, finite check)
-//   D2H   : one cudaMemcpyAsync into pinned memory
-//   Retrieve waits on the stream and scatters to the caller's per-walk arrays.
+//   host  : offsets and work items into a pinned buffer, and a table of the
+//           pieces to copy: that buffer and the callers' walk arrays
+//   device: one kernel copies every piece into one buffer [offsets | items | EPI
+//           | EPJ] (pageable host memory is read in place where the device can,
+//           otherwise the arrays are staged in pinned memory first); one kernel
+//           turns the reference AoS structs into records; the pair kernels; a
+//           pack kernel writes the reference Force structs to pinned memory
+//           (finite check)
+//   Dispatch returns when the callers' arrays have been read; Retrieve waits on
+//   the stream and copies to the caller's per-walk arrays.
+//
+// Staging 60 MB of walk arrays with memcpy took 5 ms of a 7 ms dispatch; the
+// copy kernel reads them in 0.33 ms (190 GB/s over NVLink-C2C).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -132,16 +139,17 @@ static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs 
     recheck_density(ctx, a, n_max, s, amb_total);
 }
 
-// Density rows of the items of m.
-void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s) {
+// Density rows of the items of m (longs: some may be long).
+void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s,
+                         bool longs) {
     sphk::mark_rows<sphk::ROWS_DENSITY, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-    mark_long<sphk::ROWS_DENSITY>(ctx, m, n_max, s);
+    if (longs) mark_long<sphk::ROWS_DENSITY>(ctx, m, n_max, s);
 }
 
 // Rows of the items of m, then the density sums over them.
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
-                    int n_max, int precision, cudaStream_t s, int *amb_total) {
-    launch_mark_density(ctx, m, mark_grid, n_max, s);
+                    int n_max, int precision, cudaStream_t s, int *amb_total, bool longs) {
+    launch_mark_density(ctx, m, mark_grid, n_max, s, longs);
     launch_density_sums(ctx, a, n_max, precision, s, amb_total);
 }
 
@@ -165,14 +173,14 @@ void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bo
 // (optional) is recorded between the two parts (as an external record node
 // when mid_external: inside a stream capture).
 void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
-                  int precision, cudaStream_t s, cudaEvent_t mid, bool mid_external) {
+                  int precision, cudaStream_t s, cudaEvent_t mid, bool mid_external, bool longs) {
     const bool f64 = precision == SPH_PREC_FP64;
     if (f64) {
         sphk::mark_rows<sphk::ROWS_HYDRO64, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-        mark_long<sphk::ROWS_HYDRO64>(ctx, m, a.n_i, s);
+        if (longs) mark_long<sphk::ROWS_HYDRO64>(ctx, m, a.n_i, s);
     } else {
         sphk::mark_rows<sphk::ROWS_HYDRO32, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-        mark_long<sphk::ROWS_HYDRO32>(ctx, m, a.n_i, s);
+        if (longs) mark_long<sphk::ROWS_HYDRO32>(ctx, m, a.n_i, s);
     }
     if (mid) cudaEventRecordWithFlags(mid, s, mid_external ? cudaEventRecordExternal : cudaEventRecordDefault);
     if (a.n_i <= 0) return;
@@ -211,57 +219,141 @@ __device__ __forceinline__ bool finite3(double a, double b, double c) {
     return isfinite(a) && isfinite(b) && isfinite(c);
 }
 
-__global__ void unpack_density_i(const sph_DensityEPI *in, int n, dbl4 *pm, dbl4 *vel,
-                                 long long *id, double *ksr, double *rs) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const sph_DensityEPI e = in[k];
-        pm[k] = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.mass);
-        vel[k] = make_dbl4(e.vel[0], e.vel[1], e.vel[2], 0.0);
-        id[k] = e.id;
-        ksr[k] = e.ksr;
-        rs[k] = e.rs;
+// A piece of the inputs: n 8-byte words to word dst of the device buffer.
+constexpr int COPY_WORDS = 2048;
+__global__ void __launch_bounds__(256) gather_inputs(const CopyPiece *pieces, int n, unsigned long long *dst,
+                                                     int *queue) {
+    // counters of this dispatch (the flags at 4..6 are not used on the device)
+    if (blockIdx.x == 0 && threadIdx.x < 10 && (threadIdx.x < 4 || threadIdx.x > 6)) queue[threadIdx.x] = 0;
+    for (int c = blockIdx.x; c < n; c += gridDim.x) {
+        const CopyPiece p = pieces[c];
+        unsigned long long v[COPY_WORDS / 256];
+#pragma unroll
+        for (int u = 0; u < COPY_WORDS / 256; ++u) {
+            const int k = threadIdx.x + 256 * u;
+            if (k < p.n) v[u] = p.src[k];
+        }
+#pragma unroll
+        for (int u = 0; u < COPY_WORDS / 256; ++u) {
+            const int k = threadIdx.x + 256 * u;
+            if (k < p.n) dst[p.dst + k] = v[u];
+        }
     }
 }
 
-__global__ void unpack_density_j(const sph_DensityEPJ *in, int n, dbl4 *pm, dbl4 *vel,
-                                 long long *id) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const sph_DensityEPJ e = in[k];
-        pm[k] = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.mass);
-        vel[k] = make_dbl4(e.vel[0], e.vel[1], e.vel[2], 0.0);
-        id[k] = e.id;
+// Records of one side (i or j) of a dispatch.
+struct DensitySide {
+    dbl4 *pm, *vel;
+    long long *id;
+    double *ksr, *rs;                     // i side
+    float4 *phi, *plo, *vhi, *vlo;
+};
+template <class E>
+__device__ __forceinline__ void prepare_density_one(const E *in, int k, const DensitySide &s, bool f32) {
+    const E e = in[k];
+    const dbl4 p = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.mass), v = make_dbl4(e.vel[0], e.vel[1], e.vel[2], 0.0);
+    double h = 0.0;
+    if constexpr (sizeof(E) == sizeof(sph_DensityEPI)) {
+        h = e.ksr;
+        s.ksr[k] = e.ksr;
+        s.rs[k] = e.rs;
+    }
+    s.pm[k] = p;
+    s.vel[k] = v;
+    s.id[k] = e.id;
+    float4 a, b;
+    sphk::row_record(p, h, a, b);
+    s.phi[k] = a;
+    s.plo[k] = b;
+    if (f32) {
+        sphk::velocity_record(v, a, b);
+        s.vhi[k] = a;
+        s.vlo[k] = b;
+    }
+}
+__global__ void prepare_density(const sph_DensityEPI *epi, int ni, const sph_DensityEPJ *epj, int nj, DensitySide si,
+                                DensitySide sj, bool f32) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ni + nj; k += gridDim.x * blockDim.x) {
+        if (k < ni)
+            prepare_density_one(epi, k, si, f32);
+        else
+            prepare_density_one(epj, k - ni, sj, f32);
     }
 }
 
-template <class T>
-__global__ void unpack_hydro(const T *in, int n, bool has_mass, dbl4 *pm, dbl4 *vel,
-                             long long *id, dbl4 *h1, dbl4 *h2, double2 *h3) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const T &e = in[k];
-        double m = 0.0;
-        if (has_mass) m = reinterpret_cast<const sph_HydroEPJ *>(&e)->mass;
-        pm[k] = make_dbl4(e.pos[0], e.pos[1], e.pos[2], m);
-        vel[k] = make_dbl4(e.vel[0], e.vel[1], e.vel[2], 0.0);
-        id[k] = e.id;
-        h1[k] = make_dbl4(e.hinv, e.pres, e.presc, e.bswt);
-        h2[k] = make_dbl4(e.dens, e.vsnd, e.alph, e.alphu);
-        h3[k] = make_double2(e.thrm, e.eta);
+struct HydroSide {
+    dbl4 *pm, *vel, *h1, *h2;
+    double2 *h3;
+    long long *id;
+    float4 *phi, *plo, *vhi, *vlo, *g1, *g2, *g3, *g4, *mp, *mv;
+};
+template <class E>
+__device__ __forceinline__ void prepare_hydro_one(const E *in, int k, const HydroSide &s, bool f32) {
+    const E &e = in[k];
+    double m = 0.0;
+    if constexpr (sizeof(E) == sizeof(sph_HydroEPJ)) m = e.mass;
+    const dbl4 p = make_dbl4(e.pos[0], e.pos[1], e.pos[2], m), v = make_dbl4(e.vel[0], e.vel[1], e.vel[2], 0.0);
+    const dbl4 h1 = make_dbl4(e.hinv, e.pres, e.presc, e.bswt), h2 = make_dbl4(e.dens, e.vsnd, e.alph, e.alphu);
+    const double2 h3 = make_double2(e.thrm, e.eta);
+    s.pm[k] = p;
+    s.vel[k] = v;
+    s.id[k] = e.id;
+    s.h1[k] = h1;
+    s.h2[k] = h2;
+    s.h3[k] = h3;
+    float4 a, b;
+    if (f32) {
+        sphk::HydroRecords r;
+        r.fill(p, v, h1, h2, h3);
+        s.phi[k] = r.phi; s.plo[k] = r.plo; s.vhi[k] = r.vhi; s.vlo[k] = r.vlo;
+        s.g1[k] = r.g1; s.g2[k] = r.g2; s.g3[k] = r.g3; s.g4[k] = r.g4;
+    } else {
+        sphk::row_record(p, 0.0, a, b);
+        s.plo[k] = b;
     }
+    sphk::hydro_mark_records(p, v, h1.x, h2.y, a, b);
+    s.mp[k] = a;
+    s.mv[k] = b;
 }
-
-__global__ void unpack_gravity_i(const sph_GravityEPI *in, int n, dbl4 *pe) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const sph_GravityEPI e = in[k];
-        pe[k] = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.eps2);
+__global__ void prepare_hydro(const sph_HydroEPI *epi, int ni, const sph_HydroEPJ *epj, int nj, HydroSide si,
+                              HydroSide sj, bool f32) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ni + nj; k += gridDim.x * blockDim.x) {
+        if (k < ni)
+            prepare_hydro_one(epi, k, si, f32);
+        else
+            prepare_hydro_one(epj, k - ni, sj, f32);
     }
 }
 
 // GravityEPJ and GravitySPJ share one layout (mass, pos[3], eps2).
-__global__ void unpack_gravity_j(const sph_GravityEPJ *in, int n, dbl4 *pm, double *eps2) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const sph_GravityEPJ e = in[k];
-        pm[k] = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.mass);
-        eps2[k] = e.eps2;
+__global__ void prepare_gravity(const sph_GravityEPI *epi, int ni, const sph_GravityEPJ *epj, int nj, dbl4 *i_pe,
+                                float4 *i_hi, float4 *i_lo, dbl4 *j_pm, double *j_eps2, float4 *j_hi, float4 *j_lo,
+                                bool f32) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ni + nj; k += gridDim.x * blockDim.x) {
+        float4 a, b;
+        if (k < ni) {
+            const sph_GravityEPI e = epi[k];
+            const dbl4 p = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.eps2);
+            if (f32) {
+                sphk::gravity_record(p, 0.0, e.eps2, a, b);
+                i_hi[k] = a;
+                i_lo[k] = b;
+            } else {
+                i_pe[k] = p;
+            }
+        } else {
+            const int j = k - ni;
+            const sph_GravityEPJ e = epj[j];
+            const dbl4 p = make_dbl4(e.pos[0], e.pos[1], e.pos[2], e.mass);
+            if (f32) {
+                sphk::gravity_record(p, e.mass, e.eps2, a, b);
+                j_hi[j] = a;
+                j_lo[j] = b;
+            } else {
+                j_pm[j] = p;
+                j_eps2[j] = e.eps2;
+            }
+        }
     }
 }
 
@@ -278,7 +370,7 @@ __global__ void pack_density(int n, const double *dens, const double *divv, cons
         d.np = np[k];
         d.itr = itr[k] != 0;
         out[k] = d;
-        if (!(finite3(d.dens, d.divv, d.rotv) && finite3(d.grdh, d.ksr, 0.0))) atomicOr(flag, 1);
+        if (!(finite3(d.dens, d.divv, d.rotv) && finite3(d.grdh, d.ksr, 0.0))) *flag = 1;
     }
 }
 
@@ -296,7 +388,7 @@ __global__ void pack_hydro(int n, const double *acch, const double *accg, const 
         out[k] = h;
         if (!(finite3(h.acch[0], h.acch[1], h.acch[2]) && finite3(h.accg[0], h.accg[1], h.accg[2]) &&
               finite3(h.udot, h.vsmx, h.diffu)))
-            atomicOr(flag, 1);
+            *flag = 1;
     }
 }
 
@@ -314,7 +406,7 @@ __global__ void pack_gravity(int n, const double *acc, const double *pot, const 
         g.pot = v[3];
         g.eta = v[4];
         out[k] = g;
-        if (!(finite3(g.acc[0], g.acc[1], g.acc[2]) && finite3(g.pot, g.eta, 0.0))) atomicOr(flag, 1);
+        if (!(finite3(g.acc[0], g.acc[1], g.acc[2]) && finite3(g.pot, g.eta, 0.0))) *flag = 1;
     }
 }
 
@@ -415,6 +507,9 @@ extern "C" int sph_context_create(const sph_params *p, sph_context **out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_queue, 10 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_flags, 8 * sizeof(int));
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_read, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&ctx->pageable_access, cudaDevAttrPageableMemoryAccess, prm.device);
     if (e == cudaSuccess && init_grids(ctx) != 0) e = cudaErrorInvalidDeviceFunction;
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -437,6 +532,7 @@ extern "C" int sph_context_destroy(sph_context *ctx) {
     for (int k = 0; k < 3; ++k) ctx->kind[k].release();
     if (ctx->d_queue) cudaFree(ctx->d_queue);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
+    if (ctx->ev_read) cudaEventDestroy(ctx->ev_read);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return SPH_OK;
@@ -517,6 +613,12 @@ constexpr float ROW_SLACK = 1.03f;   // row radius of the density over the first
 constexpr int LONG_NJ = 4096;    // lists beyond this are marked by a block per item
 constexpr int SPLIT_NJ = 1024;   // density and hydro: lists beyond this make smaller items
 
+int longest(const int32_t *n, int n_walk) {
+    int m = 0;
+    for (int w = 0; w < n_walk; ++w) m = std::max(m, (int)n[w]);
+    return m;
+}
+
 // Validates walk counts and fills the int32 offsets.  n_extra (gravity SPJ
 // counts) may be null.
 int walk_offsets(sph_context *ctx, int32_t n_walk, const int32_t *n_i, const int32_t *n_j,
@@ -542,8 +644,7 @@ int walk_offsets(sph_context *ctx, int32_t n_walk, const int32_t *n_i, const int
     return SPH_OK;
 }
 
-// Lays out [i_off | j_off | items | EPI | EPJ] in the kind's pinned staging
-// buffer; returns offsets of the struct regions.
+// Device buffer [i_off | j_off | items | EPI | EPJ].
 struct Layout {
     size_t off_ioff, off_joff, off_items, off_epi, off_epj, total;
 };
@@ -560,40 +661,96 @@ Layout make_layout(int n_walk, size_t n_items, size_t bytes_epi, size_t bytes_ep
     return L;
 }
 
-int stage_common(sph_context *ctx, KindState &ks, const std::vector<int> &i_off,
-                 const std::vector<int> &j_off, size_t epi_size, size_t epj_size, int chunk, int split_nj,
-                 Layout &L) {
+// One array of each walk: entries of `size` bytes, the walk's at index off of
+// the region at `base` of the device buffer.
+struct WalkArrays {
+    const void *const *ptr;
+    const int32_t *n;
+    size_t size, base;
+};
+
+// Whether the copy kernel may read the array where it is.
+bool readable(const sph_context *ctx, const void *p) {
+    return ctx->pageable_access && (reinterpret_cast<uintptr_t>(p) & 7) == 0;
+}
+
+// Builds the items and the pieces of a dispatch in the pinned buffers.  place:
+// byte offset of array a of walk w in the device buffer.
+template <class P>
+int stage(sph_context *ctx, KindState &ks, const std::vector<int> &i_off, const std::vector<int> &j_off,
+          size_t epi_size, size_t epj_size, int chunk, int split_nj, const WalkArrays *arrays, int n_arrays,
+          P place, Layout &L) {
     const int n_walk = (int)i_off.size() - 1;
     build_items(n_walk, i_off.data(), j_off.data(), chunk, split_nj, ks.items);
     L = make_layout(n_walk, ks.items.size(), epi_size * (size_t)i_off[n_walk],
                     epj_size * (size_t)j_off[n_walk]);
-    if (ks.h_in.ensure(L.total) || ks.d_in.ensure(L.total))
+    size_t staged = 0, pieces = 1 + L.off_epi / (8 * COPY_WORDS);
+    ks.in_place = false;
+    for (int a = 0; a < n_arrays; ++a)
+        for (int w = 0; w < n_walk; ++w) {
+            const size_t bytes = arrays[a].n ? arrays[a].size * (size_t)arrays[a].n[w] : 0;
+            if (!bytes) continue;
+            if (!arrays[a].ptr[w]) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
+            pieces += 1 + bytes / (8 * COPY_WORDS);
+            if (!readable(ctx, arrays[a].ptr[w])) staged += bytes;
+        }
+    if (ks.h_in.ensure(L.off_epi + staged) || ks.h_pieces.ensure(pieces) || ks.d_in.ensure(L.total))
         return set_error(ctx, SPH_ERR_CUDA, "staging allocation of %zu bytes failed", L.total);
     char *h = ks.h_in.p;
     std::memcpy(h + L.off_ioff, i_off.data(), sizeof(int) * (n_walk + 1));
     std::memcpy(h + L.off_joff, j_off.data(), sizeof(int) * (n_walk + 1));
     if (!ks.items.empty()) std::memcpy(h + L.off_items, ks.items.data(), sizeof(WorkItem) * ks.items.size());
+    ks.n_pieces = 0;
+    auto add = [&](const void *src, size_t bytes, size_t dst) {
+        const char *q = static_cast<const char *>(src);
+        for (size_t o = 0; o < bytes; o += 8 * (size_t)COPY_WORDS) {
+            const size_t b = std::min(bytes - o, 8 * (size_t)COPY_WORDS);
+            ks.h_pieces.p[ks.n_pieces++] =
+                CopyPiece{reinterpret_cast<const unsigned long long *>(q + o), (long long)((dst + o) / 8), (int)(b / 8)};
+        }
+    };
+    add(h, L.off_epi, 0);
+    size_t pos = L.off_epi;
+    for (int a = 0; a < n_arrays; ++a)
+        for (int w = 0; w < n_walk; ++w) {
+            const size_t bytes = arrays[a].n ? arrays[a].size * (size_t)arrays[a].n[w] : 0;
+            if (!bytes) continue;
+            const void *src = arrays[a].ptr[w];
+            if (readable(ctx, src)) {
+                ks.in_place = true;
+            } else {
+                std::memcpy(h + pos, src, bytes);
+                src = h + pos;
+                pos += bytes;
+            }
+            add(src, bytes, place(a, w));
+        }
     return SPH_OK;
 }
 
-int upload(sph_context *ctx, KindState &ks, const Layout &L) {
-    cudaError_t e = cudaMemcpyAsync(ks.d_in.p, ks.h_in.p, L.total, cudaMemcpyHostToDevice, ctx->stream);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "H2D");
-    return SPH_OK;
-}
-
-int finish_dispatch(sph_context *ctx, KindState &ks, int n_walk, const std::vector<int> &i_off,
-                    size_t out_size) {
-    const int ni = i_off[n_walk];
+// Copies the pieces to the device buffer and zeroes the dispatch's counters.
+int launch_gather(sph_context *ctx, KindState &ks) {
+    ctx->h_flags[ks.flag_slot] = 0;
+    gather_inputs<<<std::max(1, std::min(ks.n_pieces, 8 * ctx->sm_count)), 256, 0, ctx->stream>>>(
+        ks.h_pieces.p, ks.n_pieces, reinterpret_cast<unsigned long long *>(ks.d_in.p), ctx->d_queue);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error(ctx, e, "kernel launch");
-    if (ni > 0) {
-        e = cudaMemcpyAsync(ks.h_out.p, ks.d_out.p, out_size * ni, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) return cuda_error(ctx, e, "D2H");
+    if (e == cudaSuccess && ks.in_place && !ctx->in_functor) e = cudaEventRecord(ctx->ev_read, ctx->stream);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "input copy");
+    return SPH_OK;
+}
+
+// After the launches of a dispatch: waits until the callers' arrays have been
+// read (a functor call retrieves at once and waits there).
+int finish_dispatch(sph_context *ctx, KindState &ks, int n_walk, const std::vector<int> &i_off) {
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);   // nothing reads the callers' arrays any more
+        return cuda_error(ctx, e, "kernel launch");
     }
-    e = cudaMemcpyAsync(&ctx->h_flags[ks.flag_slot], ctx->d_queue + 4 + ks.flag_slot, sizeof(int),
-                        cudaMemcpyDeviceToHost, ctx->stream);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "D2H flag");
+    if (ks.in_place && !ctx->in_functor) {
+        e = cudaEventSynchronize(ctx->ev_read);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "input copy");
+    }
     ks.pending = true;
     ks.n_walk = n_walk;
     ks.i_off = i_off;
@@ -610,13 +767,6 @@ int begin_kind(sph_context *ctx, KindState &ks) {
     // that failed after its upload was queued; never overwrite it in flight.
     e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_error(ctx, e, "stream synchronize");
-    return SPH_OK;
-}
-
-int reset_queue_and_flag(sph_context *ctx, KindState &ks) {
-    cudaError_t e = cudaMemsetAsync(ctx->d_queue + ks.flag_slot, 0, sizeof(int), ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_queue + 4 + ks.flag_slot, 0, sizeof(int), ctx->stream);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
     return SPH_OK;
 }
 
@@ -658,53 +808,32 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
     std::vector<int> i_off, j_off;
     if ((st = walk_offsets(ctx, n_walk, n_epi, n_epj, nullptr, i_off, j_off))) return st;
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
-    Layout L;
-    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_DensityEPI), sizeof(sph_DensityEPJ),
-                           item_size(ctx, i_off[n_walk]), SPLIT_NJ, L))) return st;
-    for (int w = 0; w < n_walk; ++w) {
-        if ((n_epi[w] && !epi[w]) || (n_epj[w] && !epj[w]))
-            return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
-        if (n_epi[w]) std::memcpy(ks.h_in.p + L.off_epi + sizeof(sph_DensityEPI) * i_off[w], epi[w], sizeof(sph_DensityEPI) * n_epi[w]);
-        if (n_epj[w]) std::memcpy(ks.h_in.p + L.off_epj + sizeof(sph_DensityEPJ) * j_off[w], epj[w], sizeof(sph_DensityEPJ) * n_epj[w]);
-    }
     const int ni = i_off[n_walk], nj = j_off[n_walk];
-    if (ks.ensure_density(ni, nj)) return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
-    if (ks.h_out.ensure(sizeof(sph_Density) * (size_t)std::max(ni, 1)) ||
-        ks.d_out.ensure(sizeof(sph_Density) * (size_t)std::max(ni, 1)))
+    const int cap = std::max(256, ni / 16);
+    const WalkArrays arrays[2] = {{(const void *const *)epi, n_epi, sizeof(sph_DensityEPI), 0},
+                                  {(const void *const *)epj, n_epj, sizeof(sph_DensityEPJ), 0}};
+    Layout L;
+    auto place = [&](int a, int w) {
+        return a == 0 ? L.off_epi + sizeof(sph_DensityEPI) * i_off[w] : L.off_epj + sizeof(sph_DensityEPJ) * j_off[w];
+    };
+    if ((st = stage(ctx, ks, i_off, j_off, sizeof(sph_DensityEPI), sizeof(sph_DensityEPJ), item_size(ctx, ni),
+                    SPLIT_NJ, arrays, 2, place, L)))
+        return st;
+    if (ks.ensure_density(ni, nj) || ks.amb.ensure(cap) || ks.long_items.ensure(ks.items.size()))
+        return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
+    if (ks.h_out.ensure(sizeof(sph_Density) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
-    if ((st = upload(ctx, ks, L))) return st;
-    if ((st = reset_queue_and_flag(ctx, ks))) return st;
+    if ((st = launch_gather(ctx, ks))) return st;
     char *d = ks.d_in.p;
-    if (ni > 0)
-        unpack_density_i<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-            (const sph_DensityEPI *)(d + L.off_epi), ni, ks.a4[0].p, ks.a4[1].p, ks.id[0].p, ks.d1[0].p, ks.d1[1].p);
-    if (nj > 0)
-        unpack_density_j<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
-            (const sph_DensityEPJ *)(d + L.off_epj), nj, ks.a4[2].p, ks.a4[3].p, ks.id[1].p);
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
-    if (ni > 0) {
-        if (f32)
-            sphk::make_density_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-                ni, ks.a4[0].p, ks.a4[1].p, ks.d1[0].p, ks.f4[0].p, ks.f4[1].p, ks.f4[2].p, ks.f4[3].p);
-        else
-            sphk::make_row_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.a4[0].p, ks.d1[0].p,
-                                                                             ks.f4[0].p, ks.f4[1].p);
-    }
-    if (nj > 0) {
-        if (f32)
-            sphk::make_density_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
-                nj, ks.a4[2].p, ks.a4[3].p, nullptr, ks.f4[4].p, ks.f4[5].p, ks.f4[6].p, ks.f4[7].p);
-        else
-            sphk::make_row_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(nj, ks.a4[2].p, nullptr,
-                                                                             ks.f4[4].p, ks.f4[5].p);
-    }
+    const DensitySide si{ks.a4[0].p, ks.a4[1].p, ks.id[0].p, ks.d1[0].p, ks.d1[1].p,
+                         ks.f4[0].p, ks.f4[1].p, ks.f4[2].p, ks.f4[3].p};
+    const DensitySide sj{ks.a4[2].p, ks.a4[3].p, ks.id[1].p, nullptr, nullptr,
+                         ks.f4[4].p, ks.f4[5].p, ks.f4[6].p, ks.f4[7].p};
+    if (ni + nj > 0)
+        prepare_density<<<eltwise_grid((long long)ni + nj), 256, 0, ctx->stream>>>(
+            (const sph_DensityEPI *)(d + L.off_epi), ni, (const sph_DensityEPJ *)(d + L.off_epj), nj, si, sj, f32);
     if (!ks.items.empty()) {
-        const int cap = std::max(256, ni / 16);
-        if (ks.amb.ensure(cap) || ks.long_items.ensure(ks.items.size())) return set_error(ctx, SPH_ERR_CUDA, "allocation failed");
-        // the sweep queue and the ambiguous particles' count start empty
-        cudaError_t e = cudaMemsetAsync(ctx->d_queue + 3, 0, sizeof(int), ctx->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_queue + 7, 0, 3 * sizeof(int), ctx->stream);
-        if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
         sphk::MarkArgs m{};
         m.i_hi = ks.f4[0].p; m.i_lo = ks.f4[1].p; m.j_hi = ks.f4[4].p; m.j_lo = ks.f4[5].p;
         m.slack = ROW_SLACK;
@@ -732,13 +861,13 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         a.amb_cap = cap;
         a.amb_tol = AMB_TOL;
         launch_density(ctx, m, pair_grid(ctx, K_DENS, ctx->prm.precision, m.n_items), a, ni, ctx->prm.precision,
-                       ctx->stream);
+                       ctx->stream, nullptr, longest(n_epj, n_walk) > LONG_NJ);
     }
     if (ni > 0)
         pack_density<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
             ni, ks.o[0].p, ks.o[1].p, ks.o[2].p, ks.o[3].p, ks.o[4].p, ks.o_np.p, ks.o_itr.p,
-            (sph_Density *)ks.d_out.p, ctx->d_queue + 4 + K_DENS);
-    return finish_dispatch(ctx, ks, n_walk, i_off, sizeof(sph_Density));
+            (sph_Density *)ks.h_out.p, ctx->h_flags + K_DENS);
+    return finish_dispatch(ctx, ks, n_walk, i_off);
 }
 
 extern "C" int sph_retrieve_density(sph_context *ctx, int32_t tag, int32_t n_walk, const int32_t *n_i,
@@ -760,58 +889,35 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
     std::vector<int> i_off, j_off;
     if ((st = walk_offsets(ctx, n_walk, n_epi, n_epj, nullptr, i_off, j_off))) return st;
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
+    const int ni = i_off[n_walk], nj = j_off[n_walk];
+    const WalkArrays arrays[2] = {{(const void *const *)epi, n_epi, sizeof(sph_HydroEPI), 0},
+                                  {(const void *const *)epj, n_epj, sizeof(sph_HydroEPJ), 0}};
     Layout L;
+    auto place = [&](int a, int w) {
+        return a == 0 ? L.off_epi + sizeof(sph_HydroEPI) * i_off[w] : L.off_epj + sizeof(sph_HydroEPJ) * j_off[w];
+    };
     // FP32C: items of 32 i-particles, whose rows and so sums do not depend on
     // the size of the call
-    const bool f64 = ctx->prm.precision == SPH_PREC_FP64;
-    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_HydroEPI), sizeof(sph_HydroEPJ),
-                           f64 ? item_size(ctx, i_off[n_walk]) : 32, f64 ? SPLIT_NJ : 0, L))) return st;
-    for (int w = 0; w < n_walk; ++w) {
-        if ((n_epi[w] && !epi[w]) || (n_epj[w] && !epj[w]))
-            return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
-        if (n_epi[w]) std::memcpy(ks.h_in.p + L.off_epi + sizeof(sph_HydroEPI) * i_off[w], epi[w], sizeof(sph_HydroEPI) * n_epi[w]);
-        if (n_epj[w]) std::memcpy(ks.h_in.p + L.off_epj + sizeof(sph_HydroEPJ) * j_off[w], epj[w], sizeof(sph_HydroEPJ) * n_epj[w]);
-    }
-    const int ni = i_off[n_walk], nj = j_off[n_walk];
-    if (ks.ensure_hydro(ni, nj)) return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
-    if (ks.h_out.ensure(sizeof(sph_Hydro) * (size_t)std::max(ni, 1)) ||
-        ks.d_out.ensure(sizeof(sph_Hydro) * (size_t)std::max(ni, 1)))
+    const bool f32 = ctx->prm.precision == SPH_PREC_FP32C, f64 = !f32;
+    if ((st = stage(ctx, ks, i_off, j_off, sizeof(sph_HydroEPI), sizeof(sph_HydroEPJ), f64 ? item_size(ctx, ni) : 32,
+                    f64 ? SPLIT_NJ : 0, arrays, 2, place, L)))
+        return st;
+    if (ks.ensure_hydro(ni, nj) || ks.long_items.ensure(ks.items.size()))
+        return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
+    if (ks.h_out.ensure(sizeof(sph_Hydro) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
-    if ((st = upload(ctx, ks, L))) return st;
-    if ((st = reset_queue_and_flag(ctx, ks))) return st;
+    if ((st = launch_gather(ctx, ks))) return st;
     char *d = ks.d_in.p;
-    if (ni > 0)
-        unpack_hydro<sph_HydroEPI><<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-            (const sph_HydroEPI *)(d + L.off_epi), ni, false, ks.a4[0].p, ks.a4[1].p, ks.id[0].p,
-            ks.a4[4].p, ks.a4[5].p, ks.a2[0].p);
-    if (nj > 0)
-        unpack_hydro<sph_HydroEPJ><<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
-            (const sph_HydroEPJ *)(d + L.off_epj), nj, true, ks.a4[2].p, ks.a4[3].p, ks.id[1].p,
-            ks.a4[6].p, ks.a4[7].p, ks.a2[1].p);
-    const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
-    if (ni > 0) {
-        if (f32)
-            sphk::make_hydro_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-                ni, ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.a2[0].p, ks.f4[0].p, ks.f4[1].p, ks.f4[2].p,
-                ks.f4[3].p, ks.f4[8].p, ks.f4[9].p, ks.f4[10].p, ks.f4[14].p, ks.f4[16].p, ks.f4[17].p);
-        else
-            sphk::make_hydro_row_records<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-                ni, ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.f4[16].p, ks.f4[1].p, ks.f4[17].p);
-    }
-    if (nj > 0) {
-        if (f32)
-            sphk::make_hydro_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
-                nj, ks.a4[2].p, ks.a4[3].p, ks.a4[6].p, ks.a4[7].p, ks.a2[1].p, ks.f4[4].p, ks.f4[5].p, ks.f4[6].p,
-                ks.f4[7].p, ks.f4[11].p, ks.f4[12].p, ks.f4[13].p, ks.f4[15].p, ks.f4[18].p, ks.f4[19].p);
-        else
-            sphk::make_hydro_row_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(
-                nj, ks.a4[2].p, ks.a4[3].p, ks.a4[6].p, ks.a4[7].p, ks.f4[18].p, ks.f4[5].p, ks.f4[19].p);
-    }
+    const HydroSide si{ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.a2[0].p, ks.id[0].p, ks.f4[0].p, ks.f4[1].p,
+                       ks.f4[2].p, ks.f4[3].p, ks.f4[8].p, ks.f4[9].p, ks.f4[10].p, ks.f4[14].p, ks.f4[16].p,
+                       ks.f4[17].p};
+    const HydroSide sj{ks.a4[2].p, ks.a4[3].p, ks.a4[6].p, ks.a4[7].p, ks.a2[1].p, ks.id[1].p, ks.f4[4].p, ks.f4[5].p,
+                       ks.f4[6].p, ks.f4[7].p, ks.f4[11].p, ks.f4[12].p, ks.f4[13].p, ks.f4[15].p, ks.f4[18].p,
+                       ks.f4[19].p};
+    if (ni + nj > 0)
+        prepare_hydro<<<eltwise_grid((long long)ni + nj), 256, 0, ctx->stream>>>(
+            (const sph_HydroEPI *)(d + L.off_epi), ni, (const sph_HydroEPJ *)(d + L.off_epj), nj, si, sj, f32);
     if (!ks.items.empty()) {
-        if (ks.long_items.ensure(ks.items.size())) return set_error(ctx, SPH_ERR_CUDA, "allocation failed");
-        // no particle without a row and no long item yet
-        cudaError_t e = cudaMemsetAsync(ctx->d_queue + 8, 0, 2 * sizeof(int), ctx->stream);
-        if (e != cudaSuccess) return cuda_error(ctx, e, "memset");
         sphk::MarkArgs m{};
         m.i_hi = ks.f4[16].p; m.i_lo = ks.f4[1].p; m.j_hi = ks.f4[18].p; m.j_lo = ks.f4[5].p;
         m.i_v = ks.f4[17].p; m.j_v = ks.f4[19].p;
@@ -840,13 +946,13 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         m.i_id = a.i_id; m.j_id = a.j_id; m.fi = a.fi; m.fj = a.fj; m.fi_g2 = a.fi_g2; m.fj_g2 = a.fj_g2;
         m.i_pm = a.i_pm; m.i_vel = a.i_vel; m.i_h2 = a.i_h2; m.j_pm = a.j_pm; m.j_vel = a.j_vel; m.j_h2 = a.j_h2;
         launch_hydro(ctx, m, pair_grid(ctx, K_HYDRO, ctx->prm.precision, m.n_items), a, ctx->prm.precision,
-                     ctx->stream);
+                     ctx->stream, nullptr, false, f64 && longest(n_epj, n_walk) > LONG_NJ);
     }
     if (ni > 0)
         pack_hydro<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
-            ni, ks.o[0].p, ks.o[1].p, ks.o[2].p, ks.o[3].p, ks.o[4].p, (sph_Hydro *)ks.d_out.p,
-            ctx->d_queue + 4 + K_HYDRO);
-    return finish_dispatch(ctx, ks, n_walk, i_off, sizeof(sph_Hydro));
+            ni, ks.o[0].p, ks.o[1].p, ks.o[2].p, ks.o[3].p, ks.o[4].p, (sph_Hydro *)ks.h_out.p,
+            ctx->h_flags + K_HYDRO);
+    return finish_dispatch(ctx, ks, n_walk, i_off);
 }
 
 extern "C" int sph_retrieve_hydro(sph_context *ctx, int32_t tag, int32_t n_walk, const int32_t *n_i,
@@ -870,38 +976,30 @@ extern "C" int sph_dispatch_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
     if ((st = walk_offsets(ctx, n_walk, n_epi, n_epj, n_spj, i_off, j_off))) return st;
     if (n_walk > 0 && (!epi || !epj)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null walk arrays");
     if (n_spj && !spj) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null spj");
-    Layout L;
-    if ((st = stage_common(ctx, ks, i_off, j_off, sizeof(sph_GravityEPI), sizeof(sph_GravityEPJ), 32, 0, L))) return st;
-    static_assert(sizeof(sph_GravitySPJ) == sizeof(sph_GravityEPJ), "SPJ appended to EPJ");
-    for (int w = 0; w < n_walk; ++w) {
-        const int ns = n_spj ? n_spj[w] : 0;
-        if ((n_epi[w] && !epi[w]) || (n_epj[w] && !epj[w]) || (ns && !spj[w]))
-            return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
-        char *jdst = ks.h_in.p + L.off_epj + sizeof(sph_GravityEPJ) * j_off[w];
-        if (n_epi[w]) std::memcpy(ks.h_in.p + L.off_epi + sizeof(sph_GravityEPI) * i_off[w], epi[w], sizeof(sph_GravityEPI) * n_epi[w]);
-        if (n_epj[w]) std::memcpy(jdst, epj[w], sizeof(sph_GravityEPJ) * n_epj[w]);
-        if (ns) std::memcpy(jdst + sizeof(sph_GravityEPJ) * n_epj[w], spj[w], sizeof(sph_GravitySPJ) * ns);
-    }
     const int ni = i_off[n_walk], nj = j_off[n_walk];
+    static_assert(sizeof(sph_GravitySPJ) == sizeof(sph_GravityEPJ), "SPJ appended to EPJ");
+    const WalkArrays arrays[3] = {{(const void *const *)epi, n_epi, sizeof(sph_GravityEPI), 0},
+                                  {(const void *const *)epj, n_epj, sizeof(sph_GravityEPJ), 0},
+                                  {(const void *const *)spj, n_spj, sizeof(sph_GravitySPJ), 0}};
+    Layout L;
+    auto place = [&](int a, int w) {
+        if (a == 0) return L.off_epi + sizeof(sph_GravityEPI) * i_off[w];
+        return L.off_epj + sizeof(sph_GravityEPJ) * ((size_t)j_off[w] + (a == 2 ? n_epj[w] : 0));
+    };
+    if ((st = stage(ctx, ks, i_off, j_off, sizeof(sph_GravityEPI), sizeof(sph_GravityEPJ), 32, 0, arrays, 3, place, L)))
+        return st;
     const int slices = sphk::gravity_slices((long long)ks.items.size(), nj / std::max(n_walk, 1),
                                             2LL * resident_warps(ctx), 512);
     if (ks.ensure_gravity(ni, nj, slices)) return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
-    if (ks.h_out.ensure(sizeof(sph_Gravity) * (size_t)std::max(ni, 1)) ||
-        ks.d_out.ensure(sizeof(sph_Gravity) * (size_t)std::max(ni, 1)))
+    if (ks.h_out.ensure(sizeof(sph_Gravity) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
-    if ((st = upload(ctx, ks, L))) return st;
-    if ((st = reset_queue_and_flag(ctx, ks))) return st;
+    if ((st = launch_gather(ctx, ks))) return st;
     char *d = ks.d_in.p;
-    if (ni > 0)
-        unpack_gravity_i<<<eltwise_grid(ni), 256, 0, ctx->stream>>>((const sph_GravityEPI *)(d + L.off_epi), ni, ks.a4[0].p);
-    if (nj > 0)
-        unpack_gravity_j<<<eltwise_grid(nj), 256, 0, ctx->stream>>>((const sph_GravityEPJ *)(d + L.off_epj), nj, ks.a4[2].p, ks.d1[0].p);
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
-    if (f32 && ni > 0)
-        sphk::make_gravity_records_pe<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(ni, ks.a4[0].p, ks.f4[0].p, ks.f4[1].p);
-    if (f32 && nj > 0)
-        sphk::make_gravity_records<<<eltwise_grid(nj), 256, 0, ctx->stream>>>(nj, ks.a4[2].p, ks.d1[0].p, ks.f4[4].p,
-                                                                             ks.f4[5].p);
+    if (ni + nj > 0)
+        prepare_gravity<<<eltwise_grid((long long)ni + nj), 256, 0, ctx->stream>>>(
+            (const sph_GravityEPI *)(d + L.off_epi), ni, (const sph_GravityEPJ *)(d + L.off_epj), nj, ks.a4[0].p,
+            ks.f4[0].p, ks.f4[1].p, ks.a4[2].p, ks.d1[0].p, ks.f4[4].p, ks.f4[5].p, f32);
     if (!ks.items.empty()) {
         sphk::GravityArgs a{};
         a.i_pe = ks.a4[0].p;
@@ -926,9 +1024,9 @@ extern "C" int sph_dispatch_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
     }
     if (ni > 0)
         pack_gravity<<<eltwise_grid(32LL * ni), 256, 0, ctx->stream>>>(ni, ks.o[0].p, ks.o[1].p, ks.o[2].p, slices,
-                                                                      (sph_Gravity *)ks.d_out.p,
-                                                                      ctx->d_queue + 4 + K_GRAV);
-    return finish_dispatch(ctx, ks, n_walk, i_off, sizeof(sph_Gravity));
+                                                                      (sph_Gravity *)ks.h_out.p,
+                                                                      ctx->h_flags + K_GRAV);
+    return finish_dispatch(ctx, ks, n_walk, i_off);
 }
 
 extern "C" int sph_retrieve_gravity(sph_context *ctx, int32_t tag, int32_t n_walk, const int32_t *n_i,
@@ -939,11 +1037,21 @@ extern "C" int sph_retrieve_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
 }
 
 // ---------------------------------------------------------------- functors
+namespace {
+// A functor's dispatch is retrieved before the call returns.
+struct FunctorCall {
+    sph_context *ctx;
+    explicit FunctorCall(sph_context *c) : ctx(c) { ctx->in_functor = true; }
+    ~FunctorCall() { ctx->in_functor = false; }
+};
+}  // namespace
+
 extern "C" int sph_calc_density(sph_context *ctx, const sph_DensityEPI *epi, int32_t n_i,
                                 const sph_DensityEPJ *epj, int32_t n_j, sph_Density *force) {
     if (!ctx) return SPH_ERR_INVALID_ARGUMENT;
     if (n_i < 0 || n_j < 0 || (n_i && (!epi || !force)) || (n_j && !epj))
         return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "bad functor arguments");
+    const FunctorCall call(ctx);
     int st = sph_dispatch_density(ctx, 0, 1, &epi, &n_i, &epj, &n_j);
     if (st) return st;
     return sph_retrieve_density(ctx, 0, 1, &n_i, &force);
@@ -954,6 +1062,7 @@ extern "C" int sph_calc_hydro(sph_context *ctx, const sph_HydroEPI *epi, int32_t
     if (!ctx) return SPH_ERR_INVALID_ARGUMENT;
     if (n_i < 0 || n_j < 0 || (n_i && (!epi || !force)) || (n_j && !epj))
         return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "bad functor arguments");
+    const FunctorCall call(ctx);
     int st = sph_dispatch_hydro(ctx, 0, 1, &epi, &n_i, &epj, &n_j);
     if (st) return st;
     return sph_retrieve_hydro(ctx, 0, 1, &n_i, &force);
@@ -966,6 +1075,7 @@ int gravity_accumulate(sph_context *ctx, const sph_GravityEPI *epi, int32_t n_i,
     if (!ctx) return SPH_ERR_INVALID_ARGUMENT;
     if (n_i < 0 || n_ep < 0 || n_sp < 0 || (n_i && (!epi || !force)) || (n_ep && !epj) || (n_sp && !spj))
         return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "bad functor arguments");
+    const FunctorCall call(ctx);
     int st = sph_dispatch_gravity(ctx, 0, 1, &epi, &n_i, &epj, &n_ep, &spj, &n_sp);
     if (st) return st;
     std::vector<sph_Gravity> tmp((size_t)std::max(n_i, 1));
@@ -989,6 +1099,12 @@ extern "C" int sph_calc_gravity_ep(sph_context *ctx, const sph_GravityEPI *epi, 
 extern "C" int sph_calc_gravity_sp(sph_context *ctx, const sph_GravityEPI *epi, int32_t n_i,
                                    const sph_GravitySPJ *spj, int32_t n_j, sph_Gravity *force) {
     return gravity_accumulate(ctx, epi, n_i, nullptr, 0, spj, n_j, force);
+}
+
+// ---------------------------------------------------------------- bindings
+extern "C" void sph_member_pointers(const void *const *obj, int64_t n, int64_t offset, void **out) {
+    for (int64_t k = 0; k < n; ++k)
+        std::memcpy(&out[k], static_cast<const char *>(obj[k]) + offset, sizeof(void *));
 }
 
 // ---------------------------------------------------------------- layout

@@ -74,10 +74,21 @@ struct HostBuf {
     }
 };
 
+// A piece of a dispatch's inputs: n 8-byte words at src (pinned memory, or the
+// caller's), word dst of the device buffer.
+struct CopyPiece {
+    const unsigned long long *src;
+    long long dst;
+    int n;
+};
+
 // Buffers and dispatch state of one interaction kind (density/hydro/gravity).
 struct KindState {
     HostBuf<char> h_in, h_out;
-    DevBuf<char> d_in, d_out;
+    HostBuf<CopyPiece> h_pieces;
+    int n_pieces = 0;
+    bool in_place = false;             // some pieces are read from the caller's arrays
+    DevBuf<char> d_in;
     DevBuf<dbl4> a4[8];
     DevBuf<float4> f4[20];   // FP32C double-float records; 16..19 hydro mark records
     DevBuf<int> hl_list;               // rows of the density and hydro sums
@@ -132,8 +143,8 @@ struct KindState {
     void release() {
         h_in.release();
         h_out.release();
+        h_pieces.release();
         d_in.release();
-        d_out.release();
         for (auto &b : a4) b.release();
         for (auto &b : f4) b.release();
         hl_list.release();
@@ -157,9 +168,12 @@ struct sph_context {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     int *d_queue = nullptr;   // [0..2] work-queue counters, [3] density re-check count,
-                              // [4..6] finite flags, [7] density sweep queue,
+                              // [4..6] unused, [7] density sweep queue,
                               // [8] FP32C hydro rows that overflowed, [9] long items
-    int *h_flags = nullptr;   // pinned copies of the flags
+    int *h_flags = nullptr;   // pinned: per kind, non-finite values in the outputs
+    int pageable_access = 0;  // kernels may read pageable host memory in place
+    cudaEvent_t ev_read = nullptr;   // the callers' arrays of a dispatch have been read
+    bool in_functor = false;  // the dispatch in course is retrieved by the same call
     int grid[3][2] = {{0}};   // persistent grid per kind and precision
     int grid_stream = 0;      // persistent grid of the FP32C streamed density walk
     int grid_df = 0;          // resident blocks of the double-float hydro pass
@@ -174,12 +188,13 @@ extern const float AMB_TOL;
 int set_error(sph_context *ctx, int status, const char *fmt, ...);
 int cuda_error(sph_context *ctx, cudaError_t e, const char *what);
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items);
-void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s);
+void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s,
+                         bool longs = true);
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
-                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr);
+                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr, bool longs = true);
 void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
                            int n_max, cudaStream_t s, int *amb_total);
 void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
-                  int precision, cudaStream_t s, cudaEvent_t mid = nullptr, bool mid_external = false);
+                  int precision, cudaStream_t s, cudaEvent_t mid = nullptr, bool mid_external = false, bool longs = true);
 void launch_gravity(const sphk::GravityArgs &a, int precision, int grid, cudaStream_t s, int jtile);
 }  // namespace sphrt

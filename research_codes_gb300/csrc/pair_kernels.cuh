@@ -679,37 +679,33 @@ gravity_kernel(const GravityArgs a) {
 // Builders of the FP32C double-float records from FP64 arrays (one thread
 // per particle).  Each fills hi/lo pairs; aux lanes as documented at the
 // consumers above.
-// Density records; lo.w: h rounded up (the row radius; 0 without h).
+// Density records; lo.w: h rounded up.
 __global__ inline void make_density_records(int n, const dbl4 *pm, const dbl4 *vel, const double *h, float4 *phi,
                                             float4 *plo, float4 *vhi, float4 *vlo) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const dbl4 p = pm[k], v = vel[k];
-        const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
-        const float2 u = df_split(v.x), w = df_split(v.y), s = df_split(v.z);
-        phi[k] = make_float4(x.x, y.x, z.x, (float)p.w);
-        plo[k] = make_float4(x.y, y.y, z.y, h ? __double2float_ru(h[k]) : 0.0f);
-        vhi[k] = make_float4(u.x, w.x, s.x, 0.0f);
-        vlo[k] = make_float4(u.y, w.y, s.y, 0.0f);
+        float4 a, b;
+        row_record(pm[k], h[k], a, b);
+        phi[k] = a;
+        plo[k] = b;
+        velocity_record(vel[k], a, b);
+        vhi[k] = a;
+        vlo[k] = b;
     }
 }
 
 // Gravity records: hi = (x, y, z, mass), lo = (x, y, z, eps2).
+__device__ __forceinline__ void gravity_record(const dbl4 &p, double mass, double eps2, float4 &hi, float4 &lo) {
+    const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
+    hi = make_float4(x.x, y.x, z.x, (float)mass);
+    lo = make_float4(x.y, y.y, z.y, (float)eps2);
+}
 __global__ inline void make_gravity_records(int n, const dbl4 *pm, const double *eps2, float4 *phi, float4 *plo) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const dbl4 p = pm[k];
-        const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
-        phi[k] = make_float4(x.x, y.x, z.x, (float)p.w);
-        plo[k] = make_float4(x.y, y.y, z.y, (float)eps2[k]);
-    }
-}
-
-// The same from (x, y, z, eps2) packs without a mass (gravity i-particles).
-__global__ inline void make_gravity_records_pe(int n, const dbl4 *pe, float4 *phi, float4 *plo) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const dbl4 p = pe[k];
-        const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
-        phi[k] = make_float4(x.x, y.x, z.x, 0.0f);
-        plo[k] = make_float4(x.y, y.y, z.y, (float)p.w);
+        float4 a, b;
+        gravity_record(p, p.w, eps2[k], a, b);
+        phi[k] = a;
+        plo[k] = b;
     }
 }
 
@@ -717,25 +713,33 @@ __global__ inline void make_gravity_records_pe(int n, const dbl4 *pe, float4 *ph
 // bswt / 2), h2 = (rho, c_s, alpha, alpha_u), h3 = (thrm, eta); 1/h, h^-4 and
 // P Omega / rho^2 also as hi/lo splits of their FP64 values; and the mark
 // records (hydro_mark_records).
-__global__ inline void make_hydro_records(int n, const dbl4 *pm, const dbl4 *vel, const dbl4 *h1, const dbl4 *h2,
-                                          const double2 *h3, float4 *phi, float4 *plo, float4 *vhi, float4 *vlo,
-                                          float4 *g1, float4 *g2, float4 *g3, float4 *g4, float4 *mp, float4 *mv) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const dbl4 p = pm[k], v = vel[k], a = h1[k], b = h2[k];
-        const double2 c = h3[k];
+struct HydroRecords {
+    float4 phi, plo, vhi, vlo, g1, g2, g3, g4;
+    __device__ __forceinline__ void fill(const dbl4 &p, const dbl4 &v, const dbl4 &a, const dbl4 &b, const double2 &c) {
         const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
         const float2 u = df_split(v.x), w = df_split(v.y), s = df_split(v.z);
         const float2 P = df_split(a.y), T = df_split(c.x), Q = df_split(a.z);
         const double h4d = (a.x * a.x) * (a.x * a.x);
         const float2 H = df_split(a.x), H4 = df_split(h4d), M = df_split(p.w);
-        phi[k] = make_float4(x.x, y.x, z.x, M.x);
-        plo[k] = make_float4(x.y, y.y, z.y, M.y);
-        vhi[k] = make_float4(u.x, w.x, s.x, H.x);
-        vlo[k] = make_float4(u.y, w.y, s.y, H4.x);
-        g1[k] = make_float4(P.x, P.y, Q.x, (float)a.w);
-        g2[k] = make_float4((float)b.x, (float)b.y, (float)b.z, (float)b.w);
-        g3[k] = make_float4(T.x, T.y, (float)c.y, Q.y);
-        g4[k] = make_float4(H.x, H.y, H4.x, H4.y);
+        phi = make_float4(x.x, y.x, z.x, M.x);
+        plo = make_float4(x.y, y.y, z.y, M.y);
+        vhi = make_float4(u.x, w.x, s.x, H.x);
+        vlo = make_float4(u.y, w.y, s.y, H4.x);
+        g1 = make_float4(P.x, P.y, Q.x, (float)a.w);
+        g2 = make_float4((float)b.x, (float)b.y, (float)b.z, (float)b.w);
+        g3 = make_float4(T.x, T.y, (float)c.y, Q.y);
+        g4 = make_float4(H.x, H.y, H4.x, H4.y);
+    }
+};
+__global__ inline void make_hydro_records(int n, const dbl4 *pm, const dbl4 *vel, const dbl4 *h1, const dbl4 *h2,
+                                          const double2 *h3, float4 *phi, float4 *plo, float4 *vhi, float4 *vlo,
+                                          float4 *g1, float4 *g2, float4 *g3, float4 *g4, float4 *mp, float4 *mv) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const dbl4 p = pm[k], v = vel[k], a = h1[k], b = h2[k];
+        HydroRecords r;
+        r.fill(p, v, a, b, h3[k]);
+        phi[k] = r.phi; plo[k] = r.plo; vhi[k] = r.vhi; vlo[k] = r.vlo;
+        g1[k] = r.g1; g2[k] = r.g2; g3[k] = r.g3; g4[k] = r.g4;
         float4 m0, m1;
         hydro_mark_records(p, v, a.x, b.y, m0, m1);
         mp[k] = m0;

@@ -575,13 +575,24 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
     }
 }
 
-// Positions as double-float records with h (rounded up; 0 without h) in lo.w.
+// Position and mass as a double-float record with h (rounded up) in lo.w.
+__device__ __forceinline__ void row_record(const dbl4 &p, double h, float4 &hi, float4 &lo) {
+    const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
+    hi = make_float4(x.x, y.x, z.x, (float)p.w);
+    lo = make_float4(x.y, y.y, z.y, __double2float_ru(h));
+}
+__device__ __forceinline__ void velocity_record(const dbl4 &v, float4 &hi, float4 &lo) {
+    const float2 x = df_split(v.x), y = df_split(v.y), z = df_split(v.z);
+    hi = make_float4(x.x, y.x, z.x, 0.0f);
+    lo = make_float4(x.y, y.y, z.y, 0.0f);
+}
+
 __global__ inline void make_row_records(int n, const dbl4 *pm, const double *h, float4 *hi, float4 *lo) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const dbl4 p = pm[k];
-        const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
-        hi[k] = make_float4(x.x, y.x, z.x, (float)p.w);
-        lo[k] = make_float4(x.y, y.y, z.y, h ? __double2float_ru(h[k]) : 0.0f);
+        float4 a, b;
+        row_record(pm[k], h[k], a, b);
+        hi[k] = a;
+        lo[k] = b;
     }
 }
 

@@ -157,12 +157,38 @@ class calcGravity:
 
 # ---- multiwalk Dispatch / Retrieve -------------------------------------------
 
+# Where a numpy array object keeps its data pointer: the first member after the
+# object header (PyArrayObject's layout, what numpy's PyArray_DATA reads).
+# Checked on an array; without it every address goes through ndarray.ctypes,
+# a microsecond each.
+_DATA_OFFSET = object.__basicsize__
+_probe = np.zeros(3)
+if ctypes.c_void_p.from_address(id(_probe) + _DATA_OFFSET).value != _probe.ctypes.data:
+    _DATA_OFFSET = None
+
+
 def _ptr_array(arrs):
-    return (ctypes.c_void_p * max(len(arrs), 1))(*[a.ctypes.data if len(a) else 0 for a in arrs])
+    """Addresses of the arrays (0 for empty ones) as a C array."""
+    n = len(arrs)
+    out = (ctypes.c_void_p * max(n, 1))()
+    if _DATA_OFFSET is None or any(type(a) is not np.ndarray for a in arrs):
+        out[:n] = [a.ctypes.data if len(a) else 0 for a in arrs]
+        return out
+    obj = np.fromiter(map(id, arrs), np.uintp, n)
+    load().sph_member_pointers(ctypes.c_void_p(obj.ctypes.data), n, _DATA_OFFSET, out)
+    if not all(map(len, arrs)):
+        for k, a in enumerate(arrs):
+            if not len(a):
+                out[k] = 0
+    return out
 
 
 def _count_array(counts):
-    return (ctypes.c_int32 * max(len(counts), 1))(*[int(c) for c in counts])
+    n = len(counts)
+    out = (ctypes.c_int32 * max(n, 1))()
+    if n:
+        np.frombuffer(out, np.int32)[:n] = np.asarray(counts, np.int64)
+    return out
 
 
 def DispatchKernel_Dens(ctx, tag, n_walk, epi, n_epi, epj, n_epj):
