@@ -102,11 +102,42 @@ int pair_grid(const sph_context *ctx, int kind, int precision, int n_items) {
     return std::max(1, std::min(full, need));
 }
 
+// Long items run beside the others: first(side stream), then rest(s), joined
+// after both (in a capture the two become parallel branches).  One block per
+// SM takes half of its registers; the items of the usual kind fill the rest.
+template <class A, class B>
+static void beside(const LongSide &side, cudaStream_t s, A first, B rest) {
+    cudaEventRecord(side.fork, s);
+    cudaStreamWaitEvent(side.stream, side.fork, 0);
+    first(side.stream);
+    cudaEventRecord(side.join, side.stream);
+    rest(s);
+    cudaStreamWaitEvent(s, side.join, 0);
+}
+
 // The queued long items: a block each.
 template <int KIND>
 static void mark_long(const sph_context *ctx, const sphk::MarkArgs &m, int n_max, cudaStream_t s) {
     constexpr int W = KIND == sphk::ROWS_DENSITY ? sphk::MARK_LONG_WARPS : sphk::HYDRO_LONG_WARPS;
-    sphk::mark_rows<KIND, W, true><<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), W * 32, 0, s>>>(m);
+    sphk::mark_rows<KIND, W, true><<<std::max(1, std::min(n_max, ctx->sm_count)), W * 32, 0, s>>>(m);
+}
+
+// Rows of the items of m and of its long items: beside them where the caller
+// has queued them and gives a side stream, else after the kernel that queues
+// them (push_long).  No long items without either.
+template <int KIND>
+static void mark_all(const sph_context *ctx, const sphk::MarkArgs &m, int grid, int n_max, cudaStream_t s,
+                     const LongSide *side) {
+    auto usual = [&](cudaStream_t t) {
+        sphk::mark_rows<KIND, PAIR_WARPS><<<grid, PAIR_WARPS * 32, 0, t>>>(m);
+    };
+    auto lng = [&](cudaStream_t t) { mark_long<KIND>(ctx, m, n_max, t); };
+    if (side) {
+        beside(*side, s, lng, usual);
+    } else {
+        usual(s);
+        if (m.push_long) lng(s);
+    }
 }
 
 // FP64 recomputation of the FP32C results queued as ambiguous (their number
@@ -139,17 +170,16 @@ static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs 
     recheck_density(ctx, a, n_max, s, amb_total);
 }
 
-// Density rows of the items of m (longs: some may be long).
+// Density rows of the items of m.
 void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s,
-                         bool longs) {
-    sphk::mark_rows<sphk::ROWS_DENSITY, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-    if (longs) mark_long<sphk::ROWS_DENSITY>(ctx, m, n_max, s);
+                         const LongSide *side) {
+    mark_all<sphk::ROWS_DENSITY>(ctx, m, mark_grid, n_max, s, side);
 }
 
 // Rows of the items of m, then the density sums over them.
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
-                    int n_max, int precision, cudaStream_t s, int *amb_total, bool longs) {
-    launch_mark_density(ctx, m, mark_grid, n_max, s, longs);
+                    int n_max, int precision, cudaStream_t s, int *amb_total, const LongSide *side) {
+    launch_mark_density(ctx, m, mark_grid, n_max, s, side);
     launch_density_sums(ctx, a, n_max, precision, s, amb_total);
 }
 
@@ -157,10 +187,14 @@ void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_gr
 // over the items of w (those with long lists a block each), the sweep of the queued particles (re-walks of few) and
 // the FP64 recomputation of the ambiguous ones.
 void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
-                           int n_max, cudaStream_t s, int *amb_total) {
-    sphk::density_stream<PAIR_WARPS><<<ctx->grid_stream, PAIR_WARPS * 32, 0, s>>>(w);
-    sphk::density_stream<sphk::STREAM_LONG_WARPS, true>
-        <<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), sphk::STREAM_LONG_WARPS * 32, 0, s>>>(w);
+                           int n_max, cudaStream_t s, int *amb_total, const LongSide &side) {
+    beside(
+        side, s,
+        [&](cudaStream_t t) {
+            sphk::density_stream<sphk::STREAM_LONG_WARPS, true>
+                <<<std::max(1, std::min(n_max, ctx->sm_count)), sphk::STREAM_LONG_WARPS * 32, 0, t>>>(w);
+        },
+        [&](cudaStream_t t) { sphk::density_stream<PAIR_WARPS><<<ctx->grid_stream, PAIR_WARPS * 32, 0, t>>>(w); });
     if (sweep)
         sphk::density_sweep<false><<<std::max(1, std::min(n_max, ctx->sm_count * 6)), sphk::DSWEEP_THREADS, 0, s>>>(
             a, a.ovf, a.n_ovf, n_max, nullptr);
@@ -173,15 +207,12 @@ void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bo
 // (optional) is recorded between the two parts (as an external record node
 // when mid_external: inside a stream capture).
 void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
-                  int precision, cudaStream_t s, cudaEvent_t mid, bool mid_external, bool longs) {
+                  int precision, cudaStream_t s, cudaEvent_t mid, bool mid_external, const LongSide *side) {
     const bool f64 = precision == SPH_PREC_FP64;
-    if (f64) {
-        sphk::mark_rows<sphk::ROWS_HYDRO64, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-        if (longs) mark_long<sphk::ROWS_HYDRO64>(ctx, m, a.n_i, s);
-    } else {
-        sphk::mark_rows<sphk::ROWS_HYDRO32, PAIR_WARPS><<<mark_grid, PAIR_WARPS * 32, 0, s>>>(m);
-        if (longs) mark_long<sphk::ROWS_HYDRO32>(ctx, m, a.n_i, s);
-    }
+    if (f64)
+        mark_all<sphk::ROWS_HYDRO64>(ctx, m, mark_grid, a.n_i, s, side);
+    else
+        mark_all<sphk::ROWS_HYDRO32>(ctx, m, mark_grid, a.n_i, s, side);
     if (mid) cudaEventRecordWithFlags(mid, s, mid_external ? cudaEventRecordExternal : cudaEventRecordDefault);
     if (a.n_i <= 0) return;
     if (f64) {
@@ -843,6 +874,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         m.queue = ctx->d_queue + K_DENS;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 7;
         m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
+        m.push_long = longest(n_epj, n_walk) > LONG_NJ;
         sphk::DensityArgs a{};
         a.i_pm = ks.a4[0].p; a.i_vel = ks.a4[1].p; a.i_id = ks.id[0].p; a.i_ksr = ks.d1[0].p; a.i_rs = ks.d1[1].p;
         a.j_pm = ks.a4[2].p; a.j_vel = ks.a4[3].p; a.j_id = ks.id[1].p;
@@ -861,7 +893,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         a.amb_cap = cap;
         a.amb_tol = AMB_TOL;
         launch_density(ctx, m, pair_grid(ctx, K_DENS, ctx->prm.precision, m.n_items), a, ni, ctx->prm.precision,
-                       ctx->stream, nullptr, longest(n_epj, n_walk) > LONG_NJ);
+                       ctx->stream);
     }
     if (ni > 0)
         pack_density<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(
@@ -926,7 +958,8 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         m.j_off = (const int *)(d + L.off_joff);
         m.queue = ctx->d_queue + K_HYDRO;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 8;
-        m.long_items = f64 ? ks.long_items.p : nullptr; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
+        m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
+        m.push_long = f64 && longest(n_epj, n_walk) > LONG_NJ;
         m.o_vsmx = ks.o[3].p;
         m.sv_skip = 1;
         sphk::HydroArgs a{};
@@ -946,7 +979,7 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         m.i_id = a.i_id; m.j_id = a.j_id; m.fi = a.fi; m.fj = a.fj; m.fi_g2 = a.fi_g2; m.fj_g2 = a.fj_g2;
         m.i_pm = a.i_pm; m.i_vel = a.i_vel; m.i_h2 = a.i_h2; m.j_pm = a.j_pm; m.j_vel = a.j_vel; m.j_h2 = a.j_h2;
         launch_hydro(ctx, m, pair_grid(ctx, K_HYDRO, ctx->prm.precision, m.n_items), a, ctx->prm.precision,
-                     ctx->stream, nullptr, false, f64 && longest(n_epj, n_walk) > LONG_NJ);
+                     ctx->stream);
     }
     if (ni > 0)
         pack_hydro<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(

@@ -187,14 +187,21 @@ namespace sphrt {
 extern const float AMB_TOL;
 int set_error(sph_context *ctx, int status, const char *fmt, ...);
 int cuda_error(sph_context *ctx, cudaError_t e, const char *what);
+// A stream for long items, with the events that fork it from the caller's
+// stream and join it again.
+struct LongSide {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items);
 void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s,
-                         bool longs = true);
+                         const LongSide *side = nullptr);
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
-                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr, bool longs = true);
+                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr, const LongSide *side = nullptr);
 void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
-                           int n_max, cudaStream_t s, int *amb_total);
+                           int n_max, cudaStream_t s, int *amb_total, const LongSide &side);
 void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
-                  int precision, cudaStream_t s, cudaEvent_t mid = nullptr, bool mid_external = false, bool longs = true);
+                  int precision, cudaStream_t s, cudaEvent_t mid = nullptr, bool mid_external = false,
+                  const LongSide *side = nullptr);
 void launch_gravity(const sphk::GravityArgs &a, int precision, int grid, cudaStream_t s, int jtile);
 }  // namespace sphrt

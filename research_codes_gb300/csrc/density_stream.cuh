@@ -67,11 +67,9 @@ struct StreamArgs {
     int nbr_cap = 0;
     int nbr_warps = 0;
     float nbr_slack = 1.0f;
-    // items left to the LONG form (null: none) and their number; the listed
-    // pairs of the walk, which say what a long list is
-    WorkItem *long_items;
-    int *n_long;
-    const long long *pairs;
+    // items of the LONG form, and their number
+    const WorkItem *long_items;
+    const int *n_long;
     // when set: pair evaluations performed, [0] the three density passes
     // ((j-entries kept by the support test x i-particles) of the swept passes
     // plus the list entries of the listed ones), [1] the gradient pass
@@ -134,13 +132,13 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
     const unsigned lt = lanemask_lt();
     const int n_items = LONG ? *a.n_long : (a.n_items_dev ? *a.n_items_dev : a.n_items);
     const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
-    const int gw = LONG ? blockIdx.x : blockIdx.x * WARPS + wid;
+    // (LONG: the last gridDim.x slots, one per block)
+    const int gw = LONG ? a.nbr_warps - gridDim.x + blockIdx.x : blockIdx.x * WARPS + wid;
     // the ring (LONG: the compacted entries)
     const float *bx = LONG ? l_x : s_rx[LONG ? 0 : wid], *by = LONG ? l_y : s_ry[LONG ? 0 : wid];
     const float *bz = LONG ? l_z : s_rz[LONG ? 0 : wid], *bm = LONG ? l_m : s_rm[LONG ? 0 : wid];
     const int *bj = LONG ? l_j : s_j[LONG ? 0 : wid];
     int next = blockIdx.x;   // LONG
-    const int long_nj = a.pairs ? long_list(*a.pairs) : 0;
     // this lane's neighbour list: entry c at a.nbr[nlb + c * 32]
     const bool has_nl = a.nbr != nullptr && gw < a.nbr_warps;
     const int nlb = has_nl ? gw * a.nbr_cap * 32 + lane : 0;
@@ -165,10 +163,6 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
         const ItemRef r = decode(wi, a.j_off, a.i_list, lane);
         const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;
 
-        if (!LONG && a.long_items && nj > long_nj) {
-            if (lane == 0) a.long_items[atomicAdd(a.n_long, 1)] = wi;
-            continue;
-        }
         // i-particle relative to the centre particle c (velocity, id, mass
         // and search radius are read where they are used, keeping the
         // registers of the passes free)

@@ -24,11 +24,11 @@ namespace sphk {
 constexpr int ROW_CAP = 128;
 static_assert(ROW_CAP % 32 == 0, "eight lanes read a row four entries at a time");
 // Items with longer lists than this are taken by a whole block (the LONG forms
-// of mark_rows and density_stream).  A warp streams ~8e7 entries per second
-// and the chip ~5e11 listed pairs: beyond pairs / 16384 entries one warp's item
-// lasts about a third of the whole walk's time.
+// of mark_rows and density_stream).  On a full SM a warp streams ~1.6e7 entries
+// per second, the chip ~5e11 listed pairs: beyond pairs / 65536 entries one
+// warp's item lasts about half of the whole walk's time.
 __device__ __forceinline__ int long_list(long long pairs) {
-    return (int)min(max(pairs >> 14, 768LL), 1LL << 30);
+    return (int)min(max(pairs >> 16, 768LL), 1LL << 30);
 }
 constexpr int MARK_LONG_WARPS = 16, HYDRO_LONG_WARPS = 8;
 // Radii outside this range (or NaN) are left to the sweep: their squares
@@ -96,9 +96,12 @@ struct MarkArgs {
     int2 *info;              // per particle: entries (> ROW_CAP: none, see ovf), walk
     int2 *ovf;               // particles without a row: (particle, walk)
     int *n_ovf;
-    WorkItem *long_items;    // items left to the LONG form (null: none), and their number
+    WorkItem *long_items;    // items of the LONG form, and their number
     int *n_long;
-    const long long *pairs;  // the walks' listed pairs (null: lists beyond long_nj are long)
+    // push_long: the kernel itself moves items with lists beyond long_nj (with
+    // pairs set: beyond long_list of the walks' listed pairs) to that queue
+    bool push_long;
+    const long long *pairs;
     int long_nj;
     // hydro: velocity and sound speed in FP32
     const float4 *i_v, *j_v;
@@ -244,7 +247,7 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
             r.ii = a.i_list ? a.i_list[k] : k;
             if (threadIdx.x < 32) s_cnt[threadIdx.x] = 0;
             __syncthreads();
-        } else if (a.long_items && r.nj > long_nj) {
+        } else if (a.push_long && r.nj > long_nj) {
             if (lane == 0) a.long_items[atomicAdd(a.n_long, 1)] = wi;
             continue;
         }

@@ -437,11 +437,13 @@ __device__ __forceinline__ int cost_bucket(int nj, int sz) {
 // Histogram of the items of all walks over the cost classes (bkt[0..NBKT),
 // zero on entry).
 __global__ void item_buckets(int n, const int *n_walks, const int *i_count, const int *j_cnt, int chunk,
-                             int split_nj, int *bkt) {
+                             int split_nj, const long long *pairs, bool longs, int *bkt) {
     const int nw = *n_walks;
+    const int long_nj = longs ? sphk::long_list(*pairs) : 0x7fffffff;
     GRID_STRIDE(k, n) {
         if (k < nw) {
             const int ni = i_count[k], nj = j_cnt[k];
+            if (nj > long_nj) continue;
             const int ch = item_chunk(nj, chunk, split_nj);
             const int full = ni / ch, rest = ni - full * ch;
             if (full) atomicAdd(&bkt[cost_bucket(nj, ch)], full);
@@ -481,15 +483,16 @@ __global__ void bucket_offsets(int *bkt, int heavy) {
 
 // Number of light items (class below the heavy ones) of each walk.
 __global__ void light_counts(int n, const int *n_walks, const int *i_count, const int *j_cnt, int chunk,
-                             int split_nj, const int *bkt, int *lc) {
+                             int split_nj, const long long *pairs, bool longs, const int *bkt, int *lc) {
     const int nw = *n_walks;
     const int bh = bkt[2 * NBKT];
+    const int long_nj = longs ? sphk::long_list(*pairs) : 0x7fffffff;
     GRID_STRIDE(k, n + 1) {
         int c = 0;
         if (k < nw) {
             const int ni = i_count[k], nj = j_cnt[k];
             const int ch = item_chunk(nj, chunk, split_nj);
-            for (int c0 = 0; c0 < ni; c0 += ch) c += cost_bucket(nj, min(ch, ni - c0)) < bh ? 1 : 0;
+            for (int c0 = 0; c0 < ni && nj <= long_nj; c0 += ch) c += cost_bucket(nj, min(ch, ni - c0)) < bh ? 1 : 0;
         }
         lc[k] = c;
     }
@@ -499,34 +502,40 @@ __global__ void light_counts(int n, const int *n_walks, const int *i_count, cons
 // leaves offsets that run past the list arrays: no pair kernel may read
 // them, so the evaluation gets no work items (it is repeated, or reported).
 __global__ void drop_items_on_overflow(int *scal) {
-    if (scal[S_ERROR] & (E_LISTCAP | E_STACK)) scal[S_NITEMS] = 0;
+    if (scal[S_ERROR] & (E_LISTCAP | E_STACK)) {
+        scal[S_NITEMS] = 0;
+        scal[S_NLONG] = 0;
+    }
 }
 
 __global__ void fill_items(int n, const int *n_walks, const int *i_first, const int *i_count, int chunk,
                            int split_nj, const int *j_cnt, int *bkt, const int *light_off, WorkItem *items,
-                           int *n_items, long long *pairs) {
+                           int *n_items, const long long *pairs, WorkItem *longs, int *n_long) {
     const int nw = *n_walks;
     const int bh = bkt[2 * NBKT];
     const int n_heavy = bkt[2 * NBKT + 1];
-    long long local = 0;
+    const int long_nj = longs ? sphk::long_list(*pairs) : 0x7fffffff;
     GRID_STRIDE(k, n) {
         if (k < nw) {
             const int ni = i_count[k];
             const int nj = j_cnt[k];
             const int ch = item_chunk(nj, chunk, split_nj);
             int lpos = n_heavy + light_off[k];
+            int qpos = nj > long_nj ? atomicAdd(n_long, (ni + ch - 1) / ch) : 0;
             for (int c0 = 0; c0 < ni; c0 += ch) {
                 const int sz = min(ch, ni - c0);
+                const WorkItem it = make_int4(k, i_first[k] + c0, sz, nj * sz);
+                if (nj > long_nj) {
+                    longs[qpos++] = it;
+                    continue;
+                }
                 const int b = cost_bucket(nj, sz);
                 const int pos = (b >= bh) ? atomicAdd(&bkt[NBKT + b], 1) : lpos++;
-                items[pos] = make_int4(k, i_first[k] + c0, sz, nj * sz);
+                items[pos] = it;
             }
-            local += (long long)ni * nj;
         }
         if (k == 0) *n_items = n_heavy + light_off[nw];
     }
-    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd((unsigned long long *)pairs, (unsigned long long)local);
 }
 
 // particles still iterating (rs != 0) -> flags for the index list
@@ -551,10 +560,12 @@ __global__ void walk_particles(int n, const int *flag, const int *scan, int firs
     scal[S_NITER] = total;
     scal[S_SMALL] = small;
     scal[S_DOVF] = small ? total : 0;
-    scal[S_NLONG] = 0;
 }
 __global__ void drop_items_if_small(int *scal) {
-    if (scal[S_SMALL]) scal[S_NITEMS] = 0;
+    if (scal[S_SMALL]) {
+        scal[S_NITEMS] = 0;
+        scal[S_NLONG] = 0;
+    }
 }
 
 // the index-list segment of each active walk; when the walk is small, its
@@ -1036,6 +1047,10 @@ struct sph_system {
     bool glist_forked = false;
     long long rewalk_kernels[2] = {0, 0};   // kernel nodes of the loop body (force / step graph)
     int capturing = -1;                     // graph being captured: 0 force, 1 step
+    // the long items' streams: a captured stream stays in its graph to the end
+    // of the capture, so the loop body has one of its own
+    sphrt::LongSide sides[2];
+    const sphrt::LongSide &long_side() const { return sides[st_override && st_override == body_stream]; }
     cudaStream_t st() const { return st_override ? st_override : ctx->stream; }
     Persist persist(int k) {
         Persist p;
@@ -1102,7 +1117,7 @@ int alloc_all(sph_system *s) {
     s->amb_cap = std::max<int>(1024, s->n / 16);
     e |= s->amb.ensure(s->amb_cap) | s->r_info.ensure(n);
     e |= s->long_items.ensure(n) | s->w_csmax.ensure(n);
-    s->nbr_warps = s->ctx->grid_stream * PAIR_WARPS;
+    s->nbr_warps = s->ctx->grid_stream * PAIR_WARPS + s->ctx->sm_count;   // and the blocks of the long items
     e |= s->nbr.ensure((size_t)s->nbr_warps * NBR_CAP * 32);
     DevBuf<int> *i1[] = {&s->gflag, &s->groot, &s->gscan, &s->group_node, &s->group_first, &s->group_count,
                          &s->aflag, &s->ascan, &s->a_node, &s->a_first, &s->a_count};
@@ -1401,8 +1416,10 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
     }
     r = exclusive_scan(s, L.tlcnt.p, L.tloff.p, L.task_cap + 1, builder);
     if (r) return r;
-    sphtree::group_lists<<<grid_for(n + 1), 256, 0, st>>>(n, s->walk_num[kind], L.toff.p, L.tloff.p,
-                                                         L.task_cap, s->loff[kind].p, s->lcnt[kind].p);
+    const int *ifirst = item_first ? item_first : s->walk_first[kind];
+    const int *icount = item_count ? item_count : s->walk_count[kind];
+    sphtree::group_lists<<<grid_for(n + 1), 256, 0, st>>>(n, s->walk_num[kind], L.toff.p, L.tloff.p, L.task_cap,
+                                                         icount, s->loff[kind].p, s->lcnt[kind].p, pairs);
     const int lslot = kind == 0 ? L_LIST_D : (kind == 1 ? L_LIST_H : (kind == 2 ? L_LIST_G : L_LIST_R));
     if (eager) {
         list_total<<<1, 1, 0, st>>>(n, s->lcnt[kind].p, s->loff[kind].p, (long long)1 << 62, sc, s->lscal.p, lslot);
@@ -1433,25 +1450,26 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
             return sphrt::set_error(s->ctx, SPH_ERR_CUDA, "list pool allocation of %lld chunks failed", pool_grow_to);
         L.lpool_chunks = std::min((long long)(L.lpool.cap / sphtree::LIST_CHUNK), MAX_POOL_CHUNKS);
     }
-    // work items
-    const int *ifirst = item_first ? item_first : s->walk_first[kind];
-    const int *icount = item_count ? item_count : s->walk_count[kind];
+    // work items; those of long lists (density and hydro) in a queue of their own
+    WorkItem *longs = (kind == 2) ? nullptr : s->long_items.p;
+    if (longs) CUDA_TRY(cudaMemsetAsync(sc + S_NLONG, 0, sizeof(int), st));
     // density and hydro walks with long lists are split (their pair loops
     // drop most of the list); gravity lists are uniform and kept whole
     const int split_nj = (kind == 2) ? (1 << 30) : (s->prm.item_split_nj > 0 ? s->prm.item_split_nj : ITEM_SPLIT_NJ);
     int *bkt = sc + S_BKT;
     CUDA_TRY(cudaMemsetAsync(bkt, 0, sizeof(int) * (2 * NBKT + 2), st));
-    item_buckets<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj, bkt);
+    item_buckets<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj, pairs,
+                                              longs != nullptr, bkt);
     bucket_offsets<<<1, 32, 0, st>>>(bkt, kind == 2 ? 0 : (s->prm.heavy_classes >= 0 ? s->prm.heavy_classes
                                                                                    : SPH_HEAVY_CLASSES));
     // light items in walk order: per-walk counts (the task arrays are free
     // again once the lists are built) and their scan
     light_counts<<<grid_for(n + 1), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj,
-                                                  bkt, L.tcnt.p);
+                                                  pairs, longs != nullptr, bkt, L.tcnt.p);
     r = exclusive_scan(s, L.tcnt.p, L.toff.p, n + 1, builder);
     if (r) return r;
     fill_items<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], ifirst, icount, chunk, split_nj, s->lcnt[kind].p,
-                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs);
+                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, sc + S_NLONG);
     drop_items_on_overflow<<<1, 1, 0, st>>>(sc);
     return SPH_OK;
 }
@@ -1501,7 +1519,6 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
     m.i_list = s->ulist.p;
     m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
     m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG;
-    m.pairs = s->lscal.p + (first ? L_PAIRS_D1 : L_PAIRS_D);
     sphk::DensityArgs a{};
     a.n_eval = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_D1) : nullptr;
     a.n_pass = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_DLISTED) : nullptr;
@@ -1542,12 +1559,12 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
         w.nbr_cap = NBR_CAP;
         w.nbr_warps = s->nbr_warps;
         w.nbr_slack = lists ? s->prm.density_list_slack : 1.0f;
-        w.long_items = m.long_items; w.n_long = m.n_long; w.pairs = m.pairs;
+        w.long_items = m.long_items; w.n_long = m.n_long;
         w.n_eval = a.n_eval; w.n_pass = a.n_pass;
-        sphrt::launch_density_stream(ctx, w, !first, a, n, st, s->scal.p + S_AMBTOT);
+        sphrt::launch_density_stream(ctx, w, !first, a, n, st, s->scal.p + S_AMBTOT,
+                                     s->long_side());
     } else {
-        sphrt::launch_density(ctx, m, ctx->grid[0][0], a, n, ctx->prm.precision, st,
-                              nullptr);
+        sphrt::launch_density(ctx, m, ctx->grid[0][0], a, n, ctx->prm.precision, st, nullptr, &s->long_side());
     }
     if (first) phase_event(s, EV_DENSK_E, st);
     commit_density<<<grid_for(n), 256, 0, st>>>(n, s->rs.p, tmp, out, s->scal.p);
@@ -1756,7 +1773,6 @@ int hydro_phase(sph_system *s, bool eager) {
     // empty; no particle without a row and no long item yet
     CUDA_TRY(cudaMemsetAsync(s->r_info.p, 0, sizeof(int2) * (size_t)n, st));
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_HOVF, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_NLONG, 0, sizeof(int), st));
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
     if (s->prm.hydro_signal_skip != 0)
         walk_csmax<<<ctx->sm_count * 8, CSMAX_THREADS, 0, st>>>(s->walk_num[1], s->loff[1].p, s->jidx[1].p, s->f_mv.p,
@@ -1768,7 +1784,7 @@ int hydro_phase(sph_system *s, bool eager) {
     m.items = s->ls[0].items.p; m.n_items_dev = s->scal.p + S_NITEMS;
     m.j_off = s->loff[1].p; m.j_idx = s->jidx[1].p; m.queue = s->scal.p + S_QUEUE;
     m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_HOVF;
-    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG; m.pairs = s->lscal.p + L_PAIRS_H;
+    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG;
     m.i_id = s->id[0].p; m.j_id = m.i_id;
     m.fi = sphk::F32Part{s->f_phi.p, s->f_plo.p, s->f_vhi.p, s->f_vlo.p};
     m.fj = m.fi;
@@ -1796,7 +1812,7 @@ int hydro_phase(sph_system *s, bool eager) {
     a.rows = m.rows; a.info = m.info; a.ovf = m.ovf; a.n_ovf = m.n_ovf; a.n_i = n;
     a.mi_p = m.i_hi; a.mi_l = m.i_lo; a.mj_p = m.j_hi; a.mj_l = m.j_lo;
     sphrt::launch_hydro(ctx, m, ctx->grid[1][ctx->prm.precision == SPH_PREC_FP64], a, ctx->prm.precision, st,
-                        s->ev[EV_HK_MID], s->capturing >= 0);
+                        s->ev[EV_HK_MID], s->capturing >= 0, &s->long_side());
     phase_event(s, EV_HK_E, st);
     AlphaParams ap{s->prm.alpha_max, s->prm.alpha_min, s->prm.alphu_max, s->prm.alphu_min};
     hydro_writeback<<<grid_for(n), 256, 0, st>>>(
@@ -1982,6 +1998,13 @@ extern "C" int sph_system_create(sph_context *ctx, int64_t n, const sph_system_p
     cudaStreamCreateWithFlags(&s->side_stream, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming);
+    for (sphrt::LongSide &l : s->sides)
+        if (cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&l.fork, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&l.join, cudaEventDisableTiming) != cudaSuccess) {
+            sph_system_destroy(s);
+            return sphrt::set_error(ctx, SPH_ERR_CUDA, "streams of a system");
+        }
     cudaMemset(s->scal.p, 0, sizeof(int) * S_NI);
     cudaMemset(s->dscal.p, 0, sizeof(double) * D_NI);
     if (s->prm.quadrupole) {   // leaves keep Q = 0 (the refit writes internal nodes only)
@@ -2006,6 +2029,11 @@ extern "C" int sph_system_destroy(sph_system *s) {
     if (s->side_stream) cudaStreamDestroy(s->side_stream);
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
+    for (sphrt::LongSide &l : s->sides) {
+        if (l.stream) cudaStreamDestroy(l.stream);
+        if (l.fork) cudaEventDestroy(l.fork);
+        if (l.join) cudaEventDestroy(l.join);
+    }
     for (int k = 0; k < 2; ++k) {
         s->pos[k].release(); s->vel[k].release(); s->vel2[k].release(); s->id[k].release();
         s->istar[k].release(); s->orig[k].release(); s->uene[k].release(); s->uene2[k].release();
@@ -2717,7 +2745,8 @@ extern "C" int sph_system_adjoint_forces(sph_system *s, const double *seed, doub
     m.items = s->adj_items.p; m.n_items = n_items;
     m.j_off = as.d_off; m.j_idx = as.d_idx; m.queue = s->scal.p + S_QUEUE;
     m.rows = s->adj_rows.p; m.info = s->adj_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
-    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG; m.pairs = s->lscal.p + L_PAIRS_D1;
+    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG; m.push_long = true;
+    m.pairs = s->lscal.p + L_PAIRS_D1;
     sphrt::launch_mark_density(ctx, m, sphrt::pair_grid(ctx, 0, SPH_PREC_FP64, n_items), n, st);
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
     const int eg = grid_for(n), rg = std::min(grid_for(8LL * n, 128), 16 * ctx->sm_count);

@@ -700,16 +700,22 @@ list_tasks(ListArgs a, int *task_count, const int *task_off, int2 *tasks, int ta
 // consecutive): off[g] = task_loff[task_off[g]], cnt[g] = its entries.
 // Entries g in [n_groups, n] get the total and 0.
 // Task offsets beyond the task capacity (an overflow already flagged as an
-// error) are clamped to it.
+// error) are clamped to it.  The listed pairs, sum of i_count[g] cnt[g], are
+// added to *pairs.
 __global__ void group_lists(int n, const int *n_groups, const int *task_off, const int *task_loff, int task_cap,
-                            int *off, int *cnt) {
+                            const int *i_count, int *off, int *cnt, long long *pairs) {
     const int ng = *n_groups;
+    long long local = 0;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= n; g += gridDim.x * blockDim.x) {
         const int gg = g < ng ? g : ng;
         const int o = task_loff[min(task_off[gg], task_cap)];
+        const int c = (g < ng) ? task_loff[min(task_off[g + 1], task_cap)] - o : 0;
         off[g] = o;
-        cnt[g] = (g < ng) ? task_loff[min(task_off[g + 1], task_cap)] - o : 0;
+        cnt[g] = c;
+        if (g < ng) local += (long long)c * i_count[g];
     }
+    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(FULL, local, o);
+    if ((threadIdx.x & 31) == 0 && local) atomicAdd((unsigned long long *)pairs, (unsigned long long)local);
 }
 
 // One traversal per task (one warp each).  PASS_COUNT counts the entries of
