@@ -2,22 +2,22 @@
 // functors and the batched Dispatch/Retrieve pairs.
 //
 // Data path of one dispatch (one CUDA stream per context):
-//   host  : offsets and work items into a pinned buffer, and a table of the
-//           pieces to copy: that buffer and the callers' walk arrays
-//   device: one kernel copies every piece into one buffer [offsets | items | EPI
-//           | EPJ] (pageable host memory is read in place where the device can,
-//           otherwise the arrays are staged in pinned memory first); one kernel
-//           turns the reference AoS structs into records; the pair kernels; a
-//           pack kernel writes the reference Force structs to pinned memory
-//           (finite check)
-//   Dispatch returns when the callers' arrays have been read; Retrieve waits on
-//   the stream and copies to the caller's per-walk arrays.
+//   host  : offsets, work items and the walk arrays into one pinned buffer
+//           [offsets | items | EPI | EPJ], large ones by several threads
+//   device: a kernel copies the buffer in, a segment at a time while the host
+//           fills the next; one kernel turns the reference AoS structs into
+//           records; the pair kernels; a pack kernel writes the reference Force
+//           structs to pinned memory (finite check)
+//   Retrieve waits on the stream and copies to the caller's per-walk arrays.
 //
-// Staging 60 MB of walk arrays with memcpy took 5 ms of a 7 ms dispatch; the
-// copy kernel reads them in 0.33 ms (190 GB/s over NVLink-C2C).
+// One thread's memcpy into the buffer took 5 of a 7 ms dispatch of 64 MB.  The
+// device can read pageable arrays where they are (0.33 ms), but its first
+// access to a 4 MB region of memory that was freed and mapped again costs a
+// fault of 0.6 ms: up to 18 ms for fresh arrays scattered over the heap.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstddef>
@@ -25,6 +25,8 @@
 #include <cstring>
 #include <limits>
 #include <new>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/sph_gb300.h"
@@ -250,25 +252,19 @@ __device__ __forceinline__ bool finite3(double a, double b, double c) {
     return isfinite(a) && isfinite(b) && isfinite(c);
 }
 
-// A piece of the inputs: n 8-byte words to word dst of the device buffer.
-constexpr int COPY_WORDS = 2048;
-__global__ void __launch_bounds__(256) gather_inputs(const CopyPiece *pieces, int n, unsigned long long *dst,
-                                                     int *queue) {
-    // counters of this dispatch (the flags at 4..6 are not used on the device)
-    if (blockIdx.x == 0 && threadIdx.x < 10 && (threadIdx.x < 4 || threadIdx.x > 6)) queue[threadIdx.x] = 0;
-    for (int c = blockIdx.x; c < n; c += gridDim.x) {
-        const CopyPiece p = pieces[c];
-        unsigned long long v[COPY_WORDS / 256];
+// Copies n 16-byte words from pinned memory; the first launch of a dispatch
+// clears its counters (queue; the flags at 4..6 are not used on the device).
+__global__ void __launch_bounds__(256) copy_inputs(const uint4 *src, uint4 *dst, size_t n, int *queue) {
+    if (queue && blockIdx.x == 0 && threadIdx.x < 10 && (threadIdx.x < 4 || threadIdx.x > 6)) queue[threadIdx.x] = 0;
+    const size_t stride = (size_t)gridDim.x * 256;
+    for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n; k += 4 * stride) {
+        uint4 v[4];
 #pragma unroll
-        for (int u = 0; u < COPY_WORDS / 256; ++u) {
-            const int k = threadIdx.x + 256 * u;
-            if (k < p.n) v[u] = p.src[k];
-        }
+        for (int u = 0; u < 4; ++u)
+            if (k + u * stride < n) v[u] = src[k + u * stride];
 #pragma unroll
-        for (int u = 0; u < COPY_WORDS / 256; ++u) {
-            const int k = threadIdx.x + 256 * u;
-            if (k < p.n) dst[p.dst + k] = v[u];
-        }
+        for (int u = 0; u < 4; ++u)
+            if (k + u * stride < n) dst[k + u * stride] = v[u];
     }
 }
 
@@ -538,9 +534,6 @@ extern "C" int sph_context_create(const sph_params *p, sph_context **out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_queue, 10 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_flags, 8 * sizeof(int));
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_read, cudaEventDisableTiming);
-    if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&ctx->pageable_access, cudaDevAttrPageableMemoryAccess, prm.device);
     if (e == cudaSuccess && init_grids(ctx) != 0) e = cudaErrorInvalidDeviceFunction;
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -563,7 +556,6 @@ extern "C" int sph_context_destroy(sph_context *ctx) {
     for (int k = 0; k < 3; ++k) ctx->kind[k].release();
     if (ctx->d_queue) cudaFree(ctx->d_queue);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
-    if (ctx->ev_read) cudaEventDestroy(ctx->ev_read);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return SPH_OK;
@@ -700,13 +692,89 @@ struct WalkArrays {
     size_t size, base;
 };
 
-// Whether the copy kernel may read the array where it is.
-bool readable(const sph_context *ctx, const void *p) {
-    return ctx->pageable_access && (reinterpret_cast<uintptr_t>(p) & 7) == 0;
+// A part of an array to copy into the pinned buffer.
+struct CopyTask {
+    const char *src;
+    size_t dst, bytes;
+};
+constexpr size_t TASK_BYTES = 256 << 10;     // largest task
+constexpr size_t THREAD_BYTES = 2 << 20;     // input bytes per copying thread (~150 us; creating one takes ~15)
+constexpr size_t SEGMENT_BYTES = 8 << 20;    // bytes per copy to the device (~40 us)
+constexpr int MAX_COPY_THREADS = 8;
+
+// Copies bytes [from, to) of the pinned buffer in; the first copy of a dispatch
+// (from = 0) clears its counters.
+void launch_copy(sph_context *ctx, KindState &ks, size_t from, size_t to) {
+    const size_t n = (to - from + 15) / 16;
+    const int grid = (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 8 * ctx->sm_count));
+    copy_inputs<<<grid, 256, 0, ctx->stream>>>(reinterpret_cast<const uint4 *>(ks.h_in.p + from),
+                                               reinterpret_cast<uint4 *>(ks.d_in.p + from), n,
+                                               from == 0 ? ctx->d_queue : nullptr);
 }
 
-// Builds the items and the pieces of a dispatch in the pinned buffers.  place:
-// byte offset of array a of walk w in the device buffer.
+// Runs the tasks (ascending dst) and copies the buffer in by segments, each as
+// soon as its tasks are done.
+void run_copies(sph_context *ctx, KindState &ks, const std::vector<CopyTask> &tasks, size_t total) {
+    char *h = ks.h_in.p;
+    const size_t bytes = tasks.empty() ? 0 : tasks.back().dst + tasks.back().bytes - tasks.front().dst;
+    const int cores = (int)std::thread::hardware_concurrency();
+    const int extra = std::min<int>(std::min(MAX_COPY_THREADS, cores / 2) - 1, (int)(bytes / THREAD_BYTES) - 1);
+    if (extra < 1) {
+        for (const CopyTask &t : tasks) std::memcpy(h + t.dst, t.src, t.bytes);
+        launch_copy(ctx, ks, 0, total);
+        return;
+    }
+    const int n = (int)tasks.size();
+    // segment k: the tasks up to seg_task[k], the bytes up to seg_end[k]
+    std::vector<int> seg_task, seg_of(n);
+    std::vector<size_t> seg_end;
+    size_t from = 0;
+    for (int k = 0; k < n; ++k) {
+        const size_t next = k + 1 < n ? tasks[k + 1].dst / 256 * 256 : total;
+        seg_of[k] = (int)seg_task.size();
+        if (next - from >= SEGMENT_BYTES || k + 1 == n) {
+            // a 256-byte boundary at or before the next task: bytes of this one
+            // beyond it go with the next segment, which is copied later
+            seg_task.push_back(k + 1);
+            seg_end.push_back(next);
+            from = next;
+        }
+    }
+    const int n_seg = (int)seg_task.size();
+    std::vector<std::atomic<int>> left(n_seg);
+    for (int g = 0; g < n_seg; ++g) left[g].store(seg_task[g] - (g ? seg_task[g - 1] : 0), std::memory_order_relaxed);
+    std::atomic<int> next_task{0};
+    auto one = [&]() {
+        const int k = next_task.fetch_add(1, std::memory_order_relaxed);
+        if (k >= n) return false;
+        std::memcpy(h + tasks[k].dst, tasks[k].src, tasks[k].bytes);
+        left[seg_of[k]].fetch_sub(1, std::memory_order_release);
+        return true;
+    };
+    std::vector<std::thread> threads;
+    try {
+        threads.reserve(extra);
+        for (int t = 0; t < extra; ++t) threads.emplace_back([&]() { while (one()) {} });
+    } catch (const std::system_error &) {
+        // fewer threads: the loop below does the rest
+    }
+    int seg = 0;
+    bool more = true;
+    while (seg < n_seg) {
+        if (more)
+            more = one();
+        else
+            std::this_thread::yield();
+        while (seg < n_seg && left[seg].load(std::memory_order_acquire) == 0) {
+            launch_copy(ctx, ks, seg ? seg_end[seg - 1] : 0, seg_end[seg]);
+            ++seg;
+        }
+    }
+    for (std::thread &t : threads) t.join();
+}
+
+// Builds the items, fills the pinned buffer and copies it to the device.
+// place: byte offset of array a of walk w in the buffer.
 template <class P>
 int stage(sph_context *ctx, KindState &ks, const std::vector<int> &i_off, const std::vector<int> &j_off,
           size_t epi_size, size_t epj_size, int chunk, int split_nj, const WalkArrays *arrays, int n_arrays,
@@ -715,73 +783,41 @@ int stage(sph_context *ctx, KindState &ks, const std::vector<int> &i_off, const 
     build_items(n_walk, i_off.data(), j_off.data(), chunk, split_nj, ks.items);
     L = make_layout(n_walk, ks.items.size(), epi_size * (size_t)i_off[n_walk],
                     epj_size * (size_t)j_off[n_walk]);
-    size_t staged = 0, pieces = 1 + L.off_epi / (8 * COPY_WORDS);
-    ks.in_place = false;
-    for (int a = 0; a < n_arrays; ++a)
-        for (int w = 0; w < n_walk; ++w) {
-            const size_t bytes = arrays[a].n ? arrays[a].size * (size_t)arrays[a].n[w] : 0;
-            if (!bytes) continue;
-            if (!arrays[a].ptr[w]) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
-            pieces += 1 + bytes / (8 * COPY_WORDS);
-            if (!readable(ctx, arrays[a].ptr[w])) staged += bytes;
-        }
-    if (ks.h_in.ensure(L.off_epi + staged) || ks.h_pieces.ensure(pieces) || ks.d_in.ensure(L.total))
+    if (ks.h_in.ensure(L.total) || ks.d_in.ensure(L.total))
         return set_error(ctx, SPH_ERR_CUDA, "staging allocation of %zu bytes failed", L.total);
+    std::vector<CopyTask> tasks;
+    tasks.reserve((size_t)n_arrays * n_walk + L.total / TASK_BYTES);
+    auto add = [&](int a, int w) {
+        const size_t bytes = arrays[a].n ? arrays[a].size * (size_t)arrays[a].n[w] : 0;
+        if (!bytes) return true;
+        const char *src = static_cast<const char *>(arrays[a].ptr[w]);
+        if (!src) return false;
+        const size_t dst = place(a, w);
+        for (size_t o = 0; o < bytes; o += TASK_BYTES)
+            tasks.push_back(CopyTask{src + o, dst + o, std::min(bytes - o, TASK_BYTES)});
+        return true;
+    };
+    // in the order of the buffer: EPI of every walk, then each walk's lists
+    for (int w = 0; w < n_walk; ++w)
+        if (!add(0, w)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
+    for (int w = 0; w < n_walk; ++w)
+        for (int a = 1; a < n_arrays; ++a)
+            if (!add(a, w)) return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "null array in walk %d", w);
     char *h = ks.h_in.p;
     std::memcpy(h + L.off_ioff, i_off.data(), sizeof(int) * (n_walk + 1));
     std::memcpy(h + L.off_joff, j_off.data(), sizeof(int) * (n_walk + 1));
     if (!ks.items.empty()) std::memcpy(h + L.off_items, ks.items.data(), sizeof(WorkItem) * ks.items.size());
-    ks.n_pieces = 0;
-    auto add = [&](const void *src, size_t bytes, size_t dst) {
-        const char *q = static_cast<const char *>(src);
-        for (size_t o = 0; o < bytes; o += 8 * (size_t)COPY_WORDS) {
-            const size_t b = std::min(bytes - o, 8 * (size_t)COPY_WORDS);
-            ks.h_pieces.p[ks.n_pieces++] =
-                CopyPiece{reinterpret_cast<const unsigned long long *>(q + o), (long long)((dst + o) / 8), (int)(b / 8)};
-        }
-    };
-    add(h, L.off_epi, 0);
-    size_t pos = L.off_epi;
-    for (int a = 0; a < n_arrays; ++a)
-        for (int w = 0; w < n_walk; ++w) {
-            const size_t bytes = arrays[a].n ? arrays[a].size * (size_t)arrays[a].n[w] : 0;
-            if (!bytes) continue;
-            const void *src = arrays[a].ptr[w];
-            if (readable(ctx, src)) {
-                ks.in_place = true;
-            } else {
-                std::memcpy(h + pos, src, bytes);
-                src = h + pos;
-                pos += bytes;
-            }
-            add(src, bytes, place(a, w));
-        }
-    return SPH_OK;
-}
-
-// Copies the pieces to the device buffer and zeroes the dispatch's counters.
-int launch_gather(sph_context *ctx, KindState &ks) {
     ctx->h_flags[ks.flag_slot] = 0;
-    gather_inputs<<<std::max(1, std::min(ks.n_pieces, 8 * ctx->sm_count)), 256, 0, ctx->stream>>>(
-        ks.h_pieces.p, ks.n_pieces, reinterpret_cast<unsigned long long *>(ks.d_in.p), ctx->d_queue);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && ks.in_place && !ctx->in_functor) e = cudaEventRecord(ctx->ev_read, ctx->stream);
+    run_copies(ctx, ks, tasks, L.total);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(ctx, e, "input copy");
     return SPH_OK;
 }
 
-// After the launches of a dispatch: waits until the callers' arrays have been
-// read (a functor call retrieves at once and waits there).
+// After the launches of a dispatch.
 int finish_dispatch(sph_context *ctx, KindState &ks, int n_walk, const std::vector<int> &i_off) {
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        cudaStreamSynchronize(ctx->stream);   // nothing reads the callers' arrays any more
-        return cuda_error(ctx, e, "kernel launch");
-    }
-    if (ks.in_place && !ctx->in_functor) {
-        e = cudaEventSynchronize(ctx->ev_read);
-        if (e != cudaSuccess) return cuda_error(ctx, e, "input copy");
-    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_error(ctx, e, "kernel launch");
     ks.pending = true;
     ks.n_walk = n_walk;
     ks.i_off = i_off;
@@ -854,7 +890,6 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Density) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
-    if ((st = launch_gather(ctx, ks))) return st;
     char *d = ks.d_in.p;
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
     const DensitySide si{ks.a4[0].p, ks.a4[1].p, ks.id[0].p, ks.d1[0].p, ks.d1[1].p,
@@ -938,7 +973,6 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Hydro) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
-    if ((st = launch_gather(ctx, ks))) return st;
     char *d = ks.d_in.p;
     const HydroSide si{ks.a4[0].p, ks.a4[1].p, ks.a4[4].p, ks.a4[5].p, ks.a2[0].p, ks.id[0].p, ks.f4[0].p, ks.f4[1].p,
                        ks.f4[2].p, ks.f4[3].p, ks.f4[8].p, ks.f4[9].p, ks.f4[10].p, ks.f4[14].p, ks.f4[16].p,
@@ -1026,7 +1060,6 @@ extern "C" int sph_dispatch_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
     if (ks.ensure_gravity(ni, nj, slices)) return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Gravity) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
-    if ((st = launch_gather(ctx, ks))) return st;
     char *d = ks.d_in.p;
     const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
     if (ni + nj > 0)
@@ -1070,21 +1103,11 @@ extern "C" int sph_retrieve_gravity(sph_context *ctx, int32_t tag, int32_t n_wal
 }
 
 // ---------------------------------------------------------------- functors
-namespace {
-// A functor's dispatch is retrieved before the call returns.
-struct FunctorCall {
-    sph_context *ctx;
-    explicit FunctorCall(sph_context *c) : ctx(c) { ctx->in_functor = true; }
-    ~FunctorCall() { ctx->in_functor = false; }
-};
-}  // namespace
-
 extern "C" int sph_calc_density(sph_context *ctx, const sph_DensityEPI *epi, int32_t n_i,
                                 const sph_DensityEPJ *epj, int32_t n_j, sph_Density *force) {
     if (!ctx) return SPH_ERR_INVALID_ARGUMENT;
     if (n_i < 0 || n_j < 0 || (n_i && (!epi || !force)) || (n_j && !epj))
         return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "bad functor arguments");
-    const FunctorCall call(ctx);
     int st = sph_dispatch_density(ctx, 0, 1, &epi, &n_i, &epj, &n_j);
     if (st) return st;
     return sph_retrieve_density(ctx, 0, 1, &n_i, &force);
@@ -1095,7 +1118,6 @@ extern "C" int sph_calc_hydro(sph_context *ctx, const sph_HydroEPI *epi, int32_t
     if (!ctx) return SPH_ERR_INVALID_ARGUMENT;
     if (n_i < 0 || n_j < 0 || (n_i && (!epi || !force)) || (n_j && !epj))
         return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "bad functor arguments");
-    const FunctorCall call(ctx);
     int st = sph_dispatch_hydro(ctx, 0, 1, &epi, &n_i, &epj, &n_j);
     if (st) return st;
     return sph_retrieve_hydro(ctx, 0, 1, &n_i, &force);
@@ -1108,7 +1130,6 @@ int gravity_accumulate(sph_context *ctx, const sph_GravityEPI *epi, int32_t n_i,
     if (!ctx) return SPH_ERR_INVALID_ARGUMENT;
     if (n_i < 0 || n_ep < 0 || n_sp < 0 || (n_i && (!epi || !force)) || (n_ep && !epj) || (n_sp && !spj))
         return set_error(ctx, SPH_ERR_INVALID_ARGUMENT, "bad functor arguments");
-    const FunctorCall call(ctx);
     int st = sph_dispatch_gravity(ctx, 0, 1, &epi, &n_i, &epj, &n_ep, &spj, &n_sp);
     if (st) return st;
     std::vector<sph_Gravity> tmp((size_t)std::max(n_i, 1));

@@ -74,20 +74,9 @@ struct HostBuf {
     }
 };
 
-// A piece of a dispatch's inputs: n 8-byte words at src (pinned memory, or the
-// caller's), word dst of the device buffer.
-struct CopyPiece {
-    const unsigned long long *src;
-    long long dst;
-    int n;
-};
-
 // Buffers and dispatch state of one interaction kind (density/hydro/gravity).
 struct KindState {
     HostBuf<char> h_in, h_out;
-    HostBuf<CopyPiece> h_pieces;
-    int n_pieces = 0;
-    bool in_place = false;             // some pieces are read from the caller's arrays
     DevBuf<char> d_in;
     DevBuf<dbl4> a4[8];
     DevBuf<float4> f4[20];   // FP32C double-float records; 16..19 hydro mark records
@@ -143,7 +132,6 @@ struct KindState {
     void release() {
         h_in.release();
         h_out.release();
-        h_pieces.release();
         d_in.release();
         for (auto &b : a4) b.release();
         for (auto &b : f4) b.release();
@@ -171,9 +159,6 @@ struct sph_context {
                               // [4..6] unused, [7] density sweep queue,
                               // [8] FP32C hydro rows that overflowed, [9] long items
     int *h_flags = nullptr;   // pinned: per kind, non-finite values in the outputs
-    int pageable_access = 0;  // kernels may read pageable host memory in place
-    cudaEvent_t ev_read = nullptr;   // the callers' arrays of a dispatch have been read
-    bool in_functor = false;  // the dispatch in course is retrieved by the same call
     int grid[3][2] = {{0}};   // persistent grid per kind and precision
     int grid_stream = 0;      // persistent grid of the FP32C streamed density walk
     int grid_df = 0;          // resident blocks of the double-float hydro pass

@@ -127,3 +127,32 @@ def test_hydro_fp64_beyond_the_fp32_range(scale):
     ref = orc.hydro(epi, epj)
     for f in ("acch", "accg", "udot", "vsmx", "diffu"):
         assert rel_err(out[f], ref[f], 1e-3).max() < 1e-11, f
+
+
+@pytest.mark.parametrize("n_walk,n_j", [(3, 12), (2, 30000), (40, 9000)])
+def test_staged_arrays_by_size(n_walk, n_j):
+    """Walk arrays at odd addresses, from one short copy to several threads and
+    segments (and arrays longer than one copying task): a batch gives what the
+    walks give one by one (FP64 sums of the same rows: 1e-13)."""
+    rng = np.random.default_rng(n_j)
+
+    def odd(a):
+        raw = np.empty(a.nbytes + 1, np.uint8)
+        raw[1:] = a.view(np.uint8)
+        return raw[1:].view(a.dtype)
+
+    walks = [_cloud(7 + k, n_j + int(rng.integers(0, 50)), seed=k) for k in range(n_walk)]
+    epi, epj = [odd(a) for a, _ in walks], [odd(b) for _, b in walks]
+    n_i, n_js = [len(a) for a in epi], [len(b) for b in epj]
+    got = [np.zeros(n, abi.Density) for n in n_i]
+    with functors.Context(precision="fp64", eta=ETA) as ctx:
+        functors.DispatchKernel_Dens(ctx, 0, n_walk, epi, n_i, epj, n_js)
+        functors.RetrieveKernel_Dens(ctx, 0, n_walk, n_i, got)
+        for k in range(n_walk):
+            one = np.zeros(n_i[k], abi.Density)
+            functors.calcDensity(ctx)(epi[k], n_i[k], epj[k], n_js[k], one)
+            for f in ("dens", "ksr", "grdh", "divv", "rotv"):
+                assert np.allclose(got[k][f], one[f], rtol=1e-13, atol=1e-13 * np.abs(one[f]).max()), (k, f)
+            assert np.array_equal(got[k]["np"], one["np"])
+    one = orc.density(*walks[-1], eta=ETA, ksr_max=0.0)
+    assert rel_err(got[-1]["dens"], one["dens"], 1e-3).max() < 1e-11
