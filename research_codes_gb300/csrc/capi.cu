@@ -121,7 +121,7 @@ static void beside(const LongSide &side, cudaStream_t s, A first, B rest) {
 template <int KIND>
 static void mark_long(const sph_context *ctx, const sphk::MarkArgs &m, int n_max, cudaStream_t s) {
     constexpr int W = KIND == sphk::ROWS_DENSITY ? sphk::MARK_LONG_WARPS : sphk::HYDRO_LONG_WARPS;
-    sphk::mark_rows<KIND, W, true><<<std::max(1, std::min(n_max, ctx->sm_count)), W * 32, 0, s>>>(m);
+    sphk::mark_rows<KIND, W, true><<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), W * 32, 0, s>>>(m);
 }
 
 // Rows of the items of m and of its long items: beside them where the caller
@@ -194,7 +194,7 @@ void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bo
         side, s,
         [&](cudaStream_t t) {
             sphk::density_stream<sphk::STREAM_LONG_WARPS, true>
-                <<<std::max(1, std::min(n_max, ctx->sm_count)), sphk::STREAM_LONG_WARPS * 32, 0, t>>>(w);
+                <<<std::max(1, std::min(n_max, 2 * ctx->sm_count)), sphk::STREAM_LONG_WARPS * 32, 0, t>>>(w);
         },
         [&](cudaStream_t t) { sphk::density_stream<PAIR_WARPS><<<ctx->grid_stream, PAIR_WARPS * 32, 0, t>>>(w); });
     if (sweep)
@@ -205,7 +205,7 @@ void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bo
 
 // Hydro: signal velocities and rows of the items of m, then the pair sums
 // over them (FP32C: the double-float pass) and over the lists of the particles
-// without a row.  *a.n_ovf and *m.n_long must be zero at launch.  mid
+// without a row.  *a.n_ovf and *m.longs.n must be zero at launch.  mid
 // (optional) is recorded between the two parts (as an external record node
 // when mid_external: inside a stream capture).
 void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
@@ -255,7 +255,7 @@ __device__ __forceinline__ bool finite3(double a, double b, double c) {
 // Copies n 16-byte words from pinned memory; the first launch of a dispatch
 // clears its counters (queue; the flags at 4..6 are not used on the device).
 __global__ void __launch_bounds__(256) copy_inputs(const uint4 *src, uint4 *dst, size_t n, int *queue) {
-    if (queue && blockIdx.x == 0 && threadIdx.x < 10 && (threadIdx.x < 4 || threadIdx.x > 6)) queue[threadIdx.x] = 0;
+    if (queue && blockIdx.x == 0 && threadIdx.x < 12 && (threadIdx.x < 4 || threadIdx.x > 6)) queue[threadIdx.x] = 0;
     const size_t stride = (size_t)gridDim.x * 256;
     for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n; k += 4 * stride) {
         uint4 v[4];
@@ -532,7 +532,7 @@ extern "C" int sph_context_create(const sph_params *p, sph_context **out) {
     int cc_major = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, prm.device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_queue, 10 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_queue, 12 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_flags, 8 * sizeof(int));
     if (e == cudaSuccess && init_grids(ctx) != 0) e = cudaErrorInvalidDeviceFunction;
     if (e != cudaSuccess) {
@@ -908,7 +908,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         m.j_off = (const int *)(d + L.off_joff);
         m.queue = ctx->d_queue + K_DENS;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 7;
-        m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
+        m.longs = sphk::LongQueue{ks.long_items.p, ctx->d_queue + 9, 0}; m.long_nj = LONG_NJ;
         m.push_long = longest(n_epj, n_walk) > LONG_NJ;
         sphk::DensityArgs a{};
         a.i_pm = ks.a4[0].p; a.i_vel = ks.a4[1].p; a.i_id = ks.id[0].p; a.i_ksr = ks.d1[0].p; a.i_rs = ks.d1[1].p;
@@ -992,7 +992,7 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         m.j_off = (const int *)(d + L.off_joff);
         m.queue = ctx->d_queue + K_HYDRO;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 8;
-        m.long_items = ks.long_items.p; m.n_long = ctx->d_queue + 9; m.long_nj = LONG_NJ;
+        m.longs = sphk::LongQueue{ks.long_items.p, ctx->d_queue + 9, 0}; m.long_nj = LONG_NJ;
         m.push_long = f64 && longest(n_epj, n_walk) > LONG_NJ;
         m.o_vsmx = ks.o[3].p;
         m.sv_skip = 1;

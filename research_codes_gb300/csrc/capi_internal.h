@@ -157,7 +157,7 @@ struct sph_context {
     cudaStream_t stream = nullptr;
     int *d_queue = nullptr;   // [0..2] work-queue counters, [3] density re-check count,
                               // [4..6] unused, [7] density sweep queue,
-                              // [8] FP32C hydro rows that overflowed, [9] long items
+                              // [8] FP32C hydro rows that overflowed, [9..11] long items
     int *h_flags = nullptr;   // pinned: per kind, non-finite values in the outputs
     int grid[3][2] = {{0}};   // persistent grid per kind and precision
     int grid_stream = 0;      // persistent grid of the FP32C streamed density walk

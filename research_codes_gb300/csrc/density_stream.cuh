@@ -67,9 +67,7 @@ struct StreamArgs {
     int nbr_cap = 0;
     int nbr_warps = 0;
     float nbr_slack = 1.0f;
-    // items of the LONG form, and their number
-    const WorkItem *long_items;
-    const int *n_long;
+    LongQueue longs;        // items of the LONG form
     // when set: pair evaluations performed, [0] the three density passes
     // ((j-entries kept by the support test x i-particles) of the swept passes
     // plus the list entries of the listed ones), [1] the gradient pass
@@ -130,7 +128,8 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
     const unsigned lt = lanemask_lt();
-    const int n_items = LONG ? *a.n_long : (a.n_items_dev ? *a.n_items_dev : a.n_items);
+    __shared__ int s_next;   // LONG
+    const int n_items = LONG ? 0 : (a.n_items_dev ? *a.n_items_dev : a.n_items);
     const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
     // (LONG: the last gridDim.x slots, one per block)
     const int gw = LONG ? a.nbr_warps - gridDim.x + blockIdx.x : blockIdx.x * WARPS + wid;
@@ -138,7 +137,6 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
     const float *bx = LONG ? l_x : s_rx[LONG ? 0 : wid], *by = LONG ? l_y : s_ry[LONG ? 0 : wid];
     const float *bz = LONG ? l_z : s_rz[LONG ? 0 : wid], *bm = LONG ? l_m : s_rm[LONG ? 0 : wid];
     const int *bj = LONG ? l_j : s_j[LONG ? 0 : wid];
-    int next = blockIdx.x;   // LONG
     // this lane's neighbour list: entry c at a.nbr[nlb + c * 32]
     const bool has_nl = a.nbr != nullptr && gw < a.nbr_warps;
     const int nlb = has_nl ? gw * a.nbr_cap * 32 + lane : 0;
@@ -150,16 +148,16 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
     const double nl_hmax = (double)a.nbr_slack * 0.99998;
 
     for (;;) {
-        int item = 0;
+        WorkItem wi;
         if (LONG) {
-            item = next;
-            next += gridDim.x;
+            if (!a.longs.take(&s_next, wi)) return;
         } else {
+            int item = 0;
             if (lane == 0) item = atomicAdd(a.queue, 1);
             item = __shfl_sync(FULL, item, 0);
+            if (item >= n_items) return;
+            wi = a.items[item];
         }
-        if (item >= n_items) return;
-        const WorkItem wi = LONG ? a.long_items[item] : a.items[item];
         const ItemRef r = decode(wi, a.j_off, a.i_list, lane);
         const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;
 
@@ -469,9 +467,10 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
                 __syncwarp();
             };
             if (listed) {
-                // this lane's list, four entries per round (gathers first)
+                // this lane's list, four entries per round (gathers first);
+                // LONG: a round each for the warps, folded in order
                 const int cmax = (int)__reduce_max_sync(FULL, (unsigned)ncnt);
-                for (int c0 = 0; c0 < cmax; c0 += 4) {
+                auto round4 = [&](int c0) {
                     int jj[4];
                     float4 pj[4];
 #pragma unroll
@@ -483,7 +482,23 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (jj[u] >= 0) part += term(pj[u], pass == 2);
-                    acc.add(part);
+                };
+                if constexpr (LONG) {
+                    for (int b0 = 0; b0 < cmax; b0 += 4 * LT) {
+                        const int nq = min(LT, (cmax - b0 + 3) >> 2);
+                        for (int q = wid; q < nq; q += WARPS) {
+                            round4(b0 + 4 * q);
+                            l_part[q][0][lane] = part;
+                        }
+                        __syncthreads();
+                        for (int q = 0; q < nq; ++q) acc.add(l_part[q][0][lane]);
+                        __syncthreads();
+                    }
+                } else {
+                    for (int c0 = 0; c0 < cmax; c0 += 4) {
+                        round4(c0);
+                        acc.add(part);
+                    }
                 }
                 if (r.act) ev_list += (unsigned)ncnt;
                 ++n_listed;
@@ -501,20 +516,20 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
                                    if (build) nl_push(head, __float_as_uint(l_part[q][1][lane]));
                                    acc.add(l_part[q][0][lane]);
                                });
-                    // the warps' counts
-                    __syncthreads();
-                    if (pass == 2) {
-                        int *sum = reinterpret_cast<int *>(&l_part[0][0][0]);
-                        if (wid == 0) sum[lane] = 0;
-                        __syncthreads();
-                        atomicAdd(&sum[lane], cnt);
-                        __syncthreads();
-                        cnt = sum[lane];
-                        __syncthreads();
-                    }
                 } else {
                     sweep(rf2, false, build, run);
                 }
+            }
+            if (LONG && pass == 2) {
+                // the warps' counts
+                int *sum = reinterpret_cast<int *>(&l_part[0][0][0]);
+                __syncthreads();
+                if (wid == 0) sum[lane] = 0;
+                __syncthreads();
+                atomicAdd(&sum[lane], cnt);
+                __syncthreads();
+                cnt = sum[lane];
+                __syncthreads();
             }
             if (LONG && build) __syncthreads();   // the lists
             if (build) nl_ok = __all_sync(FULL, ncnt <= a.nbr_cap);
@@ -621,15 +636,33 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
                     pair(head + k);
                 }
             };
+            // LONG: this lane's sums to and from tile q
+            auto put = [&](int q) {
+                l_part[q][0][lane] = pg;
+                l_part[q][1][lane] = pd;
+                l_part[q][2][lane] = prx;
+                l_part[q][3][lane] = pry;
+                l_part[q][4][lane] = prz;
+                pg = 0; pd = 0; prx = 0; pry = 0; prz = 0;
+            };
+            auto take = [&](int q) {
+                pg = l_part[q][0][lane];
+                pd = l_part[q][1][lane];
+                prx = l_part[q][2][lane];
+                pry = l_part[q][3][lane];
+                prz = l_part[q][4][lane];
+                fold();
+            };
             auto run = [&](int head, int n) {
                 tile(head, n);
                 fold();
                 __syncwarp();
             };
             if (nl_ok && __all_sync(FULL, (float)h <= nl_h)) {
-                // this lane's list, two entries per round (gathers first)
+                // this lane's list, two entries per round (gathers first),
+                // folded after eight; LONG: eight entries each for the warps
                 const int cmax = (int)__reduce_max_sync(FULL, (unsigned)ncnt);
-                for (int c0 = 0; c0 < cmax; c0 += 2) {
+                auto round2 = [&](int c0) {
                     int jj[2];
                     float4 pj[2];
                     float4 vh[2];
@@ -649,9 +682,26 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
 #pragma unroll
                     for (int u = 0; u < 2; ++u)
                         if (jj[u] >= 0) gpair(pj[u], vh[u].x, vh[u].y, vh[u].z, vl[u].x, vl[u].y, vl[u].z, idj[u]);
-                    if ((c0 & 7) == 6) fold();
+                };
+                if constexpr (LONG) {
+                    const int n8 = (cmax + 1) / 8 + 1;   // folds (the last of what is left, or nothing)
+                    for (int b0 = 0; b0 < n8; b0 += LT) {
+                        const int nq = min(LT, n8 - b0);
+                        for (int q = wid; q < nq; q += WARPS) {
+                            for (int c0 = 8 * (b0 + q); c0 < min(cmax, 8 * (b0 + q) + 8); c0 += 2) round2(c0);
+                            put(q);
+                        }
+                        __syncthreads();
+                        for (int q = 0; q < nq; ++q) take(q);
+                        __syncthreads();
+                    }
+                } else {
+                    for (int c0 = 0; c0 < cmax; c0 += 2) {
+                        round2(c0);
+                        if ((c0 & 7) == 6) fold();
+                    }
+                    fold();
                 }
-                fold();
                 if (r.act) ev_list_g += (unsigned)ncnt;
                 ++n_listed;
             } else {
@@ -659,23 +709,13 @@ __global__ void __launch_bounds__(WARPS * 32, LONG ? 2 : SPH_DENSITY_MIN_BLOCKS)
                     sweep_long(support2<float>(h),
                                [&](int head, int n, int q) {
                                    tile(head, n);
-                                   l_part[q][0][lane] = pg;
-                                   l_part[q][1][lane] = pd;
-                                   l_part[q][2][lane] = prx;
-                                   l_part[q][3][lane] = pry;
-                                   l_part[q][4][lane] = prz;
                                    const bool any = pg != 0.0f || pd != 0.0f || prx != 0.0f || pry != 0.0f || prz != 0.0f;
-                                   pg = 0; pd = 0; prx = 0; pry = 0; prz = 0;
+                                   put(q);
                                    return __any_sync(FULL, any);
                                },
                                [&](int q, int head) {
                                    (void)head;
-                                   pg = l_part[q][0][lane];
-                                   pd = l_part[q][1][lane];
-                                   prx = l_part[q][2][lane];
-                                   pry = l_part[q][3][lane];
-                                   prz = l_part[q][4][lane];
-                                   fold();
+                                   take(q);
                                });
                 } else {
                     sweep(support2<float>(h), true, false, run);

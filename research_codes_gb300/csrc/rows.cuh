@@ -28,7 +28,7 @@ static_assert(ROW_CAP % 32 == 0, "eight lanes read a row four entries at a time"
 // per second, the chip ~5e11 listed pairs: beyond pairs / 65536 entries one
 // warp's item lasts about half of the whole walk's time.
 __device__ __forceinline__ int long_list(long long pairs) {
-    return (int)min(max(pairs >> 16, 768LL), 1LL << 30);
+    return (int)min(max(pairs >> 17, 768LL), 1LL << 30);
 }
 constexpr int MARK_LONG_WARPS = 16, HYDRO_LONG_WARPS = 8;
 // Radii outside this range (or NaN) are left to the sweep: their squares
@@ -80,6 +80,25 @@ struct F32Part {
     const float4 *vlo;   // vx_lo, vy_lo, vz_lo, aux
 };
 
+// Items of the LONG form: n[0] of them from the front of the array, the
+// longest, n[1] from its end (cap entries); n[2] counts those taken.
+struct LongQueue {
+    WorkItem *items;
+    int *n;
+    int cap;
+    __device__ __forceinline__ void push(const WorkItem &wi) const { items[atomicAdd(n, 1)] = wi; }
+    // the block's next item; false when there is none (slot: shared)
+    __device__ __forceinline__ bool take(int *slot, WorkItem &wi) const {
+        __syncthreads();
+        if (threadIdx.x == 0) *slot = atomicAdd(&n[2], 1);
+        __syncthreads();
+        const int k = *slot, front = n[0];
+        if (k >= front + n[1]) return false;
+        wi = items[k < front ? k : cap - 1 - (k - front)];
+        return true;
+    }
+};
+
 struct MarkArgs {
     // double-float positions; h (rounded up) in lo.w (density: i records) or
     // hi.w (hydro: i and j records)
@@ -96,8 +115,7 @@ struct MarkArgs {
     int2 *info;              // per particle: entries (> ROW_CAP: none, see ovf), walk
     int2 *ovf;               // particles without a row: (particle, walk)
     int *n_ovf;
-    WorkItem *long_items;    // items of the LONG form, and their number
-    int *n_long;
+    LongQueue longs;         // items of the LONG form
     // push_long: the kernel itself moves items with lists beyond long_nj (with
     // pairs set: beyond long_list of the walks' listed pairs) to that queue
     bool push_long;
@@ -223,20 +241,20 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
     const int wid = threadIdx.x >> 5;
     const int hw = HYDRO ? wid : 0;
     const unsigned lt = lanemask_lt();
-    const int n_items = LONG ? *a.n_long : (a.n_items_dev ? *a.n_items_dev : a.n_items);
-    int next = blockIdx.x;   // LONG
+    __shared__ int s_next;   // LONG
+    const int n_items = LONG ? 0 : (a.n_items_dev ? *a.n_items_dev : a.n_items);
     const int long_nj = a.pairs ? long_list(*a.pairs) : a.long_nj;
     for (;;) {
-        int item = 0;
+        WorkItem wi;
         if (LONG) {
-            item = next;
-            next += gridDim.x;
+            if (!a.longs.take(&s_next, wi)) return;
         } else {
+            int item = 0;
             if (lane == 0) item = atomicAdd(a.queue, 1);
             item = __shfl_sync(FULL, item, 0);
+            if (item >= n_items) return;
+            wi = a.items[item];
         }
-        if (item >= n_items) return;
-        const WorkItem wi = LONG ? a.long_items[item] : a.items[item];
         ItemRef r = decode(wi, a.j_off, a.i_list, lane);
         if (LONG) {   // a lane per particle
             r.tpi = 1;
@@ -248,7 +266,7 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
             if (threadIdx.x < 32) s_cnt[threadIdx.x] = 0;
             __syncthreads();
         } else if (a.push_long && r.nj > long_nj) {
-            if (lane == 0) a.long_items[atomicAdd(a.n_long, 1)] = wi;
+            if (lane == 0) a.longs.push(wi);
             continue;
         }
         const int tpi = r.tpi, sub = r.sub, ii = r.ii, nj = r.nj, jb = r.jb;

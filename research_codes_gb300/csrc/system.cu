@@ -48,7 +48,9 @@ constexpr int MAX_RED = 8;
 constexpr long long MAX_POOL_CHUNKS = 0x7fffffffLL / sphtree::LIST_CHUNK;
 constexpr int NBKT = 32;   // cost classes of work items (log2 of the estimated cost)
 enum { S_NGROUPS = 0, S_NACTIVE, S_NITEMS, S_QUEUE, S_ERROR, S_UNCONV, S_TOTAL, S_ITERS, S_AMB, S_AMBTOT,
-       S_NTASKS, S_NROOTS, S_POOL, S_POOLERR, S_TQUEUE, S_POOLMAX, S_HOVF, S_SMALL, S_NITER, S_DOVF, S_NLONG, S_BKT,
+       S_NTASKS, S_NROOTS, S_POOL, S_POOLERR, S_TQUEUE, S_POOLMAX, S_HOVF, S_SMALL, S_NITER, S_DOVF,
+       S_NLONG, S_NLONG_SHORTER, S_LONGS_TAKEN,   // (in this order, sphk::LongQueue)
+       S_BKT,
        S_NI = S_BKT + 2 * NBKT + 2 };
 // double scalars
 enum { D_TIME = 0, D_DT, D_KSRMAX, D_EPSU, D_DTC, D_XC, D_YC, D_ZC, D_MC, D_EKIN, D_ETHM, D_EPOT,
@@ -504,13 +506,13 @@ __global__ void light_counts(int n, const int *n_walks, const int *i_count, cons
 __global__ void drop_items_on_overflow(int *scal) {
     if (scal[S_ERROR] & (E_LISTCAP | E_STACK)) {
         scal[S_NITEMS] = 0;
-        scal[S_NLONG] = 0;
+        scal[S_NLONG] = scal[S_NLONG_SHORTER] = 0;
     }
 }
 
 __global__ void fill_items(int n, const int *n_walks, const int *i_first, const int *i_count, int chunk,
                            int split_nj, const int *j_cnt, int *bkt, const int *light_off, WorkItem *items,
-                           int *n_items, const long long *pairs, WorkItem *longs, int *n_long) {
+                           int *n_items, const long long *pairs, bool longs, sphk::LongQueue queue) {
     const int nw = *n_walks;
     const int bh = bkt[2 * NBKT];
     const int n_heavy = bkt[2 * NBKT + 1];
@@ -521,12 +523,19 @@ __global__ void fill_items(int n, const int *n_walks, const int *i_first, const 
             const int nj = j_cnt[k];
             const int ch = item_chunk(nj, chunk, split_nj);
             int lpos = n_heavy + light_off[k];
-            int qpos = nj > long_nj ? atomicAdd(n_long, (ni + ch - 1) / ch) : 0;
+            // long items: the longest from the front of their queue
+            const bool front = nj > 4LL * long_nj;
+            int qpos = 0;
+            if (nj > long_nj) {
+                qpos = atomicAdd(&queue.n[front ? 0 : 1], (ni + ch - 1) / ch);
+                if (!front) qpos = queue.cap - 1 - qpos;
+            }
             for (int c0 = 0; c0 < ni; c0 += ch) {
                 const int sz = min(ch, ni - c0);
                 const WorkItem it = make_int4(k, i_first[k] + c0, sz, nj * sz);
                 if (nj > long_nj) {
-                    longs[qpos++] = it;
+                    queue.items[qpos] = it;
+                    qpos += front ? 1 : -1;
                     continue;
                 }
                 const int b = cost_bucket(nj, sz);
@@ -564,7 +573,7 @@ __global__ void walk_particles(int n, const int *flag, const int *scan, int firs
 __global__ void drop_items_if_small(int *scal) {
     if (scal[S_SMALL]) {
         scal[S_NITEMS] = 0;
-        scal[S_NLONG] = 0;
+        scal[S_NLONG] = scal[S_NLONG_SHORTER] = 0;
     }
 }
 
@@ -1051,6 +1060,7 @@ struct sph_system {
     // of the capture, so the loop body has one of its own
     sphrt::LongSide sides[2];
     const sphrt::LongSide &long_side() const { return sides[st_override && st_override == body_stream]; }
+    sphk::LongQueue long_queue() const { return {long_items.p, scal.p + S_NLONG, n}; }
     cudaStream_t st() const { return st_override ? st_override : ctx->stream; }
     Persist persist(int k) {
         Persist p;
@@ -1117,7 +1127,7 @@ int alloc_all(sph_system *s) {
     s->amb_cap = std::max<int>(1024, s->n / 16);
     e |= s->amb.ensure(s->amb_cap) | s->r_info.ensure(n);
     e |= s->long_items.ensure(n) | s->w_csmax.ensure(n);
-    s->nbr_warps = s->ctx->grid_stream * PAIR_WARPS + s->ctx->sm_count;   // and the blocks of the long items
+    s->nbr_warps = s->ctx->grid_stream * PAIR_WARPS + 2 * s->ctx->sm_count;   // and the blocks of the long items
     e |= s->nbr.ensure((size_t)s->nbr_warps * NBR_CAP * 32);
     DevBuf<int> *i1[] = {&s->gflag, &s->groot, &s->gscan, &s->group_node, &s->group_first, &s->group_count,
                          &s->aflag, &s->ascan, &s->a_node, &s->a_first, &s->a_count};
@@ -1451,25 +1461,25 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
         L.lpool_chunks = std::min((long long)(L.lpool.cap / sphtree::LIST_CHUNK), MAX_POOL_CHUNKS);
     }
     // work items; those of long lists (density and hydro) in a queue of their own
-    WorkItem *longs = (kind == 2) ? nullptr : s->long_items.p;
-    if (longs) CUDA_TRY(cudaMemsetAsync(sc + S_NLONG, 0, sizeof(int), st));
+    const bool longs = kind != 2;
+    if (longs) CUDA_TRY(cudaMemsetAsync(sc + S_NLONG, 0, 3 * sizeof(int), st));
     // density and hydro walks with long lists are split (their pair loops
     // drop most of the list); gravity lists are uniform and kept whole
     const int split_nj = (kind == 2) ? (1 << 30) : (s->prm.item_split_nj > 0 ? s->prm.item_split_nj : ITEM_SPLIT_NJ);
     int *bkt = sc + S_BKT;
     CUDA_TRY(cudaMemsetAsync(bkt, 0, sizeof(int) * (2 * NBKT + 2), st));
     item_buckets<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj, pairs,
-                                              longs != nullptr, bkt);
+                                              longs, bkt);
     bucket_offsets<<<1, 32, 0, st>>>(bkt, kind == 2 ? 0 : (s->prm.heavy_classes >= 0 ? s->prm.heavy_classes
                                                                                    : SPH_HEAVY_CLASSES));
     // light items in walk order: per-walk counts (the task arrays are free
     // again once the lists are built) and their scan
     light_counts<<<grid_for(n + 1), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj,
-                                                  pairs, longs != nullptr, bkt, L.tcnt.p);
+                                                  pairs, longs, bkt, L.tcnt.p);
     r = exclusive_scan(s, L.tcnt.p, L.toff.p, n + 1, builder);
     if (r) return r;
     fill_items<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], ifirst, icount, chunk, split_nj, s->lcnt[kind].p,
-                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, sc + S_NLONG);
+                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, s->long_queue());
     drop_items_on_overflow<<<1, 1, 0, st>>>(sc);
     return SPH_OK;
 }
@@ -1518,7 +1528,7 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
     m.j_off = s->loff[kind].p; m.j_idx = s->jidx[kind].p; m.queue = s->scal.p + S_QUEUE;
     m.i_list = s->ulist.p;
     m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
-    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG;
+    m.longs = s->long_queue();
     sphk::DensityArgs a{};
     a.n_eval = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_EVAL_D1) : nullptr;
     a.n_pass = first ? reinterpret_cast<unsigned long long *>(s->lscal.p + L_DLISTED) : nullptr;
@@ -1559,7 +1569,7 @@ int density_walk(sph_system *s, int it, bool eager, cudaGraphConditionalHandle c
         w.nbr_cap = NBR_CAP;
         w.nbr_warps = s->nbr_warps;
         w.nbr_slack = lists ? s->prm.density_list_slack : 1.0f;
-        w.long_items = m.long_items; w.n_long = m.n_long;
+        w.longs = m.longs;
         w.n_eval = a.n_eval; w.n_pass = a.n_pass;
         sphrt::launch_density_stream(ctx, w, !first, a, n, st, s->scal.p + S_AMBTOT,
                                      s->long_side());
@@ -1784,7 +1794,7 @@ int hydro_phase(sph_system *s, bool eager) {
     m.items = s->ls[0].items.p; m.n_items_dev = s->scal.p + S_NITEMS;
     m.j_off = s->loff[1].p; m.j_idx = s->jidx[1].p; m.queue = s->scal.p + S_QUEUE;
     m.rows = s->hl_list.p; m.info = s->r_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_HOVF;
-    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG;
+    m.longs = s->long_queue();
     m.i_id = s->id[0].p; m.j_id = m.i_id;
     m.fi = sphk::F32Part{s->f_phi.p, s->f_plo.p, s->f_vhi.p, s->f_vlo.p};
     m.fj = m.fi;
@@ -2738,14 +2748,14 @@ extern "C" int sph_system_adjoint_forces(sph_system *s, const double *seed, doub
     // rows of the h passes: every j within the slack of the first guess
     sphk::make_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->h_guess.p, s->f_phi.p, s->f_plo.p);
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_DOVF, 0, 2 * sizeof(int), st));   // queue of the rowless, long items
+    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_DOVF, 0, 4 * sizeof(int), st));   // queue of the rowless, long items
     sphk::MarkArgs m{};
     m.i_hi = s->f_phi.p; m.i_lo = s->f_plo.p; m.j_hi = m.i_hi; m.j_lo = m.i_lo;
     m.slack = NBR_SLACK;
     m.items = s->adj_items.p; m.n_items = n_items;
     m.j_off = as.d_off; m.j_idx = as.d_idx; m.queue = s->scal.p + S_QUEUE;
     m.rows = s->adj_rows.p; m.info = s->adj_info.p; m.ovf = s->hl_ovf.p; m.n_ovf = s->scal.p + S_DOVF;
-    m.long_items = s->long_items.p; m.n_long = s->scal.p + S_NLONG; m.push_long = true;
+    m.longs = s->long_queue(); m.push_long = true;
     m.pairs = s->lscal.p + L_PAIRS_D1;
     sphrt::launch_mark_density(ctx, m, sphrt::pair_grid(ctx, 0, SPH_PREC_FP64, n_items), n, st);
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
