@@ -510,8 +510,9 @@ int sph_system_get_lists(sph_system *sys, int32_t kind, int32_t *n_walk, int64_t
  * values written, or minus a status code.  Eager evaluations record the
  * events directly; captured graphs (force evaluation and step) hold them as
  * external event-record nodes, so the values after a graph replay are that
- * replay's.  [3] runs on a second stream in captured graphs, overlapping
- * [1]. */
+ * replay's.  In captured graphs [3] and [4] run on a second stream, [3]
+ * overlapping [1] and [4] overlapping [5] and [8]; [9] starts when both are
+ * done. */
 int sph_system_phase_times(sph_system *sys, float *ms, int32_t n);
 
 /* Kernel launches per replay of the captured graph: step = 1 for the

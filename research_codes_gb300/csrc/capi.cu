@@ -205,19 +205,18 @@ void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bo
 
 // Hydro: signal velocities and rows of the items of m, then the pair sums
 // over them (FP32C: the double-float pass) and over the lists of the particles
-// without a row.  *a.n_ovf and *m.longs.n must be zero at launch.  mid
-// (optional) is recorded between the two parts (as an external record node
-// when mid_external: inside a stream capture).
-void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
-                  int precision, cudaStream_t s, cudaEvent_t mid, bool mid_external, const LongSide *side) {
-    const bool f64 = precision == SPH_PREC_FP64;
-    if (f64)
-        mark_all<sphk::ROWS_HYDRO64>(ctx, m, mark_grid, a.n_i, s, side);
+// without a row.  *a.n_ovf and *m.longs.n must be zero at launch.
+void launch_hydro_marks(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_i, int precision,
+                        cudaStream_t s, const LongSide *side) {
+    if (precision == SPH_PREC_FP64)
+        mark_all<sphk::ROWS_HYDRO64>(ctx, m, mark_grid, n_i, s, side);
     else
-        mark_all<sphk::ROWS_HYDRO32>(ctx, m, mark_grid, a.n_i, s, side);
-    if (mid) cudaEventRecordWithFlags(mid, s, mid_external ? cudaEventRecordExternal : cudaEventRecordDefault);
+        mark_all<sphk::ROWS_HYDRO32>(ctx, m, mark_grid, n_i, s, side);
+}
+
+void launch_hydro_sums(const sph_context *ctx, const sphk::HydroArgs &a, int precision, cudaStream_t s) {
     if (a.n_i <= 0) return;
-    if (f64) {
+    if (precision == SPH_PREC_FP64) {
         const int per_block = sphk::HROWS_THREADS / sphk::HROWS_LANES;
         sphk::hydro64_rows<<<std::max(1, std::min((a.n_i + per_block - 1) / per_block, 16 * ctx->sm_count)),
                              sphk::HROWS_THREADS, 0, s>>>(a);
@@ -1012,8 +1011,9 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         a.mi_p = m.i_hi; a.mi_l = m.i_lo; a.mj_p = m.j_hi; a.mj_l = m.j_lo;
         m.i_id = a.i_id; m.j_id = a.j_id; m.fi = a.fi; m.fj = a.fj; m.fi_g2 = a.fi_g2; m.fj_g2 = a.fj_g2;
         m.i_pm = a.i_pm; m.i_vel = a.i_vel; m.i_h2 = a.i_h2; m.j_pm = a.j_pm; m.j_vel = a.j_vel; m.j_h2 = a.j_h2;
-        launch_hydro(ctx, m, pair_grid(ctx, K_HYDRO, ctx->prm.precision, m.n_items), a, ctx->prm.precision,
-                     ctx->stream);
+        launch_hydro_marks(ctx, m, pair_grid(ctx, K_HYDRO, ctx->prm.precision, m.n_items), ni, ctx->prm.precision,
+                           ctx->stream);
+        launch_hydro_sums(ctx, a, ctx->prm.precision, ctx->stream);
     }
     if (ni > 0)
         pack_hydro<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(

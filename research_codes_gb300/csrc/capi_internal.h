@@ -185,8 +185,8 @@ void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_gr
                     int n_max, int precision, cudaStream_t s, int *amb_total = nullptr, const LongSide *side = nullptr);
 void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
                            int n_max, cudaStream_t s, int *amb_total, const LongSide &side);
-void launch_hydro(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::HydroArgs &a,
-                  int precision, cudaStream_t s, cudaEvent_t mid = nullptr, bool mid_external = false,
-                  const LongSide *side = nullptr);
+void launch_hydro_marks(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_i, int precision,
+                        cudaStream_t s, const LongSide *side = nullptr);
+void launch_hydro_sums(const sph_context *ctx, const sphk::HydroArgs &a, int precision, cudaStream_t s);
 void launch_gravity(const sphk::GravityArgs &a, int precision, int grid, cudaStream_t s, int jtile);
 }  // namespace sphrt

@@ -694,19 +694,23 @@ __global__ void post_density(int n, const dbl4 *pos, const double *dens, const d
 // Gravity write-back, hdr_gravity.hpp:107-113
 __global__ void gravity_writeback(int n, double G, const double *acc, const double *pot, const double *etas,
                                   const double *ksr, const double *grdh, const double *dens, double *accg2,
-                                  double *pot_out, double *eta_out, bool f32, int slices, double *etas_out) {
+                                  double *pot_out, double *eta_out, bool f32, int slices, double *etas_out,
+                                  double2 *h3, float4 *g3) {
     GRID_STRIDE(p, n) {
         double g[5];
         sphk::gravity_gather(acc, pot, etas, p, slices, n, g);
         for (int c = 0; c < 3; ++c) accg2[3 * p + c] = G * g[c];
         etas_out[p] = g[4];   // the derivative reads it
+        double eta;
         if (f32) {   // eta feeds the FP32 hydro records
             const float h = (float)ksr[p];
-            eta_out[p] = (double)(h * h / (float)(KSRH * KSRH) * (float)grdh[p] / (3.0f * (float)dens[p]) *
-                                  (float)g[4]);
+            eta = (double)(h * h / (float)(KSRH * KSRH) * (float)grdh[p] / (3.0f * (float)dens[p]) * (float)g[4]);
+            g3[p].z = (float)eta;
         } else {
-            eta_out[p] = ksr[p] * ksr[p] / (KSRH * KSRH) * grdh[p] / (3.0 * dens[p]) * g[4];
+            eta = ksr[p] * ksr[p] / (KSRH * KSRH) * grdh[p] / (3.0 * dens[p]) * g[4];
         }
+        eta_out[p] = eta;
+        h3[p].y = eta;   // the hydro records' field that gravity sets
         pot_out[p] = G * g[3];
     }
 }
@@ -751,9 +755,7 @@ __global__ void __launch_bounds__(CSMAX_THREADS) walk_csmax(const int *n_walks, 
 // HydroEPI/EPJ::copyFromFP, hdr_hydro.hpp:45-62 / 95-113 (umin = 0)
 __global__ void hydro_prep(int n, const double *ksr, const double *pres, const double *grdh,
                            const double *dens, const double *bswt, const double *vsnd, const double *alph,
-                           const double *alphu, const double *uene, const double *eta, dbl4 *h1, dbl4 *h2,
-                           double2 *h3, bool f32) {
-    (void)f32;
+                           const double *alphu, const double *uene, dbl4 *h1, dbl4 *h2, double2 *h3) {
     GRID_STRIDE(p, n) {
         // FP64 in both precisions: the FP32C records carry 1/h, h^-4 and
         // P Omega / rho^2 as double-float splits for the cancelling sums
@@ -761,7 +763,7 @@ __global__ void hydro_prep(int n, const double *ksr, const double *pres, const d
         const double presc = pres[p] * grdh[p] / (dens[p] * dens[p]);
         h1[p] = make_dbl4(hinv, pres[p], presc, 0.5 * bswt[p]);
         h2[p] = make_dbl4(dens[p], vsnd[p], alph[p], alphu[p]);
-        h3[p] = make_double2(fmax(uene[p] - 0.0, 0.0), eta[p]);
+        h3[p] = make_double2(fmax(uene[p] - 0.0, 0.0), 0.0);   // eta: gravity_writeback
     }
 }
 
@@ -987,7 +989,7 @@ struct sph_system {
     DevBuf<double> neps2;
     DevBuf<float4> flo, fhi, fmom, ptest;
     // FP32C double-float records (particles, hydro fields, tree monopoles)
-    DevBuf<float4> f_phi, f_plo, f_vhi, f_vlo, f_g1, f_g2, f_g3, f_g4, f_mp, f_mv, f_shi, f_slo;
+    DevBuf<float4> f_phi, f_plo, f_vhi, f_vlo, f_g1, f_g2, f_g3, f_g4, f_mp, f_mv, f_gphi, f_gplo, f_shi, f_slo;
     // per particle the j indices of its pairs (ROW_CAP per row; density rows,
     // then the hydro rows of the same evaluation), their number (density: with
     // the walk), and the particles without a row
@@ -1119,7 +1121,7 @@ int alloc_all(sph_system *s) {
     if (s->prm.quadrupole) e |= s->quad.ensure(6 * nn) | s->fq0.ensure(nn) | s->fq1.ensure(nn);
     e |= s->flo.ensure(nn) | s->fhi.ensure(nn) | s->fmom.ensure(nn) | s->ptest.ensure(n);
     DevBuf<float4> *f1[] = {&s->f_phi, &s->f_plo, &s->f_vhi, &s->f_vlo, &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4,
-                            &s->f_mp, &s->f_mv};
+                            &s->f_mp, &s->f_mv, &s->f_gphi, &s->f_gplo};
     for (auto *b : f1) e |= b->ensure(n);
     e |= s->hl_list.ensure(n * sphk::ROW_CAP) | s->hl_ovf.ensure(n);
     e |= s->f_shi.ensure(nn) | s->f_slo.ensure(nn);
@@ -1718,30 +1720,35 @@ int gravity_lists(sph_system *s, bool eager) {
     return r;
 }
 
+// The gravity kernel and write-back.  In a captured graph they follow the
+// gravity lists on side_stream, beside the hydro lists and rows: only the
+// hydro sums need its eta (gravity_join).
 int gravity_phase(sph_system *s) {
     const int n = s->n;
-    cudaStream_t st = s->st();
     sph_context *ctx = s->ctx;
-    if (s->glist_forked) CUDA_TRY(cudaStreamWaitEvent(st, s->ev_join, 0));
-    s->glist_forked = false;
-    merge_errors<<<1, 1, 0, st>>>(s->ls[1].sc, s->scal.p);
+    cudaStream_t st = s->st();
+    if (s->glist_forked) {
+        CUDA_TRY(cudaEventRecord(s->ev_fork, st));
+        CUDA_TRY(cudaStreamWaitEvent(s->side_stream, s->ev_fork, 0));
+        st = s->side_stream;
+    }
     if (ctx->prm.precision == SPH_PREC_FP32C) {
-        sphk::make_gravity_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->eps2.p, s->f_phi.p, s->f_plo.p);
+        sphk::make_gravity_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->eps2.p, s->f_gphi.p, s->f_gplo.p);
         sphk::make_gravity_records<<<grid_for(2LL * n - 1), 256, 0, st>>>(2 * n - 1, s->mom.p, s->neps2.p,
                                                                           s->f_shi.p, s->f_slo.p);
     }
-    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
+    CUDA_TRY(cudaMemsetAsync(s->ls[1].sc + S_QUEUE, 0, sizeof(int), st));
     phase_event(s, EV_GK_B, st);
     sphk::GravityArgs a{};
     a.i_pe = s->pe.p;
     a.j_pm = s->pos[0].p; a.j_eps2 = s->eps2.p;
     a.s_pm = s->mom.p; a.s_eps2 = s->neps2.p;
-    a.fi_phi = s->f_phi.p; a.fi_plo = s->f_plo.p; a.f_phi = s->f_phi.p; a.f_plo = s->f_plo.p;
+    a.fi_phi = s->f_gphi.p; a.fi_plo = s->f_gplo.p; a.f_phi = s->f_gphi.p; a.f_plo = s->f_gplo.p;
     a.f_shi = s->f_shi.p; a.f_slo = s->f_slo.p;
     a.i_list = nullptr;
     a.n_split = n;
     a.items = s->ls[1].items.p; a.n_items = 0; a.n_items_dev = s->ls[1].sc + S_NITEMS;
-    a.j_off = s->loff[2].p; a.j_idx = s->jidx[2].p; a.queue = s->scal.p + S_QUEUE;
+    a.j_off = s->loff[2].p; a.j_idx = s->jidx[2].p; a.queue = s->ls[1].sc + S_QUEUE;
     a.o_acc = s->r_acc.p; a.o_pot = s->r_pot.p; a.o_eta = s->r_eta.p;
     const bool q64 = s->prm.quadrupole && ctx->prm.precision == SPH_PREC_FP64;
     const bool q32 = s->prm.quadrupole && ctx->prm.precision != SPH_PREC_FP64;
@@ -1751,23 +1758,34 @@ int gravity_phase(sph_system *s) {
     const int jt = (ctx->prm.precision == SPH_PREC_FP32C && s->prm.gravity_jtile == 64) ? 64 : 32;
     a.slices = gravity_slices(s);
     a.o_stride = n;
+    // all resident blocks also beside the hydro lists: 200k head-on run 36.2 ms,
+    // 36.6 at 60% of them, 38.4 at 30%
     sphrt::launch_gravity(a, ctx->prm.precision,
                           jt == 64 ? ctx->grid_g64 : ctx->grid[2][ctx->prm.precision == SPH_PREC_FP64], st, jt);
     phase_event(s, EV_GK_E, st);
     gravity_writeback<<<grid_for(n), 256, 0, st>>>(n, s->prm.G, s->r_acc.p, s->r_pot.p, s->r_eta.p, s->ksr[0].p,
                                                    s->grdh.p, s->dens.p, s->accg2.p, s->pot.p, s->eta.p,
-                                                   ctx->prm.precision == SPH_PREC_FP32C, a.slices, s->r_eta.p);
+                                                   ctx->prm.precision == SPH_PREC_FP32C, a.slices, s->r_eta.p,
+                                                   s->h3.p, s->f_g3.p);
+    if (s->glist_forked) CUDA_TRY(cudaEventRecord(s->ev_join, st));
     return SPH_OK;
 }
 
-int hydro_phase(sph_system *s, bool eager) {
+int gravity_join(sph_system *s) {
+    if (s->glist_forked) CUDA_TRY(cudaStreamWaitEvent(s->st(), s->ev_join, 0));
+    s->glist_forked = false;
+    merge_errors<<<1, 1, 0, s->st()>>>(s->ls[1].sc, s->scal.p);
+    return SPH_OK;
+}
+
+// Records of the hydro pairs, but for the eta that gravity sets.
+int hydro_records(sph_system *s) {
     const int n = s->n;
     cudaStream_t st = s->st();
     sph_context *ctx = s->ctx;
-    phase_event(s, EV_HLIST_B, st);
     hydro_prep<<<grid_for(n), 256, 0, st>>>(n, s->ksr[0].p, s->pres.p, s->grdh.p, s->dens.p, s->bswt.p,
-                                            s->vsnd.p, s->alph[0].p, s->alphu[0].p, s->uene[0].p, s->eta.p,
-                                            s->h1.p, s->h2.p, s->h3.p, ctx->prm.precision == SPH_PREC_FP32C);
+                                            s->vsnd.p, s->alph[0].p, s->alphu[0].p, s->uene[0].p, s->h1.p, s->h2.p,
+                                            s->h3.p);
     if (ctx->prm.precision == SPH_PREC_FP32C)
         sphk::make_hydro_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->h1.p, s->h2.p,
                                                               s->h3.p, s->f_phi.p, s->f_plo.p, s->f_vhi.p,
@@ -1776,6 +1794,13 @@ int hydro_phase(sph_system *s, bool eager) {
     else
         sphk::make_hydro_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->vel[0].p, s->h1.p, s->h2.p,
                                                                   s->f_mp.p, s->f_plo.p, s->f_mv.p);
+    return SPH_OK;
+}
+
+int hydro_phase(sph_system *s, bool eager) {
+    const int n = s->n;
+    cudaStream_t st = s->st();
+    sph_context *ctx = s->ctx;
     int r = build_lists_and_items(s, 1, s->group_node.p, nullptr, eager, s->lscal.p + L_PAIRS_H, nullptr, nullptr,
                                   item_size(s));
     if (r) return r;
@@ -1821,8 +1846,12 @@ int hydro_phase(sph_system *s, bool eager) {
     a.o_acch = s->r_acch.p; a.o_accg = s->r_accg.p; a.o_udot = s->r_udot.p; a.o_diffu = s->r_diffu.p;
     a.rows = m.rows; a.info = m.info; a.ovf = m.ovf; a.n_ovf = m.n_ovf; a.n_i = n;
     a.mi_p = m.i_hi; a.mi_l = m.i_lo; a.mj_p = m.j_hi; a.mj_l = m.j_lo;
-    sphrt::launch_hydro(ctx, m, ctx->grid[1][ctx->prm.precision == SPH_PREC_FP64], a, ctx->prm.precision, st,
-                        s->ev[EV_HK_MID], s->capturing >= 0, &s->long_side());
+    sphrt::launch_hydro_marks(ctx, m, ctx->grid[1][ctx->prm.precision == SPH_PREC_FP64], n, ctx->prm.precision, st,
+                              &s->long_side());
+    phase_event(s, EV_HK_MID, st);
+    r = gravity_join(s);
+    if (r) return r;
+    sphrt::launch_hydro_sums(ctx, a, ctx->prm.precision, st);
     phase_event(s, EV_HK_E, st);
     AlphaParams ap{s->prm.alpha_max, s->prm.alpha_min, s->prm.alphu_max, s->prm.alphu_min};
     hydro_writeback<<<grid_for(n), 256, 0, st>>>(
@@ -1850,6 +1879,9 @@ int force_body(sph_system *s, bool eager, bool energy = true) {
                                               s->ksr[0].p, s->pres.p, s->vsnd.p, s->bswt.p, s->eps2.p, s->pe.p,
                                               s->ctx->prm.precision == SPH_PREC_FP32C);
     r = refit_tree(s, false);   // h (max h, softening) changed in the density phase
+    if (r) return r;
+    phase_event(s, EV_HLIST_B, st);
+    r = hydro_records(s);
     if (r) return r;
     r = gravity_phase(s);
     if (r) return r;
@@ -2062,7 +2094,8 @@ extern "C" int sph_system_destroy(sph_system *s) {
     s->count.release(); s->visit.release(); s->mom.release(); s->quad.release(); s->fq0.release();
     s->fq1.release();
     DevBuf<float4> *f1[] = {&s->flo, &s->fhi, &s->fmom, &s->ptest, &s->f_phi, &s->f_plo, &s->f_vhi, &s->f_vlo,
-                            &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4, &s->f_mp, &s->f_mv, &s->f_shi, &s->f_slo};
+                            &s->f_g1, &s->f_g2, &s->f_g3, &s->f_g4, &s->f_mp, &s->f_mv, &s->f_gphi, &s->f_gplo, &s->f_shi,
+                            &s->f_slo};
     for (auto *b : f1) b->release();
     s->hl_list.release(); s->hl_ovf.release();
     s->uflag.release(); s->uscan.release(); s->ulist.release(); s->a_sfirst.release(); s->a_scount.release();
