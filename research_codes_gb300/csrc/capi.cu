@@ -782,7 +782,7 @@ int stage(sph_context *ctx, KindState &ks, const std::vector<int> &i_off, const 
     build_items(n_walk, i_off.data(), j_off.data(), chunk, split_nj, ks.items);
     L = make_layout(n_walk, ks.items.size(), epi_size * (size_t)i_off[n_walk],
                     epj_size * (size_t)j_off[n_walk]);
-    if (ks.h_in.ensure(L.total) || ks.d_in.ensure(L.total))
+    if (ks.h_in.ensure(L.total) || ks.d_in.ensure(L.total, false))
         return set_error(ctx, SPH_ERR_CUDA, "staging allocation of %zu bytes failed", L.total);
     std::vector<CopyTask> tasks;
     tasks.reserve((size_t)n_arrays * n_walk + L.total / TASK_BYTES);
@@ -885,7 +885,7 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
     if ((st = stage(ctx, ks, i_off, j_off, sizeof(sph_DensityEPI), sizeof(sph_DensityEPJ), item_size(ctx, ni),
                     SPLIT_NJ, arrays, 2, place, L)))
         return st;
-    if (ks.ensure_density(ni, nj) || ks.amb.ensure(cap) || ks.long_items.ensure(ks.items.size()))
+    if (ks.ensure_density(ni, nj, cap, ks.items.size()))
         return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Density) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
@@ -968,7 +968,7 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
     if ((st = stage(ctx, ks, i_off, j_off, sizeof(sph_HydroEPI), sizeof(sph_HydroEPJ), f64 ? item_size(ctx, ni) : 32,
                     f64 ? SPLIT_NJ : 0, arrays, 2, place, L)))
         return st;
-    if (ks.ensure_hydro(ni, nj) || ks.long_items.ensure(ks.items.size()))
+    if (ks.ensure_hydro(ni, nj, ks.items.size()))
         return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Hydro) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
