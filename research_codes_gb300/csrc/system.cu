@@ -338,10 +338,28 @@ __global__ void permute(int n, const int *idx, Persist src, Persist dst) {
     }
 }
 
-// Softening of the first guess of h, for the refit after the tree build only
-// (the refit after the density phase and the gravity kernel use post_density's).
-__global__ void eps2_from_h(int n, const double *h, double *eps2) {
-    GRID_STRIDE(p, n) { eps2[p] = h[p] * h[p] * INV_KSRH2; }
+// Back to the arrays that a captured graph knows, with the softening of the
+// first guess of h for the refit after the tree build (the refit after the
+// density phase and the gravity kernel use post_density's).  One kernel: 13
+// device copies and a kernel were a third of a 10k tree build.
+__global__ void copy_back(int n, Persist src, Persist dst, double *eps2) {
+    GRID_STRIDE(p, n) {
+        const double h = src.ksr[p];
+        dst.pos[p] = src.pos[p];
+        dst.vel[p] = src.vel[p];
+        dst.vel2[p] = src.vel2[p];
+        dst.id[p] = src.id[p];
+        dst.istar[p] = src.istar[p];
+        dst.orig[p] = src.orig[p];
+        dst.uene[p] = src.uene[p];
+        dst.uene2[p] = src.uene2[p];
+        dst.alph[p] = src.alph[p];
+        dst.alph2[p] = src.alph2[p];
+        dst.alphu[p] = src.alphu[p];
+        dst.alphu2[p] = src.alphu2[p];
+        dst.ksr[p] = h;
+        eps2[p] = h * h * INV_KSRH2;
+    }
 }
 
 // compact group roots: position-indexed flags -> group arrays
@@ -394,11 +412,23 @@ __global__ void compact_active(int n, const int *scal, const int *flag, const in
     }
 }
 
-__global__ void set_int(int *p, int v) { *p = v; }
 __global__ void copy_int(const int *src, int *dst) { *dst = *src; }
 
 // list totals: offset[n-1] + count[n-1] (counts beyond the walk count are 0)
 // Task count of a list build (clamped to the task capacity, error bit beyond).
+// counters of an evaluation
+__global__ void begin_evaluation(int *scal, long long *lscal) {
+    for (int k = threadIdx.x; k < L_NI; k += blockDim.x) lscal[k] = 0;
+    if (threadIdx.x == 0) {
+        scal[S_POOLMAX] = 0;
+        scal[S_NROOTS] = 0;
+        scal[S_HOVF] = 0;
+        scal[S_AMBTOT] = 0;
+        scal[S_UNCONV] = 0;
+        scal[S_ITERS] = 1;
+    }
+}
+
 __global__ void task_total(int n, const int *toff, int cap, int *scal) {
     const int t = toff[n];
     scal[S_NTASKS] = t < cap ? t : cap;
@@ -410,6 +440,7 @@ __global__ void list_total(int n, const int *cnt, const int *off, long long cap,
     const long long tot = (long long)off[n - 1] + cnt[n - 1];
     scal[S_TOTAL] = (int)min(tot, (long long)0x7fffffff);
     lscal[lslot] = tot;
+    scal[S_POOLMAX] = max(scal[S_POOLMAX], scal[S_POOL]);
     if (tot > cap) atomicOr(&scal[S_ERROR], E_LISTCAP);
 }
 
@@ -503,16 +534,14 @@ __global__ void light_counts(int n, const int *n_walks, const int *i_count, cons
 // A list build that overflowed its buffers (capacity or stack error set)
 // leaves offsets that run past the list arrays: no pair kernel may read
 // them, so the evaluation gets no work items (it is repeated, or reported).
-__global__ void drop_items_on_overflow(int *scal) {
-    if (scal[S_ERROR] & (E_LISTCAP | E_STACK)) {
-        scal[S_NITEMS] = 0;
-        scal[S_NLONG] = scal[S_NLONG_SHORTER] = 0;
-    }
-}
-
 __global__ void fill_items(int n, const int *n_walks, const int *i_first, const int *i_count, int chunk,
                            int split_nj, const int *j_cnt, int *bkt, const int *light_off, WorkItem *items,
-                           int *n_items, const long long *pairs, bool longs, sphk::LongQueue queue) {
+                           int *n_items, const long long *pairs, bool longs, sphk::LongQueue queue,
+                           const int *error) {
+    if (*error & (E_LISTCAP | E_STACK)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *n_items = 0;
+        return;
+    }
     const int nw = *n_walks;
     const int bh = bkt[2 * NBKT];
     const int n_heavy = bkt[2 * NBKT + 1];
@@ -596,8 +625,12 @@ __global__ void walk_segments(int n, const int *scal, const int *a_first, const 
     }
 }
 
-__global__ void init_rs(int n, const double *ksr, double *rs) {
-    GRID_STRIDE(p, n) { rs[p] = 1.1 * ksr[p]; }   // hdr_density.hpp:376-379
+// h_guess: the first guess, kept for the derivative of this evaluation
+__global__ void init_rs(int n, const double *ksr, double *rs, double *h_guess) {
+    GRID_STRIDE(p, n) {
+        rs[p] = 1.1 * ksr[p];   // hdr_density.hpp:376-379
+        h_guess[p] = ksr[p];
+    }
 }
 
 struct DensOut {
@@ -1176,10 +1209,66 @@ int alloc_all(sph_system *s) {
         if (e__ != cudaSuccess) return sphrt::cuda_error(s->ctx, e__, #x); \
     } while (0)
 
+// Exclusive scan of up to SCAN_SMALL ints by one block: one launch instead of
+// the device-wide scan's two, without its pass over tile states.
+constexpr int SCAN_THREADS = 1024, SCAN_PER = 8, SCAN_STEP = SCAN_THREADS * SCAN_PER, SCAN_SMALL = 2 * SCAN_STEP;
+__global__ void __launch_bounds__(SCAN_THREADS) scan_small(const int *in, int *out, int n) {
+    __shared__ int s_v[SCAN_STEP + SCAN_STEP / 32];   // (padded: a thread's ints are consecutive)
+    __shared__ int s_w[SCAN_THREADS / 32], s_total;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const auto at = [](int k) { return k + (k >> 5); };
+    const int base = threadIdx.x * SCAN_PER;
+    int carry = 0;
+    for (int t = 0; t < n; t += SCAN_STEP) {
+        for (int k = threadIdx.x; k < SCAN_STEP; k += SCAN_THREADS) s_v[at(k)] = t + k < n ? in[t + k] : 0;
+        __syncthreads();
+        int v[SCAN_PER], sum = 0;
+#pragma unroll
+        for (int u = 0; u < SCAN_PER; ++u) {
+            v[u] = s_v[at(base + u)];
+            sum += v[u];
+        }
+        int incl = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (lane == 31) s_w[wid] = incl;
+        __syncthreads();
+        if (wid == 0) {
+            const int x = s_w[lane];
+            int w = x;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += y;
+            }
+            s_w[lane] = w - x;
+            if (lane == 31) s_total = w;
+        }
+        __syncthreads();
+        int run = carry + s_w[wid] + incl - sum;
+#pragma unroll
+        for (int u = 0; u < SCAN_PER; ++u) {
+            s_v[at(base + u)] = run;
+            run += v[u];
+        }
+        carry += s_total;
+        __syncthreads();
+        for (int k = threadIdx.x; k < SCAN_STEP; k += SCAN_THREADS)
+            if (t + k < n) out[t + k] = s_v[at(k)];
+        __syncthreads();
+    }
+}
+
 int exclusive_scan(sph_system *s, const int *in, int *out, int count = -1, int builder = 0) {
+    if (count < 0) count = s->n;
+    if (count <= SCAN_SMALL) {
+        scan_small<<<1, SCAN_THREADS, 0, s->st()>>>(in, out, count);
+        return SPH_OK;
+    }
     ListScratch &L = s->ls[builder];
     size_t bytes = L.cub_bytes;
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(L.cub.p, bytes, in, out, count < 0 ? s->n : count, s->st()));
+    CUDA_TRY(cub::DeviceScan::ExclusiveSum(L.cub.p, bytes, in, out, count, s->st()));
     return SPH_OK;
 }
 
@@ -1236,25 +1325,11 @@ int build_tree(sph_system *s) {
     const uint64_t *keys = kb.Current();
     const int *idx = vb.Current();
     permute<<<grid_for(n), 256, 0, st>>>(n, idx, s->persist(0), s->persist(1));
-    // copy back so that the persistent arrays stay at fixed addresses (graph replay)
+    copy_back<<<grid_for(n), 256, 0, st>>>(n, s->persist(1), s->persist(0), s->eps2.p);
     const size_t nb = (size_t)n;
-    CUDA_TRY(cudaMemcpyAsync(s->pos[0].p, s->pos[1].p, nb * sizeof(dbl4), cudaMemcpyDeviceToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(s->vel[0].p, s->vel[1].p, nb * sizeof(dbl4), cudaMemcpyDeviceToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(s->vel2[0].p, s->vel2[1].p, nb * sizeof(dbl4), cudaMemcpyDeviceToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(s->id[0].p, s->id[1].p, nb * sizeof(long long), cudaMemcpyDeviceToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(s->istar[0].p, s->istar[1].p, nb * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(s->orig[0].p, s->orig[1].p, nb * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    DevBuf<double> *dd[][2] = {{&s->uene[0], &s->uene[1]}, {&s->uene2[0], &s->uene2[1]},
-                               {&s->alph[0], &s->alph[1]}, {&s->alph2[0], &s->alph2[1]},
-                               {&s->alphu[0], &s->alphu[1]}, {&s->alphu2[0], &s->alphu2[1]},
-                               {&s->ksr[0], &s->ksr[1]}};
-    for (auto &d : dd)
-        CUDA_TRY(cudaMemcpyAsync(d[0]->p, d[1]->p, nb * sizeof(double), cudaMemcpyDeviceToDevice, st));
     sphtree::Nodes t = s->nodes();
     sphtree::build_radix_tree<<<grid_for(n), 256, 0, st>>>(keys, n, t);
-    set_int<<<1, 1, 0, st>>>(s->scal.p + S_NROOTS, 0);
     sphtree::mark_subtrees<<<grid_for(2LL * n - 1), 256, 0, st>>>(t, n, s->roots.p, s->scal.p + S_NROOTS);
-    eps2_from_h<<<grid_for(n), 256, 0, st>>>(n, s->ksr[0].p, s->eps2.p);
     r0 = refit_tree(s);
     if (r0) return r0;
     // groups
@@ -1310,10 +1385,6 @@ void launch_lists(int mode, int grid, const sphtree::ListArgs &a, cudaStream_t s
         sphtree::build_lists<sphtree::SYMMETRIC, sphtree::PASS_CHUNK><<<grid, th, 0, st>>>(a);
     else
         sphtree::build_lists<sphtree::GRAVITY, sphtree::PASS_CHUNK><<<grid, th, 0, st>>>(a);
-}
-
-__global__ void pool_usage(int *scal) {
-    atomicMax(&scal[S_POOLMAX], scal[S_POOL]);
 }
 
 // i-particles per density and hydro work item: halved from 32 (down to 4)
@@ -1396,7 +1467,6 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
         CUDA_TRY(cudaMemsetAsync(L.tlcnt.p, 0, sizeof(int) * (size_t)(L.task_cap + 1), st));
         CUDA_TRY(cudaMemsetAsync(sc + S_POOL, 0, 3 * sizeof(int), st));   // pool, pool error, task queue
         launch_lists(mode, tgrid, a, st);
-        pool_usage<<<1, 1, 0, st>>>(sc);
         if (!eager) break;
         int pu[2];
         CUDA_TRY(cudaMemcpyAsync(pu, sc + S_POOL, sizeof(pu), cudaMemcpyDeviceToHost, st));
@@ -1467,12 +1537,12 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
     }
     // work items; those of long lists (density and hydro) in a queue of their own
     const bool longs = kind != 2;
-    if (longs) CUDA_TRY(cudaMemsetAsync(sc + S_NLONG, 0, 3 * sizeof(int), st));
     // density and hydro walks with long lists are split (their pair loops
     // drop most of the list); gravity lists are uniform and kept whole
     const int split_nj = (kind == 2) ? (1 << 30) : (s->prm.item_split_nj > 0 ? s->prm.item_split_nj : ITEM_SPLIT_NJ);
     int *bkt = sc + S_BKT;
-    CUDA_TRY(cudaMemsetAsync(bkt, 0, sizeof(int) * (2 * NBKT + 2), st));
+    static_assert(S_BKT == S_NLONG + 3, "cleared together");
+    CUDA_TRY(cudaMemsetAsync(sc + S_NLONG, 0, sizeof(int) * (3 + 2 * NBKT + 2), st));
     item_buckets<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj, pairs,
                                               longs, bkt);
     bucket_offsets<<<1, 32, 0, st>>>(bkt, kind == 2 ? 0 : (s->prm.heavy_classes >= 0 ? s->prm.heavy_classes
@@ -1484,8 +1554,8 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
     r = exclusive_scan(s, L.tcnt.p, L.toff.p, n + 1, builder);
     if (r) return r;
     fill_items<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], ifirst, icount, chunk, split_nj, s->lcnt[kind].p,
-                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, s->long_queue());
-    drop_items_on_overflow<<<1, 1, 0, st>>>(sc);
+                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, s->long_queue(),
+                                            sc + S_ERROR);
     return SPH_OK;
 }
 
@@ -1652,12 +1722,7 @@ int density_phase(sph_system *s, bool eager) {
                                                                 s->f_plo.p, s->f_vhi.p, s->f_vlo.p);
     else
         sphk::make_row_records<<<grid_for(n), 256, 0, st>>>(n, s->pos[0].p, s->ksr[0].p, s->f_phi.p, s->f_plo.p);
-    init_rs<<<grid_for(n), 256, 0, st>>>(n, s->ksr[0].p, s->rs.p);
-    // the first guess, kept for the derivative of this evaluation
-    CUDA_TRY(cudaMemcpyAsync(s->h_guess.p, s->ksr[0].p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    set_int<<<1, 1, 0, st>>>(s->scal.p + S_ITERS, 1);
-    set_int<<<1, 1, 0, st>>>(s->scal.p + S_AMBTOT, 0);
-    set_int<<<1, 1, 0, st>>>(s->scal.p + S_UNCONV, 0);
+    init_rs<<<grid_for(n), 256, 0, st>>>(n, s->ksr[0].p, s->rs.p, s->h_guess.p);
     const int max_it = std::max(1, s->prm.max_density_iterations);
     int r = density_walk(s, 0, eager);
     if (r) return r;
@@ -1810,7 +1875,6 @@ int hydro_phase(sph_system *s, bool eager) {
     // rows of particles no work item reaches (a failed list build) stay
     // empty; no particle without a row and no long item yet
     CUDA_TRY(cudaMemsetAsync(s->r_info.p, 0, sizeof(int2) * (size_t)n, st));
-    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_HOVF, 0, sizeof(int), st));
     CUDA_TRY(cudaMemsetAsync(s->scal.p + S_QUEUE, 0, sizeof(int), st));
     if (s->prm.hydro_signal_skip != 0)
         walk_csmax<<<ctx->sm_count * 8, CSMAX_THREADS, 0, st>>>(s->walk_num[1], s->loff[1].p, s->jidx[1].p, s->f_mv.p,
@@ -1870,8 +1934,7 @@ int hydro_phase(sph_system *s, bool eager) {
 int force_body(sph_system *s, bool eager, bool energy = true) {
     const int n = s->n;
     cudaStream_t st = s->st();
-    CUDA_TRY(cudaMemsetAsync(s->lscal.p, 0, sizeof(long long) * L_NI, st));
-    CUDA_TRY(cudaMemsetAsync(s->scal.p + S_POOLMAX, 0, sizeof(int), st));
+    begin_evaluation<<<1, 32, 0, st>>>(s->scal.p, s->lscal.p);
     int r = build_tree(s);
     if (r) return r;
     r = gravity_lists(s, eager);
