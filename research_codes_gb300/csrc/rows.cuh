@@ -25,10 +25,11 @@ constexpr int ROW_CAP = 128;
 static_assert(ROW_CAP % 32 == 0, "eight lanes read a row four entries at a time");
 // Items with longer lists than this are taken by a whole block (the LONG forms
 // of mark_rows and density_stream).  On a full SM a warp streams ~1.6e7 entries
-// per second, the chip ~5e11 listed pairs: beyond pairs / 65536 entries one
-// warp's item lasts about half of the whole walk's time.
-__device__ __forceinline__ int long_list(long long pairs) {
-    return (int)min(max(pairs >> 17, 768LL), 1LL << 30);
+// per second, the chip ~5e11 listed pairs: beyond pairs / 131072 entries one
+// warp's item lasts about a quarter of the whole walk's time (200k head-on run: 37.8 ms at
+// 2^16, 37.1 at 2^17, 38.6 at 2^18, 45.9 at 2^19).
+__device__ __forceinline__ int long_list(long long pairs, int least = 768) {
+    return (int)min(max(pairs >> 17, (long long)least), 1LL << 30);
 }
 constexpr int MARK_LONG_WARPS = 16, HYDRO_LONG_WARPS = 8;
 // Radii outside this range (or NaN) are left to the sweep: their squares

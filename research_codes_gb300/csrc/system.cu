@@ -470,9 +470,9 @@ __device__ __forceinline__ int cost_bucket(int nj, int sz) {
 // Histogram of the items of all walks over the cost classes (bkt[0..NBKT),
 // zero on entry).
 __global__ void item_buckets(int n, const int *n_walks, const int *i_count, const int *j_cnt, int chunk,
-                             int split_nj, const long long *pairs, bool longs, int *bkt) {
+                             int split_nj, const long long *pairs, bool longs, int long_min, int *bkt) {
     const int nw = *n_walks;
-    const int long_nj = longs ? sphk::long_list(*pairs) : 0x7fffffff;
+    const int long_nj = longs ? sphk::long_list(*pairs, long_min) : 0x7fffffff;
     GRID_STRIDE(k, n) {
         if (k < nw) {
             const int ni = i_count[k], nj = j_cnt[k];
@@ -516,10 +516,11 @@ __global__ void bucket_offsets(int *bkt, int heavy) {
 
 // Number of light items (class below the heavy ones) of each walk.
 __global__ void light_counts(int n, const int *n_walks, const int *i_count, const int *j_cnt, int chunk,
-                             int split_nj, const long long *pairs, bool longs, const int *bkt, int *lc) {
+                             int split_nj, const long long *pairs, bool longs, int long_min, const int *bkt,
+                             int *lc) {
     const int nw = *n_walks;
     const int bh = bkt[2 * NBKT];
-    const int long_nj = longs ? sphk::long_list(*pairs) : 0x7fffffff;
+    const int long_nj = longs ? sphk::long_list(*pairs, long_min) : 0x7fffffff;
     GRID_STRIDE(k, n + 1) {
         int c = 0;
         if (k < nw) {
@@ -536,8 +537,8 @@ __global__ void light_counts(int n, const int *n_walks, const int *i_count, cons
 // them, so the evaluation gets no work items (it is repeated, or reported).
 __global__ void fill_items(int n, const int *n_walks, const int *i_first, const int *i_count, int chunk,
                            int split_nj, const int *j_cnt, int *bkt, const int *light_off, WorkItem *items,
-                           int *n_items, const long long *pairs, bool longs, sphk::LongQueue queue,
-                           const int *error) {
+                           int *n_items, const long long *pairs, bool longs, int long_min,
+                           sphk::LongQueue queue, const int *error) {
     if (*error & (E_LISTCAP | E_STACK)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *n_items = 0;
         return;
@@ -545,7 +546,7 @@ __global__ void fill_items(int n, const int *n_walks, const int *i_first, const 
     const int nw = *n_walks;
     const int bh = bkt[2 * NBKT];
     const int n_heavy = bkt[2 * NBKT + 1];
-    const int long_nj = longs ? sphk::long_list(*pairs) : 0x7fffffff;
+    const int long_nj = longs ? sphk::long_list(*pairs, long_min) : 0x7fffffff;
     GRID_STRIDE(k, n) {
         if (k < nw) {
             const int ni = i_count[k];
@@ -1537,6 +1538,12 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
     }
     // work items; those of long lists (density and hydro) in a queue of their own
     const bool longs = kind != 2;
+    // shortest list for a block of its own: a star of 10k takes 0.86 ms per
+    // evaluation at 768 entries, 0.83 at 384 for the FP32C density (whose block
+    // also shares the listed passes; 20k is slower from 128 down) and 0.82 at
+    // 2500 for hydro, whose blocks pay for putting the rows in order (20k: signal
+    // and rows 0.36 ms at 768, 0.23 at 2500); FP64 density at 1: 0.27 -> 0.37 ms
+    const int long_min = kind == 1 ? 2500 : (s->ctx->prm.precision == SPH_PREC_FP64 ? 768 : 384);
     // density and hydro walks with long lists are split (their pair loops
     // drop most of the list); gravity lists are uniform and kept whole
     const int split_nj = (kind == 2) ? (1 << 30) : (s->prm.item_split_nj > 0 ? s->prm.item_split_nj : ITEM_SPLIT_NJ);
@@ -1544,17 +1551,17 @@ int build_lists_and_items(sph_system *s, int kind, const int *walk_node, const d
     static_assert(S_BKT == S_NLONG + 3, "cleared together");
     CUDA_TRY(cudaMemsetAsync(sc + S_NLONG, 0, sizeof(int) * (3 + 2 * NBKT + 2), st));
     item_buckets<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj, pairs,
-                                              longs, bkt);
+                                              longs, long_min, bkt);
     bucket_offsets<<<1, 32, 0, st>>>(bkt, kind == 2 ? 0 : (s->prm.heavy_classes >= 0 ? s->prm.heavy_classes
                                                                                    : SPH_HEAVY_CLASSES));
     // light items in walk order: per-walk counts (the task arrays are free
     // again once the lists are built) and their scan
     light_counts<<<grid_for(n + 1), 256, 0, st>>>(n, s->walk_num[kind], icount, s->lcnt[kind].p, chunk, split_nj,
-                                                  pairs, longs, bkt, L.tcnt.p);
+                                                  pairs, longs, long_min, bkt, L.tcnt.p);
     r = exclusive_scan(s, L.tcnt.p, L.toff.p, n + 1, builder);
     if (r) return r;
     fill_items<<<grid_for(n), 256, 0, st>>>(n, s->walk_num[kind], ifirst, icount, chunk, split_nj, s->lcnt[kind].p,
-                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, s->long_queue(),
+                                            bkt, L.toff.p, L.items.p, sc + S_NITEMS, pairs, longs, long_min, s->long_queue(),
                                             sc + S_ERROR);
     return SPH_OK;
 }
