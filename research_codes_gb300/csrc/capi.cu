@@ -632,7 +632,9 @@ namespace {
 
 enum { K_DENS = 0, K_HYDRO = 1, K_GRAV = 2 };
 constexpr float ROW_SLACK = 1.03f;   // row radius of the density over the first guess of h
-constexpr int LONG_NJ = 4096;    // lists beyond this are marked by a block per item
+// Lists beyond this are marked by a block per item (hydro 21k batch 2.86 ms with none,
+// 2.23 at 4096, 1.93 at 1536, 1.98 at 1024; density 40k 2.13 / 2.04 / 2.07).
+constexpr int LONG_NJ = 1536;
 constexpr int SPLIT_NJ = 1024;   // density and hydro: lists beyond this make smaller items
 
 int longest(const int32_t *n, int n_walk) {
@@ -992,7 +994,7 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         m.queue = ctx->d_queue + K_HYDRO;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 8;
         m.longs = sphk::LongQueue{ks.long_items.p, ctx->d_queue + 9, 0}; m.long_nj = LONG_NJ;
-        m.push_long = f64 && longest(n_epj, n_walk) > LONG_NJ;
+        m.push_long = longest(n_epj, n_walk) > LONG_NJ;
         m.o_vsmx = ks.o[3].p;
         m.sv_skip = 1;
         sphk::HydroArgs a{};

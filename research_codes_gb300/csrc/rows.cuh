@@ -32,6 +32,9 @@ __device__ __forceinline__ int long_list(long long pairs, int least = 768) {
     return (int)min(max(pairs >> 17, (long long)least), 1LL << 30);
 }
 constexpr int MARK_LONG_WARPS = 16, HYDRO_LONG_WARPS = 8;
+// FP32C hydro rows: longest list (in steps of 64 entries) whose LONG form
+// keeps the row order of a warp's item
+constexpr int LONG_STEPS = 2048;
 // Radii outside this range (or NaN) are left to the sweep: their squares
 // leave the FP32 range.
 constexpr float ROW_HMIN = 1.0e-15f, ROW_HMAX = 1.0e15f;
@@ -234,6 +237,8 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
     __shared__ int s_j[WARPS][RING];   // LONG: list positions
     __shared__ long long s_id[HW][HYDRO ? RING : 1];
     __shared__ int s_cnt[LONG ? 32 : 1];
+    constexpr bool KEYS = LONG && KIND == ROWS_HYDRO32;
+    __shared__ int s_step[KEYS ? LONG_STEPS : 1];   // staged entries per step, then before it
     // hydro: 32 entries whose signal-velocity terms are due (item-frame
     // position and velocity, sound speed, |v - v_c|)
     __shared__ __align__(16) float s_sig[HW][8][HN];
@@ -257,6 +262,8 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
             wi = a.items[item];
         }
         ItemRef r = decode(wi, a.j_off, a.i_list, lane);
+        const int item_tpi = r.tpi;
+        const bool keyed = KEYS && r.nj <= 64 * LONG_STEPS;
         if (LONG) {   // a lane per particle
             r.tpi = 1;
             r.sub = 0;
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
             r.ii = a.i_list ? a.i_list[k] : k;
             if (threadIdx.x < 32) s_cnt[threadIdx.x] = 0;
             __syncthreads();
-        } else if (a.push_long && r.nj > long_nj) {
+        } else if (a.push_long && r.nj > long_nj && (KIND != ROWS_HYDRO32 || r.nj <= 64 * LONG_STEPS)) {
             if (lane == 0) a.longs.push(wi);
             continue;
         }
@@ -447,6 +454,7 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                 __syncwarp();
             };
             for (int t = t0; t < nj; t += STRIDE) {
+                int staged = 0;   // of this step
 #pragma unroll
                 for (int s = 0; s < 2; ++s) {
                     const int k = t + 32 * s + lane;
@@ -490,13 +498,14 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                         s_x[wid][slot] = px;
                         s_y[wid][slot] = py;
                         s_z[wid][slot] = pz;
-                        s_j[wid][slot] = jc;
+                        s_j[wid][slot] = keyed ? (jc << 6) | (staged + __popc(m & lt)) : jc;
                         if (HYDRO) {
                             s_h[hw][slot] = hj2;
                             s_id[hw][slot] = a.j_id[j];
                         }
                     }
                     fill += __popc(m);
+                    staged += __popc(m);
                     if (HYDRO) {
                         n_near += __popc(m);
                         const int nb = nj - t - 32 * s;
@@ -521,6 +530,7 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                         }
                     }
                 }
+                if (KEYS && keyed && lane == 0) s_step[t >> 6] = staged;
                 __syncwarp();
                 while (fill >= 32) {
                     consume(32);
@@ -552,28 +562,56 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
         if (LONG) {
             __syncthreads();
             // rows in list order: each hit's place is the number of hits at
-            // earlier list positions
+            // earlier list positions.  FP32C hydro: in the order of a warp's
+            // item, whose tpi lanes take a tile of 32 staged entries each
+            // their own residue
+            if (KEYS && keyed) {
+                if (wid == 0) {
+                    int before = 0;
+                    for (int k0 = 0; 64 * k0 < nj; k0 += 32) {
+                        const int v = 64 * (k0 + lane) < nj ? s_step[k0 + lane] : 0;
+                        int incl = v;
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int x = __shfl_up_sync(FULL, incl, o);
+                            if (lane >= o) incl += x;
+                        }
+                        if (64 * (k0 + lane) < nj) s_step[k0 + lane] = before + incl - v;
+                        before += __shfl_sync(FULL, incl, 31);
+                    }
+                }
+                __syncthreads();
+            }
+            auto key = [&](int q) {
+                if (!(KEYS && keyed)) return q;
+                const int e = s_step[q >> 12] + (q & 63);   // staged entries before it
+                return (e & ~31) << 5 | ((e & (item_tpi - 1)) << 5) | (e & 31);
+            };
             for (int i = wid; i < r.ni; i += WARPS) {
                 const int c = s_cnt[i];
                 int *row = a.rows + (size_t)__shfl_sync(FULL, ii, i) * ROW_CAP;
                 if (c > ROW_CAP) continue;
-                int pos[ROW_CAP / 32], rank[ROW_CAP / 32];
+                int pos[ROW_CAP / 32], keys[ROW_CAP / 32], rank[ROW_CAP / 32];
 #pragma unroll
                 for (int u = 0; u < ROW_CAP / 32; ++u) {
-                    pos[u] = (32 * u + lane < c) ? row[32 * u + lane] : 0x7fffffff;
+                    const bool in = 32 * u + lane < c;
+                    pos[u] = in ? row[32 * u + lane] : 0;
+                    keys[u] = in ? key(pos[u]) : 0x7fffffff;
                     rank[u] = 0;
                 }
 #pragma unroll
                 for (int v = 0; v < ROW_CAP / 32; ++v)
                     for (int q = 0; q < 32; ++q) {
-                        const int other = __shfl_sync(FULL, pos[v], q);
+                        const int other = __shfl_sync(FULL, keys[v], q);
 #pragma unroll
-                        for (int u = 0; u < ROW_CAP / 32; ++u) rank[u] += other < pos[u] ? 1 : 0;
+                        for (int u = 0; u < ROW_CAP / 32; ++u) rank[u] += other < keys[u] ? 1 : 0;
                     }
                 __syncwarp();
 #pragma unroll
                 for (int u = 0; u < ROW_CAP / 32; ++u)
-                    if (32 * u + lane < c) row[rank[u]] = a.j_idx ? a.j_idx[jb + pos[u]] : jb + pos[u];
+                    if (32 * u + lane < c) {
+                        const int k = KEYS && keyed ? pos[u] >> 6 : pos[u];
+                        row[rank[u]] = a.j_idx ? a.j_idx[jb + k] : jb + k;
+                    }
             }
             if (use) lcount = s_cnt[lane];
             if (HYDRO) {

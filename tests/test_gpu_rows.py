@@ -1,7 +1,7 @@
 """GPU tests of the neighbour-row kernels (csrc/rows.cuh and the sums over rows)
 at the sizes where they can go wrong, against the oracle: rows of 0 to more
 than ROW_CAP entries, list lengths around a streaming step (64 entries) and
-around the length that a whole block marks (4096), group sizes that
+around the length that a whole block marks (1536), group sizes that
 leave several lanes per particle, first guesses of h that leave the row
 radius, and coordinates whose squares leave the FP32 range (FP64 mode).
 
@@ -60,7 +60,7 @@ def _check(prec, epi, epj):
 @pytest.mark.parametrize("prec", ["fp32c", "fp64"])
 @pytest.mark.parametrize("n_i,n_j,guess,neighbours", [
     (1, 60, 1.0, 20.0), (3, 64, 1.0, 30.0), (32, 65, 1.0, 30.0), (33, 500, 1.0, 50.0),
-    (7, 4096, 1.0, 50.0), (37, 4097, 1.0, 50.0),     # the last list of one warp, the first of a block
+    (7, 1536, 1.0, 50.0), (37, 1537, 1.0, 50.0), (7, 4097, 1.0, 50.0),   # the last list of one warp, the first of a block
     (40, 4000, 1.0, 160.0), (40, 9000, 1.0, 160.0),   # rows beyond their capacity
     (40, 3000, 0.9, 50.0), (40, 3000, 1.25, 50.0),   # h leaves the row radius upwards and downwards
     (700, 5000, 1.0, 50.0),
@@ -103,7 +103,7 @@ def _hydro_cloud(n_i, n_j, seed, neighbours=50.0, scale=1.0, speed=1.0):
 @pytest.mark.parametrize("prec", ["fp32c", "fp64"])
 @pytest.mark.parametrize("n_i,n_j,neighbours,speed", [
     (1, 40, 20.0, 1.0), (5, 64, 20.0, 0.0), (33, 65, 20.0, 1.0), (33, 1000, 50.0, 1e-3),
-    (7, 4096, 50.0, 1.0), (37, 4097, 50.0, 30.0),   # the last list of one warp, the first of a block
+    (7, 1536, 50.0, 1.0), (37, 1537, 50.0, 30.0), (7, 4097, 50.0, 1.0),   # the last list of one warp, the first of a block
     (40, 3000, 160.0, 1.0), (40, 9000, 160.0, 1.0),  # rows beyond their capacity
 ])
 def test_hydro_rows(prec, n_i, n_j, neighbours, speed):
@@ -156,3 +156,29 @@ def test_staged_arrays_by_size(n_walk, n_j):
             assert np.array_equal(got[k]["np"], one["np"])
     one = orc.density(*walks[-1], eta=ETA, ksr_max=0.0)
     assert rel_err(got[-1]["dens"], one["dens"], 1e-3).max() < 1e-11
+
+
+@pytest.mark.parametrize("prec", ["fp32c", "fp64"])
+@pytest.mark.parametrize("n_i", [1, 5, 9, 17, 32, 40])
+def test_hydro_rows_of_a_block_equal_a_warps(prec, n_i):
+    """A list one entry under and some over the length that a block marks: the
+    added j-particles lie far away and raise no signal velocity, so the rows, and
+    the sums in their order, are the same bit for bit."""
+    epi, epj = _hydro_cloud(n_i, 1536, n_i, 50.0)
+    far = np.repeat(epj[:200], 1)
+    far["id"] += 10 ** 6
+    far["pos"] += 500.0
+    far["vsnd"] = 0.0
+    far["vel"] = epj["vel"].mean(axis=0)
+    keep = np.random.default_rng(n_i).permutation(1736)
+    mixed = np.concatenate([epj, far])[keep]
+    order = mixed[mixed["id"] < 10 ** 6]   # the same list without the far ones
+    out = []
+    with functors.Context(precision=prec, eta=ETA) as ctx:
+        for lst in (order, mixed):
+            o = np.zeros(n_i, abi.Hydro)
+            functors.calcHydro(ctx)(epi, n_i, lst, len(lst), o)
+            out.append(o)
+    for f in ("acch", "accg", "udot", "diffu"):
+        assert np.array_equal(out[0][f], out[1][f]), f
+    assert (out[1]["vsmx"] >= out[0]["vsmx"]).all()
