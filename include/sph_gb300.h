@@ -346,10 +346,10 @@ typedef struct sph_system_params {
                             cut into work items of 16, 8 or 4 i-particles (<= 0: 4096) */
     int32_t heavy_classes; /* work items of this many most expensive cost classes run
                             first, the rest in walk order (< 0: 2)                      */
-    float   density_list_slack; /* radius of the density kernel's per-lane neighbour
-                            lists over each particle's first-pass h (default 1.03): the
-                            first pass writes them, the later passes and the gradient
-                            pass read them while h stays within it; <= 0 or NaN: no
+    float   density_list_slack; /* radius of the density's neighbour lists over each
+                            particle's first guess of h (default 1.03): later passes
+                            and the gradient pass read them while h stays within it
+                            (FP64: the rows that all passes read); <= 0 or NaN: no
                             lists, every pass streams the walk's j-list; above 2 the
                             create / set_params calls fail with INVALID_ARGUMENT       */
     int32_t hydro_signal_skip; /* 1 (default): hydro tiles of 32 j-entries whose
@@ -396,7 +396,8 @@ typedef struct sph_system_stats {
                                              signal velocity only                */
     int64_t density_list_passes;          /* first walk: work-item passes after
                                              the first (second, third, gradient)
-                                             served from neighbour lists         */
+                                             served from neighbour lists (FP64:
+                                             particle passes, from rows)         */
     int64_t density_sweep_passes;         /* ... that swept the walk's j-list     */
     int64_t hydro_sv_tiles_skipped;       /* hydro 32-entry tiles whose signal-
                                              velocity terms provably could not
@@ -408,9 +409,9 @@ typedef struct sph_system_stats {
                                              (32 x the largest per-lane count of
                                              each tile); marked / slots is the
                                              lane utilisation of those loops     */
-    int64_t hydro_rows_overflowed;        /* FP32C: particles with more marked
-                                             pairs than a list row holds (summed
-                                             over the walk's whole list instead) */
+    int64_t hydro_rows_overflowed;        /* particles with more marked pairs
+                                             than a row holds (summed over the
+                                             walk's whole list instead)          */
     int32_t last_status;
 } sph_system_stats;
 
@@ -504,9 +505,9 @@ int sph_system_get_lists(sph_system *sys, int32_t kind, int32_t *n_walk, int64_t
  * step): [0] tree + groups, [1] density incl. lists and all walks,
  * [2] density pair kernel of the first walk, [3] gravity lists,
  * [4] gravity pair kernel, [5] hydro prep + lists, [6] hydro pair kernels,
- * [7] the whole force evaluation, [8] and [9] the two parts of [6] (FP32C:
- * the signal-velocity / marking kernel and the double-float pass over the
- * marked pairs; FP64: the pair kernel and nothing).  Returns the number of
+ * [7] the whole force evaluation, [8] and [9] the two parts of [6] (the
+ * signal velocities and rows, then the pair sums over the rows; in double-float
+ * arithmetic in FP32C).  Returns the number of
  * values written, or minus a status code.  Eager evaluations record the
  * events directly; captured graphs (force evaluation and step) hold them as
  * external event-record nodes, so the values after a graph replay are that

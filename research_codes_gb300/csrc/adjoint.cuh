@@ -141,7 +141,10 @@ __global__ void adj_alpha(AdjState s, AdjSeed sd, AdjAcc a) {
 
 // -------------------------------------------------------------- stage B
 // hydro pairs: seeds acch (= acc / 2 per pair sum), accg (= G acc / 2), udot / 2
-// of both ends of each pair
+// of both ends of each pair, gathered over the forward's hydro rows (a pair is
+// in the rows of both ends), eight lanes per particle: no atomics, and 1/15 of
+// the listed entries (100k, this stage and the density's: 145 -> 44 ms).  FP64
+// pipe bound.
 __global__ void __launch_bounds__(128) adj_hydro(AdjState s, AdjSeed sd, AdjAcc a) {
     const int sub = threadIdx.x & (LANES - 1);
     ADJ_PARTICLES(ip, s.n) {
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(128) adj_density_sums(AdjState s, AdjAcc a) {
 
 // ... then the pairs: what the sums of both ends pass to particle i.  The
 // terms of j's sums have -d and -u, and i stands at their other end: both
-// signs cancel, so the two ends' coefficients add.
+// signs cancel, so the two ends' coefficients add.  FP64 pipe bound (100k: 2.2 ms).
 __global__ void __launch_bounds__(128) adj_density_grad(AdjState s, AdjAcc a) {
     const int sub = threadIdx.x & (LANES - 1);
     ADJ_PARTICLES(ip, s.n) {
@@ -540,7 +543,9 @@ __global__ void __launch_bounds__(128) adj_density_grad(AdjState s, AdjAcc a) {
 }
 
 // -------------------------------------------------------------- stage H
-// the three smoothing-length passes: (rho_2, h_3) -> positions, first guess h_0
+// the three smoothing-length passes: (rho_2, h_3) -> positions, first guess h_0.
+// FP64 pipe bound (75% busy; 100k: 5.2 ms); rows of the passes are not
+// symmetric, so the j side takes atomics.
 __global__ void __launch_bounds__(128) adj_density_passes(AdjState s, AdjAcc a) {
     const int sub = threadIdx.x & (LANES - 1);
     ADJ_PARTICLES(ip, s.n) {

@@ -16,6 +16,12 @@
 //                  FP64 recomputation of FP32C results whose search-radius
 //                  decision is ambiguous.
 //
+// Bound: density_rows by the FP64 pipe (FP64) or by its launch and the latency of
+// the rows (calls: 64 targets in 13 us where one warp per 32 targets took
+// 100); eight lanes per particle keep a call of 64 on 16 warps and each pass at
+// ~8 entries per lane.  density_sweep by the longest list of a batch (29k
+// entries: 158 us; a warp took 1.6 ms).
+//
 // Both form the separations relative to the particle itself; FP32C sums a few
 // terms in FP32, folds them into Kahan pairs per lane and adds the lanes with
 // error-free transformations.

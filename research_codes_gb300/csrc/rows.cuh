@@ -13,7 +13,11 @@
 // the radius is widened over every rounding of the FP32 frame, so a row is a
 // superset of the pairs inside the radius and never depends on the precision
 // of the sums that follow; entries beyond a support add exactly zero there.
-// Bound: instruction issue and the latency of the list streaming.
+// Bound: instruction issue and the latency of the list streaming, so short
+// launches live by how many warps they keep busy: long lists go to blocks
+// (LONG), small systems get smaller items.  What rows replace: every pass over
+// all listed pairs, in FP64 at 1/60 of the FP32 rate: FP64 density call of 64
+// among 20k 2095 -> 105 us, FP64 run of 50k (density and hydro) 85 -> 40 ms.
 #pragma once
 
 #include "sph_device.cuh"
