@@ -1127,7 +1127,7 @@ void phase_event(sph_system *s, int k, cudaStream_t st) {
         cudaEventRecord(s->ev[k], st);
 }
 
-int gravity_slices(const sph_system *s);
+int max_gravity_slices(const sph_system *s);
 
 int alloc_all(sph_system *s) {
     const size_t n = (size_t)s->n;
@@ -1146,7 +1146,8 @@ int alloc_all(sph_system *s) {
     for (auto *b : d1) e |= b->ensure(n);
     DevBuf<double> *d3[] = {&s->acc, &s->acch, &s->accg1, &s->accg2, &s->r_acch, &s->r_accg, &s->staging};
     for (auto *b : d3) e |= b->ensure(3 * n);
-    const size_t parts = n * (size_t)gravity_slices(s);
+    // the precision of the context can change after this
+    const size_t parts = n * (size_t)max_gravity_slices(s);
     e |= s->r_acc.ensure(3 * parts) | s->r_pot.ensure(parts) | s->r_eta.ensure(parts);
     e |= s->np.ensure(n) | s->t_np.ensure(n) | s->t_itr.ensure(n);
     e |= s->pe.ensure(n) | s->h1.ensure(n) | s->h2.ensure(n) | s->h3.ensure(n);
@@ -1401,9 +1402,11 @@ int item_size(const sph_system *s) {
 // regroup the compensated FP32 sums (1e-9 of eta), which the derivative shows,
 // and their gravity hides behind the hydro lists (star of 10k: 1.225 ms with parts, 1.217 without).
 constexpr int MAX_SLICES = 8;
-int gravity_slices(const sph_system *s) {
-    if (s->ctx->prm.precision != SPH_PREC_FP64) return 1;
+int max_gravity_slices(const sph_system *s) {
     return sphk::gravity_slices(s->n / 24 + 1, 1024, 6LL * 16 * s->ctx->sm_count, MAX_SLICES);
+}
+int gravity_slices(const sph_system *s) {
+    return s->ctx->prm.precision == SPH_PREC_FP64 ? max_gravity_slices(s) : 1;
 }
 
 // Builds the lists of `kind` over the walks (group nodes + radii) and the
