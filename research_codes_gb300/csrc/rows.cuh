@@ -417,8 +417,10 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                 const f2 E = f2_fma(f2_add(at(7), f2_make(di, di)),
                                     f2_fma(f2_make(4.0f * pad, 4.0f * pad), RI, f2_make(4.0e-6f, 4.0e-6f)),
                                     f2_make(2.0f * verr, 2.0f * verr));
+                // NaN (r = 0 in the frame: nothing is known of w) stays NaN,
+                // which no comparison with lb skips
                 const float2 t = f2_get(f2_fma(f2_mul(DOT, NEG), RI, E));
-                return f2_get(f2_fma(f2_make(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f)), f2_make(3.0f, 3.0f),
+                return f2_get(f2_fma(f2_make(max0_nan(t.x), max0_nan(t.y)), f2_make(3.0f, 3.0f),
                                      f2_add(at(6), f2_make(vi.w, vi.w))));
             };
             // signal-velocity terms of the nb <= 32 staged entries; lb is kept

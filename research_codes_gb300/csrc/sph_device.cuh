@@ -133,6 +133,12 @@ __device__ __forceinline__ double w1_term(double q, double u, double u2, double 
 
 __device__ __forceinline__ float max0(float x) { return fmaxf(x, 0.0f); }
 __device__ __forceinline__ double max0(double x) { return fmax(x, 0.0); }
+// max(x, 0), NaN for NaN
+__device__ __forceinline__ float max0_nan(float x) {
+    float y;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
+    return y;
+}
 
 // Compensated accumulator.  In FP32 mode a warp lane sums the pairs of one
 // 32-wide j-tile in plain FP32 and folds the tile's partial sum into a Kahan

@@ -1,0 +1,92 @@
+"""GPU tests of functor calls with values at the edges of what the row kernels
+(csrc/rows.cuh, csrc/density_rows.cuh) hold in FP32: coincident particles,
+sources far outside the FP32 range of a squared distance, values that are not
+finite.
+
+Expected values are the oracle's, on the list without the sources that add
+nothing where the oracle's own arithmetic makes NaN of them.  Tolerances as in
+test_gpu_functors.py (same quantities, same reasons): FP64 1e-11, FP32C 1e-5.
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from oracle import oracle as orc
+from research_codes_gb300 import abi, functors
+
+pytestmark = pytest.mark.gpu
+
+ETA = 1.18
+TOL = {"fp64": 1e-11, "fp32c": 1e-5}
+
+
+def _ball(n_i, n_j, seed, centre=30.0, neighbours=40.0):
+    """HydroEPI / HydroEPJ of a uniform ball: the n_i sources nearest to one of
+    them as targets, sound speeds of order one, velocities of order one."""
+    rng = np.random.default_rng(seed)
+    x = rng.normal(size=(n_j, 3))
+    x *= (rng.uniform(size=n_j) ** (1.0 / 3.0) / np.linalg.norm(x, axis=1))[:, None]
+    epj = np.zeros(n_j, abi.HydroEPJ)
+    epj["id"], epj["pos"], epj["vel"] = np.arange(n_j), x + centre, rng.normal(size=(n_j, 3))
+    epj["mass"] = rng.uniform(0.5, 1.5, n_j) / n_j
+    epj["ksr"] = (neighbours / n_j) ** (1.0 / 3.0) * rng.uniform(0.8, 1.2, n_j)
+    epj["hinv"] = 1.0 / epj["ksr"]
+    epj["dens"] = 0.3 + 0.1 * (x ** 2).sum(1)
+    epj["pres"] = 1.0 - 0.5 * (x ** 2).sum(1)
+    epj["presc"] = epj["pres"] / epj["dens"] ** 2
+    epj["bswt"], epj["alph"], epj["alphu"] = rng.uniform(0.0, 0.5, n_j), 1.0, 0.05
+    epj["vsnd"] = rng.uniform(1.0, 1.3, n_j)
+    epj["thrm"], epj["eta"] = epj["pres"] / epj["dens"], 0.1 * epj["ksr"] ** 2
+    near = np.argsort(((x - x[0]) ** 2).sum(1), kind="stable")[:n_i]
+    epi = np.zeros(n_i, abi.HydroEPI)
+    for f in epi.dtype.names:
+        epi[f] = epj[f][near]
+    return epi, epj, near
+
+
+def _hydro(prec, epi, epj):
+    out = np.zeros(len(epi), abi.Hydro)
+    with functors.Context(precision=prec, eta=ETA) as ctx:
+        functors.calcHydro(ctx)(epi, len(epi), epj, len(epj), out)
+    return out
+
+
+# one target (items of one particle) and groups; lists of one warp and of a block
+SIZES = [(1, 700), (1, 4000), (40, 700), (40, 4000)]
+
+
+@pytest.mark.parametrize("prec", ["fp32c", "fp64"])
+@pytest.mark.parametrize("n_i,n_j", SIZES)
+@pytest.mark.parametrize("where,speed", [(1e16, 50.0), (1e16, 1e4), (1e3, 1e17)])
+def test_signal_velocity_of_far_and_fast_sources(prec, n_i, n_j, where, speed):
+    """The largest signal velocity is that of a source beyond the range in
+    which FP32 bounds it."""
+    epi, epj, near = _ball(n_i, n_j, 17 * n_i + n_j)
+    far = epj[~np.isin(epj["id"], near)][-1:].copy()
+    far["pos"] = epi["pos"][0] + [where, 0.0, 0.0]
+    far["vel"] = [-speed, 0.0, 0.0]
+    far["id"] += 10 ** 6
+    lst = np.concatenate([epj[: n_j // 2], far, epj[n_j // 2:]])
+    out, ref = _hydro(prec, epi, lst), orc.hydro(epi, lst)
+    assert (ref["vsmx"] > 2.0 * speed).all()
+    assert rel_err(out["vsmx"], ref["vsmx"], 1e-3).max() < TOL[prec]
+
+
+# (FP32C forms the square of the separation in FP32: 1e-18 at least; 6000 targets: items of several in FP64)
+@pytest.mark.parametrize("prec,sep", [("fp32c", 1e-9), ("fp32c", 1e-18), ("fp64", 1e-9), ("fp64", 1e-18), ("fp64", 1e-22)])
+@pytest.mark.parametrize("n_i,n_j", SIZES + [(6000, 6000)])
+def test_signal_velocity_of_close_particles(prec, sep, n_i, n_j):
+    """Two distinct particles that approach each other closer than the FP32
+    frame of their group resolves, or than FP32 squares."""
+    epi, epj, near = _ball(n_i, n_j, 19 * n_i + n_j, centre=0.0)
+    t = n_i // 2
+    epj["pos"] -= epi["pos"][t]
+    epi["pos"] -= epi["pos"][t]
+    far = np.flatnonzero(~np.isin(epj["id"], near))
+    k = far[-1] if len(far) else near[-1]
+    epj["id"][k] = 10 ** 6
+    epj["pos"][k] = [sep, 0.0, 0.0]
+    epj["vel"][k] = epi["vel"][t] - [40.0, 0.0, 0.0]
+    out, ref = _hydro(prec, epi, epj), orc.hydro(epi, epj)
+    assert ref["vsmx"][t] > 120.0
+    assert rel_err(out["vsmx"], ref["vsmx"], 1e-3).max() < TOL[prec]
