@@ -453,8 +453,10 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                     if (!exact_i && ((k & 1) ? up.y : up.x) <= lb) continue;
                     const int j = s_sj[hw][k];
                     const R vs = sig.pair(a, j, a.j_id[j] == idi);
-                    vsmx = vs > vsmx ? vs : vsmx;
-                    lb = fmaxf(lb, fminf((float)vs * 0.999997f, 3.0e38f));
+                    if (vs > vsmx) {   // (not for NaN, which raises neither)
+                        vsmx = vs;
+                        lb = fmaxf(lb, fminf((float)vs * 0.999997f, 3.0e38f));
+                    }
                 }
                 for (int o = 1; o < tpi; o <<= 1) lb = fmaxf(lb, __shfl_xor_sync(FULL, lb, o));
                 __syncwarp();

@@ -90,3 +90,17 @@ def test_signal_velocity_of_close_particles(prec, sep, n_i, n_j):
     out, ref = _hydro(prec, epi, epj), orc.hydro(epi, epj)
     assert ref["vsmx"][t] > 120.0
     assert rel_err(out["vsmx"], ref["vsmx"], 1e-3).max() < TOL[prec]
+
+
+@pytest.mark.parametrize("prec", ["fp32c", "fp64"])
+@pytest.mark.parametrize("n_i,n_j", SIZES)
+def test_signal_velocity_ignores_nan_terms(prec, n_i, n_j):
+    """Sources without a sound speed beyond every support, listed before the
+    others, leave the maximum over the others as it is."""
+    epi, epj, near = _ball(n_i, n_j, 23 * n_i + n_j)
+    nan = epj[:33].copy()
+    nan["id"] += 10 ** 6
+    nan["pos"] += 50.0
+    nan["vsnd"] = np.nan
+    out, ref = _hydro(prec, epi, np.concatenate([nan, epj])), orc.hydro(epi, epj)
+    assert rel_err(out["vsmx"], ref["vsmx"], 1e-3).max() < TOL[prec]
