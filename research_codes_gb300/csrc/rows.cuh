@@ -298,7 +298,9 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
             // of the item's extent, and 2^-47 of the global coordinates (lo
             // parts); the factor 1.0001 covers the same of the radius itself
             const float ext = fmaxf(fmaxf(fmaxf(-box.xl, box.xh), fmaxf(-box.yl, box.yh)), fmaxf(-box.zl, box.zh));
-            const float pad = 5.0e-7f * ext + 3.0e-14f * (fabsf(ch.x) + fabsf(ch.y) + fabsf(ch.z) + 3.0f * ext);
+            // (a centre without a position has no frame: every entry is marked)
+            float pad = 5.0e-7f * ext + 3.0e-14f * (fabsf(ch.x) + fabsf(ch.y) + fabsf(ch.z) + 3.0f * ext);
+            if (!(pad < 1.0e30f)) pad = INFINITY;
             // (FP32C hydro rows widen h^2 by 2e-4 alone, what FP32 sums need)
             auto reach2 = [&](float h) -> float {
                 if (KIND == ROWS_HYDRO32) return h * h * 1.0002f;

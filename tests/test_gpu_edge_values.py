@@ -104,3 +104,24 @@ def test_signal_velocity_ignores_nan_terms(prec, n_i, n_j):
     nan["vsnd"] = np.nan
     out, ref = _hydro(prec, epi, np.concatenate([nan, epj])), orc.hydro(epi, epj)
     assert rel_err(out["vsmx"], ref["vsmx"], 1e-3).max() < TOL[prec]
+
+
+@pytest.mark.parametrize("n_i,n_j", [(1, 700), (1, 4000), (5, 2000), (40, 4000), (6000, 6000)])
+@pytest.mark.parametrize("which", [0, -1])
+def test_hydro_fp64_of_a_target_without_a_position(n_i, n_j, which):
+    """NaN in one coordinate of a target: its sums are NaN, which the call
+    reports, and the others' are what they are without it."""
+    epi, epj, near = _ball(n_i, n_j, 29 * n_i + n_j)
+    epi["pos"][which, 0] = np.nan
+    out = np.zeros(n_i, abi.Hydro)
+    with functors.Context(precision="fp64", eta=ETA) as ctx:
+        with pytest.raises(abi.SPHError, match="NONFINITE"):
+            functors.calcHydro(ctx)(epi, n_i, epj, n_j, out)
+    ref = orc.hydro(epi, epj)
+    ok = np.arange(n_i) != which % n_i
+    for f in ("acch", "accg", "udot", "diffu"):
+        assert np.isnan(out[f][which]).all(), f
+        if ok.any():
+            assert rel_err(out[f][ok], ref[f][ok], 1e-3).max() < 1e-11, f
+    if ok.any():
+        assert rel_err(out["vsmx"][ok], ref["vsmx"][ok], 1e-3).max() < 1e-11
