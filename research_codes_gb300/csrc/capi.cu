@@ -288,7 +288,10 @@ __device__ __forceinline__ void prepare_density_one(const E *in, int k, const De
     s.vel[k] = v;
     s.id[k] = e.id;
     float4 a, b;
-    sphk::row_record(p, h, a, b);
+    if (f32)
+        sphk::row_record<false>(p, h, a, b);
+    else
+        sphk::row_record<true>(p, h, a, b);
     s.phi[k] = a;
     s.plo[k] = b;
     if (f32) {
@@ -334,7 +337,7 @@ __device__ __forceinline__ void prepare_hydro_one(const E *in, int k, const Hydr
         s.phi[k] = r.phi; s.plo[k] = r.plo; s.vhi[k] = r.vhi; s.vlo[k] = r.vlo;
         s.g1[k] = r.g1; s.g2[k] = r.g2; s.g3[k] = r.g3; s.g4[k] = r.g4;
     } else {
-        sphk::row_record(p, 0.0, a, b);
+        sphk::row_record<true>(p, 0.0, a, b);
         s.plo[k] = b;
     }
     sphk::hydro_mark_records(p, v, h1.x, h2.y, a, b);

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
                     if (e + 2 >= cnt) jv[g].z = -1;
                     if (e + 3 >= cnt) jv[g].w = -1;
                 }
-                const int jj[4] = {jv[g].x, jv[g].y, jv[g].z, jv[g].w};
+                int jj[4] = {jv[g].x, jv[g].y, jv[g].z, jv[g].w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     R dx, dy, dz;
@@ -327,8 +327,15 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
                     if (jj[u] >= 0) {
                         m[4 * g + u] = P.rel(a, jj[u], dx, dy, dz);
                         r[4 * g + u] = sqrt_r(dx * dx + dy * dy + dz * dz);
+                        // at an infinite distance W0(q) would be 0 * inf
+                        if (F64 && isinf(r[4 * g + u])) {
+                            r[4 * g + u] = 0;
+                            m[4 * g + u] = 0;
+                            jj[u] = -1;
+                        }
                     }
                 }
+                jv[g] = make_int4(jj[0], jj[1], jj[2], jj[3]);
             }
         }
         // three fixed-point passes, hdr_density.hpp:264-302
@@ -519,7 +526,8 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
             over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
                 R dx, dy, dz;
                 const R m = P.rel(a, j, qh, ql, dx, dy, dz);
-                const R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
+                R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
+                if (F64 && q > (R)2) q = 2;   // infinite squares: W0 would be 0 * inf
                 cnt += (q < (R)1) ? 1 : 0;
                 acc.add(density_term(q, m));
             });
@@ -532,21 +540,19 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         const long long idi = a.i_id[ii];
         PairVel<F64> V;
         V.load_i(a, ii);
-        // FP32C: the terms beyond the support are zero and need no velocity; a
-        // run of them folds one zero (further ones leave the sums as they are)
+        // the terms beyond the support are zero and need no velocity; in FP32C
+        // a run of them folds one zero (further ones leave the sums as they are)
         const R r2_far = (R)1.0002 * s.h * s.h;
         bool zero = false;
         over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
             R dx, dy, dz, ux, uy, uz;
             const R m = P.rel(a, j, qh, ql, dx, dy, dz);
-            if constexpr (!F64) {
-                if (dx * dx + dy * dy + dz * dz > r2_far) {
-                    if (!zero) gs.fold();
-                    zero = true;
-                    return;
-                }
-                zero = false;
+            if (dx * dx + dy * dy + dz * dz > r2_far) {
+                if (!F64 && !zero) gs.fold();
+                zero = true;
+                return;
             }
+            zero = false;
             V.rel(a, j, ux, uy, uz);
             gs.add(dx, dy, dz, ux, uy, uz, m, a.j_id[j] == idi, s.hinv);
             gs.fold();

@@ -53,6 +53,14 @@ __device__ __forceinline__ float2 df_split(double x) {
     return make_float2(h, (float)(x - (double)h));
 }
 
+// The same for records that FP64 sums follow: a value beyond the FP32 range
+// keeps an infinite hi part (NaN with the lo part that goes with it), so that
+// it lies outside every finite radius, as in FP64.
+__device__ __forceinline__ float2 df_split_far(double x) {
+    const float2 s = df_split(x);
+    return make_float2(s.x, isinf(s.x) ? 0.0f : s.y);
+}
+
 struct ItemRef {   // decoded work item
     int walk, jb, nj, ni, tpi, sub, li, ii, ic;
     bool act;
@@ -646,8 +654,12 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
 }
 
 // Position and mass as a double-float record with h (rounded up) in lo.w.
+// F64: of FP64 sums (df_split_far).
+template <bool F64>
 __device__ __forceinline__ void row_record(const dbl4 &p, double h, float4 &hi, float4 &lo) {
-    const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
+    const float2 x = F64 ? df_split_far(p.x) : df_split(p.x);
+    const float2 y = F64 ? df_split_far(p.y) : df_split(p.y);
+    const float2 z = F64 ? df_split_far(p.z) : df_split(p.z);
     hi = make_float4(x.x, y.x, z.x, (float)p.w);
     lo = make_float4(x.y, y.y, z.y, __double2float_ru(h));
 }
@@ -660,7 +672,7 @@ __device__ __forceinline__ void velocity_record(const dbl4 &v, float4 &hi, float
 __global__ inline void make_row_records(int n, const dbl4 *pm, const double *h, float4 *hi, float4 *lo) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         float4 a, b;
-        row_record(pm[k], h[k], a, b);
+        row_record<true>(pm[k], h[k], a, b);
         hi[k] = a;
         lo[k] = b;
     }
@@ -680,7 +692,7 @@ __global__ inline void make_hydro_row_records(int n, const dbl4 *pm, const dbl4 
                                               float4 *mp, float4 *lo, float4 *mv) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const dbl4 p = pm[k];
-        const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
+        const float2 x = df_split_far(p.x), y = df_split_far(p.y), z = df_split_far(p.z);
         float4 a, b;
         hydro_mark_records(p, vel[k], h1[k].x, h2[k].y, a, b);
         mp[k] = a;

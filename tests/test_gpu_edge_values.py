@@ -125,3 +125,61 @@ def test_hydro_fp64_of_a_target_without_a_position(n_i, n_j, which):
             assert rel_err(out[f][ok], ref[f][ok], 1e-3).max() < 1e-11, f
     if ok.any():
         assert rel_err(out["vsmx"][ok], ref["vsmx"][ok], 1e-3).max() < 1e-11
+
+
+def _density_inputs(epi, epj, guess=1.0):
+    """DensityEPI / DensityEPJ of hydro inputs; guess: first h over theirs."""
+    di, dj = np.zeros(len(epi), abi.DensityEPI), np.zeros(len(epj), abi.DensityEPJ)
+    mass = dict(zip(epj["id"].tolist(), epj["mass"].tolist()))
+    for f in ("id", "pos", "vel"):
+        di[f], dj[f] = epi[f], epj[f]
+    dj["mass"] = epj["mass"]
+    di["mass"] = [mass[k] for k in epi["id"].tolist()]
+    di["ksr"] = guess * epi["ksr"]
+    di["rs"] = 1.1 * di["ksr"]
+    return di, dj
+
+
+def _density(prec, di, dj):
+    out = np.zeros(len(di), abi.Density)
+    with functors.Context(precision=prec, eta=ETA) as ctx:
+        functors.calcDensity(ctx)(di, len(di), dj, len(dj), out)
+    return out
+
+
+# the first guess of h near (rows) and far below the final one (sweeps)
+@pytest.mark.parametrize("guess", [1.0, 0.5])
+@pytest.mark.parametrize("far", [1e39, 1e200, np.inf, -np.inf])
+@pytest.mark.parametrize("n_i,n_j", [(1, 40), (1, 700), (5, 4000), (40, 700)])
+def test_fp64_sources_at_infinite_distance(n_i, n_j, far, guess):
+    """Sources whose coordinates, or their squares, leave the FP32 or FP64
+    range add nothing to FP64 sums."""
+    epi, epj, near = _ball(n_i, n_j, 31 * n_i + n_j, neighbours=min(40.0, n_j))
+    out_of = epj[:3].copy()
+    out_of["id"] += 10 ** 6
+    out_of["pos"][:, 1] = far
+    lst = np.concatenate([epj[: n_j // 2], out_of, epj[n_j // 2:]])
+    di, dj = _density_inputs(epi, epj, guess)
+    out = _density("fp64", di, _density_inputs(epi, lst, guess)[1])
+    ref = orc.density(di, dj, eta=ETA, ksr_max=0.0)
+    for f in ("dens", "ksr", "grdh", "divv", "rotv"):
+        assert rel_err(out[f], ref[f], 1e-2).max() < 1e-11, f
+    assert np.array_equal(out["np"], ref["np"]) and np.array_equal(out["itr"], ref["itr"])
+    h, href = _hydro("fp64", epi, lst), orc.hydro(epi, epj)
+    for f in ("acch", "accg", "udot", "diffu"):
+        assert rel_err(h[f], href[f], 1e-3).max() < 1e-11, f
+
+
+@pytest.mark.parametrize("n_j", [40, 700])
+@pytest.mark.parametrize("n_i", [1, 5])
+def test_fp64_target_at_infinite_distance(n_i, n_j):
+    """A target whose squared distances leave the FP64 range: no force, and its
+    neighbours in the call keep theirs."""
+    epi, epj, near = _ball(n_i, n_j, 37 * n_i + n_j)
+    ref = orc.hydro(epi, epj)
+    epi["pos"][0, 0] = 1e200
+    out = _hydro("fp64", epi, epj)
+    for f in ("acch", "accg", "udot", "diffu"):
+        assert not out[f][0].any(), f
+        if n_i > 1:
+            assert rel_err(out[f][1:], ref[f][1:], 1e-3).max() < 1e-11, f
