@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
                 R dx, dy, dz;
                 const R m = P.rel(a, j, qh, ql, dx, dy, dz);
                 R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
-                if (F64 && q > (R)2) q = 2;   // infinite squares: W0 would be 0 * inf
+                if (q > (R)2) q = 2;   // infinite squares: W0 would be 0 * inf
                 cnt += (q < (R)1) ? 1 : 0;
                 acc.add(density_term(q, m));
             });

@@ -183,3 +183,23 @@ def test_fp64_target_at_infinite_distance(n_i, n_j):
         assert not out[f][0].any(), f
         if n_i > 1:
             assert rel_err(out[f][1:], ref[f][1:], 1e-3).max() < 1e-11, f
+
+
+@pytest.mark.parametrize("guess", [1.0, 0.5])
+@pytest.mark.parametrize("n_i,n_j", [(1, 40), (1, 700), (5, 4000), (40, 700)])
+def test_fp32c_sources_beyond_the_range_of_a_square(n_i, n_j, guess):
+    """FP32C density: sources whose squared distance is infinite in FP32 add
+    nothing, also to particles that sweep the whole list (first guess of h far
+    below the final one)."""
+    epi, epj, near = _ball(n_i, n_j, 41 * n_i + n_j, neighbours=min(40.0, n_j))
+    out_of = epj[:3].copy()
+    out_of["id"] += 10 ** 6
+    out_of["pos"][:, 1] = 1e20
+    lst = np.concatenate([epj[: n_j // 2], out_of, epj[n_j // 2:]])
+    di, dj = _density_inputs(epi, epj, guess)
+    out = _density("fp32c", di, _density_inputs(epi, lst, guess)[1])
+    ref = orc.density(di, dj, eta=ETA, ksr_max=0.0)
+    for f in ("dens", "ksr", "grdh"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < 1e-5, f
+    for f in ("divv", "rotv"):
+        assert rel_err(out[f], ref[f], 1e-2).max() < 1e-4, f
