@@ -357,7 +357,8 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const R q = r[4 * g + u] * s.hinv;
-                        part += density_term(q, m[4 * g + u]);
+                        const R t = density_term(q, m[4 * g + u]);
+                        part += q >= (R)1 ? (R)0 : t;   // beyond the support, whatever the mass
                         if (pass == 2) c += (jj[u] >= 0 && q < (R)1) ? 1 : 0;
                     }
                     acc.add(part);
@@ -470,7 +471,8 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         // visits the list entries; FP64: those that can lie within h of the
         // particle by an FP32 distance test on the double-float positions,
         // with the margins of mark_rows (h outside its range: every entry);
-        // in FP32C the test would cost what the sum does.  Indices are read a
+        // in FP32C f itself tests.  A coordinate that is NaN counts as the
+        // particle's own, as in the box test of mark_rows.  Indices are read a
         // round ahead of the records.
         auto over_list = [&](R h, auto &&f) {
             const float hf = (float)h;
@@ -510,24 +512,33 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
                             const float dx = df_diff(qh[u].x, ql[u].x, ph.x, pl.x);
                             const float dy = df_diff(qh[u].y, ql[u].y, ph.y, pl.y);
                             const float dz = df_diff(qh[u].z, ql[u].z, ph.z, pl.z);
-                            if (dx * dx + dy * dy + dz * dz > lim) continue;
+                            if (square_sum(dx, dy, dz) > lim) continue;
                         }
                         f(j[u], qh[u], ql[u]);
                     }
             }
         };
+        // Terms beyond the support are zero, whatever the mass, and need no
+        // velocity; in FP32C a run of them folds one zero (further ones leave
+        // the sums as they are).
         HState<R> s;
         s.start(a.i_ksr[ii]);
         int np = 0;
         for (int pass = 0; pass < 3; ++pass) {
             Acc<F64> acc;
             int cnt = 0;
-            const R hinv2 = s.hinv * s.hinv;
+            const R hinv2 = s.hinv * s.hinv, r2_far = (R)1.0002 * s.h * s.h;
+            bool zero = false;
             over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
                 R dx, dy, dz;
                 const R m = P.rel(a, j, qh, ql, dx, dy, dz);
-                R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
-                if (q > (R)2) q = 2;   // infinite squares: W0 would be 0 * inf
+                if (square_sum(dx, dy, dz) > r2_far) {
+                    if (!F64 && !zero) acc.add((R)0);
+                    zero = true;
+                    return;
+                }
+                zero = false;
+                const R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
                 cnt += (q < (R)1) ? 1 : 0;
                 acc.add(density_term(q, m));
             });
@@ -540,14 +551,12 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         const long long idi = a.i_id[ii];
         PairVel<F64> V;
         V.load_i(a, ii);
-        // the terms beyond the support are zero and need no velocity; in FP32C
-        // a run of them folds one zero (further ones leave the sums as they are)
         const R r2_far = (R)1.0002 * s.h * s.h;
         bool zero = false;
         over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
             R dx, dy, dz, ux, uy, uz;
             const R m = P.rel(a, j, qh, ql, dx, dy, dz);
-            if (dx * dx + dy * dy + dz * dz > r2_far) {
+            if (square_sum(dx, dy, dz) > r2_far) {
                 if (!F64 && !zero) gs.fold();
                 zero = true;
                 return;

@@ -202,7 +202,7 @@ __global__ inline void __launch_bounds__(DSWEEP_THREADS) hydro64_sweep(const Hyd
             const float dz = df_diff(qh.z, ql.z, ph.z, pl.z);
             const float h = fmaxf(ph.w, qh.w) * 1.0001f + pad;
             const bool test = ph.w >= ROW_HMIN && ph.w <= ROW_HMAX && qh.w >= ROW_HMIN && qh.w <= ROW_HMAX;
-            if ((test && dx * dx + dy * dy + dz * dz > h * h) || a.j_id[j] == idi) continue;
+            if ((test && square_sum(dx, dy, dz) > h * h) || a.j_id[j] == idi) continue;
             hydro64_pair(I, hydro64_load(a.j_pm, a.j_vel, a.j_h1, a.j_h2, a.j_h3, j), s);
         }
         double v[8] = {s.ax, s.ay, s.az, s.gx, s.gy, s.gz, s.ud, s.df};

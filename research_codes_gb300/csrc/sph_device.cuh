@@ -254,6 +254,15 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
+// x^2 + y^2 + z^2 without the coordinates that are NaN.
+template <typename R>
+__device__ __forceinline__ R square_sum(R x, R y, R z) {
+    x = max0(fabs(x));
+    y = max0(fabs(y));
+    z = max0(fabs(z));
+    return x * x + y * y + z * z;
+}
+
 // Axis-aligned box of a work item's i-particles, in the item's frame.
 template <typename R>
 struct IBox {

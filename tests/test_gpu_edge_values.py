@@ -203,3 +203,31 @@ def test_fp32c_sources_beyond_the_range_of_a_square(n_i, n_j, guess):
         assert rel_err(out[f], ref[f], 1e-3).max() < 1e-5, f
     for f in ("divv", "rotv"):
         assert rel_err(out[f], ref[f], 1e-2).max() < 1e-4, f
+
+
+# first guesses of h above the final one (rows) and far below it (sweeps)
+@pytest.mark.parametrize("prec,guess", [("fp32c", 1.2), ("fp32c", 0.5), ("fp64", 1.2), ("fp64", 0.5)])
+@pytest.mark.parametrize("field,value", [("mass", 1e39), ("mass", np.inf), ("mass", np.nan), ("pos", np.nan)])
+@pytest.mark.parametrize("n_i,n_j", [(1, 40), (1, 700), (40, 700), (5, 4000)])
+def test_density_of_unusable_sources_beyond_the_support(n_i, n_j, field, value, prec, guess):
+    """Sources beyond the support add nothing, whatever their mass (1e39: infinite
+    in FP32), nor does one that has no x but lies beyond it in y and z.  One
+    target has such a source in its row (at 1.02 times the first guess of h)."""
+    epi, epj, near = _ball(n_i, n_j, 47 * n_i + n_j, neighbours=min(40.0, n_j))
+    di, dj = _density_inputs(epi, epj)
+    di["ksr"] = guess * orc.density(di, dj, eta=ETA, ksr_max=0.0)["ksr"]
+    di["rs"] = 1.1 * di["ksr"]
+    bad = np.zeros(4, abi.DensityEPJ)
+    bad["id"] = 10 ** 6 + np.arange(4)
+    bad["mass"] = value if field == "mass" else 1.0
+    bad["pos"] = di["pos"][0] + np.array([0.0, 6.0, 8.0])
+    if n_i == 1 and guess > 1.0 and field == "mass":
+        bad["pos"][0] = di["pos"][0] + 1.02 * di["ksr"][0] * np.array([0.0, 0.6, 0.8])
+    if field == "pos":
+        bad["pos"][:, 0] = value
+    ref = orc.density(di, dj, eta=ETA, ksr_max=0.0)
+    out = _density(prec, di, np.concatenate([dj[: n_j // 2], bad, dj[n_j // 2:]]))
+    for f in ("dens", "ksr", "grdh"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < TOL[prec], f
+    for f in ("divv", "rotv"):
+        assert rel_err(out[f], ref[f], 1e-2).max() < 10 * TOL[prec], f
