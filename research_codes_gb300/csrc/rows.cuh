@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                         pz = df_diff(h.z, l.z, ch.z, cl.z);
                         float lim_j = rf2;
                         if (HYDRO) {
-                            hj2 = (h.w >= ROW_HMIN && h.w <= ROW_HMAX) ? reach2(h.w) : INFINITY;
+                            hj2 = (h.w >= 0.0f && h.w <= ROW_HMAX) ? reach2(fmaxf(h.w, ROW_HMIN)) : INFINITY;
                             lim_j = fmaxf(rf2, hj2);
                             const float ux = v.x - vc.x, uy = v.y - vc.y, uz = v.z - vc.z;
                             const float d = speed(ux, uy, uz);

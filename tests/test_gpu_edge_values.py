@@ -231,3 +231,20 @@ def test_density_of_unusable_sources_beyond_the_support(n_i, n_j, field, value, 
         assert rel_err(out[f], ref[f], 1e-3).max() < TOL[prec], f
     for f in ("divv", "rotv"):
         assert rel_err(out[f], ref[f], 1e-2).max() < 10 * TOL[prec], f
+
+
+@pytest.mark.parametrize("prec", ["fp32c", "fp64"])
+@pytest.mark.parametrize("n_i,n_j", [(1, 40), (1, 700), (40, 700), (5, 4000)])
+@pytest.mark.parametrize("h", [1e-16, 1e-39])
+def test_hydro_sources_with_a_tiny_support(n_i, n_j, h, prec):
+    """Sources whose h lies below the range of the row tests reach no target
+    but those in whose supports they are (h^-4 is infinite in FP32)."""
+    epi, epj, near = _ball(n_i, n_j, 53 * n_i + n_j)
+    tiny = epj[:3].copy()
+    tiny["id"] += 10 ** 6
+    tiny["pos"] = epi["pos"][0] + np.array([0.0, 6.0, 8.0])
+    tiny["ksr"], tiny["hinv"] = h, 1.0 / h
+    out, ref = _hydro(prec, epi, np.concatenate([epj[: n_j // 2], tiny, epj[n_j // 2:]])), orc.hydro(epi, epj)
+    for f in ("acch", "accg", "udot"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < TOL[prec], f
+    assert rel_err(out["diffu"], ref["diffu"], 1e-2).max() < 10 * TOL[prec]
