@@ -723,7 +723,8 @@ struct HydroRecords {
     float4 phi, plo, vhi, vlo, g1, g2, g3, g4;
     __device__ __forceinline__ void fill(const dbl4 &p, const dbl4 &v, const dbl4 &a, const dbl4 &b, const double2 &c) {
         const float2 x = df_split(p.x), y = df_split(p.y), z = df_split(p.z);
-        const float2 u = df_split(v.x), w = df_split(v.y), s = df_split(v.z);
+        // (velocities beyond the FP32 range: infinite signal velocities, not NaN)
+        const float2 u = df_split_far(v.x), w = df_split_far(v.y), s = df_split_far(v.z);
         const float2 P = df_split(a.y), T = df_split(c.x), Q = df_split(a.z);
         const double h4d = (a.x * a.x) * (a.x * a.x);
         const float2 H = df_split(a.x), H4 = df_split(h4d), M = df_split(p.w);

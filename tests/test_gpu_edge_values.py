@@ -248,3 +248,25 @@ def test_hydro_sources_with_a_tiny_support(n_i, n_j, h, prec):
     for f in ("acch", "accg", "udot"):
         assert rel_err(out[f], ref[f], 1e-3).max() < TOL[prec], f
     assert rel_err(out["diffu"], ref["diffu"], 1e-2).max() < 10 * TOL[prec]
+
+
+@pytest.mark.parametrize("n_i,n_j", SIZES)
+@pytest.mark.parametrize("speed", [1e39, 1e200, np.inf])
+@pytest.mark.parametrize("who", ["source", "target"])
+def test_fp32c_velocities_beyond_the_fp32_range(n_i, n_j, speed, who):
+    """An approach faster than FP32 holds is an infinite signal velocity, which
+    the call reports."""
+    epi, epj, near = _ball(n_i, n_j, 59 * n_i + n_j)
+    far = epj[~np.isin(epj["id"], near)][-1:].copy()
+    far["id"] += 10 ** 6
+    far["pos"] = epi["pos"][0] + [20.0, 1.0, 1.0]
+    lst = np.concatenate([epj[: n_j // 2], far, epj[n_j // 2:]])
+    if who == "source":
+        lst["vel"][n_j // 2] = [-speed, 0.0, 0.0]
+    else:
+        epi["vel"][0] = [speed, 0.0, 0.0]
+    out = np.zeros(n_i, abi.Hydro)
+    with functors.Context(precision="fp32c", eta=ETA) as ctx:
+        with pytest.raises(abi.SPHError, match="NONFINITE"):
+            functors.calcHydro(ctx)(epi, n_i, lst, len(lst), out)
+    assert np.isinf(out["vsmx"] if who == "source" else out["vsmx"][0]).all()
