@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
                 np = c;
             }
             s.update(sum, mi, (R)a.eta_ksrh, (R)ksr_max);
-            valid = valid && s.h <= h_row;
+            valid = valid && s.h >= (R)0 && s.h <= h_row;   // (h < 0, from a negative sum, has no radius)
         }
         // gradient pass with the final h, hdr_density.hpp:304-349
         GradSums<F64> gs;

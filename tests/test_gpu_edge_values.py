@@ -270,3 +270,22 @@ def test_fp32c_velocities_beyond_the_fp32_range(n_i, n_j, speed, who):
         with pytest.raises(abi.SPHError, match="NONFINITE"):
             functors.calcHydro(ctx)(epi, n_i, lst, len(lst), out)
     assert np.isinf(out["vsmx"] if who == "source" else out["vsmx"][0]).all()
+
+
+@pytest.mark.parametrize("n_i,n_j", [(1, 40), (1, 700), (5, 900)])
+def test_fp64_density_of_a_negative_sum(n_i, n_j):
+    """Sources of negative mass that outweigh the others make a negative h,
+    which no row radius covers: the particle sweeps the list.  The same with 200
+    massless sources beside the target, whose row overflows (FP64 sums in
+    another order: 1e-9 of what they grow to)."""
+    epi, epj, near = _ball(n_i, n_j, 43 * n_i + n_j, neighbours=min(40.0, n_j))
+    di, dj = _density_inputs(epi, epj)
+    dj["mass"][near] *= -50.0
+    extra = np.repeat(dj[near[:1]], 200)
+    extra["id"] = 10 ** 6 + np.arange(200)
+    extra["mass"] = 0.0
+    extra["pos"] += 1e-3 * np.random.default_rng(1).normal(size=(200, 3))
+    out, ref = _density("fp64", di, dj), _density("fp64", di, np.concatenate([dj, extra]))
+    assert (ref["ksr"] < 0.0).any()
+    for f in ("dens", "ksr"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < 1e-9, f
