@@ -59,25 +59,7 @@ __device__ __forceinline__ float rsqrt_r(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-
-// FP64 1/sqrt: the hardware approximation (its result has at most 21
-// significant bits, so its square is exact) and one step of Halley's third
-// order iteration, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 from one fused
-// multiply-add: five FP64 operations, relative error 2^-53 from the last
-// rounding plus (5/16) e^3 < 2^-60.  GB300 retires two FP64 operations per clock
-// and SM, and the pair loops are made of little else.  Zero and infinite
-// arguments give the exact +inf and 0 of the approximation (subnormal ones
-// count as zero), negative ones and NaN give NaN.
-__device__ __forceinline__ bool rsqrt_special(double x) {
-    return (unsigned)(__double2hiint(x) - 0x00100000) >= 0x7fe00000u;
-}
-__device__ __forceinline__ double rsqrt_r(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);
-    const double r = fma(y * e, fma(e, 0.375, 0.5), y);
-    return rsqrt_special(x) ? y : r;
-}
+__device__ __forceinline__ double rsqrt_r(double x) { return rsqrt(x); }
 
 // 1/x: FP32 via rcp.approx.ftz.f32 (relative error <= 2^-23), FP64 exact.
 __device__ __forceinline__ float rcp_r(float x) {
@@ -96,18 +78,13 @@ __device__ __forceinline__ float sqrt_q(float r2, float hinv2) {
 }
 __device__ __forceinline__ double sqrt_q(double r2, double hinv2) { return sqrt(r2 * hinv2); }
 
-// sqrt(x): FP32 by sqrt.approx; FP64 as x / sqrt(x) with one correction of the
-// residual (relative error 2^-53 from the last rounding).
+// sqrt(x): FP32 by sqrt.approx, FP64 by the library sqrt.
 __device__ __forceinline__ float sqrt_r(float x) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ double sqrt_r(double x) {
-    if (rsqrt_special(x)) return sqrt(x);
-    const double y = rsqrt_r(x), r = x * y;
-    return fma(fma(-r, r, x), 0.5 * y, r);
-}
+__device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
 
 // sqrt for bounds that carry a relative margin far above 2^-22: FP32 by
 // sqrt.approx.ftz.f32, FP64 by the library sqrt.

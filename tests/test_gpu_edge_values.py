@@ -289,3 +289,36 @@ def test_fp64_density_of_a_negative_sum(n_i, n_j):
     assert (ref["ksr"] < 0.0).any()
     for f in ("dens", "ksr"):
         assert rel_err(out[f], ref[f], 1e-3).max() < 1e-9, f
+
+
+@pytest.mark.parametrize("n_i,n_j", SIZES)
+def test_fp64_squares_below_the_normal_range(n_i, n_j):
+    """FP64 mode: 1/sqrt of squares that are subnormal (a separation of 1e-160,
+    a softening of 1e-155) is finite."""
+    epi, epj, near = _ball(n_i, n_j, 61 * n_i + n_j, centre=0.0)
+    epj["pos"] -= epi["pos"][0]
+    epi["pos"] -= epi["pos"][0]
+    k = np.flatnonzero(~np.isin(epj["id"], near))[-1]
+    epj["pos"][k] = [1e-160, 0.0, 0.0]
+    epj["vel"][k] = epi["vel"][0]
+    epj["vel"][k, 0] -= 40.0
+    # (subnormal squares have few digits: 1e-4 where they set the value)
+    out, ref = _hydro("fp64", epi, epj), orc.hydro(epi, epj)
+    assert ref["vsmx"][0] > 100.0
+    assert rel_err(out["vsmx"], ref["vsmx"], 1e-3).max() < 1e-4
+    di, dj = _density_inputs(epi, epj)
+    out, ref = _density("fp64", di, dj), orc.density(di, dj, eta=ETA, ksr_max=0.0)
+    for f in ("dens", "ksr", "grdh", "divv", "rotv"):
+        assert rel_err(out[f], ref[f], 1e-2).max() < 1e-10, f
+    gi, gj = np.zeros(n_i, abi.GravityEPI), np.zeros(n_j, abi.GravityEPJ)
+    gi["pos"], gi["eps2"] = epi["pos"], 1e-310
+    gj["pos"], gj["mass"], gj["eps2"] = epj["pos"], epj["mass"], 1e-310
+    gj["pos"][k] = 0.5
+    got = np.zeros(n_i, abi.Gravity)
+    with functors.Context(precision="fp64", eta=ETA) as ctx:
+        try:
+            functors.calcGravity(ctx)(gi, n_i, gj, n_j, got)
+        except abi.SPHError:   # (the cube in the accelerations is infinite)
+            pass
+    pot = orc.gravity(gi, gj)["pot"]
+    assert np.isfinite(pot).all() and rel_err(got["pot"], pot, 1e-3).max() < 1e-10
