@@ -269,6 +269,12 @@ __device__ __forceinline__ R density_term(R q, R m) {   // m W0(q) / c0
     return m * (u2 * u2 * ((R)1 + (R)4 * q));
 }
 
+// q >= 1, not NaN; FP64 by the high word, off the FP64 pipe
+__device__ __forceinline__ bool beyond(float q) { return q >= 1.0f; }
+__device__ __forceinline__ bool beyond(double q) {
+    return (unsigned)(__double2hiint(q) - 0x3ff00000) <= 0x7ff00000u - 0x3ff00000u;
+}
+
 constexpr int DROWS_LANES = 8;        // lanes per particle
 constexpr int DROWS_THREADS = 128;
 constexpr int DROWS_GROUPS = ROW_CAP / (4 * DROWS_LANES);   // int4 row reads per lane
@@ -328,7 +334,7 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
                         m[4 * g + u] = P.rel(a, jj[u], dx, dy, dz);
                         r[4 * g + u] = sqrt_r(dx * dx + dy * dy + dz * dz);
                         // at an infinite distance W0(q) would be 0 * inf
-                        if (F64 && isinf(r[4 * g + u])) {
+                        if (F64 && infinite(r[4 * g + u])) {
                             r[4 * g + u] = 0;
                             m[4 * g + u] = 0;
                             jj[u] = -1;
@@ -357,8 +363,8 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const R q = r[4 * g + u] * s.hinv;
-                        const R t = density_term(q, m[4 * g + u]);
-                        part += q >= (R)1 ? (R)0 : t;   // beyond the support, whatever the mass
+                        const R sum = part + density_term(q, m[4 * g + u]);
+                        part = beyond(q) ? part : sum;   // no term, whatever the mass
                         if (pass == 2) c += (jj[u] >= 0 && q < (R)1) ? 1 : 0;
                     }
                     acc.add(part);

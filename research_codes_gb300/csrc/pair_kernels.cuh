@@ -107,7 +107,7 @@ __device__ __forceinline__ void hydro64_pair(const Hydro64P &i, const Hydro64P &
     const double ux = i.v.x - j.v.x, uy = i.v.y - j.v.y, uz = i.v.z - j.v.z;
     const double r2 = dx * dx + dy * dy + dz * dz;
     const double ri = rsqrt_r(r2);
-    const double rr = isinf(r2) ? r2 : r2 * ri;   // (inf * 0 is NaN)
+    const double rr = infinite(r2) ? r2 : r2 * ri;   // (inf * 0 is NaN)
     // kernel gradients W1(q) for both smoothing lengths
     const double qi = rr * i.h1.x, qj = rr * j.h1.x;
     if (qi >= 1.0 && qj >= 1.0) return;   // beyond both supports: every term is zero

@@ -110,6 +110,9 @@ __device__ __forceinline__ double w1_term(double q, double u, double u2, double 
 
 __device__ __forceinline__ float max0(float x) { return fmaxf(x, 0.0f); }
 __device__ __forceinline__ double max0(double x) { return fmax(x, 0.0); }
+// +inf (FP64 by the high word, off the FP64 pipe)
+__device__ __forceinline__ bool infinite(float x) { return x > 3.4028235e38f; }
+__device__ __forceinline__ bool infinite(double x) { return __double2hiint(x) == 0x7ff00000; }
 // max(x, 0), NaN for NaN
 __device__ __forceinline__ float max0_nan(float x) {
     float y;
