@@ -562,11 +562,6 @@ int64_t sph_parse_hexa_rows(const char *text, int64_t len, int64_t n, int32_t nc
 int64_t sph_format_ascii_rows(int64_t n, const int64_t *id, const int64_t *istar, int32_t ncol,
                               const double *cols, const char *kinds, char *out, int64_t cap);
 
-/* ------------------------------------------------------------------------ */
-/* For language bindings: out[k] = the pointer stored `offset` bytes into
- * object k.                                                                  */
-void sph_member_pointers(const void *const *obj, int64_t n, int64_t offset, void **out);
-
 /* ABI self-description, used by the tests to check the struct layouts.
  * Writes up to n int64 values: for each struct in the order DensityEPI,
  * DensityEPJ, Density, HydroEPI, HydroEPJ, Hydro, GravityEPI, GravityEPJ,

@@ -1207,6 +1207,8 @@ extern "C" int sph_calc_gravity_sp(sph_context *ctx, const sph_GravityEPI *epi, 
 }
 
 // ---------------------------------------------------------------- bindings
+// For the Python binding alone (functors.py), not in the ABI header: the
+// pointers `offset` bytes into n objects.
 extern "C" void sph_member_pointers(const void *const *obj, int64_t n, int64_t offset, void **out) {
     for (int64_t k = 0; k < n; ++k)
         std::memcpy(&out[k], static_cast<const char *>(obj[k]) + offset, sizeof(void *));

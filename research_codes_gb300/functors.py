@@ -160,7 +160,8 @@ class calcGravity:
 # Where a numpy array object keeps its data pointer: the first member after the
 # object header (PyArrayObject's layout, what numpy's PyArray_DATA reads).
 # Checked on an array; without it every address goes through ndarray.ctypes,
-# a microsecond each.
+# a microsecond each (0.4 ms for 500 walks, 0.05 this way; the array interface
+# describes the struct dtype on every access: 4.5 ms).
 _DATA_OFFSET = object.__basicsize__
 _probe = np.zeros(3)
 if ctypes.c_void_p.from_address(id(_probe) + _DATA_OFFSET).value != _probe.ctypes.data:
@@ -169,6 +170,7 @@ if ctypes.c_void_p.from_address(id(_probe) + _DATA_OFFSET).value != _probe.ctype
 
 def _ptr_array(arrs):
     """Addresses of the arrays (0 for empty ones) as a C array."""
+    arrs = list(arrs)   # holds on to rows that exist for the loop alone
     n = len(arrs)
     out = (ctypes.c_void_p * max(n, 1))()
     if _DATA_OFFSET is None or any(type(a) is not np.ndarray for a in arrs):
