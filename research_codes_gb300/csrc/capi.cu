@@ -17,7 +17,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstddef>
@@ -25,12 +24,11 @@
 #include <cstring>
 #include <limits>
 #include <new>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/sph_gb300.h"
 #include "capi_internal.h"
+#include "host_copy.h"
 #include "pair_kernels.cuh"
 
 // ---- ABI layout checks: the reference classes' member order and padding ----
@@ -736,16 +734,6 @@ struct WalkArrays {
     size_t size, base;
 };
 
-// A part of an array to copy into the pinned buffer.
-struct CopyTask {
-    const char *src;
-    size_t dst, bytes;
-};
-constexpr size_t TASK_BYTES = 256 << 10;     // largest task
-constexpr size_t THREAD_BYTES = 2 << 20;     // input bytes per copying thread (~150 us; creating one takes ~15)
-constexpr size_t SEGMENT_BYTES = 8 << 20;    // bytes per copy to the device (~40 us)
-constexpr int MAX_COPY_THREADS = 8;
-
 // Copies bytes [from, to) of the pinned buffer in; the first copy of a dispatch
 // (from = 0) clears its counters.
 void launch_copy(sph_context *ctx, KindState &ks, size_t from, size_t to) {
@@ -754,67 +742,6 @@ void launch_copy(sph_context *ctx, KindState &ks, size_t from, size_t to) {
     copy_inputs<<<grid, 256, 0, ctx->stream>>>(reinterpret_cast<const uint4 *>(ks.h_in.p + from),
                                                reinterpret_cast<uint4 *>(ks.d_in.p + from), n,
                                                from == 0 ? ctx->d_queue : nullptr);
-}
-
-// Runs the tasks (ascending dst) and copies the buffer in by segments, each as
-// soon as its tasks are done.
-void run_copies(sph_context *ctx, KindState &ks, const std::vector<CopyTask> &tasks, size_t total) {
-    char *h = ks.h_in.p;
-    const size_t bytes = tasks.empty() ? 0 : tasks.back().dst + tasks.back().bytes - tasks.front().dst;
-    const int cores = (int)std::thread::hardware_concurrency();
-    const int extra = std::min<int>(std::min(MAX_COPY_THREADS, cores / 2) - 1, (int)(bytes / THREAD_BYTES) - 1);
-    if (extra < 1) {
-        for (const CopyTask &t : tasks) std::memcpy(h + t.dst, t.src, t.bytes);
-        launch_copy(ctx, ks, 0, total);
-        return;
-    }
-    const int n = (int)tasks.size();
-    // segment k: the tasks up to seg_task[k], the bytes up to seg_end[k]
-    std::vector<int> seg_task, seg_of(n);
-    std::vector<size_t> seg_end;
-    size_t from = 0;
-    for (int k = 0; k < n; ++k) {
-        const size_t next = k + 1 < n ? tasks[k + 1].dst / 256 * 256 : total;
-        seg_of[k] = (int)seg_task.size();
-        if (next - from >= SEGMENT_BYTES || k + 1 == n) {
-            // a 256-byte boundary at or before the next task: bytes of this one
-            // beyond it go with the next segment, which is copied later
-            seg_task.push_back(k + 1);
-            seg_end.push_back(next);
-            from = next;
-        }
-    }
-    const int n_seg = (int)seg_task.size();
-    std::vector<std::atomic<int>> left(n_seg);
-    for (int g = 0; g < n_seg; ++g) left[g].store(seg_task[g] - (g ? seg_task[g - 1] : 0), std::memory_order_relaxed);
-    std::atomic<int> next_task{0};
-    auto one = [&]() {
-        const int k = next_task.fetch_add(1, std::memory_order_relaxed);
-        if (k >= n) return false;
-        std::memcpy(h + tasks[k].dst, tasks[k].src, tasks[k].bytes);
-        left[seg_of[k]].fetch_sub(1, std::memory_order_release);
-        return true;
-    };
-    std::vector<std::thread> threads;
-    try {
-        threads.reserve(extra);
-        for (int t = 0; t < extra; ++t) threads.emplace_back([&]() { while (one()) {} });
-    } catch (const std::system_error &) {
-        // fewer threads: the loop below does the rest
-    }
-    int seg = 0;
-    bool more = true;
-    while (seg < n_seg) {
-        if (more)
-            more = one();
-        else
-            std::this_thread::yield();
-        while (seg < n_seg && left[seg].load(std::memory_order_acquire) == 0) {
-            launch_copy(ctx, ks, seg ? seg_end[seg - 1] : 0, seg_end[seg]);
-            ++seg;
-        }
-    }
-    for (std::thread &t : threads) t.join();
 }
 
 // Builds the items, fills the pinned buffer and copies it to the device.
@@ -852,7 +779,9 @@ int stage(sph_context *ctx, KindState &ks, const std::vector<int> &i_off, const 
     std::memcpy(h + L.off_joff, j_off.data(), sizeof(int) * (n_walk + 1));
     if (!ks.items.empty()) std::memcpy(h + L.off_items, ks.items.data(), sizeof(WorkItem) * ks.items.size());
     ctx->h_flags[ks.flag_slot] = 0;
-    run_copies(ctx, ks, tasks, L.total);
+    const size_t bytes = tasks.empty() ? 0 : tasks.back().dst + tasks.back().bytes - tasks.front().dst;
+    run_copies(h, tasks, L.total, extra_copy_threads(bytes),
+               [&](size_t from, size_t to) { launch_copy(ctx, ks, from, to); });
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(ctx, e, "input copy");
     return SPH_OK;
