@@ -151,17 +151,28 @@ static void recheck_density(const sph_context *ctx, const sphk::DensityArgs &a, 
         f, a.amb, a.amb_count, a.amb_cap, amb_total);
 }
 
+// FP64 rows of up to 8 particles per SM are summed by a whole warp each: their
+// chain of dependent FP64 operations is what such a call waits for.  A call of one
+// target: density 93.9 us with eight lanes, 71.3 so (78.1 by the list, before
+// rows); hydro 82.3 and 67.1 (66.3).  1000 targets: 197 and 189, hydro 391 and
+// 381; at 2000 the FP64 pipe is busy with either (326 and 358, 819 and 820).
+static bool warp_per_row(const sph_context *ctx, int n) { return n <= 8 * ctx->sm_count; }
+
 // The density sums of the particles of a.i_list (at most n_max) over their
 // rows, the sweep of the queued particles and, in FP32C, the FP64
 // recomputation of the ambiguous ones.  *a.n_ovf and *a.amb_count hold the
 // queues' counts.
 static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs &a, int n_max, int precision,
                                 cudaStream_t s, int *amb_total) {
-    const int per_block = sphk::DROWS_THREADS / sphk::DROWS_LANES;
+    const bool whole_warp = precision == SPH_PREC_FP64 && warp_per_row(ctx, n_max);
+    const int per_block = sphk::DROWS_THREADS / (whole_warp ? 32 : sphk::DROWS_LANES);
     const int rg = std::max(1, std::min((n_max + per_block - 1) / per_block, ctx->sm_count * 16));
     const int sg = std::max(1, std::min(n_max, ctx->sm_count * 6));
     if (precision == SPH_PREC_FP64) {
-        sphk::density_rows<true><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
+        if (whole_warp)
+            sphk::density_rows<true, 32><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
+        else
+            sphk::density_rows<true><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
         sphk::density_sweep<true><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr);
         return;
     }
@@ -215,9 +226,13 @@ void launch_hydro_marks(const sph_context *ctx, const sphk::MarkArgs &m, int mar
 void launch_hydro_sums(const sph_context *ctx, const sphk::HydroArgs &a, int precision, cudaStream_t s) {
     if (a.n_i <= 0) return;
     if (precision == SPH_PREC_FP64) {
-        const int per_block = sphk::HROWS_THREADS / sphk::HROWS_LANES;
-        sphk::hydro64_rows<<<std::max(1, std::min((a.n_i + per_block - 1) / per_block, 16 * ctx->sm_count)),
-                             sphk::HROWS_THREADS, 0, s>>>(a);
+        const bool whole_warp = warp_per_row(ctx, a.n_i);
+        const int per_block = sphk::HROWS_THREADS / (whole_warp ? 32 : sphk::HROWS_LANES);
+        const int grid = std::max(1, std::min((a.n_i + per_block - 1) / per_block, 16 * ctx->sm_count));
+        if (whole_warp)
+            sphk::hydro64_rows<32><<<grid, sphk::HROWS_THREADS, 0, s>>>(a);
+        else
+            sphk::hydro64_rows<sphk::HROWS_LANES><<<grid, sphk::HROWS_THREADS, 0, s>>>(a);
         sphk::hydro64_sweep<<<std::max(1, std::min(a.n_i, 2 * ctx->sm_count)), sphk::DSWEEP_THREADS, 0, s>>>(a);
         return;
     }

@@ -277,15 +277,18 @@ __device__ __forceinline__ bool beyond(double q) {
 
 constexpr int DROWS_LANES = 8;        // lanes per particle
 constexpr int DROWS_THREADS = 128;
-constexpr int DROWS_GROUPS = ROW_CAP / (4 * DROWS_LANES);   // int4 row reads per lane
 #ifndef SPH_DROWS_MIN_BLOCKS
 #define SPH_DROWS_MIN_BLOCKS 4
 #endif
 
-template <bool F64>
+// L lanes per particle: 8, or all 32 of the warp in small FP64 calls (warp_per_row).
+template <bool F64, int L = DROWS_LANES>
 __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS) density_rows(const DensityArgs a) {
     typedef typename Real<F64>::T R;
-    constexpr int L = DROWS_LANES, G = DROWS_GROUPS;
+    // a lane's entries, G groups of four: four consecutive ones of the row, or
+    // (L = 32, one group) every 32nd, those beyond the row skipped
+    constexpr int G = ROW_CAP / (4 * L);
+    static_assert(L == 8 || (L == 32 && G == 1), "8 or 32 lanes");
     if (a.err && (*a.err & a.err_mask)) return;
     if (a.skip_rows && *a.skip_rows) return;
     const int n = a.n_i_dev ? *a.n_i_dev : a.n_i;
@@ -318,7 +321,12 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
             if (g * 4 * L < cmax) {
                 const int e = g * 4 * L + 4 * sub;
                 jv[g] = make_int4(-1, -1, -1, -1);
-                if (e < cnt) {
+                if (L == 32) {
+                    if (sub < cnt) jv[g].x = row[sub];
+                    if (32 + sub < cnt) jv[g].y = row[32 + sub];
+                    if (64 + sub < cnt) jv[g].z = row[64 + sub];
+                    if (96 + sub < cnt) jv[g].w = row[96 + sub];
+                } else if (e < cnt) {
                     jv[g] = *reinterpret_cast<const int4 *>(row + e);
                     if (e + 1 >= cnt) jv[g].y = -1;
                     if (e + 2 >= cnt) jv[g].z = -1;
@@ -362,6 +370,7 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
                     R part = 0;
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
+                        if (L == 32 && 32 * u >= cmax) continue;
                         const R q = r[4 * g + u] * s.hinv;
                         const R sum = part + density_term(q, m[4 * g + u]);
                         part = beyond(q) ? part : sum;   // no term, whatever the mass

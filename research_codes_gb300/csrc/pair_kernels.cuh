@@ -159,9 +159,10 @@ __device__ __forceinline__ void hydro64_store(const HydroArgs &a, int p, const d
 // the sweep.  FP64 pipe bound (~120 instructions per pair): rows hold ~57 pairs
 // where the list holds ~900, and the old kernel tested each of those in FP64
 // (call of 256 among 20k: 2690 -> 179 us).
+// L = 32 in small calls (warp_per_row).
 constexpr int HROWS_LANES = 8, HROWS_THREADS = 128;
-__global__ inline void __launch_bounds__(HROWS_THREADS) hydro64_rows(const HydroArgs a) {
-    constexpr int L = HROWS_LANES;
+template <int L>
+__global__ void __launch_bounds__(HROWS_THREADS) hydro64_rows(const HydroArgs a) {
     const int lane = threadIdx.x & 31, sub = lane & (L - 1);
     const int gw = (blockIdx.x * HROWS_THREADS + threadIdx.x) >> 5, nw = (gridDim.x * HROWS_THREADS) >> 5;
     for (int k0 = gw * (32 / L); k0 < a.n_i; k0 += nw * (32 / L)) {
