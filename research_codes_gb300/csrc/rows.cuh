@@ -445,10 +445,14 @@ __global__ void __launch_bounds__(WARPS * 32, (KIND == ROWS_DENSITY ? 24 : 16) /
                         if (!(up.y <= lb)) m |= 2u << k;
                     }
                 } else {
-                    for (int k = sub; k < nb; k += tpi) {
-                        const float2 up = upper(k & ~1);
-                        if (!(((k & 1) ? up.y : up.x) <= lb)) m |= 1u << k;
+                    // two consecutive entries, as a packed bound holds; one
+                    // each for 32 lanes
+                    for (int k = 2 * sub & 31; k < 32; k += 2 * tpi) {
+                        const float2 up = upper(k);
+                        if (!(up.x <= lb)) m |= 1u << k;
+                        if (!(up.y <= lb)) m |= 2u << k;
                     }
+                    if (tpi == 32) m &= sub < 16 ? 0x55555555u : 0xaaaaaaaau;
                 }
                 if (exact_i) {
                     m = 0;
