@@ -163,7 +163,7 @@ static bool warp_per_row(const sph_context *ctx, int n) { return n <= 8 * ctx->s
 // recomputation of the ambiguous ones.  *a.n_ovf and *a.amb_count hold the
 // queues' counts.
 static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs &a, int n_max, int precision,
-                                cudaStream_t s, int *amb_total) {
+                                cudaStream_t s, int *amb_total, const RowlessItems *rowless) {
     const bool whole_warp = precision == SPH_PREC_FP64 && warp_per_row(ctx, n_max);
     const int per_block = sphk::DROWS_THREADS / (whole_warp ? 32 : sphk::DROWS_LANES);
     const int rg = std::max(1, std::min((n_max + per_block - 1) / per_block, ctx->sm_count * 16));
@@ -177,7 +177,23 @@ static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs 
         return;
     }
     sphk::density_rows<false><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
-    sphk::density_sweep<false><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr);
+    const int most = rowless ? rowless->most : 0x7fffffff;
+    sphk::density_sweep<false><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr, most);
+    if (rowless) {
+        const RowlessItems &r = *rowless;
+        sphk::rowless_items<<<std::max(1, std::min((r.n_walk + 3) / 4, 8 * ctx->sm_count)), 128, 0, s>>>(
+            r.n_walk, r.i_off, a.j_off, a.info, a.n_ovf, most, r.list, r.items, r.n_items);
+        sphk::StreamArgs w{};
+        w.i_pm = a.i_pm; w.fi = a.fi; w.fj = a.fj; w.i_id = a.i_id; w.j_id = a.j_id;
+        w.i_ksr = a.i_ksr; w.i_rs = a.i_rs;
+        w.items = r.items; w.n_items_dev = r.n_items; w.j_off = a.j_off; w.j_idx = a.j_idx;
+        w.i_list = r.list; w.queue = r.queue;
+        w.o_dens = a.o_dens; w.o_divv = a.o_divv; w.o_rotv = a.o_rotv; w.o_grdh = a.o_grdh; w.o_ksr = a.o_ksr;
+        w.o_np = a.o_np; w.o_itr = a.o_itr;
+        w.eta_ksrh = a.eta_ksrh; w.ksr_max = a.ksr_max; w.ksr_max_dev = a.ksr_max_dev;
+        w.amb_count = a.amb_count; w.amb = a.amb; w.amb_cap = a.amb_cap; w.amb_tol = a.amb_tol;
+        sphk::density_stream<PAIR_WARPS><<<ctx->grid_stream, PAIR_WARPS * 32, 0, s>>>(w);
+    }
     recheck_density(ctx, a, n_max, s, amb_total);
 }
 
@@ -189,9 +205,10 @@ void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int ma
 
 // Rows of the items of m, then the density sums over them.
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
-                    int n_max, int precision, cudaStream_t s, int *amb_total, const LongSide *side) {
+                    int n_max, int precision, cudaStream_t s, int *amb_total, const LongSide *side,
+                    const RowlessItems *rowless) {
     launch_mark_density(ctx, m, mark_grid, n_max, s, side);
-    launch_density_sums(ctx, a, n_max, precision, s, amb_total);
+    launch_density_sums(ctx, a, n_max, precision, s, amb_total, rowless);
 }
 
 // The FP32C density of a particle system (n_max particles): the streamed walk
@@ -265,9 +282,9 @@ __device__ __forceinline__ bool finite3(double a, double b, double c) {
 }
 
 // Copies n 16-byte words from pinned memory; the first launch of a dispatch
-// clears its counters (queue; the flags at 4..6 are not used on the device).
+// clears its counters.
 __global__ void __launch_bounds__(256) copy_inputs(const uint4 *src, uint4 *dst, size_t n, int *queue) {
-    if (queue && blockIdx.x == 0 && threadIdx.x < 12 && (threadIdx.x < 4 || threadIdx.x > 6)) queue[threadIdx.x] = 0;
+    if (queue && blockIdx.x == 0 && threadIdx.x < 12) queue[threadIdx.x] = 0;
     const size_t stride = (size_t)gridDim.x * 256;
     for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n; k += 4 * stride) {
         uint4 v[4];
@@ -699,6 +716,16 @@ int longest(const int32_t *n, int n_walk) {
     return m;
 }
 
+// FP32C density: with more rowless particles than this (a first guess of h far
+// off, or more neighbours than a row holds) items of 32, which share every list
+// entry, stream the lists instead of a block per particle.  A block takes ~0.1 us
+// of the chip per particle and 1000 entries; an item's four passes take 0.24 us
+// per entry, however many items there are.  Calls of 2000 targets (list of ~5500):
+// 0.78 ms by blocks, 1.61 by items; of 5000 (~10000) 2.12 and 2.97; batches of 10000
+// (~700) 2.2 and 1.7; of 40000 (1000 per walk) 10.5 and 3.9 (5.1 by the lists,
+// before rows); at 125 neighbours 12.8 and 5.3 (8.3).
+int rowless_most(const sph_context *ctx, int longest_list) { return ctx->sm_count * (8 + longest_list / 256); }
+
 // Validates walk counts and fills the int32 offsets.  n_extra (gravity SPJ
 // counts) may be null.
 int walk_offsets(sph_context *ctx, int32_t n_walk, const int32_t *n_i, const int32_t *n_j,
@@ -874,12 +901,14 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
     if ((st = stage(ctx, ks, i_off, j_off, sizeof(sph_DensityEPI), sizeof(sph_DensityEPJ), item_size(ctx, ni),
                     SPLIT_NJ, arrays, 2, place, L)))
         return st;
-    if (ks.ensure_density(ni, nj, cap, ks.items.size()))
+    const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
+    const int most = rowless_most(ctx, longest(n_epj, n_walk));
+    const bool many = f32 && ni > most;
+    if (ks.ensure_density(ni, nj, cap, ks.items.size(), many ? ni : 0, n_walk))
         return set_error(ctx, SPH_ERR_CUDA, "device allocation failed");
     if (ks.h_out.ensure(sizeof(sph_Density) * (size_t)std::max(ni, 1)))
         return set_error(ctx, SPH_ERR_CUDA, "output allocation failed");
     char *d = ks.d_in.p;
-    const bool f32 = ctx->prm.precision == SPH_PREC_FP32C;
     const DensitySide si{ks.a4[0].p, ks.a4[1].p, ks.id[0].p, ks.d1[0].p, ks.d1[1].p,
                          ks.f4[0].p, ks.f4[1].p, ks.f4[2].p, ks.f4[3].p};
     const DensitySide sj{ks.a4[2].p, ks.a4[3].p, ks.id[1].p, nullptr, nullptr,
@@ -915,8 +944,10 @@ extern "C" int sph_dispatch_density(sph_context *ctx, int32_t tag, int32_t n_wal
         a.amb = ks.amb.p;
         a.amb_cap = cap;
         a.amb_tol = AMB_TOL;
+        const RowlessItems rowless{(const int *)(d + L.off_ioff), n_walk, most, ks.rowless.p, ks.rowless_items.p,
+                                   ctx->d_queue + 4, ctx->d_queue + 5};
         launch_density(ctx, m, pair_grid(ctx, K_DENS, ctx->prm.precision, m.n_items), a, ni, ctx->prm.precision,
-                       ctx->stream);
+                       ctx->stream, nullptr, nullptr, many ? &rowless : nullptr);
     }
     if (ni > 0)
         pack_density<<<eltwise_grid(ni), 256, 0, ctx->stream>>>(

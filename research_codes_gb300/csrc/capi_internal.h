@@ -100,6 +100,8 @@ struct KindState {
     Slice<int2> r_info;               // rows: entries and walk per particle
     Slice<int2> amb;                  // FP64 re-check queue of the density
     Slice<int4> long_items;           // items with lists left to a block each
+    Slice<int> rowless;               // FP32C density: particles without a row, and items of them
+    Slice<int4> rowless_items;
     std::vector<int4> items;
     std::vector<int> i_off;
     bool pending = false;
@@ -125,7 +127,7 @@ struct KindState {
         layout(place);
         return 0;
     }
-    int ensure_density(size_t ni, size_t nj, size_t n_amb, size_t n_items) {
+    int ensure_density(size_t ni, size_t nj, size_t n_amb, size_t n_items, size_t n_rowless, size_t n_walk) {
         return ensure([&](Placer &put) {
             put(a4[0], ni), put(a4[1], ni), put(id[0], ni), put(d1[0], ni), put(d1[1], ni);
             put(a4[2], nj), put(a4[3], nj), put(id[1], nj);
@@ -134,6 +136,7 @@ struct KindState {
             for (int k = 0; k < 4; ++k) put(f4[k], ni), put(f4[4 + k], nj);
             put(hl_list, ni * sphk::ROW_CAP), put(r_info, ni), put(hl_ovf, ni);
             put(amb, n_amb), put(long_items, n_items);
+            if (n_rowless) put(rowless, n_rowless), put(rowless_items, n_rowless / 32 + n_walk);
         });
     }
     int ensure_hydro(size_t ni, size_t nj, size_t n_items) {
@@ -174,8 +177,8 @@ struct sph_context {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     int *d_queue = nullptr;   // [0..2] work-queue counters, [3] density re-check count,
-                              // [4..6] unused, [7] density sweep queue,
-                              // [8] FP32C hydro rows that overflowed, [9..11] long items
+                              // [4] items of rowless particles, [5] their counter, [7] density
+                              // sweep queue, [8] hydro rows that overflowed, [9..11] long items
     int *h_flags = nullptr;   // pinned: per kind, non-finite values in the outputs
     int grid[3][2] = {{0}};   // persistent grid per kind and precision
     int grid_stream = 0;      // persistent grid of the FP32C streamed density walk
@@ -196,11 +199,22 @@ struct LongSide {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
 };
+// FP32C density of a dispatch: what the items of its rowless particles need
+// (density_stream over them where they are many).
+struct RowlessItems {
+    const int *i_off;
+    int n_walk;
+    int most;   // up to this many are swept by a block each
+    int *list;
+    int4 *items;
+    int *n_items, *queue;
+};
 int pair_grid(const sph_context *ctx, int kind, int precision, int n_items);
 void launch_mark_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_max, cudaStream_t s,
                          const LongSide *side = nullptr);
 void launch_density(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, const sphk::DensityArgs &a,
-                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr, const LongSide *side = nullptr);
+                    int n_max, int precision, cudaStream_t s, int *amb_total = nullptr, const LongSide *side = nullptr,
+                    const RowlessItems *rowless = nullptr);
 void launch_density_stream(const sph_context *ctx, const sphk::StreamArgs &w, bool sweep, const sphk::DensityArgs &a,
                            int n_max, cudaStream_t s, int *amb_total, const LongSide &side);
 void launch_hydro_marks(const sph_context *ctx, const sphk::MarkArgs &m, int mark_grid, int n_i, int precision,

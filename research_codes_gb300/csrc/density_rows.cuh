@@ -53,7 +53,7 @@ struct DensityArgs {
     const int *j_idx;       // null: entries are j indices themselves
     // rows (mark_rows)
     const int *rows;
-    const int2 *info;
+    int2 *info;             // particles whose h leaves its row lose it
     int2 *ovf;              // sweep queue
     int *n_ovf;
     float slack;            // row radius over the first guess of h
@@ -417,7 +417,10 @@ __global__ void __launch_bounds__(DROWS_THREADS, F64 ? 2 : SPH_DROWS_MIN_BLOCKS)
                 ++n_rows;
             } else {
                 ++ev_swept;
-                if (row_ok) a.ovf[atomicAdd(a.n_ovf, 1)] = make_int2(ii, inf.y);
+                if (row_ok) {
+                    a.ovf[atomicAdd(a.n_ovf, 1)] = make_int2(ii, inf.y);
+                    a.info[ii].x = ROW_CAP + 1;
+                }
             }
         }
     }
@@ -452,18 +455,21 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double (*red)[DSWEEP_T
     __syncthreads();
 }
 
-// queue / n_queue: (particle, walk) to sweep (n_queue capped at queue_cap);
-// total (optional): the count is added to it.
+// queue / n_queue: (particle, walk) to sweep (n_queue capped at queue_cap;
+// nothing to do with more than `most`); total (optional): the count is added
+// to it.
 #ifndef SPH_SWEEP_U
 #define SPH_SWEEP_U 8
 #endif
 template <bool F64>
 __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArgs a, const int2 *queue,
-                                                               const int *n_queue, int queue_cap, int *total) {
+                                                               const int *n_queue, int queue_cap, int *total,
+                                                               int most = 0x7fffffff) {
     typedef typename Real<F64>::T R;
     constexpr int T = DSWEEP_THREADS, U = SPH_SWEEP_U;   // U list entries per thread in flight
     __shared__ double red[5][T / 32];
     if (a.err && (*a.err & a.err_mask)) return;
+    if (*n_queue > most) return;
     const int nq = min(*n_queue, queue_cap);
     if (total && blockIdx.x == 0 && threadIdx.x == 0) *total += *n_queue;
     const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;

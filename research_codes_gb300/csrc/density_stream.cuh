@@ -82,6 +82,32 @@ struct StreamArgs {
     unsigned long long *n_pass = nullptr;
 };
 
+// The particles without a row, walk by walk in items of 32 (one warp per
+// walk): their indices to `list`, which holds every walk's at its own offset.
+// Nothing while no more than `most` (*n_rowless) are without.
+__global__ inline void __launch_bounds__(128)
+rowless_items(int n_walk, const int *i_off, const int *j_off, const int2 *info, const int *n_rowless, int most,
+              int *list, WorkItem *items, int *n_items) {
+    if (*n_rowless <= most) return;
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_walk; w += nw) {
+        const int b = i_off[w], e = i_off[w + 1];
+        int n = 0;
+        for (int k = b; k < e; k += 32) {
+            const bool out = k + lane < e && info[k + lane].x > ROW_CAP;
+            const unsigned m = __ballot_sync(FULL, out);
+            if (out) list[b + n + __popc(m & lanemask_lt())] = k + lane;
+            n += __popc(m);
+        }
+        const int c = (n + 31) / 32;
+        int pos = 0;
+        if (lane == 0 && c > 0) pos = atomicAdd(n_items, c);
+        pos = __shfl_sync(FULL, pos, 0);
+        for (int q = lane; q < c; q += 32)
+            items[pos + q] = make_int4(w, b + 32 * q, min(32, n - 32 * q), 0);
+    }
+}
+
 template <bool B>
 struct BTag {
     static constexpr bool value = B;
