@@ -12,14 +12,15 @@
 //                  radius before the last pass is queued for the sweep.
 //   density_sweep  one block per queued particle over its walk's whole list:
 //                  particles without a row (overflow, very long lists, h
-//                  outside the row range), re-walks of few particles, and the
-//                  FP64 recomputation of FP32C results whose search-radius
+//                  outside the row range; many of them in an FP32C dispatch go
+//                  to density_stream instead), re-walks of few particles, and
+//                  the FP64 recomputation of FP32C results whose search-radius
 //                  decision is ambiguous.
 //
 // Bound: density_rows by the FP64 pipe (FP64) or by its launch and the latency of
 // the rows (calls: 64 targets in 13 us where one warp per 32 targets took
 // 100); eight lanes per particle keep a call of 64 on 16 warps and each pass at
-// ~8 entries per lane.  density_sweep by the longest list of a batch (29k
+// ~8 entries per lane (FP64 calls: a warp per particle).  density_sweep by the longest list of a batch (29k
 // entries: 150 us; a warp took 1.6 ms); indices a round ahead of the records,
 // 8 entries in flight and no velocities beyond the support: 500k evaluation
 // with five re-walks 10.29 -> 9.93 ms.

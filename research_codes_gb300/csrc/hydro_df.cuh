@@ -39,7 +39,7 @@
 
 namespace sphk {
 
-// FP32C hydro records of one particle (FP32C mode of hydro_kernel):
+// FP32C hydro records of one particle:
 //   phi (x_hi, y_hi, z_hi, mass_hi)   plo (x_lo, y_lo, z_lo, mass_lo)
 //   vhi (vx_hi, vy_hi, vz_hi, 1/h)    vlo (vx_lo, vy_lo, vz_lo, h^-4)
 //   g1  (P_hi, P_lo, presc_hi, bswt/2) g2 (dens, vsnd, alph, alphu)

@@ -38,9 +38,10 @@ constexpr int MAX_J = SPH_NOALLOC_MAX_J;
 constexpr int NOALLOC_WARPS = 4;
 constexpr int MAX_ITEMS = (MAX_I + 31) / 32;
 // Results of the parts of the lists: a call of n_i particles takes at most
-// MAX_PART / n_i parts, as many as give every resident warp (~2400) a unit.
+// MAX_PART / n_i parts, as many as give every resident warp two units (16 warps
+// on each of 152 SMs; the scratch is static, so the count is too).
 constexpr int MAX_PART = 98304;
-constexpr int UNITS = 4864;
+constexpr int UNITS = 2 * 16 * 152;
 
 // Layout of the scratch array (byte offsets, each 256-byte aligned).
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }

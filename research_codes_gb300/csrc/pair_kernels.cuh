@@ -159,7 +159,7 @@ __device__ __forceinline__ void hydro64_store(const HydroArgs &a, int p, const d
 // the sweep.  FP64 pipe bound (~120 instructions per pair): rows hold ~57 pairs
 // where the list holds ~900, and the old kernel tested each of those in FP64
 // (call of 256 among 20k: 2690 -> 179 us).
-// L = 32 in small calls (warp_per_row).
+// L = 32 in small calls (warp_per_row): the call of 256 162 -> 143 us.
 constexpr int HROWS_LANES = 8, HROWS_THREADS = 128;
 template <int L>
 __global__ void __launch_bounds__(HROWS_THREADS) hydro64_rows(const HydroArgs a) {
@@ -398,7 +398,7 @@ __device__ __forceinline__ void gravity_gather_warp(const double *acc, const dou
 
 // Bound: FP32C by instruction issue (packed FMAs and rsqrt), FP64 by the FP64
 // pipe (88% busy, 30 operations per pair).  Units of an item's list fill the
-// chip where items are few: 500 targets x 20k 411 -> 37 us, gravity of a 50k
+// chip where items are few: 500 targets x 20k 411 -> 40 us, gravity of a 50k
 // FP64 evaluation 9.9 -> 6.3 ms.
 // JT: the j-tile, list entries a warp stages in shared memory per pass (32
 // or 64; each lane loads JT / 32 of them one tile ahead) and sums in FP32

@@ -24,7 +24,12 @@
 
 namespace sphk {
 
-// Entries of a row; particles with more go to the sweep queue.
+// Entries of a row; particles with more go to the sweep queue.  128 hold the 50
+// to 64 neighbours of eta 1.18 to 1.28 within 3%; at eta 1.6 (125 neighbours) most
+// particles have no row and are swept (FP32C density: rowless_items).  Times
+// there, by the lists before rows and now: density batch of 40k in walks of 256
+// 13.1 and 3.9 ms in FP32C, 51.7 and 20.0 in FP64; hydro batch of 21k 14.5 and 4.7,
+// 83.0 and 7.9; 50k FP64 evaluation 36.2 and 35.8 ms, 50k FP32C 9.0 and 8.3.
 constexpr int ROW_CAP = 128;
 static_assert(ROW_CAP % 32 == 0, "eight lanes read a row four entries at a time");
 // Items with longer lists than this are taken by a whole block (the LONG forms
@@ -37,7 +42,8 @@ __device__ __forceinline__ int long_list(long long pairs, int least = 768) {
 }
 constexpr int MARK_LONG_WARPS = 16, HYDRO_LONG_WARPS = 8;
 // FP32C hydro rows: longest list (in steps of 64 entries) whose LONG form
-// keeps the row order of a warp's item
+// keeps the row order of a warp's item.  Calls leave longer ones to a warp;
+// in a system they go to blocks too, and their rows are in list order.
 constexpr int LONG_STEPS = 2048;
 // Radii outside this range (or NaN) are left to the sweep: their squares
 // leave the FP32 range.
@@ -223,8 +229,8 @@ struct Signal<ROWS_HYDRO64> {
 // One warp per work item streams the walk's list in steps of 64 entries.
 // LONG: a block per item of the long-item queue, its warps streaming
 // interleaved steps; the hits of all warps meet in the rows by shared
-// counters and are put into list order at the end (the same rows as one warp
-// writes).
+// counters and are put into order at the end (the same rows as one warp
+// writes; FP32C hydro: up to LONG_STEPS).
 //
 // Hydro: the signal-velocity maximum runs over every entry of the list.  A
 // term is at most c_i + c_j + 3 (|v_i - v_c| + |v_j - v_c|) with v_c the

@@ -86,14 +86,13 @@ __device__ __forceinline__ float sqrt_r(float x) {
 }
 __device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
 
-// sqrt for bounds that carry a relative margin far above 2^-22: FP32 by
-// sqrt.approx.ftz.f32, FP64 by the library sqrt.
+// sqrt for bounds that carry a relative margin far above 2^-22, by
+// sqrt.approx.ftz.f32.
 __device__ __forceinline__ float sqrt_bound(float x) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ double sqrt_bound(double x) { return sqrt(x); }
 
 // Radial kernel-gradient factor W1(q)/c1 with u = (1-q)_+ (hdr_kernel.hpp:251-257).
 // The reference's form u^4 - u^3 (1+4q) subtracts two nearly equal terms for
@@ -145,7 +144,7 @@ struct Acc<true> {
     __device__ __forceinline__ double value() const { return s; }
 };
 
-// Sum / max over the `tpi` consecutive lanes that share one i-particle
+// Sum over the `tpi` consecutive lanes that share one i-particle
 // (tpi is a power of two <= 32; every lane of the warp must call it).
 __device__ __forceinline__ double seg_sum(double v, int tpi) {
     for (int o = tpi >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
@@ -153,10 +152,6 @@ __device__ __forceinline__ double seg_sum(double v, int tpi) {
 }
 __device__ __forceinline__ long long seg_sum(long long v, int tpi) {
     for (int o = tpi >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    return v;
-}
-__device__ __forceinline__ double seg_max(double v, int tpi) {
-    for (int o = tpi >> 1; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL, v, o));
     return v;
 }
 
@@ -214,16 +209,8 @@ __device__ __forceinline__ float warp_min(float v) {
     for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(FULL, v, o));
     return v;
 }
-__device__ __forceinline__ double warp_min(double v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(FULL, v, o));
-    return v;
-}
 __device__ __forceinline__ float warp_max(float v) {
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULL, v, o));
-    return v;
-}
-__device__ __forceinline__ double warp_max(double v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL, v, o));
     return v;
 }
 

@@ -412,10 +412,6 @@ __global__ void compact_active(int n, const int *scal, const int *flag, const in
     }
 }
 
-__global__ void copy_int(const int *src, int *dst) { *dst = *src; }
-
-// list totals: offset[n-1] + count[n-1] (counts beyond the walk count are 0)
-// Task count of a list build (clamped to the task capacity, error bit beyond).
 // counters of an evaluation
 __global__ void begin_evaluation(int *scal, long long *lscal) {
     for (int k = threadIdx.x; k < L_NI; k += blockDim.x) lscal[k] = 0;
@@ -429,12 +425,14 @@ __global__ void begin_evaluation(int *scal, long long *lscal) {
     }
 }
 
+// Task count of a list build (clamped to the task capacity, error bit beyond).
 __global__ void task_total(int n, const int *toff, int cap, int *scal) {
     const int t = toff[n];
     scal[S_NTASKS] = t < cap ? t : cap;
     if (t > cap) atomicOr(&scal[S_ERROR], E_LISTCAP);
 }
 
+// list totals: offset[n-1] + count[n-1] (counts beyond the walk count are 0)
 __global__ void list_total(int n, const int *cnt, const int *off, long long cap, int *scal, long long *lscal,
                            int lslot) {
     const long long tot = (long long)off[n - 1] + cnt[n - 1];
