@@ -418,7 +418,7 @@ __global__ void prepare_gravity(const sph_GravityEPI *epi, int ni, const sph_Gra
 
 // Results go to pinned memory: a block's structs through shared memory, so that
 // the link sees consecutive words (bound by it: 40k density structs took 89 us
-// written struct by struct, 17 us so).
+// written struct by struct, 16 us so).
 constexpr int PACK_THREADS = 256;
 template <class T>
 __device__ __forceinline__ void write_structs(T *s, const T &v, T *out, int k0, int n) {

@@ -20,10 +20,11 @@
 // Bound: density_rows by the FP64 pipe (FP64) or by its launch and the latency of
 // the rows (calls: 64 targets in 13 us where one warp per 32 targets took
 // 100); eight lanes per particle keep a call of 64 on 16 warps and each pass at
-// ~8 entries per lane (FP64 calls: a warp per particle).  density_sweep by the longest list of a batch (29k
-// entries: 150 us; a warp took 1.6 ms); indices a round ahead of the records,
-// 8 entries in flight and no velocities beyond the support: 500k evaluation
-// with five re-walks 10.29 -> 9.93 ms.
+// ~8 entries per lane (FP64 calls: a warp per particle).  density_sweep by the
+// longest list of a batch (29k entries: 100 us, 150 without the distance test; a
+// warp took 1.6 ms); indices a round ahead of the records, 8 entries in flight
+// and no velocities beyond the support: 500k evaluation with five re-walks
+// 10.29 -> 9.93 ms.
 //
 // Both form the separations relative to the particle itself; FP32C sums a few
 // terms in FP32, folds them into Kahan pairs per lane and adds the lanes with
