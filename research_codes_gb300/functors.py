@@ -186,10 +186,16 @@ def _ptr_array(arrs):
 
 
 def _count_array(counts):
+    """Counts as a C array, each as int() takes it."""
     n = len(counts)
     out = (ctypes.c_int32 * max(n, 1))()
-    if n:
-        np.frombuffer(out, np.int32)[:n] = np.asarray(counts, np.int64)
+    a = counts
+    if type(a) in (list, tuple) and set(map(type, a)) == {int}:
+        a = np.array(a)
+    if type(a) is np.ndarray and a.ndim == 1 and a.dtype.kind in "iu":
+        np.frombuffer(out, np.int32)[:n] = a
+    else:
+        out[:n] = list(map(int, counts))
     return out
 
 

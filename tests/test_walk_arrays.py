@@ -3,6 +3,7 @@ import ctypes
 
 import numpy as np
 import pytest
+import torch
 
 from research_codes_gb300 import _lib, abi, functors
 
@@ -44,6 +45,27 @@ def test_addresses_of_rows_that_exist_for_the_loop_alone():
 def test_counts():
     for c in ([], [3], (1, 2, 3), np.arange(5), np.arange(5, dtype=np.uint8), [2.0, 7.0]):
         assert list(functors._count_array(c))[:len(c)] == [int(x) for x in c]
+
+
+class _Int:
+    def __int__(self):
+        return 4
+
+
+@pytest.mark.parametrize("counts", [
+    np.array([np.nan, 1.0]), np.array([np.inf]), [float("nan")], [None], np.array(["2020"], "M8[Y]"),
+    np.array([[1], [2]]), {2: 1, 3: 1}, [2 ** 70 + 3, 1], [2 ** 63, -1], np.array([2 ** 63 + 5], np.uint64),
+    ["3", b"7"], [True, _Int()], np.array([1.5, 2.0]), torch.tensor([1, 2]), [torch.tensor(3), torch.tensor([4])],
+], ids=str)
+def test_counts_are_taken_as_int_takes_them(counts):
+    """What int() refuses is refused, what it accepts is accepted (low 32 bits)."""
+    try:
+        want = [ctypes.c_int32(int(c)).value for c in counts]
+    except (TypeError, ValueError, OverflowError) as e:
+        with pytest.raises(type(e)):
+            functors._count_array(counts)
+    else:
+        assert list(functors._count_array(counts)) == want
 
 
 def test_the_binding_helper_is_not_part_of_the_abi():
