@@ -173,7 +173,14 @@ static void launch_density_sums(const sph_context *ctx, const sphk::DensityArgs 
             sphk::density_rows<true, 32><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
         else
             sphk::density_rows<true><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);
-        sphk::density_sweep<true><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr);
+        // More particles without a row than SMs: a warp each.  Calls (list of
+        // ~1100 to 4500) of 128: 146 us by warps and 135 by blocks; of 256: 166 and
+        // 183, of 600: 217 and 300; of 4096 (~12500) 1.2 and 2.4 ms.
+        const int most = ctx->sm_count;
+        if (n_max > most)
+            sphk::density_sweep_warps<<<std::min(n_max / sphk::SWEEP_WARPS + 1, 4 * ctx->sm_count),
+                                        sphk::SWEEP_WARPS * 32, 0, s>>>(a, a.ovf, a.n_ovf, n_max, most);
+        sphk::density_sweep<true><<<sg, sphk::DSWEEP_THREADS, 0, s>>>(a, a.ovf, a.n_ovf, n_max, nullptr, most);
         return;
     }
     sphk::density_rows<false><<<rg, sphk::DROWS_THREADS, 0, s>>>(a);

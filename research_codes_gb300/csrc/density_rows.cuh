@@ -13,9 +13,10 @@
 //   density_sweep  one block per queued particle over its walk's whole list:
 //                  particles without a row (overflow, very long lists, h
 //                  outside the row range; many of them in an FP32C dispatch go
-//                  to density_stream instead), re-walks of few particles, and
-//                  the FP64 recomputation of FP32C results whose search-radius
-//                  decision is ambiguous.
+//                  to density_stream instead, in FP64 to density_sweep_warps),
+//                  re-walks of few particles, and the FP64 recomputation of
+//                  FP32C results whose search-radius decision is ambiguous.
+//   density_sweep_warps  the same with a warp per particle (FP64).
 //
 // Bound: density_rows by the FP64 pipe (FP64) or by its launch and the latency of
 // the rows (calls: 64 targets in 13 us where one warp per 32 targets took
@@ -24,7 +25,9 @@
 // longest list of a batch (29k entries: 100 us, 150 without the distance test; a
 // warp took 1.6 ms); indices a round ahead of the records, 8 entries in flight
 // and no velocities beyond the support: 500k evaluation with five re-walks
-// 10.29 -> 9.93 ms.
+// 10.29 -> 9.93 ms.  FP64: a step of 32 list entries holds two or three within
+// reach, and the FP64 pipe takes a warp's instruction whole; collected and summed
+// 32 at a time, a call of 64 without rows takes 135 us, 154 one by one.
 //
 // Both form the separations relative to the particle itself; FP32C sums a few
 // terms in FP32, folds them into Kahan pairs per lane and adds the lanes with
@@ -458,24 +461,55 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double (*red)[DSWEEP_T
 }
 
 // queue / n_queue: (particle, walk) to sweep (n_queue capped at queue_cap;
-// nothing to do with more than `most`); total (optional): the count is added
-// to it.
+// with more than `most` in FP32C nothing, in FP64 the lists that are left by
+// density_sweep_warps); total (optional): the count is added to it.
 #ifndef SPH_SWEEP_U
 #define SPH_SWEEP_U 8
 #endif
+// FP64: longest list of a queue of n that a warp takes: at about n entries a warp
+// needs as long for it as the chip for the rest of the queue, at 16384 ~0.2 ms.
+__host__ __device__ __forceinline__ int sweep_long(int n) { return n > 16384 ? n : 16384; }
 template <bool F64>
 __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArgs a, const int2 *queue,
                                                                const int *n_queue, int queue_cap, int *total,
                                                                int most = 0x7fffffff) {
     typedef typename Real<F64>::T R;
     constexpr int T = DSWEEP_THREADS, U = SPH_SWEEP_U;   // U list entries per thread in flight
+    constexpr int RING = 512;                            // < 32 left over + a round of 32 U
+    static_assert(32 * (U + 1) <= RING, "hits of a round");
     __shared__ double red[5][T / 32];
+    __shared__ int s_hit[F64 ? T / 32 : 1][RING];        // a warp's entries within reach
+    __shared__ int s_todo[F64 ? T : 1], s_n;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned lt = lanemask_lt();
     if (a.err && (*a.err & a.err_mask)) return;
-    if (*n_queue > most) return;
     const int nq = min(*n_queue, queue_cap);
+    const bool many = *n_queue > most;
+    if (!F64 && many) return;
     if (total && blockIdx.x == 0 && threadIdx.x == 0) *total += *n_queue;
     const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
-    for (int e = blockIdx.x; e < nq; e += gridDim.x) {
+    // many: T particles of the queue at a time, those with the longest lists
+    const int step = many ? T : 1, nj_warp = sweep_long(nq);
+    for (int e0 = blockIdx.x * step; e0 < nq; e0 += gridDim.x * step)
+    for (int td = 0;; ++td) {
+        int e = e0;
+        if (many) {
+            if (td == 0) {
+                __syncthreads();
+                if (threadIdx.x == 0) s_n = 0;
+                __syncthreads();
+                const int k = e0 + threadIdx.x;
+                if (F64 && k < nq) {
+                    const int w = queue[k].y;
+                    if (a.j_off[w + 1] - a.j_off[w] > nj_warp) s_todo[atomicAdd(&s_n, 1)] = k;
+                }
+                __syncthreads();
+            }
+            if (td >= s_n) break;
+            e = s_todo[F64 ? td : 0];
+        } else if (td > 0) {
+            break;
+        }
         const int2 pw = queue[e];
         const int ii = pw.x;
         if (a.n_j > 0 && (ii < 0 || ii >= a.n_j)) {
@@ -493,10 +527,10 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         const double mi = a.i_pm[ii].w;
         // visits the list entries; FP64: those that can lie within h of the
         // particle by an FP32 distance test on the double-float positions,
-        // with the margins of mark_rows (h outside its range: every entry);
-        // in FP32C f itself tests.  A coordinate that is NaN counts as the
-        // particle's own, as in the box test of mark_rows.  Indices are read a
-        // round ahead of the records.
+        // with the margins of mark_rows (h outside its range: every entry), 32
+        // at a time; in FP32C f itself tests.  A coordinate that is NaN counts
+        // as the particle's own, as in the box test of mark_rows.  Indices are
+        // read a round ahead of the records.
         auto over_list = [&](R h, auto &&f) {
             const float hf = (float)h;
             const float pad = 3.0e-14f * (fabsf(ph.x) + fabsf(ph.y) + fabsf(ph.z));
@@ -511,8 +545,9 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
                     next[u] = (k < je) ? (a.j_idx ? a.j_idx[k] : k) : -1;
                 }
             };
+            int head = 0, fill = 0;
             indices(jb + threadIdx.x);
-            for (int k0 = jb + threadIdx.x; k0 < je; k0 += T * U) {
+            for (int b = jb + 32 * wid; b < je; b += T * U) {
                 int j[U];
                 float4 qh[U], ql[U];
 #pragma unroll
@@ -527,19 +562,38 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
                         ql[u] = __ldg(&a.fj.plo[j[u]]);
                     }
                 }
-                indices(k0 + T * U);
+                indices(b + lane + T * U);
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (j[u] >= 0) {
-                        if constexpr (F64) {
+                for (int u = 0; u < U; ++u) {
+                    if constexpr (F64) {
+                        bool hit = j[u] >= 0;
+                        if (hit) {
                             const float dx = df_diff(qh[u].x, ql[u].x, ph.x, pl.x);
                             const float dy = df_diff(qh[u].y, ql[u].y, ph.y, pl.y);
                             const float dz = df_diff(qh[u].z, ql[u].z, ph.z, pl.z);
-                            if (square_sum(dx, dy, dz) > lim) continue;
+                            hit = !(square_sum(dx, dy, dz) > lim);
                         }
+                        const unsigned m = __ballot_sync(FULL, hit);
+                        if (hit) s_hit[wid][(head + fill + __popc(m & lt)) & (RING - 1)] = j[u];
+                        fill += __popc(m);
+                    } else if (j[u] >= 0) {
                         f(j[u], qh[u], ql[u]);
                     }
+                }
+                if constexpr (F64) {
+                    __syncwarp();
+                    for (; fill >= 32; fill -= 32, head += 32) f(s_hit[wid][(head + lane) & (RING - 1)], ph, pl);
+                    __syncwarp();
+                }
             }
+            if constexpr (F64) {
+                if (lane < fill) f(s_hit[wid][(head + lane) & (RING - 1)], ph, pl);
+                __syncwarp();
+            }
+        };
+        // farther than r2_far; a coordinate that is NaN counts as zero
+        auto far_off = [](R r2, R dx, R dy, R dz, R r2_far) {
+            return r2 > r2_far || (r2 != r2 && square_sum(dx, dy, dz) > r2_far);
         };
         // Terms beyond the support are zero, whatever the mass, and need no
         // velocity; in FP32C a run of them folds one zero (further ones leave
@@ -554,14 +608,14 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
             bool zero = false;
             over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
                 R dx, dy, dz;
-                const R m = P.rel(a, j, qh, ql, dx, dy, dz);
-                if (square_sum(dx, dy, dz) > r2_far) {
+                const R m = P.rel(a, j, qh, ql, dx, dy, dz), r2 = dx * dx + dy * dy + dz * dz;
+                if (far_off(r2, dx, dy, dz, r2_far)) {
                     if (!F64 && !zero) acc.add((R)0);
                     zero = true;
                     return;
                 }
                 zero = false;
-                const R q = sqrt_q(dx * dx + dy * dy + dz * dz, hinv2);
+                const R q = sqrt_q(r2, hinv2);
                 cnt += (q < (R)1) ? 1 : 0;
                 acc.add(density_term(q, m));
             });
@@ -578,8 +632,8 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         bool zero = false;
         over_list(s.h, [&](int j, const float4 &qh, const float4 &ql) {
             R dx, dy, dz, ux, uy, uz;
-            const R m = P.rel(a, j, qh, ql, dx, dy, dz);
-            if (square_sum(dx, dy, dz) > r2_far) {
+            const R m = P.rel(a, j, qh, ql, dx, dy, dz), r2 = dx * dx + dy * dy + dz * dz;
+            if (far_off(r2, dx, dy, dz, r2_far)) {
                 if (!F64 && !zero) gs.fold();
                 zero = true;
                 return;
@@ -593,6 +647,152 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
         block_sum(v, red);
         if (threadIdx.x == 0) {
             density_finish<R>(a, ii, pw.y, s, (R)v[0], (R)v[1], (R)v[2], (R)v[3], (R)v[4], np, ksr_max);
+            if (a.n_eval) {
+                atomicAdd(a.n_eval, 3ull * (unsigned long long)(je - jb));
+                atomicAdd(a.n_eval + 1, (unsigned long long)(je - jb));
+            }
+        }
+    }
+}
+
+// FP64: a warp per queued particle where there are many (more than `least`) and
+// its list is not far longer than the others' (sweep_long).  Entries within
+// 1.1 h are kept in shared memory for the passes whose h stays within that;
+// SWEEP_CAP hold 125 neighbours four times.
+// Bound by FP64 pairs and the latency of the list's records (a block of
+// density_sweep fills an SM and waits for both and for its barriers).  Density of
+// 200k particles at 125 neighbours 58.7 -> 12.6 ms (36.0 by the lists before rows;
+// 17.7 at 12 warps per SM, 13.4 at 20), with a first guess of h 20% low at 55
+// neighbours 134 -> 23 ms (42.7).
+constexpr int SWEEP_CAP = 512, SWEEP_WARPS = 4;
+__global__ inline void __launch_bounds__(SWEEP_WARPS * 32, 4)
+density_sweep_warps(const DensityArgs a, const int2 *queue, const int *n_queue, int queue_cap, int least) {
+    constexpr int U = 4;   // list entries per lane in flight
+    static_assert(SWEEP_CAP >= 64 * U, "a round of hits and the room for another");
+    __shared__ int s_hit[SWEEP_WARPS][SWEEP_CAP];
+    if (a.err && (*a.err & a.err_mask)) return;
+    if (*n_queue <= least) return;
+    const int nq = min(*n_queue, queue_cap), nj_warp = sweep_long(nq);
+    const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned lt = lanemask_lt();
+    int *hits = s_hit[wid];
+    for (int e = blockIdx.x * SWEEP_WARPS + wid; e < nq; e += gridDim.x * SWEEP_WARPS) {
+        const int2 pw = queue[e];
+        const int ii = pw.x;
+        if (a.n_j > 0 && (ii < 0 || ii >= a.n_j)) {
+            if (lane == 0) atomicOr(a.err_out, a.bounds_bit);
+            continue;   // warp-uniform
+        }
+        const int jb = a.j_off[pw.y], je = a.j_off[pw.y + 1];
+        if (je - jb > nj_warp) continue;
+        if (a.n_j > 0 && (jb < 0 || je < jb || (long long)je > a.list_cap)) {
+            if (lane == 0) atomicOr(a.err_out, a.bounds_bit);
+            continue;   // warp-uniform
+        }
+        PairPos<true> P;
+        P.load_i(a, ii);
+        const float4 ph = a.fi.phi[ii], pl = a.fi.plo[ii];
+        const float pad = 3.0e-14f * (fabsf(ph.x) + fabsf(ph.y) + fabsf(ph.z));
+        int n = 0;            // hits
+        double h_hits = -1.0;   // all within this radius are there
+        // f(j) for the entries that can lie within h, as in density_sweep
+        auto over_list = [&](double h, auto &&f) {
+            const bool scan = !(h >= 0.0 && h <= h_hits);
+            bool all = true;
+            float lim = INFINITY;
+            int b = jb;
+            if (scan) {
+                const float hf = (float)(1.1 * h), rad = hf * 1.0001f + pad;
+                if (hf >= ROW_HMIN && hf <= ROW_HMAX) lim = rad * rad;
+                n = 0;
+            }
+            for (bool last = false; !last;) {
+                if (scan && b < je) {
+                    int j[U];
+                    float4 qh[U], ql[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int k = b + 32 * u + lane;
+                        j[u] = k < je ? (a.j_idx ? a.j_idx[k] : k) : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (a.n_j > 0 && j[u] >= a.n_j) {
+                            atomicOr(a.err_out, a.bounds_bit);
+                            j[u] = -1;
+                        }
+                        if (j[u] >= 0) {
+                            qh[u] = __ldg(&a.fj.phi[j[u]]);
+                            ql[u] = __ldg(&a.fj.plo[j[u]]);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        bool hit = j[u] >= 0;
+                        if (hit) {
+                            const float dx = df_diff(qh[u].x, ql[u].x, ph.x, pl.x);
+                            const float dy = df_diff(qh[u].y, ql[u].y, ph.y, pl.y);
+                            const float dz = df_diff(qh[u].z, ql[u].z, ph.z, pl.z);
+                            hit = !(square_sum(dx, dy, dz) > lim);
+                        }
+                        const unsigned m = __ballot_sync(FULL, hit);
+                        if (hit) hits[n + __popc(m & lt)] = j[u];
+                        n += __popc(m);
+                    }
+                    b += 32 * U;
+                    __syncwarp();
+                }
+                last = !scan || b >= je;
+                if (last || n > SWEEP_CAP - 32 * U) {
+                    for (int k = lane; k < n; k += 32) f(hits[k]);
+                    if (!last) {
+                        n = 0;
+                        all = false;
+                    }
+                    __syncwarp();
+                }
+            }
+            if (scan) h_hits = all && lim < INFINITY ? 1.1 * h : -1.0;
+        };
+        auto far_off = [](double r2, double dx, double dy, double dz, double r2_far) {
+            return r2 > r2_far || (r2 != r2 && square_sum(dx, dy, dz) > r2_far);
+        };
+        HState<double> s;
+        s.start(a.i_ksr[ii]);
+        int np = 0;
+        for (int pass = 0; pass < 3; ++pass) {
+            double sum = 0.0;
+            int cnt = 0;
+            const double hinv2 = s.hinv * s.hinv, r2_far = 1.0002 * s.h * s.h;
+            over_list(s.h, [&](int j) {
+                double dx, dy, dz;
+                const double m = P.rel(a, j, dx, dy, dz), r2 = dx * dx + dy * dy + dz * dz;
+                if (far_off(r2, dx, dy, dz, r2_far)) return;
+                const double q = sqrt_q(r2, hinv2);
+                cnt += (q < 1.0) ? 1 : 0;
+                sum += density_term(q, m);
+            });
+            np = __reduce_add_sync(FULL, cnt);
+            s.update(seg_sum(sum, 32), P.p.w, a.eta_ksrh, ksr_max);
+        }
+        GradSums<true> gs;
+        const long long idi = a.i_id[ii];
+        PairVel<true> V;
+        V.load_i(a, ii);
+        const double r2_far = 1.0002 * s.h * s.h;
+        over_list(s.h, [&](int j) {
+            double dx, dy, dz, ux, uy, uz;
+            const double m = P.rel(a, j, dx, dy, dz), r2 = dx * dx + dy * dy + dz * dz;
+            if (far_off(r2, dx, dy, dz, r2_far)) return;
+            V.rel(a, j, ux, uy, uz);
+            gs.add(dx, dy, dz, ux, uy, uz, m, a.j_id[j] == idi, s.hinv);
+        });
+        gs.fold();
+        const double sg = seg_sum(gs.g.value(), 32), sd = seg_sum(gs.d.value(), 32);
+        const double sx = seg_sum(gs.rx.value(), 32), sy = seg_sum(gs.ry.value(), 32), sz = seg_sum(gs.rz.value(), 32);
+        if (lane == 0) {
+            density_finish<double>(a, ii, pw.y, s, sg, sd, sx, sy, sz, np, ksr_max);
             if (a.n_eval) {
                 atomicAdd(a.n_eval, 3ull * (unsigned long long)(je - jb));
                 atomicAdd(a.n_eval + 1, (unsigned long long)(je - jb));

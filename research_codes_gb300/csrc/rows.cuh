@@ -27,9 +27,9 @@ namespace sphk {
 // Entries of a row; particles with more go to the sweep queue.  128 hold the 50
 // to 64 neighbours of eta 1.18 to 1.28 within 3%; at eta 1.6 (125 neighbours) most
 // particles have no row and are swept (FP32C density: rowless_items).  Times
-// there, by the lists before rows and now: density batch of 40k in walks of 256
-// 13.1 and 3.9 ms in FP32C, 51.7 and 20.0 in FP64; hydro batch of 21k 14.5 and 4.7,
-// 83.0 and 7.9; 50k FP64 evaluation 36.2 and 35.8 ms, 50k FP32C 9.0 and 8.3.
+// there, by the lists before rows and now: density batch of 20k in walks of 300
+// 4.8 and 2.9 ms in FP32C, 21.4 and 3.7 in FP64; hydro batch 10.5 and 4.6, 37.9 and
+// 5.7; evaluation of 200k 16.4 and 16.1 ms in FP32C, 86.2 and 60.3 in FP64.
 constexpr int ROW_CAP = 128;
 static_assert(ROW_CAP % 32 == 0, "eight lanes read a row four entries at a time");
 // Items with longer lists than this are taken by a whole block (the LONG forms
