@@ -2,7 +2,8 @@
 around the number from which a warp takes each of them (152 on 152 SMs), more
 entries within reach than a warp keeps (512), lists that stay with a block
 beside them (more than 16384 entries), first guesses of h that every pass
-outgrows, and sources that add nothing, against the oracle.
+outgrows, and sources that add nothing; FP64 hydro sums of particles without
+rows; against the oracle.
 
 Tolerances: FP64 1e-11, as in test_gpu_functors.py; Omega, div v and |rot v| as
 sums, to 1e-11 of the sum of their terms' magnitudes (see test_gpu_rowless.py).
@@ -13,6 +14,7 @@ import pytest
 from conftest import rel_err
 from oracle import oracle as orc
 from research_codes_gb300 import abi, functors
+from test_gpu_edge_values import _ball, _hydro
 from test_gpu_rowless import _batch, _magnitudes
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +74,13 @@ def test_sources_that_add_nothing(field, value, guess):
         bad["pos"][:, 1] = value
     epi, epj = _batch([350] * 2, 500, 1.18, guess, 15)
     _check(epi, epj, 1.18, bad)
+
+
+@pytest.mark.parametrize("n_i", [1, 40, 700])
+@pytest.mark.parametrize("n_j,neighbours", [(700, 200), (700, 700), (4000, 300), (4000, 3000)])
+def test_hydro_sums_of_particles_without_rows(n_i, n_j, neighbours):
+    """A few to all entries of a round of a block (1024) within reach."""
+    epi, epj, near = _ball(n_i, n_j, 17 * n_i + n_j, neighbours=neighbours)
+    out, ref = _hydro("fp64", epi, epj), orc.hydro(epi, epj)
+    for f in ("acch", "accg", "udot", "vsmx", "diffu"):
+        assert rel_err(out[f], ref[f], 1e-3).max() < 1e-11, f
