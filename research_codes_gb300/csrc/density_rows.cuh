@@ -466,9 +466,11 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double (*red)[DSWEEP_T
 #ifndef SPH_SWEEP_U
 #define SPH_SWEEP_U 8
 #endif
-// FP64: longest list of a queue of n that a warp takes: at about n entries a warp
-// needs as long for it as the chip for the rest of the queue, at 16384 ~0.2 ms.
-__host__ __device__ __forceinline__ int sweep_long(int n) { return n > 16384 ? n : 16384; }
+// FP64: longest list of a queue of n that a warp takes: up to 12 n entries, but
+// not so many that a warp would need longer for it than the chip for the rest of
+// the queue (n), or 0.2 ms (16384).  50k FP64 steps, whose few hundred particles
+// without rows have lists of up to 50k: 27.7 ms; with 16384 for every queue 40.4.
+__device__ __forceinline__ int sweep_long(int n) { return n < 1366 ? 12 * n : (n > 16384 ? n : 16384); }
 template <bool F64>
 __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArgs a, const int2 *queue,
                                                                const int *n_queue, int queue_cap, int *total,
@@ -488,9 +490,9 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
     if (!F64 && many) return;
     if (total && blockIdx.x == 0 && threadIdx.x == 0) *total += *n_queue;
     const double ksr_max = a.ksr_max_dev ? *a.ksr_max_dev : a.ksr_max;
-    // many: T particles of the queue at a time, those with the longest lists
+    // many: of T particles of the queue at a time those with the longest lists
     const int step = many ? T : 1, nj_warp = sweep_long(nq);
-    for (int e0 = blockIdx.x * step; e0 < nq; e0 += gridDim.x * step)
+    for (int e0 = blockIdx.x; e0 < nq; e0 += gridDim.x * step)
     for (int td = 0;; ++td) {
         int e = e0;
         if (many) {
@@ -498,7 +500,7 @@ __global__ void __launch_bounds__(DSWEEP_THREADS) density_sweep(const DensityArg
                 __syncthreads();
                 if (threadIdx.x == 0) s_n = 0;
                 __syncthreads();
-                const int k = e0 + threadIdx.x;
+                const int k = e0 + threadIdx.x * gridDim.x;
                 if (F64 && k < nq) {
                     const int w = queue[k].y;
                     if (a.j_off[w + 1] - a.j_off[w] > nj_warp) s_todo[atomicAdd(&s_n, 1)] = k;

@@ -1,9 +1,9 @@
 """GPU tests of FP64 density dispatches whose particles have no usable row:
 around the number from which a warp takes each of them (152 on 152 SMs), more
 entries within reach than a warp keeps (512), lists that stay with a block
-beside them (more than 16384 entries), first guesses of h that every pass
-outgrows, and sources that add nothing; FP64 hydro sums of particles without
-rows; against the oracle.
+beside them (more than twelve times the queue, or 16384 entries), first guesses
+of h that every pass outgrows, and sources that add nothing; FP64 hydro sums of
+particles without rows; against the oracle.
 
 Tolerances: FP64 1e-11, as in test_gpu_functors.py; Omega, div v and |rot v| as
 sums, to 1e-11 of the sum of their terms' magnitudes (see test_gpu_rowless.py).
@@ -57,6 +57,14 @@ def test_long_lists_beside_the_others(n_long):
     epi, epj = _batch([200] * 4, 300, 1.18, 0.5, 11)
     a, b = _batch([3], n_long, 1.6, 1.2, 13)
     _check(epi[:2] + a + epi[2:], epj[:2] + b + epj[2:], 1.18)
+
+
+@pytest.mark.parametrize("n_long", [2400, 2401])
+def test_long_lists_by_the_length_of_the_queue(n_long):
+    """200 without a row: a warp takes lists of up to 2400 entries."""
+    epi, epj = _batch([160], 300, 1.18, 0.5, 17)
+    a, b = _batch([40], n_long, 1.18, 0.5, 19)
+    _check(epi + a, epj + b, 1.18)
 
 
 @pytest.mark.parametrize("field,value", [("mass", np.inf), ("mass", np.nan), ("pos", np.nan), ("all", 1e39), ("all", 1e200),
