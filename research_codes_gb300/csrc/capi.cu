@@ -715,6 +715,11 @@ constexpr float ROW_SLACK = 1.03f;   // row radius of the density over the first
 // Lists beyond this are marked by a block per item (hydro 21k batch 2.86 ms with none,
 // 2.23 at 4096, 1.93 at 1536, 1.98 at 1024; density 40k 2.13 / 2.04 / 2.07).
 constexpr int LONG_NJ = 1536;
+// FP32C hydro calls of few items (32 targets each, so that rows keep a warp's
+// order): a warp per list leaves the chip idle.  Calls of 16, 32 and 64 targets 158,
+// 172 and 199 us by warps at 125 neighbours, 123, 125 and 132 by blocks; at 55
+// neighbours 145, 163 and 180, 139, 153 and 161; of 8 (list of 187) 124 and 127.
+constexpr int LONG_NJ_FEW = 256;
 constexpr int SPLIT_NJ = 1024;   // density and hydro: lists beyond this make smaller items
 
 int longest(const int32_t *n, int n_walk) {
@@ -1018,8 +1023,9 @@ extern "C" int sph_dispatch_hydro(sph_context *ctx, int32_t tag, int32_t n_walk,
         m.j_off = (const int *)(d + L.off_joff);
         m.queue = ctx->d_queue + K_HYDRO;
         m.rows = ks.hl_list.p; m.info = ks.r_info.p; m.ovf = ks.hl_ovf.p; m.n_ovf = ctx->d_queue + 8;
-        m.longs = sphk::LongQueue{ks.long_items.p, ctx->d_queue + 9, 0}; m.long_nj = LONG_NJ;
-        m.push_long = longest(n_epj, n_walk) > LONG_NJ;
+        m.longs = sphk::LongQueue{ks.long_items.p, ctx->d_queue + 9, 0};
+        m.long_nj = f32 && m.n_items <= ctx->sm_count ? LONG_NJ_FEW : LONG_NJ;
+        m.push_long = longest(n_epj, n_walk) > m.long_nj;
         m.o_vsmx = ks.o[3].p;
         m.sv_skip = 1;
         sphk::HydroArgs a{};
