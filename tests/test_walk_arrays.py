@@ -56,6 +56,7 @@ class _Int:
     np.array([np.nan, 1.0]), np.array([np.inf]), [float("nan")], [None], np.array(["2020"], "M8[Y]"),
     np.array([[1], [2]]), {2: 1, 3: 1}, [2 ** 70 + 3, 1], [2 ** 63, -1], np.array([2 ** 63 + 5], np.uint64),
     ["3", b"7"], [True, _Int()], np.array([1.5, 2.0]), torch.tensor([1, 2]), [torch.tensor(3), torch.tensor([4])],
+    [np.int64(7), np.int32(-2)], (2 ** 31, 5), [3, np.float64(3.7)], (np.uint64(2 ** 63 + 9),),
 ], ids=str)
 def test_counts_are_taken_as_int_takes_them(counts):
     """What int() refuses is refused, what it accepts is accepted (low 32 bits)."""
